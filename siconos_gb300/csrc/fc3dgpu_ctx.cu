@@ -18,7 +18,7 @@
 #include "fc3dgpu_sweep_launch.h"
 #include "fc3dgpu_fast64.h"
 #include "fc3dgpu_layout.cuh"
-#include "fc3dgpu_local.cuh"
+#include "fc3dgpu_local64.cuh"
 #include "fc3dgpu_mlp.h"
 
 namespace fc3dgpu {

@@ -18,7 +18,7 @@
 #include <mutex>
 
 #include "fc3dgpu.h"
-#include "fc3dgpu_local.cuh"
+#include "fc3dgpu_local64.cuh"
 
 extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 

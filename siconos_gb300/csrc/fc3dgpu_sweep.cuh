@@ -18,7 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "fc3dgpu_layout.cuh"
-#include "fc3dgpu_local.cuh"
+#include "fc3dgpu_local64.cuh"
 
 namespace fc3dgpu {
 
