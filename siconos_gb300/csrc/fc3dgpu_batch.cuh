@@ -46,7 +46,7 @@ __device__ __forceinline__ double scene_full_error(const SweepArgs<Real>& a, int
 }
 
 template <typename Real>
-__device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene, WorkList<Real>& wk) {
+__device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene, typename RangeList<Real>::type& wk) {
   const SweepArgs<Real>& a = b.base;
   const int ncol = b.scene_ncol[scene];
   const int* sptr = b.scene_sptr + (size_t)scene * (FC3D_MAX_COLOURS + 1);
@@ -77,7 +77,7 @@ __device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene,
     sweep++;
     double acc[3] = {0.0, 0.0, 0.0};
     for (int c = 0; c < ncol; c++) {
-      process_range_compact<Real>(a, sptr[c], sptr[c + 1], (Real)local_tol, acc[0], acc[1], wk, nullptr);
+      process_range<Real>(a, sptr[c], sptr[c + 1], (Real)local_tol, acc[0], acc[1], wk, nullptr);
       __syncthreads();
     }
     double s[3];
@@ -154,7 +154,7 @@ __device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene,
 
 template <typename Real>
 __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_batch_kernel(const BatchArgs<Real> b) {
-  __shared__ WorkList<Real> wk;
+  __shared__ typename RangeList<Real>::type wk;
   __shared__ int s_next;
   for (;;) {
     if (threadIdx.x == 0) s_next = atomicAdd(b.queue, 1);

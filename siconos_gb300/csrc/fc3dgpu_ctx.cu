@@ -692,6 +692,7 @@ struct fc3dgpu_ctx {
   BUF(float, r32);
   BUF(double, rpli64);
   BUF(float, rpli32);
+  BUF(unsigned char, cost);
   BUF(double, u64);
   // control
   BUF(double, partials);
@@ -884,7 +885,7 @@ extern "C" void fc3dgpu_ctx_destroy(fc3dgpu_ctx* c) {
   void* ptrs[] = {c->rowptr, c->colidx, c->blocks, c->qo, c->muo, c->ro, c->uo, c->deg, c->gptr64, c->gptr,
                   c->cursor, c->adj, c->key, c->colour, c->blockhist, c->counts, c->sptr_d, c->perm, c->iperm,
                   c->rowlen, c->dpos, c->slab_nslot, c->slab_off, c->W64, c->W32, c->col, c->D64, c->D32,
-                  c->rho64, c->rho32, c->q64, c->q32, c->mu64, c->mu32, c->r64, c->r32, c->rpli64, c->rpli32,
+                  c->rho64, c->rho32, c->q64, c->q32, c->mu64, c->mu32, c->r64, c->r32, c->rpli64, c->rpli32, c->cost,
                   c->u64, c->partials, c->barrier, c->status, c->scratch, c->scratch64, c->out, c->trace,
                   c->counters, c->timeline, c->scene_off, c->grp, c->scounts, c->snslab, c->sncol, c->sbase,
                   c->ssptr, c->sorder, c->snormq, c->sbudget, c->squeue, c->sout32, c->sout64, c->feat,
@@ -1279,6 +1280,7 @@ static int build_layout(fc3dgpu_ctx* c, int nc, long long nnzb, int kind, int ns
   CK(ensure(&c->r32, &c->r32_cap, ((size_t)npad + 1) * 4));
   CK(ensure(&c->rpli64, &c->rpli64_cap, (size_t)npad));
   CK(ensure(&c->rpli32, &c->rpli32_cap, (size_t)npad));
+  CK(ensure(&c->cost, &c->cost_cap, (size_t)npad));
   CK(ensure(&c->u64, &c->u64_cap, (size_t)npad * 3));
   CK(cudaMemsetAsync(c->W64, 0, sizeof(double) * nw, s));
   CK(cudaMemsetAsync(c->D64, 0, sizeof(double) * nslab * 9 * FC3D_SLAB, s));
@@ -1581,6 +1583,7 @@ static void fill_args(fc3dgpu_ctx* c, fc3dgpu::SweepArgs<Real>& a, const Real* W
   a.rho = rho;
   a.r = r;
   a.rpli = rpli;
+  a.cost = c->cost;
   a.u = c->u64;
   a.partials = c->partials;
   a.barrier = c->barrier;
@@ -2084,6 +2087,7 @@ static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st
       a.max_sweeps = out[3] == 0.0 ? 0 : budget;
     }
     if (!(converged32 && a.max_sweeps == 0)) {
+      if (a.max_sweeps > 0) CK(cudaMemsetAsync(c->cost, 0, (size_t)c->npad, s));
       CK(cudaMemsetAsync(c->barrier, 0, FC3D_BARRIER_WORDS * sizeof(unsigned), s));
       CK(launch64(a));
       c->launches++;
@@ -2285,6 +2289,7 @@ static int record_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
   }
   k_batch_budget<<<grid1d(ns), 256, 0, s>>>(ns, c->sout32, p->fp32_only ? 0 : p->max_iter, c->sbudget);
   {
+    CK(cudaMemsetAsync(c->cost, 0, (size_t)c->npad, s));
     BatchArgs<double> b;
     fill_args<double>(c, b.base, c->W64, c->D64, c->q64, c->mu64, c->rho64, c->r64, c->rpli64);
     b.base.max_sweeps = p->max_iter;

@@ -40,6 +40,7 @@ __device__ __forceinline__ uint32_t ie_rsqrt_seed(uint32_t f) {
 __device__ __forceinline__ uint32_t ie_mulhi(uint32_t a, uint32_t b) { return __umulhi(a, b); }
 __device__ __forceinline__ uint64_t ie_bits(double x) { return (uint64_t)__double_as_longlong(x); }
 __device__ __forceinline__ double ie_double(uint64_t x) { return __longlong_as_double((long long)x); }
+#define IE_AS_FLOAT(u) __uint_as_float(u)
 #define IE_FN __device__ __forceinline__
 #define IE_SLOW static __device__ __noinline__
 #else
@@ -71,6 +72,7 @@ static inline double ie_double(uint64_t u) {
   memcpy(&x, &u, 8);
   return x;
 }
+#define IE_AS_FLOAT(u) ie_host_as_float(u)
 #define IE_FN static inline
 #define IE_SLOW static
 #endif
@@ -195,6 +197,25 @@ IE_FN int64_t ie_order(double a) {
 IE_FN bool ie_nan(double a) { return (ie_bits(a) << 1) > 0xffe0000000000000ull; }
 IE_FN bool ie_lt(double a, double b) { return ie_order(a) < ie_order(b) && !ie_nan(a) && !ie_nan(b); }
 IE_FN bool ie_le(double a, double b) { return ie_order(a) <= ie_order(b) && !ie_nan(a) && !ie_nan(b); }
+// a <= b and a < b of operands with the sign bit clear
+IE_FN bool ie_le_pos(double a, double b) { return ie_bits(a) <= ie_bits(b) && ie_bits(b) <= 0x7ff0000000000000ull; }
+IE_FN bool ie_lt_pos(double a, double b) { return ie_bits(a) < ie_bits(b) && ie_bits(b) <= 0x7ff0000000000000ull; }
+// a > 0
+IE_FN bool ie_positive(double a) { return ie_bits(a) - 1ull < 0x7ff0000000000000ull; }
 IE_FN double ie_abs(double a) { return ie_double(ie_bits(a) & 0x7fffffffffffffffull); }
+
+// |a| in FP32, truncated (relative error under 2^-23); 0 below the FP32
+// normal range, infinity above it and for NaN.  A conversion instruction
+// would take the FP64 unit.
+IE_FN uint32_t ie_float_bits(double a) {
+  const uint64_t x = ie_bits(a);
+  const uint32_t h = ((uint32_t)(x >> 32) & 0x7fffffffu) - 0x38000000u;  // exponent rebiased by 896
+  const uint32_t f = (h << 3) | ((uint32_t)x >> 29);
+  return (int32_t)h < 0x00100000 ? 0u : (h >= 0x0ff00000u ? 0x7f800000u : f);
+}
+IE_FN float ie_float(double a) { return IE_AS_FLOAT(ie_float_bits(a)); }
+IE_FN float ie_float_signed(double a) {
+  return IE_AS_FLOAT(ie_float_bits(a) | ((uint32_t)(ie_bits(a) >> 32) & 0x80000000u));
+}
 
 }  // namespace fc3dgpu

@@ -46,6 +46,7 @@ struct SweepArgs {
   // state
   Real* r;                      // AoS (npad + 1) * 3, entry npad is zero
   Real* rpli;                   // npad
+  unsigned char* cost;          // npad: cost class of each contact's last FP64 local solve (order of work only)
   double* u;                    // AoS npad * 3 (FP64 full error output)
   // reductions and control
   double* partials;             // gridDim.x * 4

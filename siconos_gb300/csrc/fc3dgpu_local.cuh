@@ -241,6 +241,7 @@ struct LocalProblem {
   int mode;       // 0: the reference's hybrid; 1: damped Newton only
   Real residual;  // SOLVER_RESIDUAL of the local options
   int n_newton, n_pli, n_ls;  // work counters
+  bool slip;                  // FP64: the last Newton ended at a slipping point
 };
 
 template <typename Real>

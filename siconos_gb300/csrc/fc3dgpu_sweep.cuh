@@ -18,7 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "fc3dgpu_layout.cuh"
-#include "fc3dgpu_local64.cuh"
+#include "fc3dgpu_coop64.cuh"
 
 namespace fc3dgpu {
 
@@ -550,6 +550,279 @@ __device__ __forceinline__ void process_range_compact(const SweepArgs<Real>& a, 
   }
 }
 
+// ---- the FP64 colour, one lane or three lanes a contact -------------------
+// Cost classes of a contact, from its last local solve: 2 min(Newton
+// iterations, 3), one more when it slips, the last class after a PLI loop.
+#define FC3D_COSTS 8
+// Contacts of a pass up to which the block solves them on three lanes each
+// (a round of its warps takes FC3D_COOP_GROUPS a warp); more are solved one
+// a lane.
+#define FC3D_COOP_MAX 80
+
+struct WorkList64 {
+  // component-major by row of the pass (slab * 32 + lane)
+  double q[3][FC3D_PASS_SLABS * FC3D_SLAB];
+  double ro[3][FC3D_PASS_SLABS * FC3D_SLAB];
+  int count[FC3D_COSTS * FC3D_PASS_SLABS + 1];  // class-major; then the exclusive prefix sums
+  unsigned short row[FC3D_PASS_SLABS * FC3D_SLAB];
+};
+
+// Component `comp` of row (slab, lane)'s q + sum over its off-diagonal
+// blocks, in the reference's slot order.
+__device__ __forceinline__ double row_product64(const SweepArgs<double>& a, int slab, int lane, int comp) {
+  const long long base = a.slab_off[slab];
+  const int ns = a.slab_nslot[slab];
+  double acc = a.q[((size_t)slab * 3 + comp) * FC3D_SLAB + lane];
+  constexpr int CH = 8;
+  for (int t0 = 0; t0 < ns; t0 += CH) {
+    int pj[CH];
+    double wv[CH][3];
+#pragma unroll
+    for (int k = 0; k < CH; k++) {
+      const size_t sl = (size_t)(base + (t0 + k < ns ? t0 + k : 0));
+      pj[k] = t0 + k < ns ? __ldg(&a.col[sl * FC3D_SLAB + lane]) : a.npad;
+      const double* wp = a.W + (sl * 9 + comp) * FC3D_SLAB + lane;
+#pragma unroll
+      for (int e = 0; e < 3; e++) wv[k][e] = t0 + k < ns ? __ldg(&wp[3 * e * FC3D_SLAB]) : 0.0;
+    }
+    double rv[CH][3];
+#pragma unroll
+    for (int k = 0; k < CH; k++) load_r3<double>(a.r, pj[k], rv[k]);
+#pragma unroll
+    for (int k = 0; k < CH; k++)
+      if (t0 + k < ns) {
+        acc += wv[k][0] * rv[k][0];
+        acc += wv[k][1] * rv[k][1];
+        acc += wv[k][2] * rv[k][2];
+      }
+  }
+  return acc;
+}
+
+__device__ __forceinline__ unsigned char cost_class(int newton, int pli, bool slip) {
+  return (unsigned char)(pli > 0 ? FC3D_COSTS - 1 : 2 * (newton < 3 ? newton : 3) + (slip ? 1 : 0));
+}
+
+__device__ __forceinline__ void count_work(const SweepArgs<double>& a, int newton, int pli, int ls) {
+  atomicAdd(&a.counters[0], (unsigned long long)newton);
+  atomicAdd(&a.counters[1], (unsigned long long)pli);
+  atomicAdd(&a.counters[2], (unsigned long long)ls);
+  atomicAdd(&a.counters[3], 1ULL);
+  atomicMax(&a.counters[4], (unsigned long long)newton);
+}
+
+// Contact of row x of the pass (first slab ps) on one lane.
+__device__ __forceinline__ void solve_lane64(const SweepArgs<double>& a, const WorkList64& wk, int ps, int x,
+                                             double ltol, double& dr2, double& rr2) {
+  const int sl = ps + x / FC3D_SLAB, k = x % FC3D_SLAB, pp = sl * FC3D_SLAB + k;
+  LocalProblem<double> L;
+#pragma unroll
+  for (int e = 0; e < 9; e++) L.M[e] = __ldg(&a.D[((size_t)sl * 9 + e) * FC3D_SLAB + k]);
+  L.q[0] = wk.q[0][x];
+  L.q[1] = wk.q[1][x];
+  L.q[2] = wk.q[2][x];
+  L.mu = __ldg(&a.mu[(size_t)sl * FC3D_SLAB + k]);
+  L.rhoN = __ldg(&a.rho[((size_t)sl * 2) * FC3D_SLAB + k]);
+  L.rhoT = __ldg(&a.rho[((size_t)sl * 2 + 1) * FC3D_SLAB + k]);
+  L.rho_pli = __ldcg(&a.rpli[pp]);
+  L.tol = ltol;
+  L.newton_max = a.newton_max;
+  L.pli_max = a.pli_max;
+  L.ls_max = a.ls_max;
+  L.mode = a.local_mode;
+  L.n_newton = 0;
+  L.n_pli = 0;
+  L.n_ls = 0;
+  L.slip = false;
+  const double o[3] = {wk.ro[0][x], wk.ro[1][x], wk.ro[2][x]};
+  double rn[3] = {o[0], o[1], o[2]};
+  local_solve(L, rn);
+  double keep[3];
+  nsgs_accept(a, L, o, rn, keep);
+  double* rp = a.r + (size_t)pp * FC3D_RSTRIDE;
+  rp[0] = keep[0];
+  rp[1] = keep[1];
+  rp[2] = keep[2];
+  a.rpli[pp] = L.rho_pli;
+  a.cost[pp] = cost_class(L.n_newton, L.n_pli, L.slip);
+  const double d0 = o[0] - rn[0], d1 = o[1] - rn[1], d2 = o[2] - rn[2];
+  dr2 += d0 * d0 + d1 * d1 + d2 * d2;
+  rr2 += keep[0] * keep[0] + keep[1] * keep[1] + keep[2] * keep[2];
+  if (a.counters) count_work(a, L.n_newton, L.n_pli, L.n_ls);
+}
+
+// Contacts wk.row[t0 .. t1) of the pass, three lanes each, by one warp
+// (at most FC3D_COOP_GROUPS; the spare groups repeat the first contact
+// without storing it).
+__device__ __forceinline__ void solve_coop64(const SweepArgs<double>& a, const WorkList64& wk, int ps, int t0, int t1,
+                                             double ltol, double& dr2, double& rr2) {
+  const int lane = threadIdx.x & 31;
+  const bool spare = lane >= 3 * FC3D_COOP_GROUPS;
+  CoopLane c;
+  const int g = spare ? 0 : lane / 3;
+  c.base = 3 * g;
+  c.i = lane - (spare ? 3 * FC3D_COOP_GROUPS : c.base);
+  const bool act = !spare && t0 + g < t1;
+  const int x = wk.row[act ? t0 + g : t0];
+  const int sl = ps + x / FC3D_SLAB, k = x % FC3D_SLAB, pp = sl * FC3D_SLAB + k;
+  CoopProblem P;
+#pragma unroll
+  for (int e = 0; e < 9; e++) P.M[e] = __ldg(&a.D[((size_t)sl * 9 + e) * FC3D_SLAB + k]);
+  P.m0 = c.i == 0 ? P.M[0] : (c.i == 1 ? P.M[1] : P.M[2]);
+  P.m1 = c.i == 0 ? P.M[3] : (c.i == 1 ? P.M[4] : P.M[5]);
+  P.m2 = c.i == 0 ? P.M[6] : (c.i == 1 ? P.M[7] : P.M[8]);
+  P.q = wk.q[c.i][x];
+  P.mu = __ldg(&a.mu[(size_t)sl * FC3D_SLAB + k]);
+  P.rhoN = __ldg(&a.rho[((size_t)sl * 2) * FC3D_SLAB + k]);
+  P.rhoT = __ldg(&a.rho[((size_t)sl * 2 + 1) * FC3D_SLAB + k]);
+  P.rho_i = c.i == 0 ? P.rhoN : P.rhoT;
+  double rpli = __ldcg(&a.rpli[pp]);
+  const double o = wk.ro[c.i][x];
+  double rn = o;
+  CoopCount n = {0, 0, 0, false};
+  const double residual = coop_local_solve(c, P, act, a, ltol, rn, rpli, n);
+  if (a.relax) rn = a.omega * rn + (1.0 - a.omega) * o;
+  const bool discard = a.filter && (!finite64(residual) || residual > 1.0);
+  const double keep = discard ? o : rn;
+  if (act) a.r[(size_t)pp * FC3D_RSTRIDE + c.i] = keep;
+  const double d = o - rn;
+  const double d2 = coop_sum(c, d * d), k2 = coop_sum(c, keep * keep);
+  if (act && c.i == 0) {
+    a.rpli[pp] = rpli;
+    a.cost[pp] = cost_class(n.newton, n.pli, n.slip);
+    dr2 += d2;
+    rr2 += k2;
+    if (a.counters) count_work(a, n.newton, n.pli, n.ls);
+  }
+}
+
+// One colour's slabs [lo, hi) of this block in FP64, in passes of up to
+// FC3D_PASS_SLABS slabs.  What bounds it: FP64 warp instructions (see
+// fc3dgpu_local64.cuh), so
+//   - the row products are split by component: a (slab, component) unit is a
+//     third of a slab's chain and the units spread over all the SM's
+//     quarters (each component keeps the reference's slot order);
+//   - contacts with q_n > -eps are the local solver's trivial take-off
+//     (onecontact.c:234-245), finished at once;
+//   - the others are listed by the cost class of their previous solve, the
+//     longest first, so that the lanes of a warp end together (listed in slab
+//     order a warp runs the 3 to 4 iterations of its slowest lane for a mean
+//     of 1.6);
+//   - up to FC3D_COOP_MAX of them are solved on three lanes each.
+__device__ __forceinline__ void process_range64(const SweepArgs<double>& a, int lo, int hi, double ltol, double& dr2,
+                                                double& rr2, WorkList64& wk, unsigned long long* tl) {
+  constexpr int NWB = BlockDim<double>::value / 32;
+  constexpr int MAXR = (FC3D_PASS_SLABS + NWB - 1) / NWB;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int ps = lo; ps < hi; ps += FC3D_PASS_SLABS) {
+    const int np = min(FC3D_PASS_SLABS, hi - ps);
+    for (int u = w; u < 3 * np; u += NWB) {
+      const int i = u / 3, comp = u - 3 * i, slab = ps + i, p = slab * FC3D_SLAB + lane;
+      double acc = 0, ro = 0;
+      if (__ldg(&a.perm[p]) >= 0) {
+        ro = __ldcg(&a.r[(size_t)p * FC3D_RSTRIDE + comp]);
+        acc = row_product64(a, slab, lane, comp);
+      }
+      wk.q[comp][i * FC3D_SLAB + lane] = acc;
+      wk.ro[comp][i * FC3D_SLAB + lane] = ro;
+    }
+    __syncthreads();
+    unsigned mine[MAXR];
+    int cls[MAXR];
+#pragma unroll
+    for (int j = 0; j < MAXR; j++) {
+      const int i = w + j * NWB;
+      cls[j] = -1;
+      mine[j] = 0;
+      if (i < np) {
+        const int p = (ps + i) * FC3D_SLAB + lane, x = i * FC3D_SLAB + lane;
+        if (__ldg(&a.perm[p]) >= 0) {
+          if (ie_lt(-DBL_EPSILON, wk.q[0][x])) {
+            const double ro[3] = {wk.ro[0][x], wk.ro[1][x], wk.ro[2][x]};
+            double* rp = a.r + (size_t)p * FC3D_RSTRIDE;
+            if (a.relax) {
+              takeoff_relaxed(a, ro, rp, dr2, rr2);
+            } else {
+              rp[0] = 0;
+              rp[1] = 0;
+              rp[2] = 0;
+              dr2 += ro[0] * ro[0] + ro[1] * ro[1] + ro[2] * ro[2];
+            }
+          } else {
+            cls[j] = FC3D_COSTS - 1 - min((int)a.cost[p], FC3D_COSTS - 1);
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < FC3D_COSTS; b++) {
+          const unsigned m = __ballot_sync(0xffffffffu, cls[j] == b);
+          if (cls[j] == b) mine[j] = m;
+          if (lane == 0) wk.count[b * np + i] = __popc(m);
+        }
+      }
+    }
+    __syncthreads();
+    if (w == 0) {
+      // exclusive prefix sums of the counts, 32 at a time
+      int carry = 0;
+      for (int k0 = 0; k0 < FC3D_COSTS * np; k0 += 32) {
+        const int v = k0 + lane < FC3D_COSTS * np ? wk.count[k0 + lane] : 0;
+        int s = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, s, d);
+          if (lane >= d) s += y;
+        }
+        if (k0 + lane < FC3D_COSTS * np) wk.count[k0 + lane] = carry + s - v;
+        carry += __shfl_sync(0xffffffffu, s, 31);
+      }
+      if (lane == 0) wk.count[FC3D_COSTS * np] = carry;
+    }
+    __syncthreads();
+    const int total = wk.count[FC3D_COSTS * np];
+    if (tl && threadIdx.x == 0) {
+      tl[0] = globaltimer_ns();
+      tl[1] = (unsigned long long)total;
+    }
+#pragma unroll
+    for (int j = 0; j < MAXR; j++)
+      if (cls[j] >= 0) {
+        const int i = w + j * NWB;
+        wk.row[wk.count[cls[j] * np + i] + __popc(mine[j] & ((1u << lane) - 1))] =
+            (unsigned short)(i * FC3D_SLAB + lane);
+      }
+    __syncthreads();
+    if (total <= FC3D_COOP_MAX && a.local_mode == 0) {
+      // a quarter of the list to each SM quarter's first warp, the rest to
+      // its second
+      const int cpw = min(FC3D_COOP_GROUPS, max(1, (total + 3) / 4));
+      const int t0 = w * cpw;
+      if (t0 < total) solve_coop64(a, wk, ps, t0, min(total, t0 + cpw), ltol, dr2, rr2);
+    } else {
+      for (int t = threadIdx.x; t < total; t += blockDim.x) solve_lane64(a, wk, ps, wk.row[t], ltol, dr2, rr2);
+    }
+    __syncthreads();
+  }
+}
+
+// A block's share of a colour without staging: the FP32 or the FP64 form.
+template <typename Real>
+struct RangeList {
+  using type = WorkList<Real>;
+};
+template <>
+struct RangeList<double> {
+  using type = WorkList64;
+};
+template <typename Real>
+__device__ __forceinline__ void process_range(const SweepArgs<Real>& a, int lo, int hi, Real ltol, double& dr2,
+                                              double& rr2, typename RangeList<Real>::type& wk,
+                                              unsigned long long* tl) {
+  if constexpr (sizeof(Real) == sizeof(double))
+    process_range64(a, lo, hi, ltol, dr2, rr2, wk, tl);
+  else
+    process_range_compact<Real>(a, lo, hi, ltol, dr2, rr2, wk, tl);
+}
+
 // Issue the bulk copies of W, col and q for slabs [lo, hi) into the
 // staging buffers (one thread).  The caller made sure the previous
 // contents were consumed (block barrier + proxy fence).
@@ -897,7 +1170,7 @@ __device__ __forceinline__ bool full_error_phase(const SweepArgs<Real>& a, int s
 
 template <typename Real, int T>
 __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_kernel(const SweepArgs<Real> a) {
-  __shared__ WorkList<Real> wk;
+  __shared__ typename RangeList<Real>::type wk;
   __shared__ __align__(8) unsigned long long stage_bar;
 
   extern __shared__ __align__(128) unsigned char stage[];
@@ -953,7 +1226,7 @@ __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_kernel(const Sw
       } else if (T == 1) {
         int lo, hi;
         block_range(s0, a.sptr[c + 1], lo, hi);
-        process_range_compact<Real>(a, lo, hi, (Real)local_tol, acc[0], acc[1], wk,
+        process_range<Real>(a, lo, hi, (Real)local_tol, acc[0], acc[1], wk,
                                     tl ? a.timeline + ((size_t)c * gridDim.x + blockIdx.x) * FC3D_TL_STRIDE + 2 : nullptr);
       } else {
         for (int u = gw; u < nunits; u += tw) {
