@@ -2,51 +2,127 @@
 //
 // The problems are one block-diagonal union layout (rows permuted by
 // problem, then colour, each (problem, colour) group padded to 32-row slabs).
-// Each block pulls whole problems from a work queue ordered by decreasing
-// size, and runs every sweep of its problem with block barriers between
-// colours -- no grid-wide synchronisation at all.  Within a problem the
-// arithmetic is that of the single-problem kernel (same row product, same
-// local solver, same reference convergence logic with fc3d_compute_error and
-// the tolerance manager), so each problem's iterates equal a solo solve's.
+// problem, then colour, each (problem, colour) group padded to 32-row slabs).
+// A problem is solved by one block, or by a team of blocks that splits every
+// colour's slabs evenly and meets at a bounded barrier of its own between
+// colours; blocks without a team, and teams that are done, pull problems one
+// by one from a work queue ordered by decreasing size.  There is no grid-wide
+// synchronisation.  Within a problem the arithmetic is that of the
+// single-problem kernel (same row product, same local solver, same reference
+// convergence logic with fc3d_compute_error and the tolerance manager), so
+// each problem's iterates equal a solo solve's.
+//
+// What bounds a sweep of one problem is its rounds of slabs per block, each a
+// latency chain, so a batch with few problems is as slow as its largest
+// problem on one SM; the teams (batch_plan in fc3dgpu_ctx.cu) give the large
+// problems the idle SMs.  48 lattices of 130 to 8,901 contacts, 100 FP32
+// sweeps: 28.3 ms one block each, 7.6 ms in teams; 200 lattices, 30 sweeps:
+// 11.1 and 7.2 ms; in FP64, 48 lattices and 100 sweeps, 50 ms in teams.
 #pragma once
 #include "fc3dgpu_batch_args.cuh"
 #include "fc3dgpu_sweep.cuh"
 
 namespace fc3dgpu {
 
-__device__ __forceinline__ void block_reduce3(double v[3], double out[3]) {
-  __shared__ double sh[FC3D_BLOCK_MAX / 32][3];
+// The blocks that share a problem: `size` of them from block `first` on.
+struct BatchTeam {
+  int first, size, rank;
+  unsigned epoch;  // barriers passed (the blocks of a team pass the same ones)
+};
+
+// Orders every write of the team before it, reactions in global memory
+// included, ahead of every read after it.  False when a block of the team did
+// not arrive within the poll limit (recorded in the status).
+__device__ __forceinline__ bool team_sync(BatchTeam& t, unsigned* flags, unsigned long long limit, int* status) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (t.size == 1) return true;
+  t.epoch++;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    if (lane == 0) st_release_u32(&flags[blockIdx.x * FC3D_FLAG_STRIDE], t.epoch);
+    unsigned long long n = 0;
+    int ok = 1;
+    for (;;) {
+      bool mine = true;
+      for (int k = lane; k < t.size; k += 32)
+        mine &= (ld_relaxed_u32(&flags[(t.first + k) * FC3D_FLAG_STRIDE]) >= t.epoch);
+      if (__all_sync(0xffffffffu, mine)) break;
+      if (++n > limit) {
+        ok = 0;
+        if (lane == 0) atomicOr(status, 1);
+        break;
+      }
+      if (n > 256) __nanosleep(32);
+    }
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    if (lane == 0) s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// Sums of three values per thread over the team in a fixed order (warp tree,
+// warps in order, blocks in order), the same bits in every thread.  The block
+// sums of a team go through a ring of two slots in global memory: a block
+// writes slot k & 1 only after the barrier of call k - 1, which every block
+// passes after reading call k - 2's slot.
+struct TeamSum {
+  double warp[FC3D_BLOCK_MAX / 32][3];
+};
+template <typename Real>
+__device__ __forceinline__ bool team_reduce3(const BatchArgs<Real>& b, BatchTeam& t, TeamSum& S, double v[3],
+                                             double out[3]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     double x = v[i];
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[w][i] = x;
+    if (lane == 0) S.warp[w][i] = x;
   }
   __syncthreads();
+  double s[3] = {0.0, 0.0, 0.0};
+  for (int k = 0; k < (int)(blockDim.x >> 5); k++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) s[i] += S.warp[k][i];
+  if (t.size == 1) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) out[i] = s[i];
+    __syncthreads();
+    return true;
+  }
+  double* ring = b.team_part + (size_t)(t.epoch & 1) * FC3D_BATCH_BLOCKS * 4;
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int i = 0; i < 3; i++) __stcg(&ring[4 * blockIdx.x + i], s[i]);
+  if (!team_sync(t, b.base.barrier, b.base.spin_limit, b.base.status)) return false;
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    double s = 0.0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); k++) s += sh[k][i];
-    out[i] = s;
+    double x = 0.0;
+    for (int k = 0; k < t.size; k++) x += __ldcg(&ring[4 * (t.first + k) + i]);
+    out[i] = x;
   }
-  __syncthreads();
+  return true;
 }
 
 template <typename Real>
-__device__ __forceinline__ double scene_full_error(const SweepArgs<Real>& a, int p0, int p1, double norm_q) {
+__device__ __forceinline__ bool scene_full_error(const BatchArgs<Real>& b, int p0, int p1, double norm_q,
+                                                 BatchTeam& t, TeamSum& S, double& full) {
   double v[3], s[3];
-  full_error_rows(a, v, p0, p1, threadIdx.x, blockDim.x);
-  block_reduce3(v, s);
+  full_error_rows(b.base, v, p0, p1, t.rank * blockDim.x + threadIdx.x, t.size * blockDim.x);
+  if (!team_reduce3(b, t, S, v, s)) return false;
   double e = sqrt(s[0]);
   const double scal = fmax(norm_q, fmax(sqrt(s[2]), sqrt(s[1])));
   if (fabs(scal) > DBL_EPSILON) e /= scal;
-  return e;
+  full = e;
+  return true;
 }
 
+// All sweeps of one problem; false when a wait of the team gave up.
 template <typename Real>
-__device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene, typename RangeList<Real>::type& wk) {
+__device__ __forceinline__ bool solve_scene(const BatchArgs<Real>& b, int scene, typename RangeList<Real>::type& wk,
+                                            BatchTeam& t, TeamSum& S) {
   const SweepArgs<Real>& a = b.base;
   const int ncol = b.scene_ncol[scene];
   const int* sptr = b.scene_sptr + (size_t)scene * (FC3D_MAX_COLOURS + 1);
@@ -59,9 +135,9 @@ __device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene,
   bool converged = false;
   if (a.mode == 1 && b.scene_out_prev && b.scene_out_prev[(size_t)scene * 8 + 3] == 0.0) {
     // the FP32 iterate met the tolerance in FP32 arithmetic: FP64 check first
-    full = scene_full_error(a, p0, p1, norm_q);
+    if (!scene_full_error(b, p0, p1, norm_q, t, S, full)) return false;
     if (full < a.user_tol) {
-      if (threadIdx.x == 0) {
+      if (t.rank == 0 && threadIdx.x == 0) {
         double* o = b.scene_out + (size_t)scene * 8;
         o[0] = 0;
         o[1] = b.scene_out_prev[(size_t)scene * 8 + 1];
@@ -70,25 +146,28 @@ __device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene,
         o[4] = working;
         o[5] = local_tol;
       }
-      return;
+      return true;
     }
   }
   while (sweep < max_sweeps) {
     sweep++;
     double acc[3] = {0.0, 0.0, 0.0};
     for (int c = 0; c < ncol; c++) {
-      process_range<Real>(a, sptr[c], sptr[c + 1], (Real)local_tol, acc[0], acc[1], wk, nullptr);
-      __syncthreads();
+      const int s0 = sptr[c], n = sptr[c + 1] - s0;
+      process_range<Real>(a, s0 + n * t.rank / t.size, s0 + n * (t.rank + 1) / t.size, (Real)local_tol, acc[0],
+                          acc[1], wk, nullptr);
+      // the barrier of the sums closes the last colour
+      if (c + 1 < ncol && !team_sync(t, a.barrier, a.spin_limit, a.status)) return false;
     }
     double s[3];
-    block_reduce3(acc, s);
+    if (!team_reduce3(b, t, S, acc, s)) return false;
     incr = sqrt(s[0]);
     const double nr = sqrt(s[1]);
     if (fabs(nr) > DBL_EPSILON) incr /= nr;
     bool stop = false;
     if (a.mode == 1) {
       if (incr < working) {
-        full = scene_full_error(a, p0, p1, norm_q);
+        if (!scene_full_error(b, p0, p1, norm_q, t, S, full)) return false;
         if (full <= a.user_tol) {
           converged = true;
           stop = true;
@@ -118,7 +197,7 @@ __device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene,
       // the reference's adaptive test on this precision's iterate, against
       // max(tol, switch_tol), as in the single-problem kernel
       if (!stop && incr < working) {
-        full = scene_full_error(a, p0, p1, norm_q);
+        if (!scene_full_error(b, p0, p1, norm_q, t, S, full)) return false;
         const double target = fmax(a.user_tol, a.switch_tol);
         if (full <= target) {
           converged = true;
@@ -135,13 +214,13 @@ __device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene,
   }
   int info = 1;
   if (a.mode == 1) {
-    full = scene_full_error(a, p0, p1, norm_q);
+    if (!scene_full_error(b, p0, p1, norm_q, t, S, full)) return false;
     info = full < a.user_tol ? 0 : 1;
     if (sweep == max_sweeps && info > 0) info = -20;
   } else {
     info = converged ? 0 : 1;
   }
-  if (threadIdx.x == 0) {
+  if (t.rank == 0 && threadIdx.x == 0) {
     double* o = b.scene_out + (size_t)scene * 8;
     o[0] = sweep;
     o[1] = incr;
@@ -155,16 +234,63 @@ __device__ __forceinline__ void solve_scene(const BatchArgs<Real>& b, int scene,
 template <typename Real>
 __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_batch_kernel(const BatchArgs<Real> b) {
   __shared__ typename RangeList<Real>::type wk;
+  __shared__ TeamSum S;
   __shared__ int s_next;
+  BatchTeam t = {(int)blockIdx.x, 1, 0, 0};
+  if (b.teams) {
+    const int4 m = b.teams[blockIdx.x];
+    if (m.y > 1) {
+      t.first = m.x;
+      t.size = m.y;
+      t.rank = (int)blockIdx.x - m.x;
+      if (!solve_scene<Real>(b, b.order[m.z], wk, t, S)) return;
+      __syncthreads();
+      t.size = 1;
+      t.rank = 0;
+    }
+  }
   for (;;) {
     if (threadIdx.x == 0) s_next = atomicAdd(b.queue, 1);
     __syncthreads();
-    const int k = s_next;
+    const int k = b.team_scenes + s_next;
     __syncthreads();
     if (k >= b.nscenes) break;
-    solve_scene<Real>(b, b.order[k], wk);
+    if (!solve_scene<Real>(b, b.order[k], wk, t, S)) return;
     __syncthreads();
   }
+}
+
+// Launch of `grid` blocks, co-resident (a cooperative launch) when some of
+// them form teams.
+template <typename Real>
+static cudaError_t launch_batch_t(const BatchArgs<Real>& b, int grid, cudaStream_t s) {
+  if (grid < 1 || grid > FC3D_BATCH_BLOCKS) return cudaErrorInvalidConfiguration;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(BlockDim<Real>::value);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = b.teams ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, nsgs_batch_kernel<Real>, b);
+}
+
+// Resident blocks of the batched kernel on the current device.
+template <typename Real>
+static cudaError_t batch_grid_t(int* grid) {
+  auto kern = nsgs_batch_kernel<Real>;
+  int dev = 0, nsm = 0, per_sm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BlockDim<Real>::value, 0);
+  if (e != cudaSuccess) return e;
+  if (per_sm < 1) return cudaErrorInvalidConfiguration;
+  *grid = nsm * per_sm < FC3D_BATCH_BLOCKS ? nsm * per_sm : FC3D_BATCH_BLOCKS;
+  return cudaSuccess;
 }
 
 }  // namespace fc3dgpu

@@ -2,6 +2,11 @@
 #pragma once
 #include "fc3dgpu_layout.cuh"
 
+// Most blocks of a batched launch
+#define FC3D_BATCH_BLOCKS 1024
+// Warps of a block of the FP32 batched kernel
+#define FC3D_BATCH_WARPS32 10
+
 namespace fc3dgpu {
 
 template <typename Real>
@@ -13,7 +18,13 @@ struct BatchArgs {
   const int* scene_sptr;     // nscenes x (FC3D_MAX_COLOURS + 1), absolute slab indices
   const double* scene_normq; // |q| of each problem
   const int* scene_budget;   // sweep budget of each problem (nullptr: base.max_sweeps)
-  int* queue;                // next problem index, zero at launch
+  int* queue;                // next problem of the queue, zero at launch
+  // teams: per block (first block, size, problem in `order`, unused) with
+  // size 1 for none; the first team_scenes problems of `order` have teams, the
+  // others are queued.  nullptr: no teams.
+  const int4* teams;
+  int team_scenes;
+  double* team_part;         // 2 slots x FC3D_BATCH_BLOCKS x 4 block sums of the teams
   double* scene_out;         // nscenes x 8: sweeps, incr, full error, info, working tol, local tol
   // outputs of the previous (FP32) phase, or nullptr: a problem whose FP32
   // iterate met the tolerance gets its FP64 error checked before any sweep

@@ -638,6 +638,50 @@ static cudaError_t ensure(T** p, size_t* cap, size_t n) {
   T* name = nullptr; \
   size_t name##_cap = 0
 
+// Teams of a batched launch of `resident` blocks.  A block takes `step` slabs
+// of a colour in one round (its warps), and a sweep's time goes with the
+// rounds of the slowest block: every problem gets the blocks that bring it
+// down to m rounds, with the smallest m for which the blocks suffice.  With
+// more problems than blocks no m does; then the problems above 1.25 times the
+// mean load of a block are split down to that and the others stay one block
+// each in the queue.  slabs: slabs of a colour per problem, decreasing.
+struct BatchPlan {
+  int grid = 0, team_scenes = 0;
+  std::vector<int4> teams;  // one entry per block, empty without teams
+};
+static BatchPlan batch_plan(const std::vector<int>& slabs, int resident, int step) {
+  const int ns = (int)slabs.size();
+  BatchPlan P;
+  P.grid = resident < ns ? resident : ns;
+  auto need = [&](int n, int load) { return (n + load - 1) / load; };
+  int load = 0;
+  if (ns <= resident) {
+    for (int m = 1; load == 0; m++) {
+      long long blocks = 0;
+      for (int n : slabs) blocks += need(n, m * step);
+      if (blocks <= resident) load = m * step;
+    }
+  } else {
+    long long total = 0;
+    for (int n : slabs) total += n;
+    load = (int)((total * 5) / (4LL * resident));
+    load = ((load > 0 ? load : 1) + step - 1) / step * step;
+  }
+  std::vector<int4> t;
+  for (int k = 0; k < ns && need(slabs[k], load) > 1; k++) {
+    const int size = need(slabs[k], load), first = (int)t.size();
+    if (first + size > resident) break;
+    for (int r = 0; r < size; r++) t.push_back(make_int4(first, size, k, 0));
+    P.team_scenes++;
+  }
+  if (P.team_scenes == 0) return P;
+  P.grid = (int)t.size() + (ns - P.team_scenes);
+  if (P.grid > resident) P.grid = resident;
+  for (int b = (int)t.size(); b < P.grid; b++) t.push_back(make_int4(b, 1, 0, 0));
+  P.teams = t;
+  return P;
+}
+
 struct fc3dgpu_ctx {
   int device = 0;
   int nsm = 0;
@@ -752,10 +796,13 @@ struct fc3dgpu_ctx {
   BUF(int, squeue);
   BUF(double, sout32);
   BUF(double, sout64);
+  std::vector<int> scene_slabs_h;  // slabs of a colour, by decreasing problem size (an estimate: six colours)
+  BUF(int4, steams);               // teams of the FP32, FP64 and fast FP64 launches
+  BUF(double, steam_part);
   cudaGraphExec_t batch_graph = nullptr;
   fc3dgpu_params batch_graph_params;
-  // resident blocks of the batched kernels (FP32, FP64, fast FP64), set before capture
-  int batch_grid32 = 0, batch_grid64 = 0, batch_grid64f = 0;
+  // launches of the batched kernels (FP32, FP64, fast FP64), set before capture
+  BatchPlan batch_plans[3];
   // neighbourhood synchronisation: block neighbour lists per grid size
   struct Nbr {
     int grid = 0;
@@ -888,7 +935,7 @@ extern "C" void fc3dgpu_ctx_destroy(fc3dgpu_ctx* c) {
                   c->rho64, c->rho32, c->q64, c->q32, c->mu64, c->mu32, c->r64, c->r32, c->rpli64, c->rpli32, c->cost,
                   c->u64, c->partials, c->barrier, c->status, c->scratch, c->scratch64, c->out, c->trace,
                   c->counters, c->timeline, c->scene_off, c->grp, c->scounts, c->snslab, c->sncol, c->sbase,
-                  c->ssptr, c->sorder, c->snormq, c->sbudget, c->squeue, c->sout32, c->sout64, c->feat,
+                  c->ssptr, c->sorder, c->snormq, c->sbudget, c->squeue, c->sout32, c->sout64, c->steams, c->steam_part, c->feat,
                   c->prop, c->rbak, c->gapo, c->cbA, c->cbB, c->cframe, c->cpoint, c->bpos, c->bmass,
                   c->binert, c->bvel, c->bdeg, c->bptr, c->blist, c->crowlen, c->qsum, c->wtmp, c->wdiff,
                   c->flow_dptr, c->flow_dep, c->flow_done, c->flow_need, c->flow_sptr, c->flow_part,
@@ -1237,6 +1284,8 @@ static int build_layout(fc3dgpu_ctx* c, int nc, long long nnzb, int kind, int ns
     std::vector<int> order(nscenes);
     for (int g = 0; g < nscenes; g++) order[g] = g;
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return scene_nc[x] > scene_nc[y]; });
+    c->scene_slabs_h.resize(nscenes);
+    for (int k = 0; k < nscenes; k++) c->scene_slabs_h[k] = (scene_nc[order[k]] + 6 * FC3D_SLAB - 1) / (6 * FC3D_SLAB);
     CK(ensure(&c->sorder, &c->sorder_cap, (size_t)nscenes));
     CK(cudaMemcpyAsync(c->sorder, order.data(), sizeof(int) * nscenes, cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));
@@ -2252,11 +2301,22 @@ extern "C" int fc3dgpu_colour(int nc, const int64_t* rowptr, const int64_t* coli
 // persistent launch per precision, the whole sequence captured once in a
 // CUDA graph and replayed while the parameters stay the same.
 // ---------------------------------------------------------------------------
+// The teams of launch `which` (0 FP32, 1 FP64, 2 fast FP64) for the kernel;
+// its barrier flags start at zero.
+template <typename Real>
+static int attach_teams(fc3dgpu_ctx* c, fc3dgpu::BatchArgs<Real>& b, int which) {
+  const BatchPlan& P = c->batch_plans[which];
+  b.teams = P.teams.empty() ? nullptr : c->steams + (size_t)which * FC3D_BATCH_BLOCKS;
+  b.team_scenes = P.team_scenes;
+  b.team_part = c->steam_part;
+  if (b.teams) CK(cudaMemsetAsync(c->barrier, 0, FC3D_BARRIER_WORDS * sizeof(unsigned), c->stream));
+  return 0;
+}
+
 static int record_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
   using namespace fc3dgpu;
   cudaStream_t s = c->stream;
   const int ns = c->nscenes;
-  int g = 0;
   CK(cudaMemsetAsync(c->squeue, 0, 2 * sizeof(int), s));
   CK(cudaMemsetAsync(c->sout32, 0, sizeof(double) * 8 * ns, s));
   const bool mixed = p->precision == 0 || p->precision == 2;
@@ -2284,7 +2344,8 @@ static int record_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
     b.queue = c->squeue;
     b.scene_out = c->sout32;
     b.scene_out_prev = nullptr;
-    CK(launch_batch_f32(b, c->batch_grid32, s, &g));
+    if (int rc = attach_teams(c, b, 0)) return rc;
+    CK(launch_batch_f32(b, c->batch_plans[0].grid, s));
     k_r32_to_r64<<<grid1d(c->npad), 256, 0, s>>>(c->npad, c->r32, c->rpli32, c->r64, c->rpli64);
   }
   k_batch_budget<<<grid1d(ns), 256, 0, s>>>(ns, c->sout32, p->fp32_only ? 0 : p->max_iter, c->sbudget);
@@ -2312,10 +2373,12 @@ static int record_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
     b.queue = c->squeue + 1;
     b.scene_out = c->sout64;
     b.scene_out_prev = mixed ? c->sout32 : nullptr;
-    if (p->precision >= 2)
-      CK(fc3dgpu_launch_batch_f64_fast(&b, c->batch_grid64f, s, &g));
+    const int which = p->precision >= 2 ? 2 : 1;
+    if (int rc = attach_teams(c, b, which)) return rc;
+    if (which == 2)
+      CK(fc3dgpu_launch_batch_f64_fast(&b, c->batch_plans[2].grid, s));
     else
-      CK(launch_batch_f64(b, c->batch_grid64, s, &g));
+      CK(launch_batch_f64(b, c->batch_plans[1].grid, s));
   }
   return 0;
 }
@@ -2343,9 +2406,22 @@ extern "C" int fc3dgpu_ctx_solve_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p, 
       fc3dgpu_set_error("fc3dgpu_ctx_solve_batch: precision must be 0-3 and local_mode32 0 or 1");
       return NUMERICS_ERR_INVALID_OPTION;
     }
-    CK(batch_grid_f32(&c->batch_grid32));
-    CK(batch_grid_f64(&c->batch_grid64));
-    CK(fc3dgpu_batch_grid_f64_fast(&c->batch_grid64f));
+    int resident[3];
+    CK(batch_grid_f32(&resident[0]));
+    CK(batch_grid_f64(&resident[1]));
+    CK(fc3dgpu_batch_grid_f64_fast(&resident[2]));
+    CK(ensure(&c->steams, &c->steams_cap, (size_t)3 * FC3D_BATCH_BLOCKS));
+    CK(ensure(&c->steam_part, &c->steam_part_cap, (size_t)2 * FC3D_BATCH_BLOCKS * 4));
+    for (int k = 0; k < 3; k++) {
+      // an FP32 block takes a slab per warp and round; an FP64 colour's time
+      // goes with its slabs
+      c->batch_plans[k] = batch_plan(c->scene_slabs_h, resident[k], k == 0 ? FC3D_BATCH_WARPS32 : 1);
+      const std::vector<int4>& t = c->batch_plans[k].teams;
+      if (!t.empty())
+        CK(cudaMemcpyAsync(c->steams + (size_t)k * FC3D_BATCH_BLOCKS, t.data(), sizeof(int4) * t.size(),
+                           cudaMemcpyHostToDevice, s));
+    }
+    CK(cudaStreamSynchronize(s));
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     int rc = record_batch(c, p);

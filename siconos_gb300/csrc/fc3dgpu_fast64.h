@@ -10,5 +10,5 @@
 // args: a fc3dgpu::SweepArgs<double>; lanes 1, 2, 4 or 8; as launch_sweep_f64.
 cudaError_t fc3dgpu_launch_sweep_f64_fast(const void* args, int lanes, int max_grid, cudaStream_t s, int* grid);
 // args: a fc3dgpu::BatchArgs<double>; as launch_batch_f64 / batch_grid_f64.
-cudaError_t fc3dgpu_launch_batch_f64_fast(const void* args, int max_grid, cudaStream_t s, int* grid);
+cudaError_t fc3dgpu_launch_batch_f64_fast(const void* args, int grid, cudaStream_t s);
 cudaError_t fc3dgpu_batch_grid_f64_fast(int* grid);

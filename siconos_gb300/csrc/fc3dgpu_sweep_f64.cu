@@ -67,30 +67,11 @@ int sweep_grid_f64(int lanes) {
   }
 }
 
-// Resident blocks of the batched kernel on the current device, queried
-// outside any stream capture; the caller keeps the figure with its context.
-cudaError_t batch_grid_f64(int* grid) {
-  auto kern = nsgs_batch_kernel<double>;
-  int dev = 0, nsm = 0, per_sm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BlockDim<double>::value, 0);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  *grid = nsm * per_sm;
-  return cudaSuccess;
-}
+// Queried outside any stream capture; the caller keeps the figure with its
+// context.
+cudaError_t batch_grid_f64(int* grid) { return batch_grid_t<double>(grid); }
 
-// One block per problem, at most max_grid (batch_grid_f64) resident blocks.
-cudaError_t launch_batch_f64(const BatchArgs<double>& b, int max_grid, cudaStream_t s, int* grid) {
-  if (max_grid < 1) return cudaErrorInvalidConfiguration;
-  const int g = max_grid < b.nscenes ? max_grid : b.nscenes;
-  *grid = g;
-  nsgs_batch_kernel<double><<<g, BlockDim<double>::value, 0, s>>>(b);
-  return cudaGetLastError();
-}
+cudaError_t launch_batch_f64(const BatchArgs<double>& b, int grid, cudaStream_t s) { return launch_batch_t(b, grid, s); }
 
 void warm_batch_kernel_f64() {
   cudaFuncAttributes fa;

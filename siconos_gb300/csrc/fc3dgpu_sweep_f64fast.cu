@@ -50,27 +50,9 @@ cudaError_t fc3dgpu_launch_sweep_f64_fast(const void* args, int lanes, int max_g
   }
 }
 
-cudaError_t fc3dgpu_batch_grid_f64_fast(int* grid) {
-  using namespace fc3dgpu_fast64;
-  auto kern = nsgs_batch_kernel<double>;
-  int dev = 0, nsm = 0, per_sm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BlockDim<double>::value, 0);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  *grid = nsm * per_sm;
-  return cudaSuccess;
-}
+cudaError_t fc3dgpu_batch_grid_f64_fast(int* grid) { return fc3dgpu_fast64::batch_grid_t<double>(grid); }
 
-cudaError_t fc3dgpu_launch_batch_f64_fast(const void* args, int max_grid, cudaStream_t s, int* grid) {
+cudaError_t fc3dgpu_launch_batch_f64_fast(const void* args, int grid, cudaStream_t s) {
   using namespace fc3dgpu_fast64;
-  const BatchArgs<double>& b = *static_cast<const BatchArgs<double>*>(args);
-  if (max_grid < 1) return cudaErrorInvalidConfiguration;
-  const int g = max_grid < b.nscenes ? max_grid : b.nscenes;
-  *grid = g;
-  nsgs_batch_kernel<double><<<g, BlockDim<double>::value, 0, s>>>(b);
-  return cudaGetLastError();
+  return launch_batch_t(*static_cast<const BatchArgs<double>*>(args), grid, s);
 }

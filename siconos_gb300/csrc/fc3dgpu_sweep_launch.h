@@ -20,11 +20,11 @@ void warm_sweep_kernels();
 template <typename Real>
 struct BatchArgs;
 // Batched kernel: resident blocks on the current device (query outside any
-// stream capture), and the launch of min(max_grid, problems) blocks.
+// stream capture), and the launch of `grid` of them.
 cudaError_t batch_grid_f32(int* grid);
 cudaError_t batch_grid_f64(int* grid);
-cudaError_t launch_batch_f32(const BatchArgs<float>& b, int max_grid, cudaStream_t s, int* grid);
-cudaError_t launch_batch_f64(const BatchArgs<double>& b, int max_grid, cudaStream_t s, int* grid);
+cudaError_t launch_batch_f32(const BatchArgs<float>& b, int grid, cudaStream_t s);
+cudaError_t launch_batch_f64(const BatchArgs<double>& b, int grid, cudaStream_t s);
 void warm_batch_kernel_f32();
 void warm_batch_kernel_f64();
 int sweep_grid_f64(int lanes);
