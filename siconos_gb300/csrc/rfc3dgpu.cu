@@ -4,7 +4,8 @@
 // row its blocks sorted by (original) column, the column stored permuted,
 // each a 5x5 column-major block; q, mu, mu_r, rho, r, u in permuted order.
 // One cooperative launch runs every sweep: a colour's contacts are spread
-// over all threads of the grid, a grid barrier separates colours, and the
+// over the whole grid (five lanes a contact in FP64, one in FP32), a grid
+// barrier separates colours, and the
 // convergence logic runs on the device with the same bits in every block.
 // FP64 without FMA contraction, in the reference's operation order; in mixed
 // precision FP32 sweeps of the same loop run first and the FP64 loop starts
@@ -21,6 +22,7 @@
 #include <vector>
 
 #include "rfc3dgpu.h"
+#include "rfc3dgpu_coop.cuh"
 
 extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 
@@ -537,6 +539,66 @@ __device__ __forceinline__ void sweep_colours(const ArgsT<Real>& a, Real local_t
   }
 }
 
+// sweep_colours in FP64, five lanes a contact and six contacts a warp
+// (rfc3dgpu_coop.cuh).
+__device__ __forceinline__ void sweep_colours_coop(const Args& a, double local_tol, double v[2],
+                                                   cg::grid_group& g) {
+  const int lane = threadIdx.x & 31;
+  const bool spare = lane >= 5 * RFC3D_COOP_GROUPS;
+  RLane c;
+  const int grp = spare ? 0 : lane / 5;
+  c.base = 5 * grp;
+  c.i = lane - (spare ? 5 * RFC3D_COOP_GROUPS : c.base);
+  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (int col = 0; col < a.ncol; col++) {
+    const int end = a.cptr[col + 1];
+    for (int first = a.cptr[col] + gw * RFC3D_COOP_GROUPS; first < end; first += nw * RFC3D_COOP_GROUPS) {
+      // spare groups repeat the warp's first contact without storing it
+      const bool have = !spare && first + grp < end;
+      const int p = have ? first + grp : first;
+      double s = 0.0;
+      const int s0 = a.rp[p], s1 = a.rp[p + 1];
+      for (int sl = s0; sl < s1; sl++) {
+        const int j = a.col[sl];
+        if (j == p) continue;
+        const double* blk = a.W + 25 * (size_t)sl + c.i;
+        double x[5], w[5];
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+          x[k] = __ldcg(&a.r[5 * (size_t)j + k]);
+          w[k] = __ldg(&blk[5 * k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 5; k++) s += w[k] * x[k];
+      }
+      RProblem P;
+      P.q = a.q[5 * (size_t)p + c.i] + s;
+      const double old = __ldcg(&a.r[5 * (size_t)p + c.i]);
+      const double* d = a.W + 25 * (size_t)(s0 + a.dpos[p]);
+#pragma unroll
+      for (int e = 0; e < 25; e++) P.M[e] = __ldg(&d[e]);
+      P.mu = a.mu[p];
+      P.mur = a.mur[p];
+      P.rho = a.rho[p];
+      const bool off = ie_lt(-DBL_EPSILON, rget(P.q, c.base));  // take-off
+      double rl = old;
+      if (rany(have && !off)) rlocal_solve(c, P, have && !off, DBL_EPSILON, local_tol, a.local_max, rl);
+      if (off) rl = 0.0;
+      const double dr = old - rl;
+      const double d2 = rsum(c, dr * dr);
+      const double r2 = rsum(c, rl * rl);
+      if (have) {
+        __stcg(&a.r[5 * (size_t)p + c.i], rl);
+        if (c.i == 0) {
+          v[0] += d2;
+          v[1] += r2;
+        }
+      }
+    }
+    if (col + 1 < a.ncol) grid_sync(g);
+  }
+}
+
 __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
   __shared__ Reduce R;
   cg::grid_group g = cg::this_grid();
@@ -549,7 +611,7 @@ __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
   while (iter < a.max_iter && not_conv) {
     ++iter;
     double v[2] = {0.0, 0.0};
-    sweep_colours<double>(a, local_tol, v, g);
+    sweep_colours_coop(a, local_tol, v, g);
     grid_sum<2>(v, a, R, g);
     err = sqrt(v[0]);
     const double nr = sqrt(v[1]);
@@ -693,7 +755,7 @@ struct rfc3dgpu_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
-  int nc = 0, ncol = 0, max_colour = 0, blocks = 1, threads = NT;
+  int nc = 0, ncol = 0, max_colour = 0, blocks = 1, threads = NT, blocks32 = 1, threads32 = NT;
   double norm_q = 0.0;
   std::vector<int> perm, iperm, colour;
   std::vector<double> rho_host;
@@ -904,19 +966,23 @@ extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* 
   c->ncol = ncol;
   c->max_colour = 0;
   for (int k = 0; k < ncol; k++) c->max_colour = std::max(c->max_colour, cptr[k + 1] - cptr[k]);
-  // grid: the largest colour spread over as many SMs as it fills (the local
-  // Newton is bound by the FP64 pipe of each SM), smaller blocks when it
-  // fills fewer SMs than the device has; all blocks resident (cooperative)
+  // grids of the FP64 kernels (six contacts a warp) and the FP32 one (one a
+  // lane): the largest colour spread over as many SMs as it fills (both are
+  // bound by each SM's arithmetic), smaller blocks when it fills fewer SMs
+  // than the device has, one block (no grid barrier) when one holds it; all
+  // blocks resident (cooperative)
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-  int threads = NT;
-  while (threads > 32 && (c->max_colour + threads - 1) / threads < sms) threads /= 2;
-  int per_sm = 0, per_sm32 = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rfc3d_nsgs, threads, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm32, k_rfc3d_sweeps32, threads, 0);
-  const int resident = std::max(1, std::min(std::min(per_sm, per_sm32) * sms, MAX_BLOCKS));
-  c->threads = threads;
-  c->blocks = std::max(1, std::min((c->max_colour + threads - 1) / threads, resident));
+  auto shape = [&](const void* kernel, int per_warp, int& threads, int& blocks) {
+    auto blocks_of = [&](int t) { return (c->max_colour + t / 32 * per_warp - 1) / (t / 32 * per_warp); };
+    threads = NT;
+    while (threads > 32 && blocks_of(threads) > 1 && blocks_of(threads) < sms) threads /= 2;
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
+    blocks = std::max(1, std::min(blocks_of(threads), std::max(1, std::min(per_sm * sms, MAX_BLOCKS))));
+  };
+  shape((const void*)k_rfc3d_nsgs, RFC3D_COOP_GROUPS, c->threads, c->blocks);
+  shape((const void*)k_rfc3d_sweeps32, 32, c->threads32, c->blocks32);
   return 0;
 }
 
@@ -979,9 +1045,9 @@ static ArgsT<float> args32_of(const rfc3dgpu_ctx* c) {
 }
 
 template <typename K, typename A>
-static cudaError_t launch(rfc3dgpu_ctx* c, K kernel, A& a) {
+static cudaError_t launch(rfc3dgpu_ctx* c, K kernel, A& a, int blocks, int threads) {
   void* params[] = {&a};
-  return cudaLaunchCooperativeKernel((const void*)kernel, dim3(c->blocks), dim3(c->threads), params, 0, c->stream);
+  return cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(threads), params, 0, c->stream);
 }
 
 extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, double local_tol, int local_max_iter,
@@ -1005,7 +1071,7 @@ extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, dou
     a.stall_window = c->stall;
     k_rfc3d_to_f32<<<(n5 + 255) / 256, 256, 0, c->stream>>>(n5, c->r, c->r32);
     KR(cudaGetLastError());
-    KR(launch(c, k_rfc3d_sweeps32, a));
+    KR(launch(c, k_rfc3d_sweeps32, a, c->blocks32, c->threads32));
     KR(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
     KR(cudaStreamSynchronize(c->stream));
     sweeps32 = (int)out[0];
@@ -1023,7 +1089,7 @@ extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, dou
   a.local_max = local_max_iter;
   a.trace = c->trace + std::min(sweeps32, TRACE_CAP);
   a.trace_cap = TRACE_CAP - std::min(sweeps32, TRACE_CAP);
-  KR(launch(c, k_rfc3d_nsgs, a));
+  KR(launch(c, k_rfc3d_nsgs, a, c->blocks, c->threads));
   KR(cudaEventRecord(c->ev[1], c->stream));
   KR(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
   KR(cudaStreamSynchronize(c->stream));
@@ -1062,7 +1128,7 @@ extern "C" int rfc3dgpu_ctx_compute_error(rfc3dgpu_ctx* c, double norm_q, double
   KR(cudaSetDevice(c->device));
   Args a = args_of(c);
   a.norm_q = norm_q;
-  KR(launch(c, k_rfc3d_error, a));
+  KR(launch(c, k_rfc3d_error, a, c->blocks, c->threads));
   KR(cudaMemcpyAsync(error, c->out + 1, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   KR(cudaStreamSynchronize(c->stream));
   return 0;
