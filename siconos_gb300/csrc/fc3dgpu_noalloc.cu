@@ -9,8 +9,21 @@
 // the device and stall their other streams in the middle of a time step, or
 // fail because the pool has taken the memory).
 //
-// The reduction order is fixed by the chunking (256 contacts per chunk,
-// chunks summed in index order), so the result does not depend on the grid.
+// The reduction order is fixed by the chunking (chunk_of(nc) contacts per
+// chunk, chunks summed in index order), so the result does not depend on the
+// grid.
+//
+// What bounds it: the FP64 unit (a warp instruction in 64 cycles per SM
+// quarter: 9 fused multiply-adds a block of W against 72 bytes, 21 us of
+// arithmetic against 13 us of HBM time for 94,400 contacts), and below some
+// 20,000 contacts one row's chain of them.  So three threads share a row, one
+// component each (a third of the chain, and their loads of a block and stores
+// of the velocity are contiguous), then one thread a contact forms the
+// natural map from shared memory; chunks are small, so that few contacts
+// still reach every SM and the last round is short; and the completion
+// tickets rotate instead of being cleared by a copy operation before every
+// launch.  21.2 -> 9.0 us at 16 contacts, 33.6 -> 16.9 at 23,200, 76.2 -> 41.3 at
+// 94,400, 210 -> 147 at 320,400 (back to back on the device).
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
@@ -25,95 +38,131 @@ extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 namespace fc3dgpu {
 namespace noalloc {
 
-constexpr int CHUNK = 256;  // contacts per chunk = threads per block
-constexpr int MAX_CHUNKS = FC3DGPU_NOALLOC_MAX_CONTACTS / CHUNK;
-static_assert(MAX_CHUNKS * CHUNK == FC3DGPU_NOALLOC_MAX_CONTACTS, "limit must be a multiple of the chunk");
-// 3 partial sums per chunk, then one 256-byte line holding the ticket
+// Contacts per chunk: 64, or 256 where 64 would make more chunks than the
+// last block sums quickly (and than the scratch holds).
+constexpr int SMALL_CHUNK = 64, LARGE_CHUNK = 256;
+constexpr int SMALL_MAX = 1 << 19;  // contacts
+static int chunk_of(int nc) { return nc <= SMALL_MAX ? SMALL_CHUNK : LARGE_CHUNK; }
+constexpr int MAX_CHUNKS = FC3DGPU_NOALLOC_MAX_CONTACTS / LARGE_CHUNK;
+static_assert(MAX_CHUNKS * LARGE_CHUNK == FC3DGPU_NOALLOC_MAX_CONTACTS, "limit must be a multiple of the chunk");
+static_assert(SMALL_MAX / SMALL_CHUNK <= MAX_CHUNKS, "the scratch holds the small chunks");
+// 3 partial sums per chunk, then one 256-byte line of SLOTS completion slots
+// (ticket, bad-input flag).  A call takes the next slot; a launch that
+// completes leaves its slot at zero and clears the one half a turn ahead,
+// which makes an interrupted launch harmless.
+constexpr int SLOTS = 16;
 constexpr int SCRATCH_DOUBLES = 3 * MAX_CHUNKS + 32;
 static_assert(SCRATCH_DOUBLES * 8 == FC3DGPU_NOALLOC_SCRATCH_BYTES, "header states the scratch size");
 
 static __device__ __align__(256) double g_scratch[SCRATCH_DOUBLES];
 
+// Sums of three values over the first CH threads of the block (the others
+// pass nothing), warps in order; every thread gets them.
+template <int CH>
 __device__ __forceinline__ void block_sum3(double v[3], double (*sh)[3]) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x < CH) {
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    double x = v[k];
+    for (int k = 0; k < 3; k++) {
+      double x = v[k];
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[w][k] = x;
+      for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      if (lane == 0) sh[w][k] = x;
+    }
   }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    double s = 0.0;
-    for (int i = 0; i < CHUNK / 32; i++) s += sh[i][k];
+    double s = sh[0][k];
+#pragma unroll
+    for (int i = 1; i < CH / 32; i++) s += sh[i][k];
     v[k] = s;
   }
-  __syncthreads();
 }
 
 // Rows are read in the caller's block-CSR order (the diagonal block at its
 // own position), as SBM_gemv_3x3 does (SparseBlockMatrix.c:360-419).  A row
 // pointer or column index out of range is not followed: the error becomes
 // NaN.
-__global__ void __launch_bounds__(CHUNK) k_error_noalloc(int nc, long long nnz, const int64_t* __restrict__ rowptr,
-                                                         const int64_t* __restrict__ colidx,
-                                                         const double* __restrict__ blocks,
-                                                         const double* __restrict__ q, const double* __restrict__ mu,
-                                                         const double* __restrict__ r, double norm_q,
-                                                         double* __restrict__ velocity, double* __restrict__ error,
-                                                         double* __restrict__ scratch) {
-  __shared__ double sh[CHUNK / 32][3];
+template <int CH>
+__global__ void __launch_bounds__(3 * CH) k_error_noalloc(int nc, long long nnz, const int64_t* __restrict__ rowptr,
+                                                          const int64_t* __restrict__ colidx,
+                                                          const double* __restrict__ blocks,
+                                                          const double* __restrict__ q, const double* __restrict__ mu,
+                                                          const double* __restrict__ r, double norm_q,
+                                                          double* __restrict__ velocity, double* __restrict__ error,
+                                                          double* __restrict__ scratch, int slot) {
+  __shared__ double su[3 * CH], sr[3 * CH];
+  __shared__ double sh[CH / 32][3];
   __shared__ int last;
-  __shared__ int bad_any;
   double* part = scratch;
-  unsigned* ticket = reinterpret_cast<unsigned*>(scratch + 3 * MAX_CHUNKS);
-  unsigned* bad = ticket + 1;
-  const int nchunks = (nc + CHUNK - 1) / CHUNK;
+  unsigned* slots = reinterpret_cast<unsigned*>(scratch + 3 * MAX_CHUNKS);
+  unsigned *ticket = slots + 2 * slot, *bad = ticket + 1;
+  const int nchunks = (nc + CH - 1) / CH;
   int badl = 0;
+  const int t = threadIdx.x, comp = t % 3;
   for (int ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
-    const int i = ch * CHUNK + threadIdx.x;
-    double v[3] = {0.0, 0.0, 0.0};
+    const size_t x0 = (size_t)3 * ch * CH + t;  // the thread's entry of the vectors
+    const int i = ch * CH + t / 3;
     if (i < nc) {
-      double u[3] = {q[3 * (size_t)i], q[3 * (size_t)i + 1], q[3 * (size_t)i + 2]};
-      const double rr[3] = {r[3 * (size_t)i], r[3 * (size_t)i + 1], r[3 * (size_t)i + 2]};
+      double u = q[x0];
       const long long b0 = rowptr[i], b1 = rowptr[i + 1];
       if (b0 < 0 || b1 < b0 || b1 > nnz) {
         badl = 1;
       } else {
-        for (long long b = b0; b < b1; b++) {
-          const long long j = colidx[b];
-          if (j < 0 || j >= nc) {
-            badl = 1;
-            continue;
-          }
-          double wv[9];
+        // blocks four at a time: their columns, then their values and
+        // reactions, are requested together; a column out of range reads
+        // contact 0 and flags the input
+        constexpr int U = 4;
+        for (long long b = b0; b < b1; b += U) {
+          long long j[U];
+          double wv[U][3], rv[U][3];
 #pragma unroll
-          for (int e = 0; e < 9; e++) wv[e] = blocks[9 * b + e];
-          const double rj[3] = {r[3 * j], r[3 * j + 1], r[3 * j + 2]};
-          mvp3x3(wv, rj, u);
+          for (int k = 0; k < U; k++) {
+            j[k] = b + k < b1 ? __ldg(&colidx[b + k]) : 0;
+            if (j[k] < 0 || j[k] >= nc) {
+              badl = 1;
+              j[k] = 0;
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < U; k++)
+#pragma unroll
+            for (int e = 0; e < 3; e++) {
+              wv[k][e] = b + k < b1 ? __ldg(&blocks[9 * (b + k) + 3 * e + comp]) : 0.0;
+              rv[k][e] = b + k < b1 ? __ldg(&r[3 * j[k] + e]) : 0.0;
+            }
+#pragma unroll
+          for (int k = 0; k < U; k++)
+            if (b + k < b1)
+#pragma unroll
+              for (int e = 0; e < 3; e++) u = fma(wv[k][e], rv[k][e], u);
         }
       }
-      v[0] = unitary_error2(rr, u, mu[i]);
-      v[1] = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-      v[2] = rr[0] * rr[0] + rr[1] * rr[1] + rr[2] * rr[2];
-      if (velocity) {
-        velocity[3 * (size_t)i] = u[0];
-        velocity[3 * (size_t)i + 1] = u[1];
-        velocity[3 * (size_t)i + 2] = u[2];
-      }
+      su[t] = u;
+      sr[t] = r[x0];
+      if (velocity) velocity[x0] = u;
     }
-    block_sum3(v, sh);
-    if (threadIdx.x == 0) {
+    __syncthreads();
+    double v[3] = {0.0, 0.0, 0.0};
+    const int i1 = ch * CH + t;
+    if (t < CH && i1 < nc) {
+      const double uu[3] = {su[3 * t], su[3 * t + 1], su[3 * t + 2]}, rr[3] = {sr[3 * t], sr[3 * t + 1], sr[3 * t + 2]};
+      v[0] = unitary_error2<double>(rr, uu, mu[i1]);
+      v[1] = fma(uu[2], uu[2], fma(uu[1], uu[1], uu[0] * uu[0]));
+      v[2] = fma(rr[2], rr[2], fma(rr[1], rr[1], rr[0] * rr[0]));
+    }
+    block_sum3<CH>(v, sh);
+    if (t == 0) {
       part[3 * ch] = v[0];
       part[3 * ch + 1] = v[1];
       part[3 * ch + 2] = v[2];
     }
+    __syncthreads();  // sh and the vectors are free for the next chunk
   }
-  if (__syncthreads_or(badl) && threadIdx.x == 0) atomicOr(bad, 1u);
+  if (__syncthreads_or(badl) && t == 0) atomicOr(bad, 1u);
   // the last block to finish sums the chunk partials in chunk order
-  if (threadIdx.x == 0) {
+  if (t == 0) {
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
@@ -121,22 +170,25 @@ __global__ void __launch_bounds__(CHUNK) k_error_noalloc(int nc, long long nnz, 
   if (!last) return;
   __threadfence();
   double v[3] = {0.0, 0.0, 0.0};
-  for (int ch = threadIdx.x; ch < nchunks; ch += CHUNK) {
-    v[0] += __ldcg(&part[3 * ch]);
-    v[1] += __ldcg(&part[3 * ch + 1]);
-    v[2] += __ldcg(&part[3 * ch + 2]);
+  if (t < CH) {
+#pragma unroll 4
+    for (int ch = t; ch < nchunks; ch += CH) {
+      v[0] += __ldcg(&part[3 * ch]);
+      v[1] += __ldcg(&part[3 * ch + 1]);
+      v[2] += __ldcg(&part[3 * ch + 2]);
+    }
   }
-  block_sum3(v, sh);
-  if (threadIdx.x == 0) bad_any = (int)atomicOr(bad, 0u);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double e = sqrt(v[0]);
-    const double scal = fmax(norm_q, fmax(sqrt(v[2]), sqrt(v[1])));
-    if (fabs(scal) > DBL_EPSILON) e /= scal;
-    *error = bad_any ? __longlong_as_double(0x7ff8000000000000LL) : e;
-    // leave the ticket and the flag at zero for the next call
+  block_sum3<CH>(v, sh);
+  if (t == 0) {
+    double e = ie_sqrt(v[0]);
+    const double scal = fmax(norm_q, fmax(ie_sqrt(v[2]), ie_sqrt(v[1])));
+    if (fabs(scal) > DBL_EPSILON) e = ie_div(e, scal);
+    *error = atomicOr(bad, 0u) ? __longlong_as_double(0x7ff8000000000000LL) : e;
     *ticket = 0u;
     *bad = 0u;
+    const int ahead = (slot + SLOTS / 2) % SLOTS;
+    slots[2 * ahead] = 0u;
+    slots[2 * ahead + 1] = 0u;
   }
 }
 
@@ -151,6 +203,7 @@ struct Entry {
   void* ctx;
   double* addr;
   int sms;
+  unsigned calls;
 };
 Entry g_entry[MAX_DEVICES];
 typedef int (*CtxGetCurrent)(void**);  // cuCtxGetCurrent, through the runtime
@@ -162,7 +215,7 @@ static void* current_context() {
   return ctx;
 }
 
-int setup(int dev, double** addr, int* sms) {
+int setup(int dev, double** addr, int* sms, int* slot) {
   std::lock_guard<std::mutex> lock(g_mutex);
   if (!g_ctx_current) {
     void* fn = nullptr;
@@ -199,6 +252,7 @@ int setup(int dev, double** addr, int* sms) {
   }
   *addr = en.addr;
   *sms = en.sms;
+  *slot = (int)(en.calls++ % SLOTS);
   return 0;
 }
 
@@ -261,22 +315,21 @@ extern "C" int fc3dgpu_compute_error_device(int nc, int64_t nnz, const int64_t* 
       return NUMERICS_ERR_INVALID_ARGUMENT;
     }
   double* scratch = nullptr;
-  int sms = 0;
-  int rc = setup(dev, &scratch, &sms);
+  int sms = 0, slot = 0;
+  int rc = setup(dev, &scratch, &sms, &slot);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the ticket and the bad-input flag must be zero at launch; a launch that
-  // completes leaves them zero, this makes an interrupted one harmless
-  e = cudaMemsetAsync(scratch + 3 * MAX_CHUNKS, 0, 2 * sizeof(unsigned), s);
-  if (e == cudaSuccess) {
-    const int nchunks = (nc + CHUNK - 1) / CHUNK;
-    int grid = 4 * sms;
+  auto launch = [&](auto kernel, int chunk, int per_sm) {
+    const int nchunks = (nc + chunk - 1) / chunk;
+    int grid = per_sm * sms;
     if (grid > nchunks) grid = nchunks;
     if (grid < 1) grid = 1;
-    k_error_noalloc<<<grid, CHUNK, 0, s>>>(nc, (long long)nnz, rowptr, colidx, blocks, q, mu, reaction, norm_q,
-                                           velocity, error, scratch);
-    e = cudaGetLastError();
-  }
+    kernel<<<grid, 3 * chunk, 0, s>>>(nc, (long long)nnz, rowptr, colidx, blocks, q, mu, reaction, norm_q, velocity,
+                                      error, scratch, slot);
+    return cudaGetLastError();
+  };
+  e = chunk_of(nc) == SMALL_CHUNK ? launch(k_error_noalloc<SMALL_CHUNK>, SMALL_CHUNK, 8)
+                                  : launch(k_error_noalloc<LARGE_CHUNK>, LARGE_CHUNK, 2);
   if (e != cudaSuccess) {
     fc3dgpu_set_error("fc3dgpu_compute_error_device: %s", cudaGetErrorString(e));
     return NUMERICS_ERR_UNKNOWN;
