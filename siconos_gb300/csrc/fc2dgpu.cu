@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "fc2dgpu.h"
+#include "fc3dgpu_ieee64.cuh"
 
 extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 
@@ -58,6 +59,15 @@ struct Args {
   const T* det;     // determinant of each row's diagonal block
   const T* q;
   const T* mu;
+  // the sweep's copy of the rows, coalesced: contact k of colour c is lane
+  // k % 32 of slab sp[c] + k / 32; per slab its slots (off-diagonal blocks of
+  // its longest row, in row order), per slot and lane the permuted column
+  // (-1: none) and the block's entries (a00, a01, a10, a11)
+  const int* sp;
+  const int2* slab;  // (first slot, slots)
+  const int* scol;
+  const T* sW;
+  const T* D;       // 4 per contact: its diagonal block, column-major
   double* r;        // the reactions (FP64, permuted order)
   T* rw;            // the sweep's copy in HBM when it is not replicated
   double* u;
@@ -91,6 +101,16 @@ struct ClusterTeam {
       cl.sync();
   }
   __device__ __forceinline__ void sync_all() { cl.sync(); }
+  // the barrier in two halves: what stands between them overlaps its latency
+  __device__ __forceinline__ void arrive() {
+    if (size() > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  }
+  __device__ __forceinline__ void wait() {
+    if (size() > 1)
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else
+      __syncthreads();
+  }
 };
 
 struct GridTeam {
@@ -106,6 +126,8 @@ struct GridTeam {
       g.sync();
   }
   __device__ __forceinline__ void sync_all() { sync(); }
+  __device__ __forceinline__ void arrive() {}
+  __device__ __forceinline__ void wait() { sync(); }
 };
 
 // Where the sweep keeps the reactions.  HBM: read past L1 (ld.global.cg)
@@ -138,14 +160,15 @@ struct Reactions {
   }
 };
 
-template <typename T, typename V>
-__device__ __forceinline__ void mvp2x2(const T* a, const V v, T* y) {
-  const V a01 = __ldg(reinterpret_cast<const V*>(a));
-  const V a23 = __ldg(reinterpret_cast<const V*>(a) + 1);
-  y[0] += a01.x * v.x;
-  y[1] += a01.y * v.x;
-  y[0] += a23.x * v.y;
-  y[1] += a23.y * v.y;
+// Component `comp` alone of reaction j
+template <bool REP, typename Team>
+__device__ __forceinline__ void put_component(const Reactions<double, REP>& rx, int j, int comp, double x, Team& t) {
+  if constexpr (REP && !Team::grid) {
+    const int cs = t.size();
+    for (int k = 0; k < cs; k++) reinterpret_cast<double*>(t.cl.map_shared_rank(rx.rs, k))[2 * j + comp] = x;
+  } else {
+    __stcg(rx.rw + 2 * (size_t)j + comp, x);
+  }
 }
 
 // Team-wide sum of N values per thread, in a fixed order (xor-shuffle tree
@@ -162,6 +185,52 @@ struct Reduce {
   T bcast[4];
   int calls;
 };
+
+// The sum of two FP64 values: the same steps as trees of depth log2 (an FP64
+// addition takes 64 cycles, so the sums over warps and blocks in order above
+// cost more than a colour): the two values share each butterfly, 16 lanes
+// each.
+template <typename Team>
+__device__ __forceinline__ void team_sum2(double v[2], Reduce<double>& R, Team& team, double* gpart) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, which = lane >> 4, k16 = lane & 15;
+  auto tree = [&](double x) {
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+  // lanes 0-15 take over value 0, lanes 16-31 value 1
+  const double send = which ? v[0] : v[1], keep = which ? v[1] : v[0];
+  const double x = tree(keep + __shfl_xor_sync(0xffffffffu, send, 16));
+  if (k16 == 0) R.warp[w][which] = x;
+  __syncthreads();
+  const int slot = R.calls & 1, nw = blockDim.x >> 5;
+  double* gslot = gpart + (size_t)slot * GRID_MAX * 4;
+  if (w == 0) {
+    const double y = tree(k16 < nw ? R.warp[k16][which] : 0.0);
+    if (k16 == 0) {
+      if constexpr (Team::grid)
+        __stcg(&gslot[4 * blockIdx.x + which], y);
+      else
+        R.part[slot][which] = y;
+    }
+  }
+  team.sync();
+  if (w == 0) {
+    double y = 0.0;
+    if constexpr (Team::grid) {
+      for (int b = k16; b < (int)gridDim.x; b += 16) y += __ldcg(&gslot[4 * b + which]);
+    } else if (k16 < team.size()) {
+      y = team.cl.map_shared_rank(&R.part[slot][0], k16)[which];
+    }
+    y = tree(y);
+    if (k16 == 0) R.bcast[which] = y;
+    if (lane == 0) R.calls++;
+  }
+  __syncthreads();
+  v[0] = R.bcast[0];
+  v[1] = R.bcast[1];
+  __syncthreads();
+}
 
 template <int N, typename T, typename Team>
 __device__ __forceinline__ void team_sum(T v[N], Reduce<T>& R, Team& team, double* gpart) {
@@ -187,14 +256,24 @@ __device__ __forceinline__ void team_sum(T v[N], Reduce<T>& R, Team& team, doubl
   }
   team.sync();
   if constexpr (Team::grid) {
-    // thread 0 adds the blocks' partials in order
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < N; i++) {
-        T s = 0;
-        for (int b = 0; b < (int)gridDim.x; b++) s += (T)__ldcg(&gslot[4 * b + i]);
-        R.bcast[i] = s;
+    // the blocks' partials added in order; a warp fetches 32 of them at once
+    if (w == 0) {
+      T s[N];
+#pragma unroll
+      for (int i = 0; i < N; i++) s[i] = 0;
+      for (int b = 0; b < (int)gridDim.x; b += 32) {
+        const int n = min(32, (int)gridDim.x - b);
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+          const T mine = lane < n ? (T)__ldcg(&gslot[4 * (b + lane) + i]) : T(0);
+          for (int k = 0; k < n; k++) s[i] += __shfl_sync(0xffffffffu, mine, k);
+        }
       }
-      R.calls++;
+      if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i++) R.bcast[i] = s[i];
+        R.calls++;
+      }
     }
   } else if (w == 0) {
     // lane k fetches block k's partials (the remote loads overlap), lane 0
@@ -286,6 +365,215 @@ __device__ __forceinline__ void local_solve(const T* W, T D, const T* q, T mu, T
   }
 }
 
+// Slots of a row loaded together, ahead of their products.
+#define FC2D_NB 8
+
+// The static inputs of a contact (its first slots' columns and entries),
+// loaded before the barrier that releases its colour.
+template <typename T>
+struct Row;
+template <>
+struct Row<float> {
+  int p, first, slots;  // the contact, its slab's slots
+  int col[FC2D_NB];
+  float4 w[FC2D_NB];
+  float2 q;
+  float4 d;  // diagonal block
+  float det, mu;
+};
+template <>
+struct Row<double> {
+  int p, first, slots;
+  int col[FC2D_NB];
+  double2 w[FC2D_NB];  // row `comp` of the blocks
+  double q;
+};
+
+template <typename T>
+__device__ __forceinline__ void load_slots(const Args<T>& a, Row<T>& x, int t0, int lane, int comp) {
+#pragma unroll
+  for (int k = 0; k < FC2D_NB; k++) {
+    x.col[k] = -1;
+    if (t0 + k < x.slots) {
+      const size_t e = (size_t)(x.first + t0 + k) * 32 + lane;
+      x.col[k] = __ldg(&a.scol[e]);
+      if constexpr (sizeof(T) == sizeof(float))
+        x.w[k] = __ldg(reinterpret_cast<const float4*>(a.sW) + e);
+      else
+        x.w[k] = __ldg(reinterpret_cast<const double2*>(a.sW) + 2 * e + comp);
+    }
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void load_row(const Args<T>& a, int c, int k, int comp, Row<T>& x) {
+  const int2 s = __ldg(&a.slab[__ldg(&a.sp[c]) + (k >> 5)]);
+  x.first = s.x;
+  x.slots = s.y;
+  x.p = __ldg(&a.cptr[c]) + k;
+  const size_t p = (size_t)x.p;
+  load_slots(a, x, 0, k & 31, comp);
+  if constexpr (sizeof(T) == sizeof(float)) {
+    x.q = __ldg(reinterpret_cast<const float2*>(a.q) + p);
+    x.d = __ldg(reinterpret_cast<const float4*>(a.D) + p);
+    x.det = __ldg(&a.det[p]);
+    x.mu = __ldg(&a.mu[p]);
+  } else {
+    x.q = __ldg(&a.q[2 * p + comp]);
+  }
+}
+
+// A contact of the FP32 sweep on one lane: its neighbours' reactions are
+// fetched together, then the products run in the row's order
+// (SBM_row_prod_no_diag_2x2: every block on the diagonal is left out).
+template <bool REP, typename Team>
+__device__ __forceinline__ void contact32(const Args<float>& a, const Reactions<float, REP>& rx, int k, Row<float>& x,
+                                          float& x0, float& x1, float P[2], Team& team) {
+  const int p = x.p;
+  const float2 old = rx.get(p);
+  float ql[2] = {x.q.x, x.q.y};
+  for (int t0 = 0;; t0 += FC2D_NB) {
+    float2 r[FC2D_NB];
+#pragma unroll
+    for (int i = 0; i < FC2D_NB; i++)
+      if (x.col[i] >= 0) r[i] = rx.get(x.col[i]);
+#pragma unroll
+    for (int i = 0; i < FC2D_NB; i++)
+      if (x.col[i] >= 0) {
+        ql[0] += x.w[i].x * r[i].x;
+        ql[1] += x.w[i].z * r[i].x;
+        ql[0] += x.w[i].y * r[i].y;
+        ql[1] += x.w[i].w * r[i].y;
+      }
+    if (t0 + FC2D_NB >= x.slots) break;
+    load_slots(a, x, t0 + FC2D_NB, k & 31, 0);
+  }
+  const float W[4] = {x.d.x, x.d.y, x.d.z, x.d.w};
+  P[0] = old.x;
+  P[1] = old.y;
+  local_solve<float>(W, x.det, ql, x.mu, P);
+  x0 = old.x - P[0];
+  x1 = old.y - P[1];
+  rx.put(p, P[0], P[1], team);
+}
+
+// A contact of the FP64 sweep on two lanes, one component each.  The sweep
+// is bound by FP64 warp instructions (64 cycles each on an SM quarter whatever
+// their lanes do), so the two rows of every product and the two quotients of
+// the local solve run side by side; divisions and comparisons are the integer
+// forms of fc3dgpu_ieee64.cuh.  The bits are local_solve's.  Every lane of the
+// warp calls it; `act` false stores nothing.
+template <bool REP, typename Team>
+__device__ __forceinline__ void contact64(const Args<double>& a, const Reactions<double, REP>& rx, int k, int comp,
+                                          bool act, Row<double>& x, double& dx, double& pn, Team& team) {
+  using namespace fc3dgpu;
+  const int p = x.p;
+  const double2 o = rx.get(p);
+  const double old = comp ? o.y : o.x;
+  double y = x.q;
+  for (int t0 = 0;; t0 += FC2D_NB) {
+    double2 r[FC2D_NB];
+#pragma unroll
+    for (int i = 0; i < FC2D_NB; i++)
+      if (x.col[i] >= 0) r[i] = rx.get(x.col[i]);
+#pragma unroll
+    for (int i = 0; i < FC2D_NB; i++)
+      if (x.col[i] >= 0) {
+        y += x.w[i].x * r[i].x;
+        y += x.w[i].y * r[i].y;
+      }
+    if (t0 + FC2D_NB >= x.slots) break;
+    load_slots(a, x, t0 + FC2D_NB, k & 31, comp);
+  }
+  const double z = __shfl_xor_sync(0xffffffffu, y, 1);
+  const double q0 = comp ? z : y, q1 = comp ? y : z;
+  const double2 n = __ldg(reinterpret_cast<const double2*>(a.D) + 2 * (size_t)p);      // Wnn, Wtn
+  const double2 t = __ldg(reinterpret_cast<const double2*>(a.D) + 2 * (size_t)p + 1);  // Wnt, Wtt
+  const double mu = __ldg(&a.mu[p]), det = __ldg(&a.det[p]);
+  double P = 0.0;
+  const bool contact = !ie_positive(q0);
+  // P = -(adjugate q) / D, component by component
+  const double s = (comp ? -n.y : t.y) * q0 + (comp ? n.x : -t.x) * q1;
+  const double f = ie_div(-s, det);
+  const double g = __shfl_xor_sync(0xffffffffu, f, 1);
+  const double P0 = comp ? g : f, P1 = comp ? f : g;
+  if (contact) {
+    P = f;
+    const double muPn = mu * P0;
+    if (ie_lt(muPn, ie_abs(P1))) {
+      // slip backward (P1 + mu P0 < 0) or forward
+      const bool back = ie_lt(P1, -muPn);
+      const double b = back ? n.x - mu * t.x : n.x + mu * t.x;
+      const double S0 = ie_div(-q0, b);
+      P = comp ? (back ? -mu : mu) * S0 : S0;
+    }
+  }
+  dx = old - P;
+  pn = P;
+  if (act) put_component<REP, Team>(rx, p, comp, P, team);
+}
+
+// All colours of one sweep; v gets this thread's sums |r_old - r_new|^2 and
+// |r_new|^2.  row: the static inputs of the thread's first contact of colour
+// 0, loaded; left loaded for the next sweep.
+template <bool REP, typename Team>
+__device__ __forceinline__ void sweep_colours(const Args<float>& a, const Reactions<float, REP>& rx, int g0, int G,
+                                              Row<float>& row, float v[2], Team& team) {
+  auto size = [&](int c) { return __ldg(&a.cptr[c + 1]) - __ldg(&a.cptr[c]); };
+  int n = size(0), next;
+  for (int c = 0; c < a.ncol; c++, n = next) {
+    const int cn = c + 1 < a.ncol ? c + 1 : 0;
+    next = size(cn);
+    float x0 = 0.f, x1 = 0.f, P[2] = {0.f, 0.f};
+    for (int k = g0; k < n; k += G) {
+      if (k != g0) {
+        // the sums of the contact before, in the sweep's order
+        v[0] += x0 * x0 + x1 * x1;
+        v[1] += P[0] * P[0] + P[1] * P[1];
+        load_row(a, c, k, 0, row);
+      }
+      contact32(a, rx, k, row, x0, x1, P, team);
+    }
+    if (c + 1 < a.ncol) team.arrive();
+    if (g0 < next) load_row(a, cn, g0, 0, row);
+    if (g0 < n) {
+      v[0] += x0 * x0 + x1 * x1;
+      v[1] += P[0] * P[0] + P[1] * P[1];
+    }
+    if (c + 1 < a.ncol) team.wait();
+  }
+}
+
+template <bool REP, typename Team>
+__device__ __forceinline__ void sweep_colours(const Args<double>& a, const Reactions<double, REP>& rx, int g0, int G,
+                                              Row<double>& row, double v[2], Team& team) {
+  const int comp = g0 & 1, h0 = g0 >> 1, H = G >> 1;
+  const int lead = (g0 & ~31) >> 1;  // the warp's first contact, present while any of the warp's is
+  auto size = [&](int c) { return __ldg(&a.cptr[c + 1]) - __ldg(&a.cptr[c]); };
+  int n = size(0), next;
+  for (int c = 0; c < a.ncol; c++, n = next) {
+    const int cn = c + 1 < a.ncol ? c + 1 : 0;
+    next = size(cn);
+    double dx = 0.0, pn = 0.0;
+    for (int j = 0; lead + j < n; j += H) {
+      const bool act = h0 + j < n;
+      const int k = act ? h0 + j : lead + j;
+      if (j > 0) {
+        v[0] += dx * dx;
+        v[1] += pn * pn;
+      }
+      if (j > 0 || !act) load_row(a, c, k, comp, row);
+      contact64(a, rx, k, comp, act, row, dx, pn, team);
+      if (!act) dx = pn = 0.0;
+    }
+    if (c + 1 < a.ncol) team.arrive();
+    if (h0 < next) load_row(a, cn, h0, comp, row);
+    v[0] += dx * dx;
+    v[1] += pn * pn;
+    if (c + 1 < a.ncol) team.wait();
+  }
+}
+
 // Bring the FP64 reactions into the sweep's copy (replica or FP32 copy in
 // HBM); the cluster barrier keeps other blocks from writing into a copy
 // before it is filled.
@@ -334,12 +622,20 @@ __device__ __forceinline__ void close_reactions(const Args<T>& a, const Reaction
 }
 
 // All sweeps of one problem (or of one precision phase of it) in one launch
-// of one thread-block cluster or one cooperative grid (the Team).  A colour's contacts are spread over the
-// cluster's threads (contact lo + g, lo + g + G, ... for global thread g of
-// G: a contact always lands on the same block, so its W row stays in that
-// SM's L1); the hardware cluster barrier (release / acquire) separates
-// colours, the barrier of the error reduction closing the last one, and the
-// convergence logic runs on the device with the same bits in every block.
+// of one thread-block cluster or one cooperative grid (the Team).  A colour's
+// contacts are spread over the team's threads, one a thread in FP32 and one a
+// pair of threads in FP64 (contact k, k + G, ... for place k of G: a contact
+// always lands on the same block, so its W row stays in that SM's L1).  What
+// bounds a colour is its dependent chain: the rows are stored coalesced
+// (read by rows, each lane touched its own lines and a colour of 5,000
+// contacts queued on the L1's tags) and loaded before the barrier that
+// releases the colour; the light-error terms are summed behind the barrier's
+// arrival.  Granular problems, us a sweep before and after: FP64 37.4 and 24.6
+// at 367 contacts, 49.2 and 34.9 at 7,002, 75.3 and 34.4 at 28,008; FP32 12.5
+// and 10.1, 16.5 and 14.2, 26.7 and 20.3.  The hardware cluster barrier
+// (release / acquire) separates colours, the barrier of the error reduction
+// closing the last one, and the convergence logic runs on the device with the
+// same bits in every block.
 // The light error's |r|^2 is summed over the new reactions as they are made
 // (each contact is updated once per sweep, so it is |r|^2 after the sweep).
 // A phase that follows another starts its sweep count, budget and trace
@@ -360,50 +656,28 @@ __global__ void __launch_bounds__(NT_MAX, 1) k_fc2d_nsgs(const Args<T> a) {
   const int budget = a.max_iter - done;
   T tolerance = (T)a.tol, err = (T)INFINITY, best = (T)INFINITY;
   int iter = 0, not_conv = 1, since_best = 0;
+  Row<T> row;
+  {
+    const int comp = sizeof(T) == sizeof(double) ? g0 & 1 : 0, k = sizeof(T) == sizeof(double) ? g0 >> 1 : g0;
+    if (k < a.cptr[1] - a.cptr[0]) load_row(a, 0, k, comp, row);
+  }
   while (iter < budget && not_conv) {
     ++iter;
     T v[2] = {0, 0};
-    for (int c = 0; c < a.ncol; c++) {
-      for (int p = a.cptr[c] + g0; p < a.cptr[c + 1]; p += G) {
-        const V old = rx.get(p);
-        T ql[2] = {a.q[2 * p], a.q[2 * p + 1]};
-        const int s0 = a.rp[p], s1 = a.rp[p + 1], sd = s0 + a.dpos[p];
-        // every block on the diagonal is left out (SBM_row_prod_no_diag_2x2);
-        // a row of up to NB blocks has all its neighbours' reactions fetched
-        // before the first product (one memory round trip, not one per
-        // block), then the products run in the row's order
-        constexpr int NB = sizeof(T) == sizeof(float) ? 16 : 8;
-        if (s1 - s0 <= NB) {
-          int cj[NB];
-          V rj[NB];
-#pragma unroll
-          for (int k = 0; k < NB; k++)
-            if (k < s1 - s0) cj[k] = a.col[s0 + k];
-#pragma unroll
-          for (int k = 0; k < NB; k++)
-            if (k < s1 - s0 && cj[k] != p) rj[k] = rx.get(cj[k]);
-#pragma unroll
-          for (int k = 0; k < NB; k++)
-            if (k < s1 - s0 && cj[k] != p) mvp2x2(a.W + 4 * (size_t)(s0 + k), rj[k], ql);
-        } else {
-          for (int s = s0; s < s1; s++) {
-            const int j = a.col[s];
-            if (j != p) mvp2x2(a.W + 4 * (size_t)s, rx.get(j), ql);
-          }
-        }
-        T P[2] = {old.x, old.y};
-        local_solve<T>(a.W + 4 * (size_t)sd, a.det[p], ql, a.mu[p], P);
-        const T x0 = old.x - P[0], x1 = old.y - P[1];
-        v[0] += x0 * x0 + x1 * x1;
-        v[1] += P[0] * P[0] + P[1] * P[1];
-        rx.put(p, P[0], P[1], team);
-      }
-      if (c + 1 < a.ncol) team.sync();
+    sweep_colours(a, rx, g0, G, row, v, team);
+    if constexpr (sizeof(T) == sizeof(double))
+      team_sum2(v, R, team, a.part);
+    else
+      team_sum<2>(v, R, team, a.part);
+    if constexpr (sizeof(T) == sizeof(double)) {
+      const double nr = fc3dgpu::ie_sqrt(v[1]);
+      err = fc3dgpu::ie_sqrt(v[0]);
+      if (fabs(nr) > DBL_EPSILON) err = fc3dgpu::ie_div(err, nr);
+    } else {
+      err = sqrt(v[0]);
+      const T nr = sqrt(v[1]);
+      if (fabs(nr) > (T)DBL_EPSILON) err /= nr;
     }
-    team_sum<2>(v, R, team, a.part);
-    err = sqrt(v[0]);
-    const T nr = sqrt(v[1]);
-    if (fabs(nr) > (T)DBL_EPSILON) err /= nr;
     if (a.trace && lead && done + iter <= TRACE_CAP) a.trace[done + iter - 1] = (double)err;
     if (a.mode == FP32_PHASE) {
       if (err < best) {
@@ -466,14 +740,18 @@ __global__ void __launch_bounds__(NT_MAX, 1) k_fc2d_error(const Args<double> a) 
 // ---------------------------------------------------------------------------
 using namespace fc2dgpu;
 
+// A launch: a cluster of cs blocks, or a cooperative grid of `blocks`; the
+// reactions in HBM or replicated in shared memory.
+struct Shape {
+  bool grid = false, rep = false;
+  int cs = 1, nt = 128, blocks = 1;
+};
+
 struct fc2dgpu_ctx {
   int device = 0;
   int cs_req = 0, nt_req = 0;  // launch shape asked for (0 = automatic)
   int rep_req = 0;             // reactions: 0 automatic, 1 in HBM, 2 replicated in shared memory
-  int cs = 1, nt = 128;        // launch shape of the current problem
-  bool rep = false;
-  bool grid = false;           // a cooperative grid of `blocks` blocks instead of a cluster
-  int blocks = 1;
+  Shape s32, s64;              // launch shapes of the current problem's FP32 and FP64 kernels
   int max_colour = 0;          // contacts in the largest colour
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -482,6 +760,10 @@ struct fc2dgpu_ctx {
   double norm_q = 0.0;
   std::vector<int> perm, iperm, colour;
   int *cptr = nullptr, *rp = nullptr, *col = nullptr, *dpos = nullptr;
+  int *sp = nullptr, *scol = nullptr;
+  int2* slab = nullptr;
+  double *sW = nullptr, *D = nullptr;
+  float *sW32 = nullptr, *D32 = nullptr;
   double *W = nullptr, *det = nullptr, *q = nullptr, *mu = nullptr, *r = nullptr, *u = nullptr, *trace = nullptr,
          *out = nullptr, *part = nullptr;
   // FP32 copies for the first phase of a mixed-precision solve
@@ -506,11 +788,15 @@ static void choose_shape(fc2dgpu_ctx* c);
 
 static void free_problem(fc2dgpu_ctx* c) {
   void* ptrs[] = {c->cptr, c->rp, c->col, c->dpos, c->W, c->det, c->q, c->mu, c->r, c->u,
-                  c->W32, c->det32, c->q32, c->mu32, c->r32};
+                  c->sp, c->scol, c->slab, c->sW, c->D, c->sW32, c->D32, c->W32, c->det32, c->q32, c->mu32, c->r32};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   c->cptr = c->rp = c->col = c->dpos = nullptr;
   c->W = c->det = c->q = c->mu = c->r = c->u = nullptr;
+  c->sp = c->scol = nullptr;
+  c->slab = nullptr;
+  c->sW = c->D = nullptr;
+  c->sW32 = c->D32 = nullptr;
   c->W32 = c->det32 = c->q32 = c->mu32 = c->r32 = nullptr;
   c->nc = 0;
 }
@@ -667,6 +953,52 @@ extern "C" int fc2dgpu_ctx_set_problem(fc2dgpu_ctx* c, int nc, const int64_t* ro
     if (e == cudaSuccess) e = upload(&c->mu32, mu32);
     if (e == cudaSuccess) e = upload(&c->r32, zero32);
   }
+  // the sweeps' coalesced copy of the rows (Args::slab)
+  {
+    std::vector<int> sp(ncol + 1, 0);
+    for (int k = 0; k < ncol; k++) sp[k + 1] = sp[k] + (cptr[k + 1] - cptr[k] + 31) / 32;
+    std::vector<int2> slab(sp[ncol]);
+    int slots = 0;
+    auto off_diagonal = [&](int p) {
+      int n = 0;
+      for (int s = rp[p]; s < rp[p + 1]; s++) n += col[s] != p;
+      return n;
+    };
+    for (int k = 0; k < ncol; k++)
+      for (int b = sp[k]; b < sp[k + 1]; b++) {
+        const int p0 = cptr[k] + 32 * (b - sp[k]), p1 = std::min(p0 + 32, cptr[k + 1]);
+        int m = 0;
+        for (int p = p0; p < p1; p++) m = std::max(m, off_diagonal(p));
+        slab[b] = make_int2(slots, m);
+        slots += m;
+      }
+    std::vector<int> scol((size_t)slots * 32, -1);
+    std::vector<double> sW((size_t)slots * 128, 0.0), D(4 * (size_t)nc);
+    for (int k = 0; k < ncol; k++)
+      for (int p = cptr[k]; p < cptr[k + 1]; p++) {
+        const int b = sp[k] + (p - cptr[k]) / 32, lane = (p - cptr[k]) % 32;
+        size_t slot = (size_t)slab[b].x;
+        for (int s = rp[p]; s < rp[p + 1]; s++) {
+          if (col[s] == p) continue;
+          const size_t x = slot++ * 32 + lane;
+          scol[x] = col[s];
+          const double* w = &W[4 * (size_t)s];
+          sW[4 * x] = w[0];
+          sW[4 * x + 1] = w[2];
+          sW[4 * x + 2] = w[1];
+          sW[4 * x + 3] = w[3];
+        }
+        for (int i = 0; i < 4; i++) D[4 * (size_t)p + i] = W[4 * ((size_t)rp[p] + dpos[p]) + i];
+      }
+    const std::vector<float> sW32(sW.begin(), sW.end()), D32(D.begin(), D.end());
+    if (e == cudaSuccess) e = upload(&c->sp, sp);
+    if (e == cudaSuccess) e = upload(&c->slab, slab);
+    if (e == cudaSuccess) e = upload(&c->scol, scol);
+    if (e == cudaSuccess) e = upload(&c->sW, sW);
+    if (e == cudaSuccess) e = upload(&c->D, D);
+    if (e == cudaSuccess) e = upload(&c->sW32, sW32);
+    if (e == cudaSuccess) e = upload(&c->D32, D32);
+  }
   if (e != cudaSuccess) {
     free_problem(c);
     fc3dgpu_set_error("fc2dgpu_ctx_set_problem: %s", cudaGetErrorString(e));
@@ -780,27 +1112,34 @@ static bool cluster_fits(fc2dgpu_ctx* c, int cs, int nt, bool rep) {
 // goes to a cooperative grid over every SM instead (grid barrier, about
 // 1-2 us, instead of the cluster's 0.3 us; the FP64 pipes of all SMs).
 constexpr int GRID_FROM = CS_MAX * NT_MAX;
+// In FP64 the FP64 units of a cluster's SMs bound a colour from far fewer
+// contacts (cluster and grid, us a sweep: 40.7 and 35.2 with 2,401 contacts in
+// the largest colour, 67.5 and 34.6 with 4,828; 26 on a cluster with 514,
+// where the grid's barriers alone take 8 more than the cluster's).
+constexpr int GRID64_FROM = 1000;
 
-static void choose_grid(fc2dgpu_ctx* c) {
-  int nt = c->nt_req > 0 ? c->nt_req : 256;
-  nt = std::min(std::max(nt / 32 * 32, 32), NT_MAX);
+static Shape grid_shape(fc2dgpu_ctx* c, int nt, int lanes) {
+  Shape s;
   int sms = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  // FP64: the largest colour over all SMs, one pass each
+  if (nt <= 0) nt = lanes == 1 ? 256 : std::min(256, std::max(32, (lanes * c->max_colour / std::max(sms, 1) + 31) / 32 * 32));
+  nt = std::min(std::max(nt / 32 * 32, 32), NT_MAX);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fc2d_nsgs<double, false, GridTeam>, nt, 0);
   const int resident = std::max(1, std::min(per_sm * sms, GRID_MAX));
-  c->grid = true;
-  c->rep = false;
-  c->nt = nt;
-  c->cs = 1;
-  c->blocks = std::max(1, std::min((c->max_colour + nt - 1) / nt, resident));
+  s.grid = true;
+  s.nt = nt;
+  s.blocks = std::max(1, std::min((lanes * c->max_colour + nt - 1) / nt, resident));
+  return s;
 }
 
 static void choose_shape(fc2dgpu_ctx* c) {
   if (c->cs_req < 0 || (c->cs_req == 0 && c->rep_req != 2 && c->max_colour > GRID_FROM)) {
-    choose_grid(c);
+    c->s32 = grid_shape(c, c->nt_req, 1);
+    c->s64 = c->cs_req < 0 ? c->s32 : grid_shape(c, c->nt_req, 2);
     return;
   }
-  c->grid = false;
+  Shape s;
   int cs = c->cs_req, nt = c->nt_req;
   if (cs <= 0) {
     const int want = (c->max_colour + 63) / 64;  // about 64 contacts per SM and colour
@@ -816,23 +1155,30 @@ static void choose_shape(fc2dgpu_ctx* c) {
   if (rep && c->rep_req == 0 && !cluster_fits(c, cs, nt, true)) rep = false;
   if (c->cs_req <= 0)
     while (cs > 1 && !cluster_fits(c, cs, nt, rep)) cs /= 2;
-  c->cs = cs;
-  c->nt = nt;
-  c->rep = rep;
+  s.cs = cs;
+  s.nt = nt;
+  s.rep = rep;
+  c->s32 = c->s64 = s;
+  // FP64 takes two threads a contact
+  if (c->nt_req == 0) {
+    const int nt2 = std::min(NT_MAX, 2 * nt);
+    if (cluster_fits(c, cs, nt2, rep)) c->s64.nt = nt2;
+  }
+  if (c->cs_req == 0 && c->rep_req == 0 && c->max_colour > GRID64_FROM) c->s64 = grid_shape(c, c->nt_req, 2);
 }
 
 template <typename K, typename A>
-static cudaError_t launch_grid(fc2dgpu_ctx* c, K kernel, const A& a) {
+static cudaError_t launch_grid(fc2dgpu_ctx* c, const Shape& s, K kernel, const A& a) {
   void* params[] = {(void*)&a};
-  return cudaLaunchCooperativeKernel((const void*)kernel, dim3(c->blocks), dim3(c->nt), params, 0, c->stream);
+  return cudaLaunchCooperativeKernel((const void*)kernel, dim3(s.blocks), dim3(s.nt), params, 0, c->stream);
 }
 
 template <typename K, typename A>
-static cudaError_t launch(fc2dgpu_ctx* c, K kernel, const A& a, size_t smem) {
-  cudaError_t e = prepare(kernel, c->cs, smem);
+static cudaError_t launch(fc2dgpu_ctx* c, const Shape& s, K kernel, const A& a, size_t smem) {
+  cudaError_t e = prepare(kernel, s.cs, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = config(c, c->cs, c->nt, smem, attr);
+  cudaLaunchConfig_t cfg = config(c, s.cs, s.nt, smem, attr);
   return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
@@ -864,9 +1210,9 @@ extern "C" int fc2dgpu_ctx_set_launch(fc2dgpu_ctx* c, int cluster_blocks, int th
 
 extern "C" int fc2dgpu_ctx_launch_shape(fc2dgpu_ctx* c, int* cluster_blocks, int* threads, int* reactions) {
   if (!c) return NUMERICS_ERR_INVALID_ARGUMENT;
-  if (cluster_blocks) *cluster_blocks = c->grid ? -c->blocks : c->cs;
-  if (threads) *threads = c->nt;
-  if (reactions) *reactions = c->rep ? 2 : 1;
+  if (cluster_blocks) *cluster_blocks = c->s32.grid ? -c->s32.blocks : c->s32.cs;
+  if (threads) *threads = c->s32.nt;
+  if (reactions) *reactions = c->s32.rep ? 2 : 1;
   return 0;
 }
 
@@ -880,6 +1226,11 @@ static Args<double> args64(const fc2dgpu_ctx* c) {
   a.col = c->col;
   a.dpos = c->dpos;
   a.W = c->W;
+  a.sp = c->sp;
+  a.slab = c->slab;
+  a.scol = c->scol;
+  a.sW = c->sW;
+  a.D = c->D;
   a.det = c->det;
   a.q = c->q;
   a.mu = c->mu;
@@ -903,6 +1254,11 @@ static Args<float> args32(const fc2dgpu_ctx* c) {
   a.col = c->col;
   a.dpos = c->dpos;
   a.W = c->W32;
+  a.sp = c->sp;
+  a.slab = c->slab;
+  a.scol = c->scol;
+  a.sW = c->sW32;
+  a.D = c->D32;
   a.det = c->det32;
   a.q = c->q32;
   a.mu = c->mu32;
@@ -942,9 +1298,10 @@ extern "C" int fc2dgpu_ctx_compute_error(fc2dgpu_ctx* c, double norm_q, double* 
   K2(cudaSetDevice(c->device));
   Args<double> a = args64(c);
   a.norm_q = norm_q;
-  K2(c->grid ? launch_grid(c, k_fc2d_error<false, GridTeam>, a)
-     : c->rep ? launch(c, k_fc2d_error<true, ClusterTeam>, a, rep_bytes(c))
-              : launch(c, k_fc2d_error<false, ClusterTeam>, a, 0));
+  const Shape& s = c->s64;
+  K2(s.grid  ? launch_grid(c, s, k_fc2d_error<false, GridTeam>, a)
+     : s.rep ? launch(c, s, k_fc2d_error<true, ClusterTeam>, a, rep_bytes(c))
+             : launch(c, s, k_fc2d_error<false, ClusterTeam>, a, 0));
   K2(cudaMemcpyAsync(error, c->out + 1, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   K2(cudaStreamSynchronize(c->stream));
   return 0;
@@ -989,14 +1346,16 @@ extern "C" int fc2dgpu_ctx_solve(fc2dgpu_ctx* c, double tol, int max_iter, int e
     b.mode = FP32_PHASE;
     b.switch_tol = c->switch_tol > 0.0 ? c->switch_tol : std::max(tol, 1e-6);
     b.stall = c->stall;
-    K2(c->grid  ? launch_grid(c, k_fc2d_nsgs<float, false, GridTeam>, b)
-       : c->rep ? launch(c, k_fc2d_nsgs<float, true, ClusterTeam>, b, sizeof(float2) * (size_t)c->nc)
-                : launch(c, k_fc2d_nsgs<float, false, ClusterTeam>, b, 0));
+    const Shape& s = c->s32;
+    K2(s.grid  ? launch_grid(c, s, k_fc2d_nsgs<float, false, GridTeam>, b)
+       : s.rep ? launch(c, s, k_fc2d_nsgs<float, true, ClusterTeam>, b, sizeof(float2) * (size_t)c->nc)
+               : launch(c, s, k_fc2d_nsgs<float, false, ClusterTeam>, b, 0));
     a.before = c->out + 4;
   }
-  K2(c->grid  ? launch_grid(c, k_fc2d_nsgs<double, false, GridTeam>, a)
-     : c->rep ? launch(c, k_fc2d_nsgs<double, true, ClusterTeam>, a, rep_bytes(c))
-              : launch(c, k_fc2d_nsgs<double, false, ClusterTeam>, a, 0));
+  const Shape& s = c->s64;
+  K2(s.grid  ? launch_grid(c, s, k_fc2d_nsgs<double, false, GridTeam>, a)
+     : s.rep ? launch(c, s, k_fc2d_nsgs<double, true, ClusterTeam>, a, rep_bytes(c))
+             : launch(c, s, k_fc2d_nsgs<double, false, ClusterTeam>, a, 0));
   K2(cudaEventRecord(c->ev[1], c->stream));
   double out[8];
   K2(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
