@@ -451,9 +451,18 @@ __global__ void k_r32_to_r64(int npad, const float* __restrict__ r32, const floa
   }
 }
 
+// The FP32 reactions of a solve's start, with the stamps of the dataflow sweep
+// in their fourth words: sweep 0, and for the zero entry every sweep.
 __global__ void k_r64_to_r32(int npad, const double* __restrict__ r64, float* __restrict__ r32) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npad; p += gridDim.x * blockDim.x)
-    for (int a = 0; a < 3; a++) r32[4 * (size_t)p + a] = (float)r64[4 * (size_t)p + a];
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= npad; p += gridDim.x * blockDim.x) {
+    float4 v = make_float4(0.f, 0.f, 0.f, __int_as_float(p < npad ? 0 : 0x7fffffff));
+    if (p < npad) {
+      v.x = (float)r64[4 * (size_t)p];
+      v.y = (float)r64[4 * (size_t)p + 1];
+      v.z = (float)r64[4 * (size_t)p + 2];
+    }
+    reinterpret_cast<float4*>(r32)[p] = v;
+  }
 }
 
 // The 17 warm-start features of every row (padding rows: zeros): the
@@ -761,6 +770,7 @@ struct fc3dgpu_ctx {
   int flow_on = 1;
   int flow_state = 0;
   int flow_nw = 0, flow_maxslot = 0;
+  bool flow_symmetric = false;  // every block has its transpose's place in W
   int flow_want = 0;  // warps per block of the dataflow sweep asked for (0: default)
   // measuring autotuner (per layout): chosen FP32 variant and FP64 lanes,
   // and the measured device time of one sweep of every candidate
@@ -1816,6 +1826,9 @@ static int prepare_flow(fc3dgpu_ctx* c) {
   CK(cudaMemcpyAsync(c->flow_dptr, sptr_sym.data(), sizeof(int) * (nslab + 1), cudaMemcpyHostToDevice, s));
   if (!sym.empty()) CK(cudaMemcpyAsync(c->flow_dep, sym.data(), sizeof(int) * sym.size(), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(c->flow_need, need.data(), sizeof(int2) * nslab, cudaMemcpyHostToDevice, s));
+  int missing = 0;
+  CK(check_flow_symmetric(c->npad, c->perm, c->slab_nslot, c->slab_off, c->col, c->scratch, s));
+  CK(cudaMemcpyAsync(&missing, c->scratch, sizeof(int), cudaMemcpyDeviceToHost, s));
   // offsets of the per-slab records (filled before each solve's FP32 sweeps)
   std::vector<long long> roff((size_t)nslab + 1, 0);
   for (int t = 0; t < nslab; t++) roff[t + 1] = roff[t] + flow_rec_floats(c->slab_nslot_h[t]);
@@ -1823,7 +1836,8 @@ static int prepare_flow(fc3dgpu_ctx* c) {
   CK(ensure(&c->flow_rec, &c->flow_rec_cap, (size_t)std::max(roff[nslab], 1LL)));
   CK(cudaMemcpyAsync(c->flow_rec_off, roff.data(), sizeof(long long) * (nslab + 1), cudaMemcpyHostToDevice, s));
   CK(cudaStreamSynchronize(s));
-  c->launches += 2;
+  c->flow_symmetric = missing == 0;
+  c->launches += 3;
   c->flow_nw = nw;
   c->flow_maxslot = maxslot;
   c->flow_state = 1;
@@ -2052,7 +2066,7 @@ static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st
     }
     // the FP32 sweeps start from the context's reaction (the FP64 iterate of
     // a previous solve, a warm start, or what fc3dgpu_ctx_set_r gave)
-    k_r64_to_r32<<<grid1d(c->npad), 256, 0, s>>>(c->npad, c->r64, c->r32);
+    k_r64_to_r32<<<grid1d(c->npad + 1), 256, 0, s>>>(c->npad, c->r64, c->r32);
     CK(cudaGetLastError());
     c->launches++;
     bool flow = lanes == 1 && use_flow && !a.counters;
@@ -2076,6 +2090,13 @@ static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st
       f.buf_bytes = flow_buf_bytes(c->flow_maxslot);
       f.rec = c->flow_rec;
       f.rec_off = c->flow_rec_off;
+      f.stamped = c->flow_symmetric ? 1 : 0;
+      f.split = 0;
+      if (f.stamped) {
+        int sms = 0;
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+        while (f.split < 5 && ((long long)c->nslab << (f.split + 1)) <= (long long)sms * c->flow_nw) f.split++;
+      }
       CK(cudaMemsetAsync(c->flow_done, 0, sizeof(unsigned) * c->nslab, s));
       CK(pack_flow_records(c->nslab, c->slab_off, c->slab_nslot, c->W32, c->col, c->q32, c->D32, c->mu32, c->rho32,
                            c->flow_rec_off, c->flow_rec, s));

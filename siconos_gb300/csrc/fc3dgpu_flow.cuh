@@ -18,24 +18,36 @@
 // (fc3d_nsgs.c:711-875 visiting the contacts colour by colour): every row
 // reads the reactions a sequential sweep would read.
 //
-// Each slab carries an arrival counter that every neighbour increments
-// after each of its updates.  A neighbour of an earlier colour cannot
-// update sweep k + 1 before s has updated sweep k, and one of a later colour
-// cannot update sweep k before s has, so while s waits for sweep k its
-// counter never exceeds  n * k - n_later  (n neighbours, n_later of them of
-// a later colour) and reaches it exactly when all of them are done: one
-// acquire load of the slab's own counter replaces a load per neighbour.
-// The (sweep, colour)
-// order of the waits is acyclic and every warp is resident (cooperative
-// launch), so the earliest unfinished slab can always proceed.  The light
-// error of a sweep (fc3d_nsgs.c:80-96) and the stop rules still need one
-// grid barrier per sweep.
+// How a warp knows: where W's block pattern is symmetric (every Delassus
+// operator), each reaction carries the sweep that wrote it in its fourth word
+// and the row product's loads are repeated until every stamp is the one the
+// sweep needs.  A neighbour of an earlier colour cannot write sweep k + 1
+// before s has written sweep k, and one of a later colour cannot write sweep
+// k before s has, so the value found is exactly the sequential sweep's.  There
+// is no fence, no counter and no extra round trip: a neighbour's store is seen
+// by the load that needs it, contact by contact.  Contacts depend on contacts
+// and not slabs on slabs, so a slab's rows may be spread over several warps
+// (1 << split), as far as the warps reach: fewer rows a warp mean a shorter
+// gather and a smaller largest local solve.  FP32 sweep with stamps, and with
+// counters before: 22.2 and 34.8 us at 11,600 contacts, 29.8 and 36.7 at
+// 96,780, 45.0 and 55.1 at 320,400, 92 and 124 at 761,600.
+//
+// Otherwise each slab carries an arrival counter that every neighbour
+// increments (after a fence) after each of its updates; by the same argument
+// while s waits for sweep k its counter never exceeds  n * k - n_later  (n
+// neighbours, n_later of them of a later colour) and reaches it exactly when
+// all of them are done: one acquire load of the slab's own counter.
+//
+// The (sweep, colour) order of the waits is acyclic and every warp is
+// resident (cooperative launch), so the earliest unfinished slab can always
+// proceed.  The light error of a sweep (fc3d_nsgs.c:80-96) and the stop rules
+// still need one grid barrier per sweep.
 //
 // While a warp waits for a slab's columns, the bulk-copy engine brings that
 // slab's W, column indices, q, diagonal block, mu and rho (one record per
 // slab, packed before the sweeps) into the warp's shared-memory buffer; the
 // next slab's copy is issued as soon as the current one's inputs are in
-// registers.
+// registers.  A warp with one slab keeps its record there.
 #pragma once
 #include "fc3dgpu_sweep.cuh"
 
@@ -193,6 +205,37 @@ __device__ __forceinline__ void flow_signal(const FlowArgs& f, int d0, int d1, i
   for (int i = i0 + 64; i < d1; i += 32) atomicAdd(&f.done[__ldg(&f.dep[i]) & 0x7fffffff], 1u);
 }
 
+// Stamped reactions: the fourth word of a reaction holds the sweep that wrote
+// it, and the 16 bytes are stored and loaded by single 128-bit accesses, which
+// are single-copy atomic, so a reaction and its stamp always belong together
+// and no fence or counter is needed.
+__device__ __forceinline__ void st_stamped(float* r, int p, const float x[3], int stamp) {
+  const unsigned long long lo = (unsigned long long)__float_as_uint(x[0]) | ((unsigned long long)__float_as_uint(x[1]) << 32);
+  const unsigned long long hi = (unsigned long long)__float_as_uint(x[2]) | ((unsigned long long)(unsigned)stamp << 32);
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(
+                   r + (size_t)p * FC3D_RSTRIDE),
+               "l"(lo), "l"(hi)
+               : "memory");
+}
+
+struct Stamped {
+  float x[3];
+  int stamp;
+};
+__device__ __forceinline__ Stamped ld_stamped(const float* r, int p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(r + (size_t)p * FC3D_RSTRIDE)
+               : "memory");
+  Stamped v;
+  v.x[0] = __uint_as_float((unsigned)lo);
+  v.x[1] = __uint_as_float((unsigned)(lo >> 32));
+  v.x[2] = __uint_as_float((unsigned)hi);
+  v.stamp = (int)(hi >> 32);
+  return v;
+}
+
 // Row product, take-off test and local solve of the 32 rows of slab s from
 // the warp's buffer; issues the copy of slab `next` (or none when next < 0)
 // once the buffer is read.
@@ -209,10 +252,14 @@ struct FlowRow {
   unsigned need_a, need_b;  // wait for sweep k: counter >= need_a * k - need_b
 };
 
-__device__ __forceinline__ FlowRow flow_static(const SweepArgs<float>& a, const FlowArgs& f, int s, int lane) {
+// rl: the lane's row of the slab, or beyond it for a lane without one.
+template <bool STAMP>
+__device__ __forceinline__ FlowRow flow_static(const SweepArgs<float>& a, const FlowArgs& f, int s, int rl, int lane) {
   FlowRow x;
-  x.row = __ldg(&a.perm[s * FC3D_SLAB + lane]) >= 0;
+  x.row = rl < FC3D_SLAB && __ldg(&a.perm[s * FC3D_SLAB + rl]) >= 0;
   x.ns = __ldg(&a.slab_nslot[s]);
+  x.ro[0] = x.ro[1] = x.ro[2] = 0.f;
+  if (STAMP) return x;
   x.d0 = __ldg(&f.dptr[s]);
   x.d1 = __ldg(&f.dptr[s + 1]);
   x.dep0 = x.d0 + lane < x.d1 ? __ldg(&f.dep[x.d0 + lane]) : 0;
@@ -220,7 +267,6 @@ __device__ __forceinline__ FlowRow flow_static(const SweepArgs<float>& a, const 
   const int2 nd = __ldg(&f.need[s]);
   x.need_a = (unsigned)nd.x;
   x.need_b = (unsigned)nd.y;
-  x.ro[0] = x.ro[1] = x.ro[2] = 0.f;
   return x;
 }
 
@@ -230,9 +276,15 @@ __device__ __forceinline__ void flow_own_r(const SweepArgs<float>& a, int s, int
 
 // The new reaction of the lane's row goes to rn (zero on take-off); the
 // light-error sums are left to the caller, after the slab's release.
-__device__ __forceinline__ void flow_slab(const SweepArgs<float>& a, const FlowArgs& f, int s, const FlowNext& next,
-                                          unsigned char* buf, unsigned long long* bar, int lane, float ltol,
-                                          float rn[3], unsigned long long* tl, const FlowRow& x) {
+// STAMP: the columns' reactions are loaded until their stamps are those
+// sweep `sweep` needs (this sweep's of an earlier colour, a smaller row; the
+// last one's of a later colour); false when the poll limit ran out.  refill
+// is false when the buffer already holds the next slab (the same one).
+template <bool STAMP>
+__device__ __forceinline__ bool flow_slab(const SweepArgs<float>& a, const FlowArgs& f, int s, const FlowNext& next,
+                                          unsigned char* buf, unsigned long long* bar, int rl, int lane, float ltol,
+                                          float rn[3], unsigned long long* tl, const FlowRow& x, int sweep,
+                                          bool refill) {
   const int ns = x.ns;
   const float* Ws = reinterpret_cast<const float*>(buf);
   const int* Cs = reinterpret_cast<const int*>(buf + (size_t)ns * 9 * FC3D_SLAB * 4);
@@ -240,27 +292,63 @@ __device__ __forceinline__ void flow_slab(const SweepArgs<float>& a, const FlowA
   const float* Ds = Qs + 3 * FC3D_SLAB;
   const float* Ms = Ds + 9 * FC3D_SLAB;
   const float* Rs = Ms + FC3D_SLAB;
-  const int p = s * FC3D_SLAB + lane;
+  const int p = s * FC3D_SLAB + rl;
   const float ro[3] = {x.ro[0], x.ro[1], x.ro[2]};
   float acc[3] = {0.f, 0.f, 0.f};
-  bool work = false;
+  bool work = false, ok = true;
   LocalProblem<float> L;
   if (x.row) {
-    acc[0] = Qs[lane];
-    acc[1] = Qs[FC3D_SLAB + lane];
-    acc[2] = Qs[2 * FC3D_SLAB + lane];
-    constexpr int CH = 16;
+    acc[0] = Qs[rl];
+    acc[1] = Qs[FC3D_SLAB + rl];
+    acc[2] = Qs[2 * FC3D_SLAB + rl];
+    // slots gathered together: 10 cover a sphere lattice's rows in one round
+    // trip and leave 10 warps without spills (16: 54 us a sweep for 45 on the
+    // 60x60x30 lattice)
+    constexpr int CH = 10;
     for (int t0 = 0; t0 < ns; t0 += CH) {
       float rv[CH][3];
+      if (STAMP) {
+        int pj[CH], need[CH];
+        unsigned late = 0;  // columns not there yet
 #pragma unroll
-      for (int k = 0; k < CH; k++) {
-        const int pj = t0 + k < ns ? Cs[(t0 + k) * FC3D_SLAB + lane] : a.npad;
-        load_r3<float>(a.r, pj, rv[k]);
+        for (int k = 0; k < CH; k++) {
+          pj[k] = t0 + k < ns ? Cs[(t0 + k) * FC3D_SLAB + rl] : a.npad;
+          need[k] = sweep - (pj[k] > p ? 1 : 0);
+          const Stamped v = ld_stamped(a.r, pj[k]);
+          rv[k][0] = v.x[0];
+          rv[k][1] = v.x[1];
+          rv[k][2] = v.x[2];
+          late |= (v.stamp < need[k] ? 1u : 0u) << k;
+        }
+        unsigned long long n = 0;
+        while (late) {
+          if (++n > a.spin_limit) {
+            atomicOr(a.status, 1);
+            ok = false;
+            break;
+          }
+          if (n > FC3D_FLOW_SPIN) __nanosleep(FC3D_FLOW_SLEEP_NS);
+#pragma unroll
+          for (int k = 0; k < CH; k++)
+            if (late >> k & 1u) {
+              const Stamped v = ld_stamped(a.r, pj[k]);
+              rv[k][0] = v.x[0];
+              rv[k][1] = v.x[1];
+              rv[k][2] = v.x[2];
+              if (v.stamp >= need[k]) late &= ~(1u << k);
+            }
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+          const int pj = t0 + k < ns ? Cs[(t0 + k) * FC3D_SLAB + rl] : a.npad;
+          load_r3<float>(a.r, pj, rv[k]);
+        }
       }
 #pragma unroll
       for (int k = 0; k < CH; k++) {
         if (t0 + k < ns) {
-          const float* wp = Ws + (size_t)(t0 + k) * 9 * FC3D_SLAB + lane;
+          const float* wp = Ws + (size_t)(t0 + k) * 9 * FC3D_SLAB + rl;
           float wv[9];
 #pragma unroll
           for (int e = 0; e < 9; e++) wv[e] = wp[e * FC3D_SLAB];
@@ -268,18 +356,24 @@ __device__ __forceinline__ void flow_slab(const SweepArgs<float>& a, const FlowA
         }
       }
     }
-    if (acc[0] > -Eps<float>::v()) {
-      float* rp = a.r + (size_t)p * FC3D_RSTRIDE;
-      rp[0] = 0;
-      rp[1] = 0;
-      rp[2] = 0;
+    if (!ok) {
+    } else if (acc[0] > -Eps<float>::v()) {
+      if (STAMP) {
+        const float zero[3] = {0.f, 0.f, 0.f};
+        st_stamped(a.r, p, zero, sweep);
+      } else {
+        float* rp = a.r + (size_t)p * FC3D_RSTRIDE;
+        rp[0] = 0;
+        rp[1] = 0;
+        rp[2] = 0;
+      }
     } else {
       work = true;
 #pragma unroll
-      for (int e = 0; e < 9; e++) L.M[e] = Ds[e * FC3D_SLAB + lane];
-      L.mu = Ms[lane];
-      L.rhoN = Rs[lane];
-      L.rhoT = Rs[FC3D_SLAB + lane];
+      for (int e = 0; e < 9; e++) L.M[e] = Ds[e * FC3D_SLAB + rl];
+      L.mu = Ms[rl];
+      L.rhoN = Rs[rl];
+      L.rhoT = Rs[FC3D_SLAB + rl];
       L.q[0] = acc[0];
       L.q[1] = acc[1];
       L.q[2] = acc[2];
@@ -290,7 +384,8 @@ __device__ __forceinline__ void flow_slab(const SweepArgs<float>& a, const FlowA
     tl[3] = globaltimer_ns();
     tl[5] = (unsigned long long)__popc(wmask);
   }
-  if (lane == 0) {
+  if (STAMP && !__all_sync(0xffffffffu, ok)) return false;
+  if (lane == 0 && refill) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     flow_issue(f, next, buf, bar);
   }
@@ -307,18 +402,31 @@ __device__ __forceinline__ void flow_slab(const SweepArgs<float>& a, const FlowA
     rn[0] = ro[0];
     rn[1] = ro[1];
     rn[2] = ro[2];
-    local_solve(L, rn);
-    float* rp = a.r + (size_t)p * FC3D_RSTRIDE;
-    rp[0] = rn[0];
-    rp[1] = rn[1];
-    rp[2] = rn[2];
+    if (STAMP) {
+      // a contact is released as soon as it is solved, not when the slowest
+      // of its warp is
+      LocalState<float> S;
+      const bool done = local_solve_newton(L, rn, S);
+      if (done) st_stamped(a.r, p, rn, sweep);
+      if (!done) {
+        local_solve_rest(L, rn, S);
+        st_stamped(a.r, p, rn, sweep);
+      }
+    } else {
+      local_solve(L, rn);
+      float* rp = a.r + (size_t)p * FC3D_RSTRIDE;
+      rp[0] = rn[0];
+      rp[1] = rn[1];
+      rp[2] = rn[2];
+    }
     a.rpli[p] = L.rho_pli;
   }
   __syncwarp();
   if (tl) tl[7] = globaltimer_ns();
+  return true;
 }
 
-template <int NW>
+template <int NW, bool STAMP>
 __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<float> a, const FlowArgs f) {
   extern __shared__ __align__(128) unsigned char flow_smem[];
   __shared__ __align__(8) unsigned long long bars[NW];
@@ -331,13 +439,19 @@ __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<f
   }
   __syncwarp();
   const int gw = blockIdx.x * NW + w, tw = gridDim.x * NW;
+  // a warp takes whole slabs, or with stamps a part of one (32 >> split rows)
+  const int sh = STAMP ? f.split : 0, units = a.nslab << sh;
+  auto row_of = [&](int u) {
+    if (!STAMP) return lane;
+    return lane < (FC3D_SLAB >> sh) ? (u & ((1 << sh) - 1)) * (FC3D_SLAB >> sh) + lane : FC3D_SLAB;
+  };
   unsigned parity = 0;
   bool pending = false, failed = false;
   FlowRow xs;  // the static inputs of the warp's next slab
-  if (gw < a.nslab) {
-    if (lane == 0) flow_issue(f, flow_next(a, f, gw), buf, bar);
+  if (gw < units) {
+    if (lane == 0) flow_issue(f, flow_next(a, f, gw >> sh), buf, bar);
     pending = true;
-    xs = flow_static(a, f, gw, lane);
+    xs = flow_static<STAMP>(a, f, gw >> sh, row_of(gw), lane);
   }
   // Light errors run one sweep behind: at the end of sweep j a block
   // publishes its partial sums of sweep j (slot j mod 4 of f.part) and its
@@ -383,17 +497,18 @@ __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<f
     sweep++;
     double acc[2] = {0.0, 0.0};
     const bool record = a.timeline && sweep == a.timeline_sweep && lane == 0;
-    for (int s = gw; s < a.nslab && !failed; s += tw) {
+    for (int u = gw; u < units && !failed; u += tw) {
+      const int s = u >> sh, rl = row_of(u);
       unsigned long long* tl = record ? a.timeline + (size_t)s * FC3D_TL_STRIDE : nullptr;
       if (tl) tl[0] = globaltimer_ns();
       // the next slab of this warp: later in this sweep, else the first one
       // of the next sweep (fetched even when no sweep follows; awaited at exit)
-      const int sn = s + tw < a.nslab ? s + tw : gw;
-      const FlowNext next = flow_next(a, f, sn);
+      const int un = u + tw < units ? u + tw : gw;
+      const FlowNext next = flow_next(a, f, un >> sh);
       FlowRow x = xs;
-      xs = flow_static(a, f, sn, lane);
-      flow_own_r(a, s, lane, x);
-      if (!flow_wait_deps(a, f, s, x.need_a * (unsigned)sweep - x.need_b, lane)) {
+      xs = flow_static<STAMP>(a, f, un >> sh, row_of(un), lane);
+      flow_own_r(a, s, rl, x);
+      if (!STAMP && !flow_wait_deps(a, f, s, x.need_a * (unsigned)sweep - x.need_b, lane)) {
         failed = true;
         break;
       }
@@ -409,8 +524,13 @@ __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<f
       }
       if (tl) tl[2] = globaltimer_ns();
       float rn[3];
-      flow_slab(a, f, s, next, buf, bar, lane, (float)a.local_tol, rn, tl, x);
-      pending = true;
+      // a warp with one slab keeps its record in the buffer
+      const bool refill = !STAMP || un != u;
+      if (!flow_slab<STAMP>(a, f, s, next, buf, bar, rl, lane, (float)a.local_tol, rn, tl, x, sweep, refill)) {
+        failed = true;
+        break;
+      }
+      pending = refill;
       if (x.row) {
         // light-error sums (fc3d_nsgs.c:80-96), while the reaction stores
         // drain: squares in FP32, sums in FP64 (the FP64 pipe is a small
@@ -421,7 +541,7 @@ __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<f
       }
       __syncwarp();
       if (tl) tl[4] = globaltimer_ns();
-      flow_signal(f, x.d0, x.d1, x.dep0, x.dep1, lane);
+      if (!STAMP) flow_signal(f, x.d0, x.d1, x.dep0, x.dep1, lane);
     }
     flow_block_sum<2, NW>(acc, f.part + blockIdx.x * 8 + (sweep & 3) * 2);
     e_prev = e_last;
@@ -486,6 +606,26 @@ __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<f
     a.out[3] = converged ? 0 : 1;
     a.out[4] = working;
     a.out[5] = a.local_tol;
+  }
+}
+
+// Sets *missing when some row reads a column whose row does not read it back
+// (a block pattern that is not symmetric).
+__global__ void k_flow_symmetric(int npad, const int* __restrict__ perm, const int* __restrict__ slab_nslot,
+                                 const long long* __restrict__ slab_off, const int* __restrict__ col,
+                                 int* __restrict__ missing) {
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npad; p += gridDim.x * blockDim.x) {
+    if (perm[p] < 0) continue;
+    const int s = p / FC3D_SLAB, k = p % FC3D_SLAB;
+    for (int t = 0; t < slab_nslot[s]; t++) {
+      const int j = col[(size_t)(slab_off[s] + t) * FC3D_SLAB + k];
+      if (j < 0 || j >= npad) continue;
+      const int d = j / FC3D_SLAB, l = j % FC3D_SLAB;
+      bool back = false;
+      for (int u = 0; u < slab_nslot[d] && !back; u++)
+        back = col[(size_t)(slab_off[d] + u) * FC3D_SLAB + l] == p;
+      if (!back) *missing = 1;
+    }
   }
 }
 

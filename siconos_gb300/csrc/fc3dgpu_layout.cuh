@@ -134,6 +134,8 @@ struct FlowArgs {
   int maxslot;         // slots of one slab the buffer holds
   const float* rec;          // per slab one record of its sweep inputs (flow_rec_floats)
   const long long* rec_off;  // float offset of slab s's record in rec
+  int stamped;         // wait on the reactions' stamps instead of the counters
+  int split;           // with stamps: a slab's rows are spread over 1 << split warps (0 to 5)
 };
 
 // Per-slab record of the FP32 inputs of a slab with ns slots, back to back:

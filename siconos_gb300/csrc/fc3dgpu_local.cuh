@@ -418,16 +418,26 @@ __device__ __forceinline__ void keep_or_discard(LocalProblem<Real>& L, Real r[3]
   }
 }
 
-// fc3d_onecontact_nonsmooth_Newton_solvers_solve (onecontact.c:221-290) with
-// the hybrid strategy; r holds the contact's current reaction on entry.
+// What the second part of a local solve takes over from the first: the best
+// reaction so far and its natural-map error.
 template <typename Real>
-__device__ __forceinline__ void local_solve(LocalProblem<Real>& L, Real r[3]) {
+struct LocalState {
+  Real rb[3];
+  Real cur;
+};
+
+// fc3d_onecontact_nonsmooth_Newton_solvers_solve (onecontact.c:221-290) with
+// the hybrid strategy; r holds the contact's current reaction on entry.  In
+// two parts, so that the contacts the first one finishes (it returns true)
+// can be stored while the others of the warp go on.
+template <typename Real>
+__device__ __forceinline__ bool local_solve_newton(LocalProblem<Real>& L, Real r[3], LocalState<Real>& S) {
   if (L.q[0] > -Eps<Real>::v()) {
     r[0] = 0;
     r[1] = 0;
     r[2] = 0;
     L.residual = 0;
-    return;
+    return true;
   }
   if (L.mode == 1) {
     // accelerator mode of the FP32 sweeps: the damped Newton alone, from
@@ -441,25 +451,33 @@ __device__ __forceinline__ void local_solve(LocalProblem<Real>& L, Real r[3]) {
       r[1] = r0[1];
       r[2] = r0[2];
     }
-    return;
+    return true;
   }
-  Real rb[3] = {r[0], r[1], r[2]};
-  Real cur = local_error(L, r);
+  S.rb[0] = r[0];
+  S.rb[1] = r[1];
+  S.rb[2] = r[2];
+  S.cur = local_error(L, r);
   newton_damped(L, r);
-  keep_or_discard(L, r, rb, cur);
-  if (cur <= L.tol) {
-    L.residual = cur;
-    return;
+  keep_or_discard(L, r, S.rb, S.cur);
+  L.residual = S.cur;
+  return S.cur <= L.tol || !(S.cur >= L.tol);
+}
+
+template <typename Real>
+__device__ __forceinline__ void local_solve_rest(LocalProblem<Real>& L, Real r[3], LocalState<Real>& S) {
+  pli_solve(L, r);
+  keep_or_discard(L, r, S.rb, S.cur);
+  if (!(S.cur < L.tol)) {
+    newton_damped(L, r);
+    keep_or_discard(L, r, S.rb, S.cur);
   }
-  if (cur >= L.tol) {
-    pli_solve(L, r);
-    keep_or_discard(L, r, rb, cur);
-    if (!(cur < L.tol)) {
-      newton_damped(L, r);
-      keep_or_discard(L, r, rb, cur);
-    }
-  }
-  L.residual = cur;
+  L.residual = S.cur;
+}
+
+template <typename Real>
+__device__ __forceinline__ void local_solve(LocalProblem<Real>& L, Real r[3]) {
+  LocalState<Real> S;
+  if (!local_solve_newton(L, r, S)) local_solve_rest(L, r, S);
 }
 
 // rho from the diagonal block, split spectral norm strategy

@@ -51,15 +51,21 @@ cudaError_t launch_sweep_f32(const SweepArgs<float>& a, int lanes, int max_grid,
   }
 }
 
+template <int NW>
+static void warm_flow_t(cudaFuncAttributes* fa) {
+  cudaFuncGetAttributes(fa, nsgs_flow_kernel<NW, false>);
+  cudaFuncGetAttributes(fa, nsgs_flow_kernel<NW, true>);
+}
+
 void warm_sweep_kernels() {
   cudaFuncAttributes fa;
   cudaFuncGetAttributes(&fa, nsgs_kernel<float, 1>);
   cudaFuncGetAttributes(&fa, nsgs_kernel<float, 2>);
   cudaFuncGetAttributes(&fa, nsgs_kernel<float, 4>);
   cudaFuncGetAttributes(&fa, nsgs_kernel<float, 8>);
-  cudaFuncGetAttributes(&fa, nsgs_flow_kernel<12>);
-  cudaFuncGetAttributes(&fa, nsgs_flow_kernel<10>);
-  cudaFuncGetAttributes(&fa, nsgs_flow_kernel<8>);
+  warm_flow_t<12>(&fa);
+  warm_flow_t<10>(&fa);
+  warm_flow_t<8>(&fa);
   warm_sweep_kernels_f64();
 }
 
@@ -91,9 +97,9 @@ int flow_warps(int maxslot, int want) {
   return 0;
 }
 
-template <int NW>
+template <int NW, bool STAMP>
 static cudaError_t launch_flow_t(const SweepArgs<float>& a, const FlowArgs& f, cudaStream_t s, int* grid) {
-  auto kern = nsgs_flow_kernel<NW>;
+  auto kern = nsgs_flow_kernel<NW, STAMP>;
   const size_t smem = (size_t)NW * f.buf_bytes;
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -112,11 +118,16 @@ static cudaError_t launch_flow_t(const SweepArgs<float>& a, const FlowArgs& f, c
   return cudaLaunchCooperativeKernel((const void*)kern, dim3(g), dim3(NW * 32), args, smem, s);
 }
 
+template <int NW>
+static cudaError_t launch_flow_n(const SweepArgs<float>& a, const FlowArgs& f, cudaStream_t s, int* grid) {
+  return f.stamped ? launch_flow_t<NW, true>(a, f, s, grid) : launch_flow_t<NW, false>(a, f, s, grid);
+}
+
 cudaError_t launch_flow_f32(const SweepArgs<float>& a, const FlowArgs& f, int nw, cudaStream_t s, int* grid) {
   switch (nw) {
-    case 12: return launch_flow_t<12>(a, f, s, grid);
-    case 10: return launch_flow_t<10>(a, f, s, grid);
-    case 8: return launch_flow_t<8>(a, f, s, grid);
+    case 12: return launch_flow_n<12>(a, f, s, grid);
+    case 10: return launch_flow_n<10>(a, f, s, grid);
+    case 8: return launch_flow_n<8>(a, f, s, grid);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -127,6 +138,14 @@ cudaError_t pack_flow_records(int nslab, const long long* slab_off, const int* s
   if (nslab <= 0) return cudaSuccess;
   const int grid = nslab < 4096 ? nslab : 4096;
   k_flow_pack<<<grid, 256, 0, s>>>(nslab, slab_off, slab_nslot, W, col, q, D, mu, rho, rec_off, rec);
+  return cudaGetLastError();
+}
+
+cudaError_t check_flow_symmetric(int npad, const int* perm, const int* slab_nslot, const long long* slab_off,
+                                 const int* col, int* missing, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(missing, 0, sizeof(int), s);
+  if (e != cudaSuccess || npad <= 0) return e;
+  k_flow_symmetric<<<(npad + 255) / 256, 256, 0, s>>>(npad, perm, slab_nslot, slab_off, col, missing);
   return cudaGetLastError();
 }
 

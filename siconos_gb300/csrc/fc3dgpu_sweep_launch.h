@@ -38,6 +38,9 @@ cudaError_t launch_flow_f32(const SweepArgs<float>& a, const FlowArgs& f, int nw
 cudaError_t pack_flow_records(int nslab, const long long* slab_off, const int* slab_nslot, const float* W,
                               const int* col, const float* q, const float* D, const float* mu, const float* rho,
                               const long long* rec_off, float* rec, cudaStream_t s);
+// *missing (device) = 1 when the block pattern is not symmetric.
+cudaError_t check_flow_symmetric(int npad, const int* perm, const int* slab_nslot, const long long* slab_off,
+                                 const int* col, int* missing, cudaStream_t s);
 cudaError_t build_flow_deps(int nslab, int npad, int ncol, const int* sptr_d, const int* perm, const int* slab_nslot,
                             const long long* slab_off, const int* col, const int* dptr, int* count, int* dep,
                             cudaStream_t s);
