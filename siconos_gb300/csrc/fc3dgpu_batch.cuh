@@ -229,6 +229,7 @@ __device__ __forceinline__ bool solve_scene(const BatchArgs<Real>& b, int scene,
     o[4] = working;
     o[5] = local_tol;
   }
+  return true;
 }
 
 template <typename Real>
