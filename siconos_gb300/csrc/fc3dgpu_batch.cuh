@@ -119,10 +119,29 @@ __device__ __forceinline__ bool scene_full_error(const BatchArgs<Real>& b, int p
   return true;
 }
 
-// All sweeps of one problem; false when a wait of the team gave up.
+// How a block sweeps a problem's colours.  ColourSweep: colour by colour, the
+// team's barrier between them (the sums' barrier closes the last one).
 template <typename Real>
-__device__ __forceinline__ bool solve_scene(const BatchArgs<Real>& b, int scene, typename RangeList<Real>::type& wk,
-                                            BatchTeam& t, TeamSum& S) {
+struct ColourSweep {
+  typename RangeList<Real>::type& wk;
+  __device__ __forceinline__ void open(const BatchArgs<Real>&, const int*, int, const BatchTeam&) {}
+  __device__ __forceinline__ bool sweep(const BatchArgs<Real>& b, const int* sptr, int ncol, int, Real local_tol,
+                                        double acc[3], BatchTeam& t) {
+    const SweepArgs<Real>& a = b.base;
+    for (int c = 0; c < ncol; c++) {
+      const int s0 = sptr[c], n = sptr[c + 1] - s0;
+      process_range<Real>(a, s0 + n * t.rank / t.size, s0 + n * (t.rank + 1) / t.size, local_tol, acc[0], acc[1], wk,
+                          nullptr);
+      if (c + 1 < ncol && !team_sync(t, a.barrier, a.spin_limit, a.status)) return false;
+    }
+    return true;
+  }
+  __device__ __forceinline__ void close(const BatchArgs<Real>&) {}
+};
+
+// All sweeps of one problem; false when a wait of the team gave up.
+template <typename Real, typename Sweep>
+__device__ __forceinline__ bool solve_scene(const BatchArgs<Real>& b, int scene, Sweep& sw, BatchTeam& t, TeamSum& S) {
   const SweepArgs<Real>& a = b.base;
   const int ncol = b.scene_ncol[scene];
   const int* sptr = b.scene_sptr + (size_t)scene * (FC3D_MAX_COLOURS + 1);
@@ -149,16 +168,11 @@ __device__ __forceinline__ bool solve_scene(const BatchArgs<Real>& b, int scene,
       return true;
     }
   }
+  if (max_sweeps > 0) sw.open(b, sptr, ncol, t);
   while (sweep < max_sweeps) {
     sweep++;
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int c = 0; c < ncol; c++) {
-      const int s0 = sptr[c], n = sptr[c + 1] - s0;
-      process_range<Real>(a, s0 + n * t.rank / t.size, s0 + n * (t.rank + 1) / t.size, (Real)local_tol, acc[0],
-                          acc[1], wk, nullptr);
-      // the barrier of the sums closes the last colour
-      if (c + 1 < ncol && !team_sync(t, a.barrier, a.spin_limit, a.status)) return false;
-    }
+    if (!sw.sweep(b, sptr, ncol, sweep, (Real)local_tol, acc, t)) return false;
     double s[3];
     if (!team_reduce3(b, t, S, acc, s)) return false;
     incr = sqrt(s[0]);
@@ -212,6 +226,7 @@ __device__ __forceinline__ bool solve_scene(const BatchArgs<Real>& b, int scene,
     }
     if (stop) break;
   }
+  sw.close(b);
   int info = 1;
   if (a.mode == 1) {
     if (!scene_full_error(b, p0, p1, norm_q, t, S, full)) return false;
@@ -232,9 +247,9 @@ __device__ __forceinline__ bool solve_scene(const BatchArgs<Real>& b, int scene,
   return true;
 }
 
-template <typename Real>
-__global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_batch_kernel(const BatchArgs<Real> b) {
-  __shared__ typename RangeList<Real>::type wk;
+// The block's problems: its team's, then the queue's.
+template <typename Real, typename Sweep>
+__device__ __forceinline__ void batch_problems(const BatchArgs<Real>& b, Sweep& sw) {
   __shared__ TeamSum S;
   __shared__ int s_next;
   BatchTeam t = {(int)blockIdx.x, 1, 0, 0};
@@ -244,7 +259,11 @@ __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_batch_kernel(co
       t.first = m.x;
       t.size = m.y;
       t.rank = (int)blockIdx.x - m.x;
-      if (!solve_scene<Real>(b, b.order[m.z], wk, t, S)) return;
+      const bool ok = solve_scene<Real>(b, b.order[m.z], sw, t, S);
+      if (!ok) {
+        sw.close(b);
+        return;
+      }
       __syncthreads();
       t.size = 1;
       t.rank = 0;
@@ -256,9 +275,19 @@ __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_batch_kernel(co
     const int k = b.team_scenes + s_next;
     __syncthreads();
     if (k >= b.nscenes) break;
-    if (!solve_scene<Real>(b, b.order[k], wk, t, S)) return;
+    if (!solve_scene<Real>(b, b.order[k], sw, t, S)) {
+      sw.close(b);
+      return;
+    }
     __syncthreads();
   }
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_batch_kernel(const BatchArgs<Real> b) {
+  __shared__ typename RangeList<Real>::type wk;
+  ColourSweep<Real> sw = {wk};
+  batch_problems<Real>(b, sw);
 }
 
 // Launch of `grid` blocks, co-resident (a cooperative launch) when some of

@@ -465,6 +465,13 @@ __global__ void k_r64_to_r32(int npad, const double* __restrict__ r64, float* __
   }
 }
 
+// The stamps alone, the reactions as they are (a batch's FP32 sweeps start
+// from them).
+__global__ void k_reset_stamps(int npad, float* __restrict__ r32) {
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= npad; p += gridDim.x * blockDim.x)
+    r32[4 * (size_t)p + 3] = __int_as_float(p < npad ? 0 : 0x7fffffff);
+}
+
 // The 17 warm-start features of every row (padding rows: zeros): the
 // diagonal block (column-major), q, mu, the current reaction, the gap of
 // the row's contact (gapo in the caller's order, or 0).
@@ -770,6 +777,7 @@ struct fc3dgpu_ctx {
   int flow_on = 1;
   int flow_state = 0;
   int flow_nw = 0, flow_maxslot = 0;
+  int batch_flow = 0;  // the batch's FP32 sweeps as dataflow: 0 not decided, 1 yes, -1 no
   bool flow_symmetric = false;  // every block has its transpose's place in W
   int flow_want = 0;  // warps per block of the dataflow sweep asked for (0: default)
   // measuring autotuner (per layout): chosen FP32 variant and FP64 lanes,
@@ -1365,6 +1373,7 @@ static int build_layout(fc3dgpu_ctx* c, int nc, long long nnzb, int kind, int ns
   c->colour_kind = kind;
   for (auto& n : c->nbrc) n.grid = 0;  // the rows' owners changed
   c->flow_state = 0;
+  c->batch_flow = 0;
   c->tuned = 0;
   return 0;
 }
@@ -1535,6 +1544,12 @@ extern "C" int fc3dgpu_ctx_flow(fc3dgpu_ctx* c, int on) {
   if (!c) return -1;
   const int old = c->flow_on;
   c->flow_on = on ? 1 : 0;
+  if (old != c->flow_on && c->batch_graph) {
+    // recorded for the other form
+    cudaGraphExecDestroy(c->batch_graph);
+    c->batch_graph = nullptr;
+  }
+  c->batch_flow = 0;
   return old;
 }
 
@@ -1755,6 +1770,49 @@ static size_t staging_sizes(fc3dgpu_ctx* c, int grid, unsigned* wb, unsigned* cb
   return tot;
 }
 
+// Whether the block pattern is symmetric (the stamped dataflow sweeps need
+// it), and the places of the slabs' records.
+static int prepare_records(fc3dgpu_ctx* c) {
+  using namespace fc3dgpu;
+  cudaStream_t s = c->stream;
+  const int nslab = c->nslab;
+  int missing = 0;
+  CK(check_flow_symmetric(c->npad, c->perm, c->slab_nslot, c->slab_off, c->col, c->scratch, s));
+  CK(cudaMemcpyAsync(&missing, c->scratch, sizeof(int), cudaMemcpyDeviceToHost, s));
+  // offsets of the per-slab records (filled before each solve's FP32 sweeps)
+  std::vector<long long> roff((size_t)nslab + 1, 0);
+  for (int t = 0; t < nslab; t++) roff[t + 1] = roff[t] + flow_rec_floats(c->slab_nslot_h[t]);
+  CK(ensure(&c->flow_rec_off, &c->flow_rec_off_cap, (size_t)nslab + 1));
+  CK(ensure(&c->flow_rec, &c->flow_rec_cap, (size_t)std::max(roff[nslab], 1LL)));
+  CK(cudaMemcpyAsync(c->flow_rec_off, roff.data(), sizeof(long long) * (nslab + 1), cudaMemcpyHostToDevice, s));
+  CK(cudaStreamSynchronize(s));
+  c->flow_symmetric = missing == 0;
+  c->launches++;
+  return 0;
+}
+
+// Decides c->batch_flow for a batch layout; *resident: blocks of its FP32
+// kernel that fit the device.
+static int prepare_batch_flow(fc3dgpu_ctx* c, int* resident) {
+  using namespace fc3dgpu;
+  int maxslot = 0, grid = 0;
+  for (int s = 0; s < c->nslab; s++) maxslot = std::max(maxslot, c->slab_nslot_h[s]);
+  CK(batch_flow_grid_f32(maxslot, &grid));
+  if (c->batch_flow == 0) {
+    c->batch_flow = -1;
+    if (c->flow_on && !c->counters_on && grid > 0) {
+      if (int rc = prepare_records(c)) return rc;
+      c->flow_maxslot = maxslot;
+      if (c->flow_symmetric) c->batch_flow = 1;
+    }
+  }
+  if (c->batch_flow == 1)
+    *resident = grid;
+  else
+    CK(batch_grid_f32(resident));
+  return 0;
+}
+
 // Column-slab lists of the dataflow sweep for the current layout; leaves
 // c->flow_state 1 when the sweep applies, -1 when not (slabs longer than
 // FC3D_FLOW_MAXSLOT or than the per-warp buffers allow).
@@ -1826,18 +1884,8 @@ static int prepare_flow(fc3dgpu_ctx* c) {
   CK(cudaMemcpyAsync(c->flow_dptr, sptr_sym.data(), sizeof(int) * (nslab + 1), cudaMemcpyHostToDevice, s));
   if (!sym.empty()) CK(cudaMemcpyAsync(c->flow_dep, sym.data(), sizeof(int) * sym.size(), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(c->flow_need, need.data(), sizeof(int2) * nslab, cudaMemcpyHostToDevice, s));
-  int missing = 0;
-  CK(check_flow_symmetric(c->npad, c->perm, c->slab_nslot, c->slab_off, c->col, c->scratch, s));
-  CK(cudaMemcpyAsync(&missing, c->scratch, sizeof(int), cudaMemcpyDeviceToHost, s));
-  // offsets of the per-slab records (filled before each solve's FP32 sweeps)
-  std::vector<long long> roff((size_t)nslab + 1, 0);
-  for (int t = 0; t < nslab; t++) roff[t + 1] = roff[t] + flow_rec_floats(c->slab_nslot_h[t]);
-  CK(ensure(&c->flow_rec_off, &c->flow_rec_off_cap, (size_t)nslab + 1));
-  CK(ensure(&c->flow_rec, &c->flow_rec_cap, (size_t)std::max(roff[nslab], 1LL)));
-  CK(cudaMemcpyAsync(c->flow_rec_off, roff.data(), sizeof(long long) * (nslab + 1), cudaMemcpyHostToDevice, s));
-  CK(cudaStreamSynchronize(s));
-  c->flow_symmetric = missing == 0;
-  c->launches += 3;
+  if (int rc = prepare_records(c)) return rc;
+  c->launches += 2;
   c->flow_nw = nw;
   c->flow_maxslot = maxslot;
   c->flow_state = 1;
@@ -2366,7 +2414,20 @@ static int record_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
     b.scene_out = c->sout32;
     b.scene_out_prev = nullptr;
     if (int rc = attach_teams(c, b, 0)) return rc;
-    CK(launch_batch_f32(b, c->batch_plans[0].grid, s));
+    if (c->batch_flow == 1) {
+      FlowArgs f = {};
+      f.maxslot = c->flow_maxslot;
+      f.buf_bytes = flow_buf_bytes(c->flow_maxslot);
+      f.rec = c->flow_rec;
+      f.rec_off = c->flow_rec_off;
+      f.stamped = 1;
+      k_reset_stamps<<<grid1d(c->npad + 1), 256, 0, s>>>(c->npad, c->r32);
+      CK(pack_flow_records(c->nslab, c->slab_off, c->slab_nslot, c->W32, c->col, c->q32, c->D32, c->mu32, c->rho32,
+                           c->flow_rec_off, c->flow_rec, s));
+      CK(launch_batch_flow_f32(b, f, c->batch_plans[0].grid, s));
+    } else {
+      CK(launch_batch_f32(b, c->batch_plans[0].grid, s));
+    }
     k_r32_to_r64<<<grid1d(c->npad), 256, 0, s>>>(c->npad, c->r32, c->rpli32, c->r64, c->rpli64);
   }
   k_batch_budget<<<grid1d(ns), 256, 0, s>>>(ns, c->sout32, p->fp32_only ? 0 : p->max_iter, c->sbudget);
@@ -2428,15 +2489,15 @@ extern "C" int fc3dgpu_ctx_solve_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p, 
       return NUMERICS_ERR_INVALID_OPTION;
     }
     int resident[3];
-    CK(batch_grid_f32(&resident[0]));
+    if (int rc = prepare_batch_flow(c, &resident[0])) return rc;
     CK(batch_grid_f64(&resident[1]));
     CK(fc3dgpu_batch_grid_f64_fast(&resident[2]));
     CK(ensure(&c->steams, &c->steams_cap, (size_t)3 * FC3D_BATCH_BLOCKS));
     CK(ensure(&c->steam_part, &c->steam_part_cap, (size_t)2 * FC3D_BATCH_BLOCKS * 4));
     for (int k = 0; k < 3; k++) {
-      // an FP32 block takes a slab per warp and round; an FP64 colour's time
-      // goes with its slabs
-      c->batch_plans[k] = batch_plan(c->scene_slabs_h, resident[k], k == 0 ? FC3D_BATCH_WARPS32 : 1);
+      // by colours an FP32 block takes a slab per warp and round; an FP64
+      // colour's and a dataflow sweep's time goes with the block's slabs
+      c->batch_plans[k] = batch_plan(c->scene_slabs_h, resident[k], k == 0 && c->batch_flow != 1 ? FC3D_BATCH_WARPS32 : 1);
       const std::vector<int4>& t = c->batch_plans[k].teams;
       if (!t.empty())
         CK(cudaMemcpyAsync(c->steams + (size_t)k * FC3D_BATCH_BLOCKS, t.data(), sizeof(int4) * t.size(),

@@ -1,5 +1,5 @@
 // float instantiations of the persistent coloured NSGS kernel.
-#include "fc3dgpu_batch.cuh"
+#include "fc3dgpu_batch_flow.cuh"
 #include "fc3dgpu_flow.cuh"
 #include "fc3dgpu_sweep.cuh"
 #include "fc3dgpu_sweep_launch.h"
@@ -162,6 +162,38 @@ cudaError_t build_flow_deps(int nslab, int npad, int ncol, const int* sptr_d, co
 cudaError_t batch_grid_f32(int* grid) { return batch_grid_t<float>(grid); }
 
 cudaError_t launch_batch_f32(const BatchArgs<float>& b, int grid, cudaStream_t s) { return launch_batch_t(b, grid, s); }
+
+// Resident blocks of the dataflow form with per-warp buffers for slabs of up
+// to maxslot slots; 0 when they do not fit.
+cudaError_t batch_flow_grid_f32(int maxslot, int* grid) {
+  int dev = 0, nsm = 0, per_sm = 0;
+  *grid = 0;
+  if (maxslot > FC3D_FLOW_MAXSLOT || flow_warps(maxslot, FC3D_BATCH_WARPS32) != FC3D_BATCH_WARPS32) return cudaSuccess;
+  const int smem = (int)(FC3D_BATCH_WARPS32 * flow_buf_bytes(maxslot));
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(nsgs_batch_flow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nsgs_batch_flow_kernel, FC3D_BATCH_WARPS32 * 32, smem);
+  if (e == cudaSuccess) *grid = nsm * per_sm < FC3D_BATCH_BLOCKS ? nsm * per_sm : FC3D_BATCH_BLOCKS;
+  return e;
+}
+
+cudaError_t launch_batch_flow_f32(const BatchArgs<float>& b, const FlowArgs& f, int grid, cudaStream_t s) {
+  if (grid < 1 || grid > FC3D_BATCH_BLOCKS) return cudaErrorInvalidConfiguration;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(FC3D_BATCH_WARPS32 * 32);
+  cfg.dynamicSmemBytes = (size_t)FC3D_BATCH_WARPS32 * f.buf_bytes;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = b.teams ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, nsgs_batch_flow_kernel, b, f);
+}
 
 void warm_batch_kernel_f32() {
   cudaFuncAttributes fa;

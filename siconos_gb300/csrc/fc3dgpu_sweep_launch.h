@@ -23,6 +23,8 @@ struct BatchArgs;
 // stream capture), and the launch of `grid` of them.
 cudaError_t batch_grid_f32(int* grid);
 cudaError_t batch_grid_f64(int* grid);
+cudaError_t batch_flow_grid_f32(int maxslot, int* grid);
+cudaError_t launch_batch_flow_f32(const BatchArgs<float>& b, const FlowArgs& f, int grid, cudaStream_t s);
 cudaError_t launch_batch_f32(const BatchArgs<float>& b, int grid, cudaStream_t s);
 cudaError_t launch_batch_f64(const BatchArgs<double>& b, int grid, cudaStream_t s);
 void warm_batch_kernel_f32();

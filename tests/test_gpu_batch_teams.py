@@ -9,14 +9,18 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dims", [[(20, 19, 9), (3, 3, 2), (12, 11, 6)], [(2, 2, 1), (25, 24, 12)]],
                          ids=["three", "tiny-and-large"])
-@pytest.mark.parametrize("precision", [0, 1], ids=["fp32", "fp64"])
-def test_team_equals_solo_bitwise(gpu, dims, precision):
+@pytest.mark.parametrize("precision,flow", [(0, True), (0, False), (1, True)], ids=["fp32", "fp32-colours", "fp64"])
+def test_team_equals_solo_bitwise(gpu, dims, precision, flow):
     from siconos_gb300 import scene
     from siconos_gb300.device import DeviceSolver
     scs = [scene.lattice(*d, seed=50 + k, mu=0.3 + 0.2 * k) for k, d in enumerate(dims)]
     kw = dict(tol=1e-300, max_iter=12, precision=precision, fp32_only=1 - precision)
-    gpu.load_batch(scs)
-    st = gpu.solve_batch(**kw)
+    gpu.flow(flow)  # the FP32 sweeps as dataflow, or colour by colour
+    try:
+        gpu.load_batch(scs)
+        st = gpu.solve_batch(**kw)
+    finally:
+        gpu.flow(True)
     rb, ub = gpu.get_batch()
     solo = DeviceSolver(0)
     solo.flow(False)  # the coloured FP32 kernel, whose stop rules the batch has (the dataflow stops a sweep later)
