@@ -263,12 +263,15 @@ int fc3dgpu_ctx_staging(fc3dgpu_ctx *ctx, int on);
  * with its own, 0 a grid-wide barrier after every colour.  Both give the same
  * iterates.  Returns the previous setting. */
 int fc3dgpu_ctx_sync(fc3dgpu_ctx *ctx, int neighbourhood);
-/* FP32 sweeps as a slab dataflow (1, default): each warp updates whole
- * 32-row slabs once the slabs holding their columns reached the state the
- * sequential sweep in colour order reads (per-slab completion counters, no
- * barrier between colours); 0 the coloured kernel above.  The same sweep
- * either way.  Applies with one lane per contact when no slab has more
- * than 16 off-diagonal slots.  Returns the previous setting. */
+/* Sweeps as a dataflow (1, default): each warp updates its rows once the
+ * reactions they read have the state the sequential sweep in colour order
+ * reads (a sweep number stored with each reaction, or per-slab completion
+ * counters where the block pattern is not symmetric; no barrier between
+ * colours); 0 the coloured kernel above.  The same sweep either way.  Applies
+ * with one lane per contact, in FP32 when no slab has more than 16
+ * off-diagonal slots, in FP64 (bit-exact arithmetic, no timeline) on a
+ * symmetric pattern with at most 110 contacts a colour and SM.  Returns the
+ * previous setting. */
 int fc3dgpu_ctx_flow(fc3dgpu_ctx *ctx, int on);
 /* Warps per block of the dataflow sweep: 8, 10 or 12 (0: the default, 10,
  * or the autotuner's choice); fewer when the per-warp buffers of the current

@@ -465,6 +465,21 @@ __global__ void k_r64_to_r32(int npad, const double* __restrict__ r64, float* __
   }
 }
 
+// The FP64 reactions with sweep 0's stamps (fc3dgpu_flow64.cuh), the zero
+// entry with every sweep's.
+__global__ void k_stamp64(int npad, const double* __restrict__ r64, double* __restrict__ rs) {
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= npad; p += gridDim.x * blockDim.x) {
+    ulonglong2 a = make_ulonglong2(0, 0x7fffffffull << 32), b = a;
+    if (p < npad) {
+      const unsigned long long r1 = (unsigned long long)__double_as_longlong(r64[4 * (size_t)p + 1]);
+      a = make_ulonglong2((unsigned long long)__double_as_longlong(r64[4 * (size_t)p]), r1 & 0xffffffffull);
+      b = make_ulonglong2((unsigned long long)__double_as_longlong(r64[4 * (size_t)p + 2]), r1 >> 32);
+    }
+    reinterpret_cast<ulonglong2*>(rs)[2 * (size_t)p] = a;
+    reinterpret_cast<ulonglong2*>(rs)[2 * (size_t)p + 1] = b;
+  }
+}
+
 // The stamps alone, the reactions as they are (a batch's FP32 sweeps start
 // from them).
 __global__ void k_reset_stamps(int npad, float* __restrict__ r32) {
@@ -753,6 +768,8 @@ struct fc3dgpu_ctx {
   BUF(double, rpli64);
   BUF(float, rpli32);
   BUF(unsigned char, cost);
+  BUF(double, rs64);      // stamped FP64 reactions of the dataflow sweeps
+  int symmetric = -1;     // the block pattern: 1 symmetric, 0 not, -1 not looked at
   BUF(double, u64);
   // control
   BUF(double, partials);
@@ -778,7 +795,6 @@ struct fc3dgpu_ctx {
   int flow_state = 0;
   int flow_nw = 0, flow_maxslot = 0;
   int batch_flow = 0;  // the batch's FP32 sweeps as dataflow: 0 not decided, 1 yes, -1 no
-  bool flow_symmetric = false;  // every block has its transpose's place in W
   int flow_want = 0;  // warps per block of the dataflow sweep asked for (0: default)
   // measuring autotuner (per layout): chosen FP32 variant and FP64 lanes,
   // and the measured device time of one sweep of every candidate
@@ -950,7 +966,7 @@ extern "C" void fc3dgpu_ctx_destroy(fc3dgpu_ctx* c) {
   void* ptrs[] = {c->rowptr, c->colidx, c->blocks, c->qo, c->muo, c->ro, c->uo, c->deg, c->gptr64, c->gptr,
                   c->cursor, c->adj, c->key, c->colour, c->blockhist, c->counts, c->sptr_d, c->perm, c->iperm,
                   c->rowlen, c->dpos, c->slab_nslot, c->slab_off, c->W64, c->W32, c->col, c->D64, c->D32,
-                  c->rho64, c->rho32, c->q64, c->q32, c->mu64, c->mu32, c->r64, c->r32, c->rpli64, c->rpli32, c->cost,
+                  c->rho64, c->rho32, c->q64, c->q32, c->mu64, c->mu32, c->r64, c->r32, c->rpli64, c->rpli32, c->cost, c->rs64,
                   c->u64, c->partials, c->barrier, c->status, c->scratch, c->scratch64, c->out, c->trace,
                   c->counters, c->timeline, c->scene_off, c->grp, c->scounts, c->snslab, c->sncol, c->sbase,
                   c->ssptr, c->sorder, c->snormq, c->sbudget, c->squeue, c->sout32, c->sout64, c->steams, c->steam_part, c->feat,
@@ -1374,6 +1390,7 @@ static int build_layout(fc3dgpu_ctx* c, int nc, long long nnzb, int kind, int ns
   for (auto& n : c->nbrc) n.grid = 0;  // the rows' owners changed
   c->flow_state = 0;
   c->batch_flow = 0;
+  c->symmetric = -1;
   c->tuned = 0;
   return 0;
 }
@@ -1658,6 +1675,7 @@ static void fill_args(fc3dgpu_ctx* c, fc3dgpu::SweepArgs<Real>& a, const Real* W
   a.r = r;
   a.rpli = rpli;
   a.cost = c->cost;
+  a.rs = nullptr;
   a.u = c->u64;
   a.partials = c->partials;
   a.barrier = c->barrier;
@@ -1770,25 +1788,33 @@ static size_t staging_sizes(fc3dgpu_ctx* c, int grid, unsigned* wb, unsigned* cb
   return tot;
 }
 
-// Whether the block pattern is symmetric (the stamped dataflow sweeps need
-// it), and the places of the slabs' records.
+// c->symmetric of the current layout: every block has its transpose's place
+// in W (the stamped dataflow sweeps need it).
+static int look_symmetric(fc3dgpu_ctx* c) {
+  if (c->symmetric >= 0) return 0;
+  cudaStream_t s = c->stream;
+  int missing = 0;
+  CK(fc3dgpu::check_flow_symmetric(c->npad, c->perm, c->slab_nslot, c->slab_off, c->col, c->scratch, s));
+  CK(cudaMemcpyAsync(&missing, c->scratch, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  c->symmetric = missing ? 0 : 1;
+  c->launches++;
+  return 0;
+}
+
+// The places of the FP32 dataflow's per-slab records (filled before each
+// solve's FP32 sweeps).
 static int prepare_records(fc3dgpu_ctx* c) {
   using namespace fc3dgpu;
   cudaStream_t s = c->stream;
   const int nslab = c->nslab;
-  int missing = 0;
-  CK(check_flow_symmetric(c->npad, c->perm, c->slab_nslot, c->slab_off, c->col, c->scratch, s));
-  CK(cudaMemcpyAsync(&missing, c->scratch, sizeof(int), cudaMemcpyDeviceToHost, s));
-  // offsets of the per-slab records (filled before each solve's FP32 sweeps)
   std::vector<long long> roff((size_t)nslab + 1, 0);
   for (int t = 0; t < nslab; t++) roff[t + 1] = roff[t] + flow_rec_floats(c->slab_nslot_h[t]);
   CK(ensure(&c->flow_rec_off, &c->flow_rec_off_cap, (size_t)nslab + 1));
   CK(ensure(&c->flow_rec, &c->flow_rec_cap, (size_t)std::max(roff[nslab], 1LL)));
   CK(cudaMemcpyAsync(c->flow_rec_off, roff.data(), sizeof(long long) * (nslab + 1), cudaMemcpyHostToDevice, s));
   CK(cudaStreamSynchronize(s));
-  c->flow_symmetric = missing == 0;
-  c->launches++;
-  return 0;
+  return look_symmetric(c);
 }
 
 // Decides c->batch_flow for a batch layout; *resident: blocks of its FP32
@@ -1803,7 +1829,7 @@ static int prepare_batch_flow(fc3dgpu_ctx* c, int* resident) {
     if (c->flow_on && !c->counters_on && grid > 0) {
       if (int rc = prepare_records(c)) return rc;
       c->flow_maxslot = maxslot;
-      if (c->flow_symmetric) c->batch_flow = 1;
+      if (c->symmetric == 1) c->batch_flow = 1;
     }
   }
   if (c->batch_flow == 1)
@@ -1983,6 +2009,7 @@ static int autotune(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
       c->tune_lanes32 = ls[i];
     }
   }
+  c->flow_on = flow_on;
   for (int i = 0; i < 4; i++) {
     c->tune_ms64[i] = INFINITY;
     if (!all) continue;
@@ -1994,7 +2021,6 @@ static int autotune(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
     }
   }
   if (!all) best64 = 0.f;  // one lane per contact, unmeasured
-  c->flow_on = flow_on;
   c->flow_want = want;
   if (c->flow_state == 1) c->flow_nw = c->tune_flow ? c->tune_nw : flow_warps(c->flow_maxslot, want);
   c->timeline = tl;
@@ -2053,6 +2079,25 @@ extern "C" int fc3dgpu_ctx_solve(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgp
     if (int rc = autotune(c, p)) return rc;
   }
   return solve_impl(c, p, st);
+}
+
+// The FP64 sweeps as dataflow (a.rs set), where the block pattern is symmetric
+// and a block has few contacts of a colour: the stamped reactions of the
+// solve's start.
+static int attach_flow64(fc3dgpu_ctx* c, fc3dgpu::SweepArgs<double>& a) {
+  using namespace fc3dgpu;
+  int dev = 0, sms = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (c->npad > (long long)FC3D_FLOW64_MAX * c->ncol * sms) return 0;
+  if (int rc = look_symmetric(c)) return rc;
+  if (c->symmetric != 1) return 0;
+  CK(ensure(&c->rs64, &c->rs64_cap, ((size_t)c->npad + 1) * 4));
+  k_stamp64<<<grid1d(c->npad + 1), 256, 0, c->stream>>>(c->npad, c->r64, c->rs64);
+  CK(cudaGetLastError());
+  c->launches++;
+  a.rs = c->rs64;
+  return 0;
 }
 
 static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st) {
@@ -2138,7 +2183,7 @@ static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st
       f.buf_bytes = flow_buf_bytes(c->flow_maxslot);
       f.rec = c->flow_rec;
       f.rec_off = c->flow_rec_off;
-      f.stamped = c->flow_symmetric ? 1 : 0;
+      f.stamped = c->symmetric == 1 ? 1 : 0;
       f.split = 0;
       if (f.stamped) {
         int sms = 0;
@@ -2205,7 +2250,11 @@ static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st
       a.max_sweeps = out[3] == 0.0 ? 0 : budget;
     }
     if (!(converged32 && a.max_sweeps == 0)) {
-      if (a.max_sweeps > 0) CK(cudaMemsetAsync(c->cost, 0, (size_t)c->npad, s));
+      if (a.max_sweeps > 0) {
+        CK(cudaMemsetAsync(c->cost, 0, (size_t)c->npad, s));
+        if (lanes64 == 1 && !fast64 && c->flow_on && !c->timeline)
+          if (int rc = attach_flow64(c, a)) return rc;
+      }
       CK(cudaMemsetAsync(c->barrier, 0, FC3D_BARRIER_WORDS * sizeof(unsigned), s));
       CK(launch64(a));
       c->launches++;

@@ -22,6 +22,9 @@
 
 #define FC3D_SLAB 32
 #define FC3D_MAX_COLOURS 128
+// Contacts a colour and block up to which the FP64 sweeps go as dataflow
+// (measured in fc3dgpu_flow64.cuh)
+#define FC3D_FLOW64_MAX 110
 
 namespace fc3dgpu {
 
@@ -46,6 +49,7 @@ struct SweepArgs {
   // state
   Real* r;                      // AoS (npad + 1) * 3, entry npad is zero
   Real* rpli;                   // npad
+  double* rs;                   // FP64 dataflow: stamped reactions, (npad + 1) * 4 (null: sweeps by colours)
   unsigned char* cost;          // npad: cost class of each contact's last FP64 local solve (order of work only)
   double* u;                    // AoS npad * 3 (FP64 full error output)
   // reductions and control

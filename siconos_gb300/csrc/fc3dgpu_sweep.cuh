@@ -1104,6 +1104,12 @@ __device__ __forceinline__ bool process_colour_staged(const SweepArgs<Real>& a, 
   return true;
 }
 
+}  // namespace fc3dgpu
+
+#include "fc3dgpu_flow64.cuh"
+
+namespace fc3dgpu {
+
 // u = q + W r for every row in CSR block order (diagonal at its own slot
 // position, SBM_gemv_3x3, SparseBlockMatrix.c:360-419) and the partial sums
 // of the squared natural-map error, |u|^2 and |r|^2.  FP64 only.
@@ -1168,7 +1174,9 @@ __device__ __forceinline__ bool full_error_phase(const SweepArgs<Real>& a, int s
   return true;
 }
 
-template <typename Real, int T>
+// FLOW (FP64): the sweeps as dataflow (fc3dgpu_flow64.cuh) instead of by
+// colours.
+template <typename Real, int T, bool FLOW = false>
 __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_kernel(const SweepArgs<Real> a) {
   __shared__ typename RangeList<Real>::type wk;
   __shared__ __align__(8) unsigned long long stage_bar;
@@ -1200,10 +1208,17 @@ __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_kernel(const Sw
   double incr = INFINITY, full = INFINITY, best = INFINITY;
   int sweep = 0, best_sweep = 0;
   bool converged = false;
+  const int rows64 = FLOW ? flow64_rows(a.sptr, a.ncol, gridDim.x) : 0;
   while (sweep < a.max_sweeps) {
     sweep++;
     double acc[2] = {0.0, 0.0};
-    for (int c = 0; c < a.ncol; c++) {
+    if constexpr (FLOW) {
+      if (!flow64_sweep(a, a.sptr, a.ncol, rows64, blockIdx.x, gridDim.x, sweep, local_tol, acc[0],
+                        acc[1])) return;
+      block_sum<2>(acc, a.partials + blockIdx.x * 8);
+      if (!grid_barrier(a.barrier, epoch, a.spin_limit, a.status)) return;
+    }
+    for (int c = 0; c < (FLOW ? 0 : a.ncol); c++) {
       const int s0 = a.sptr[c], nunits = (a.sptr[c + 1] - s0) * T;
       const bool tl = a.timeline && sweep == a.timeline_sweep && threadIdx.x == 0;
       if (tl) {

@@ -8,9 +8,9 @@ namespace fc3dgpu {
 // The grid is queried at every launch (a few microseconds of host work
 // against a solve of milliseconds): no launch state is kept between calls, so
 // contexts on different host threads and devices never share any.
-template <int T>
+template <int T, bool FLOW = false>
 static cudaError_t launch_t(const SweepArgs<double>& a, int max_grid, size_t smem, cudaStream_t s, int* grid) {
-  auto kern = nsgs_kernel<double, T>;
+  auto kern = nsgs_kernel<double, T, FLOW>;
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -41,7 +41,7 @@ static int grid_t() {
 cudaError_t launch_sweep_f64(const SweepArgs<double>& a, int lanes, int max_grid, size_t smem, cudaStream_t s,
                              int* grid) {
   switch (lanes) {
-    case 1: return launch_t<1>(a, max_grid, smem, s, grid);
+    case 1: return a.rs ? launch_t<1, true>(a, max_grid, smem, s, grid) : launch_t<1>(a, max_grid, smem, s, grid);
     case 2: return launch_t<2>(a, max_grid, 0, s, grid);
     case 4: return launch_t<4>(a, max_grid, 0, s, grid);
     case 8: return launch_t<8>(a, max_grid, 0, s, grid);
@@ -52,6 +52,7 @@ cudaError_t launch_sweep_f64(const SweepArgs<double>& a, int lanes, int max_grid
 void warm_sweep_kernels_f64() {
   cudaFuncAttributes fa;
   cudaFuncGetAttributes(&fa, nsgs_kernel<double, 1>);
+  cudaFuncGetAttributes(&fa, nsgs_kernel<double, 1, true>);
   cudaFuncGetAttributes(&fa, nsgs_kernel<double, 2>);
   cudaFuncGetAttributes(&fa, nsgs_kernel<double, 4>);
   cudaFuncGetAttributes(&fa, nsgs_kernel<double, 8>);

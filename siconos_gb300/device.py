@@ -76,7 +76,7 @@ class DeviceSolver:
         return int(self.L.fc3dgpu_ctx_spin_limit(self.ctx, polls))
 
     def flow(self, on: bool) -> bool:
-        """Slab-dataflow FP32 sweeps (True) or the coloured kernel (False);
+        """Dataflow sweeps (True) or the coloured kernel (False);
         returns the previous setting."""
         return bool(self.L.fc3dgpu_ctx_flow(self.ctx, int(on)))
 
