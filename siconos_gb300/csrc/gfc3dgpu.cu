@@ -21,13 +21,22 @@
 //   phase A (degree-of-freedom rows)  t = q + H r_{k-1};  [diagonal M:
 //       v_k = t / M_ii]  and the error terms of iteration k - 1: H r_{k-1}
 //       and M v_{k-1} (gfc3d_compute_error.c:87-109 of r_{k-1}, v_{k-1});
-//   grid barrier; the stop decision on iteration k - 1's error;
+//   grid barrier;
 //   phase B (components, general M)  v_k = LU solve of t; grid barrier;
 //   phase C (contacts)  u_k = b + H^T v_k, r_k = proj(r_{k-1} - (u_N + mu
-//       |u_T|, u_T)), the complementarity terms of (r_k, u_k); grid barrier.
-// The error of iteration k is thus known after phase A of iteration k + 1;
-// a stop leaves r_k, u_k and v_k (v double-buffered) as the reference's loop
-// leaves them.  Every product and update follows the reference's operation
+//       |u_T|, u_T)), the complementarity terms of (r_k, u_k); beside it one
+//       warp of each block forms iteration k - 1's error and the stop
+//       decision; grid barrier.
+// r, u and v are double-buffered, so a stop on iteration k - 1 leaves its r, u
+// and v as the reference's loop leaves them, phase C of iteration k aside.
+//
+// What bounds an iteration is the FP64 pipe (a warp instruction holds it 64
+// cycles whatever its lanes do): 1.30 M warp instructions at 192,000 dofs and
+// 94,400 contacts, of which 0.43 M are the products.  So the stop decision is
+// one warp's work, not every warp's (0.5 M); block sums take 6 additions a
+// warp, not 15; roots, divisions and the cone's comparisons are those of
+// fc3dgpu_ieee64.cuh on the integer pipes; what the error and the update
+// share is formed once.  GFIG  Every product and update follows the reference's operation
 // order (row sums from +0.0 in column order, then added to q or b; the
 // projection as projectionOnCone), compiled without FMA contraction, so the
 // iterates are the reference's bit for bit; the norms are fixed-order block
@@ -42,6 +51,7 @@
 #include <numeric>
 #include <vector>
 
+#include "fc3dgpu_local64.cuh"
 #include "fc3dgpu_sweep.cuh"
 #include "gfc3dgpu.h"
 
@@ -52,7 +62,7 @@ namespace gfc3dgpu {
 using fc3dgpu::grid_barrier;
 using fc3dgpu::project_cone;
 
-constexpr int NT = 512;            // threads per block
+constexpr int NT = 1024;           // threads per block, one block an SM
 constexpr int NW = NT / 32;
 constexpr int GRID_MAX = 1024;     // blocks at most
 constexpr int TRACE_CAP = 1 << 16;
@@ -90,14 +100,14 @@ struct Args {
   const double* tval;
   const double* b;
   const double* mu;
-  double* r;     // m + 1 (r[m] = 0)
-  double* u;     // m
-  double* v0;    // n + 1 each (v[n] = 0): v of the odd iterations in v1, even in v0
-  double* v1;
+  // iterates of the even iterations (and the start) in [0], odd in [1]
+  double* r[2];  // m + 1 each (r[m] = 0)
+  double* u[2];  // m each
+  double* v[2];  // n + 1 each (v[n] = 0)
   double* t;     // n
   // solve
   double tol;
-  int max_iter, freq, mode;  // mode 0 solve, 1 error of (r, v0) only, 2 v0 = M^-1 q only
+  int max_iter, freq, mode;  // mode 0 solve, 1 error of (r[0], v[0]) only, 2 v[0] = M^-1 q only
   double norm_q;
   unsigned* flags;
   double* part;  // [2][GRID_MAX][8]
@@ -105,49 +115,62 @@ struct Args {
   unsigned long long spin_limit;
   double* trace;
   int trace_cap;
-  double* out;  // iterations, error, info, buffer of the result's v
+  double* out;  // iterations, error, info, buffer of the result
 };
 
-// Sum of N values over the block in a fixed order, written to out[0..N).
-template <int N>
-__device__ __forceinline__ void bsum(double v[N], double* out) {
-  __shared__ double sh[NW][N];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// Sums of three values over the warp: of e[0] in lane 0, e[1] in lane 8, e[2]
+// in lane 16.  Each step adds half the values of half the lanes, so 6
+// additions in place of 15.
+__device__ __forceinline__ double wsum3(const double e[3]) {
+  const unsigned full = 0xffffffffu;
+  const bool b16 = threadIdx.x & 16, b8 = threadIdx.x & 8;
+  const double x = (b16 ? e[2] : e[0]) + __shfl_xor_sync(full, b16 ? e[0] : e[2], 16);
+  const double y = e[1] + __shfl_xor_sync(full, e[1], 16);
+  double z = (b8 ? y : x) + __shfl_xor_sync(full, b8 ? x : y, 8);
 #pragma unroll
-  for (int i = 0; i < N; i++) {
-    double x = v[i];
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[w][i] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x < N) {
-    double s = 0.0;
-    for (int k = 0; k < NW; k++) s += sh[k][threadIdx.x];
-    out[threadIdx.x] = s;
-  }
-  __syncthreads();
+  for (int o = 4; o >= 1; o >>= 1) z += __shfl_xor_sync(full, z, o);
+  return z;
 }
 
-// Slot i of every block's partials (stride 8) summed in a fixed order.
-template <int N>
-__device__ __forceinline__ void gsum(const double* part, int slot, double out[N]) {
-  __shared__ double res[8];
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
+// Sums of three values over the block in a fixed order, written to out[0..3)
+__device__ __forceinline__ void bsum3(const double e[3], double* out) {
+  __shared__ double sh[NW][3];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const double z = wsum3(e);
+  if ((lane & 7) == 0 && lane < 24) sh[w][lane >> 3] = z;
+  __syncthreads();
+  if (w < 3) {
+    double x = sh[lane][w];
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-      double s = 0.0;
-      for (int bl = lane; bl < (int)gridDim.x; bl += 32) s += __ldcg(&part[bl * 8 + slot + i]);
+    for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane == 0) out[w] = x;
+  }
+}
+static_assert(NW == 32, "bsum3 sums the warps of a block in one warp");
+
+// Six sums over every block's partials (stride 8) by one warp, in a fixed
+// order: slots 0-2 of pa in lanes 0-2, slots 3-5 of pc in lanes 3-5.
+__device__ __forceinline__ double gsum6(const double* pa, const double* pc) {
+  const int lane = threadIdx.x & 31;
+  double sa[3] = {0.0, 0.0, 0.0}, sc[3] = {0.0, 0.0, 0.0};
+#pragma unroll 2
+  for (int bl = lane; bl < (int)gridDim.x; bl += 32) {
+    double x[6];
 #pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) res[i] = s;
+    for (int i = 0; i < 3; i++) {
+      x[i] = __ldcg(&pa[bl * 8 + i]);
+      x[3 + i] = __ldcg(&pc[bl * 8 + 3 + i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      sa[i] += x[i];
+      sc[i] += x[3 + i];
     }
   }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < N; i++) out[i] = res[i];
-  __syncthreads();
+  const double za = wsum3(sa), zc = wsum3(sc);
+  const int src = lane % 3 * 8;
+  const double ga = __shfl_sync(0xffffffffu, za, src), gc = __shfl_sync(0xffffffffu, zc, src);
+  return lane < 3 ? ga : gc;
 }
 
 // acc + a b: two roundings as the reference computes it, or (FAST, the
@@ -158,6 +181,9 @@ __device__ __forceinline__ double madd(double acc, double a, double b) {
   if (FAST) return fma(a, b, acc);
   return acc + a * b;
 }
+// 0.0 + a b, the first term of a row sum: a fused multiply-add with +0.0 is
+// exactly that, rounding and sign of zero included
+__device__ __forceinline__ double mfirst(double a, double b) { return fma(a, b, 0.0); }
 
 // Rank of the calling warp for the grid-stride slab loops: consecutive ranks
 // go to different blocks, so the slabs left over after equal shares fall
@@ -174,8 +200,8 @@ __device__ __forceinline__ double* part_of(const Args& a, int parity) {
 // |q + H r - M v|^2); vcur receives t / M_ii for a diagonal M (when non
 // null), else t is stored.  no_h: t = q (no contact).
 template <bool FAST>
-__device__ __forceinline__ void phase_a(const Args& a, bool err, const double* vprev, double* vcur, bool store,
-                                        bool no_h, double e[3]) {
+__device__ __forceinline__ void phase_a(const Args& a, bool err, const double* r, const double* vprev, double* vcur,
+                                        bool store, bool no_h, double e[3]) {
   const int lane = threadIdx.x & 31;
   const int gw = warp_rank(), tw = (gridDim.x * NT) >> 5;
   for (int s = gw; s < a.nslab_d; s += tw) {
@@ -185,46 +211,50 @@ __device__ __forceinline__ void phase_a(const Args& a, bool err, const double* v
     if (!no_h) {
       const long long o = a.hoff[s];
       const int ns = a.hns[s];
+      constexpr int CH = 6;
       int k = 0;
-      for (; k + 4 <= ns; k += 4) {
-        double hv[4], rv[4];
+      for (; k + CH <= ns; k += CH) {
+        double hv[CH], rv[CH];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < CH; j++) {
           const size_t p = (size_t)(o + k + j) * 32 + lane;
           hv[j] = __ldg(&a.hval[p]);
-          rv[j] = __ldcg(&a.r[__ldg(&a.hcol[p])]);
+          rv[j] = __ldcg(&r[__ldg(&a.hcol[p])]);
         }
 #pragma unroll
-        for (int j = 0; j < 4; j++) sh = madd<FAST>(sh, hv[j], rv[j]);
+        for (int j = 0; j < CH; j++) sh = j == 0 && k == 0 ? mfirst(hv[j], rv[j]) : madd<FAST>(sh, hv[j], rv[j]);
       }
       for (; k < ns; k++) {
         const size_t p = (size_t)(o + k) * 32 + lane;
-        sh = madd<FAST>(sh, __ldg(&a.hval[p]), __ldcg(&a.r[__ldg(&a.hcol[p])]));
+        sh = madd<FAST>(sh, __ldg(&a.hval[p]), __ldcg(&r[__ldg(&a.hcol[p])]));
       }
     }
     if (!row) continue;
     const double qi = __ldg(&a.q[i]);
     // dgemv with beta 1: 1.0 * q + 1.0 * s (the loop), daxpy q + 1.0 * tmp
     // (the error): both q + s
-    const double ti = no_h ? qi : qi + 1.0 * sh;
+    const double ti = no_h ? qi : qi + sh;
+    const double md = a.mdiag ? __ldg(&a.mdiag[i]) : 0.0;
     if (err) {
-      const long long o = a.moff[s];
-      const int ns = a.mns[s];
       double sm = 0.0;
-      for (int k = 0; k < ns; k++) {
-        const size_t p = (size_t)(o + k) * 32 + lane;
-        sm = madd<FAST>(sm, __ldg(&a.mval[p]), __ldcg(&vprev[__ldg(&a.mcol[p])]));
+      if (a.mdiag) {
+        sm = mfirst(md, __ldcg(&vprev[i]));
+      } else {
+        const long long o = a.moff[s];
+        const int ns = a.mns[s];
+        for (int k = 0; k < ns; k++) {
+          const size_t p = (size_t)(o + k) * 32 + lane;
+          sm = madd<FAST>(sm, __ldg(&a.mval[p]), __ldcg(&vprev[__ldg(&a.mcol[p])]));
+        }
       }
-      const double hr = 0.0 + 1.0 * sh;    // NM_gemv(1.0, H, r, 0.0, tmp)
-      const double mv = 0.0 + -1.0 * sm;   // NM_gemv(-1.0, M, v, 0.0, tmp)
-      const double t1 = ti + 1.0 * mv;     // tmp_1 += 1.0 * tmp
-      e[0] += hr * hr;
-      e[1] += mv * mv;
-      e[2] += t1 * t1;
+      const double t1 = ti - sm;  // tmp_1 += NM_gemv(-1.0, M, v, 0.0, tmp)
+      e[0] = fma(sh, sh, e[0]);
+      e[1] = fma(sm, sm, e[1]);
+      e[2] = fma(t1, t1, e[2]);
     }
     if (!store) continue;
     if (vcur)
-      vcur[i] = ti / __ldg(&a.mdiag[i]);
+      vcur[i] = fc3dgpu::ie_div(ti, md);
     else
       a.t[i] = ti;
   }
@@ -301,24 +331,12 @@ __device__ __forceinline__ void phase_b(const Args& a, double* v) {
   }
 }
 
-// fc3d_unitary_compute_and_add_error (fc3d_compute_error.c:42-56)
-__device__ __forceinline__ double unitary_error(const double r[3], const double u[3], double mu) {
-  double w[3];
-  w[0] = r[0] - u[0] - mu * sqrt(u[1] * u[1] + u[2] * u[2]);
-  w[1] = r[1] - u[1];
-  w[2] = r[2] - u[2];
-  project_cone<double>(w, mu);
-  w[0] = r[0] - w[0];
-  w[1] = r[1] - w[1];
-  w[2] = r[2] - w[2];
-  return w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
-}
-
 // Phase C over the contact slabs (one warp per slab): u = b + H^T v, the
-// projected update of r (gfc3d_nsgs.c:150-165) when `update`, and the
+// projected update of r (gfc3d_nsgs.c:150-165) unless rnew is null, and the
 // error terms e[0..2] (|u|^2, |r|^2, complementarity) of the result.
 template <bool FAST>
-__device__ __forceinline__ void phase_c(const Args& a, const double* v, bool update, double e[3]) {
+__device__ __forceinline__ void phase_c(const Args& a, const double* v, const double* rold, double* rnew, double* unew,
+                                        double e[3]) {
   const int lane = threadIdx.x & 31;
   const int gw = warp_rank(), tw = (gridDim.x * NT) >> 5;
   for (int s = gw; s < a.nslab_c; s += tw) {
@@ -339,11 +357,10 @@ __device__ __forceinline__ void phase_c(const Args& a, const double* v, bool upd
         tv[j][2] = __ldg(&a.tval[pv + 64]);
       }
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        acc[0] = madd<FAST>(acc[0], tv[j][0], vv[j]);
-        acc[1] = madd<FAST>(acc[1], tv[j][1], vv[j]);
-        acc[2] = madd<FAST>(acc[2], tv[j][2], vv[j]);
-      }
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+          acc[d] = j == 0 && k == 0 ? mfirst(tv[j][d], vv[j]) : madd<FAST>(acc[d], tv[j][d], vv[j]);
     }
     for (; k < ns; k++) {
       const size_t p = (size_t)(o + k) * 32 + lane;
@@ -357,57 +374,64 @@ __device__ __forceinline__ void phase_c(const Args& a, const double* v, bool upd
     double u[3], r[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      u[d] = 1.0 * __ldg(&a.b[3 * c + d]) + 1.0 * acc[d];  // dgemv^T with beta 1
-      r[d] = __ldcg(&a.r[3 * c + d]);
+      u[d] = __ldg(&a.b[3 * c + d]) + acc[d];  // dgemv^T with beta 1
+      r[d] = __ldcg(&rold[3 * c + d]);
     }
     const double mu = __ldg(&a.mu[c]);
-    if (update) {
-      const double normUT = sqrt(u[1] * u[1] + u[2] * u[2]);
-      const double an = 1.0;
-      r[0] -= an * (u[0] + mu * normUT);
-      r[1] -= an * u[1];
-      r[2] -= an * u[2];
+    const double mun = mu * fc3dgpu::ie_sqrt(u[1] * u[1] + u[2] * u[2]);
+    if (rnew) {
+      r[0] -= u[0] + mun;
+      r[1] -= u[1];
+      r[2] -= u[2];
       project_cone<double>(r, mu);
 #pragma unroll
-      for (int d = 0; d < 3; d++) a.r[3 * c + d] = r[d];
+      for (int d = 0; d < 3; d++) rnew[3 * c + d] = r[d];
     }
 #pragma unroll
-    for (int d = 0; d < 3; d++) a.u[3 * c + d] = u[d];
-    e[0] += u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-    e[1] += r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-    e[2] += unitary_error(r, u, mu);
+    for (int d = 0; d < 3; d++) unew[3 * c + d] = u[d];
+    // fc3d_unitary_compute_and_add_error (fc3d_compute_error.c:42-56)
+    double w[3] = {r[0] - u[0] - mun, r[1] - u[1], r[2] - u[2]};
+    project_cone<double>(w, mu);
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      w[d] = r[d] - w[d];
+      e[0] = fma(u[d], u[d], e[0]);
+      e[1] = fma(r[d], r[d], e[1]);
+      e[2] = fma(w[d], w[d], e[2]);
+    }
   }
 }
 
-// gfc3d_compute_error from the grid sums of phase A (slot 0-2) and phase C
-// (slot 3-5).
-__device__ __forceinline__ double error_of(const Args& a, const double sa[3], const double sc[3]) {
-  const double min_rel = sqrt(DBL_EPSILON);
-  const double norm_hr = sqrt(sa[0]), norm_mv = sqrt(sa[1]);
-  const double rel = fmax(a.norm_q, fmax(norm_mv, norm_hr));
-  double err = sqrt(sa[2]);
-  if (fabs(rel) > min_rel) err = err / rel;
-  const double norm_u = sqrt(sc[0]), norm_r = sqrt(sc[1]);
-  double ec = sqrt(sc[2]);
-  const double rel2 = fmax(norm_u, norm_r);
-  if (fabs(rel2) > min_rel) ec = ec / rel2;
-  return err + ec;
+// gfc3d_compute_error from the six sums of gsum6, the same in every lane of
+// the warp: the roots side by side in lanes 0-5, the quotients in 0 and 1.
+__device__ __forceinline__ double error_of(const Args& a, double sum) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const double min_rel = 1.4901161193847656e-08;  // sqrt(DBL_EPSILON) = 2^-26
+  const double root = fc3dgpu::ie_sqrt(sum);
+  const double norm_hr = __shfl_sync(full, root, 0), norm_mv = __shfl_sync(full, root, 1);
+  const double norm_u = __shfl_sync(full, root, 3), norm_r = __shfl_sync(full, root, 4);
+  const double num = __shfl_sync(full, root, lane == 0 ? 2 : 5);
+  const double rel = lane == 0 ? fmax(a.norm_q, fmax(norm_mv, norm_hr)) : fmax(norm_u, norm_r);
+  const double part = fabs(rel) > min_rel ? fc3dgpu::ie_div(num, rel) : num;
+  return __shfl_sync(full, part, 0) + __shfl_sync(full, part, 1);
 }
 
 template <bool FAST>
-__global__ void __launch_bounds__(NT) k_gfc3d(Args a) {
+__global__ void __launch_bounds__(NT, 1) k_gfc3d(Args a) {
+  __shared__ int s_stop;
   unsigned epoch = 0;
   const bool diag = a.mdiag != nullptr;
-  double* vb[2] = {a.v0, a.v1};
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
   if (a.mode == 2) {
     // v = M^-1 q (gfc3d_driver's no-contact case)
     double e[3] = {0, 0, 0};
-    phase_a<FAST>(a, false, nullptr, diag ? a.v0 : nullptr, true, true, e);
+    phase_a<FAST>(a, false, nullptr, nullptr, diag ? a.v[0] : nullptr, true, true, e);
     if (!diag) {
       if (!grid_barrier(a.flags, epoch, a.spin_limit, a.status)) return;
-      phase_b(a, a.v0);
+      phase_b(a, a.v[0]);
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (first) {
       a.out[0] = 0;
       a.out[1] = 0.0;
       a.out[2] = 0;
@@ -416,25 +440,29 @@ __global__ void __launch_bounds__(NT) k_gfc3d(Args a) {
     return;
   }
   if (a.mode == 1) {
-    // the error of (r, v0) with u = b + H^T v0 (max_iter 0, or an error
+    // the error of (r, v) with u = b + H^T v (max_iter 0, or an error
     // evaluation alone)
     double ec[3] = {0, 0, 0}, ea[3] = {0, 0, 0};
-    phase_c<FAST>(a, a.v0, false, ec);
-    bsum<3>(ec, part_of(a, 0) + blockIdx.x * 8 + 3);
-    phase_a<FAST>(a, true, a.v0, nullptr, false, false, ea);
-    bsum<3>(ea, part_of(a, 0) + blockIdx.x * 8);
+    phase_c<FAST>(a, a.v[0], a.r[0], nullptr, a.u[0], ec);
+    bsum3(ec, part_of(a, 0) + blockIdx.x * 8 + 3);
+    phase_a<FAST>(a, true, a.r[0], a.v[0], nullptr, false, false, ea);
+    __syncthreads();
+    bsum3(ea, part_of(a, 0) + blockIdx.x * 8);
     if (!grid_barrier(a.flags, epoch, a.spin_limit, a.status)) return;
-    double sa[3], sc[3];
-    gsum<3>(part_of(a, 0), 0, sa);
-    gsum<3>(part_of(a, 0), 3, sc);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      a.out[0] = 0;
-      a.out[1] = error_of(a, sa, sc);
-      a.out[2] = -1;
-      a.out[3] = 0;
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+      const double err = error_of(a, gsum6(part_of(a, 0), part_of(a, 0)));
+      if (first) {
+        a.out[0] = 0;
+        a.out[1] = err;
+        a.out[2] = -1;
+        a.out[3] = 0;
+      }
     }
     return;
   }
+  // The last warp of a block has the fewest slabs: it decides.
+  const bool decides = (threadIdx.x >> 5) == NW - 1;
+  const bool writes = blockIdx.x == 0 && threadIdx.x == NT - 32;
   double eff = 1.0;  // the error the reference's loop holds (1.0 before any evaluation)
   int k = 0;
   for (;;) {
@@ -443,36 +471,36 @@ __global__ void __launch_bounds__(NT) k_gfc3d(Args a) {
     // phase A of iteration k, with the error terms of iteration k - 1
     double ea[3] = {0, 0, 0};
     const bool final_only = k > a.max_iter;  // the error of the last iterate alone
-    phase_a<FAST>(a, k >= 2, vb[prev], diag ? vb[cur] : nullptr, !final_only, false, ea);
-    bsum<3>(ea, part_of(a, cur) + blockIdx.x * 8);
+    phase_a<FAST>(a, k >= 2, a.r[prev], a.v[prev], diag ? a.v[cur] : nullptr, !final_only, false, ea);
+    if (k >= 2) bsum3(ea, part_of(a, cur) + blockIdx.x * 8);
     if (!grid_barrier(a.flags, epoch, a.spin_limit, a.status)) return;
-    if (k >= 2) {
-      double sa[3], sc[3];
-      gsum<3>(part_of(a, cur), 0, sa);
-      gsum<3>(part_of(a, prev), 3, sc);
-      const int it = k - 1;
-      const double err = error_of(a, sa, sc);
-      if (a.freq <= 0 || it % a.freq == 0) eff = err;
-      if (a.trace && it - 1 < a.trace_cap && blockIdx.x == 0 && threadIdx.x == 0) a.trace[it - 1] = eff;
-      const bool conv = eff < a.tol;
-      if (conv || it >= a.max_iter) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (!diag && !final_only) {
+      phase_b(a, a.v[cur]);
+      if (!grid_barrier(a.flags, epoch, a.spin_limit, a.status)) return;
+    }
+    if (decides) {
+      bool stop = false;
+      if (k >= 2) {
+        const int it = k - 1;
+        const double err = error_of(a, gsum6(part_of(a, cur), part_of(a, prev)));
+        if (a.freq <= 0 || it % a.freq == 0) eff = err;
+        if (a.trace && it - 1 < a.trace_cap && writes) a.trace[it - 1] = eff;
+        const bool conv = eff < a.tol;
+        stop = conv || it >= a.max_iter;
+        if (stop && writes) {
           a.out[0] = it;
           // at the budget the reference evaluates the error once more
           a.out[1] = it >= a.max_iter ? err : eff;
           a.out[2] = conv ? 0 : 1;
           a.out[3] = prev;
         }
-        return;
       }
-    }
-    if (!diag) {
-      phase_b(a, vb[cur]);
-      if (!grid_barrier(a.flags, epoch, a.spin_limit, a.status)) return;
+      if ((threadIdx.x & 31) == 0) s_stop = stop;
     }
     double ec[3] = {0, 0, 0};
-    phase_c<FAST>(a, vb[cur], true, ec);
-    bsum<3>(ec, part_of(a, cur) + blockIdx.x * 8 + 3);
+    if (!final_only) phase_c<FAST>(a, a.v[cur], a.r[prev], a.r[cur], a.u[cur], ec);
+    bsum3(ec, part_of(a, cur) + blockIdx.x * 8 + 3);  // its barrier publishes s_stop
+    if (s_stop) return;
     if (!grid_barrier(a.flags, epoch, a.spin_limit, a.status)) return;
   }
 }
@@ -570,11 +598,12 @@ struct gfc3dgpu_ctx {
   int *hns = nullptr, *hcol = nullptr, *mns = nullptr, *mcol = nullptr, *tns = nullptr, *tcol = nullptr;
   int *cptr = nullptr, *cdof = nullptr, *piv = nullptr;
   double *hval = nullptr, *mval = nullptr, *tval = nullptr, *q = nullptr, *mdiag = nullptr, *lu = nullptr;
-  double *b = nullptr, *mu = nullptr, *r = nullptr, *u = nullptr, *v[2] = {nullptr, nullptr}, *t = nullptr;
+  double *b = nullptr, *mu = nullptr, *t = nullptr;
+  double *r[2] = {nullptr, nullptr}, *u[2] = {nullptr, nullptr}, *v[2] = {nullptr, nullptr};
   unsigned* flags = nullptr;
   double *part = nullptr, *trace = nullptr, *out = nullptr;
   int* status = nullptr;
-  int vcur = 0;  // buffer holding the current global velocity
+  int cur = 0;  // buffer holding the current r, u and v
   int trace_len = 0;
 };
 
@@ -590,13 +619,13 @@ struct gfc3dgpu_ctx {
 static void free_problem(gfc3dgpu_ctx* c) {
   void* ptrs[] = {c->hoff, c->moff, c->toff, c->luoff, c->hns, c->hcol, c->mns, c->mcol, c->tns, c->tcol,
                   c->cptr, c->cdof, c->piv, c->hval, c->mval, c->tval, c->q, c->mdiag, c->lu, c->b,
-                  c->mu, c->r, c->u, c->v[0], c->v[1], c->t};
+                  c->mu, c->r[0], c->r[1], c->u[0], c->u[1], c->v[0], c->v[1], c->t};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   c->hoff = c->moff = c->toff = c->luoff = nullptr;
   c->hns = c->hcol = c->mns = c->mcol = c->tns = c->tcol = c->cptr = c->cdof = c->piv = nullptr;
-  c->hval = c->mval = c->tval = c->q = c->mdiag = c->lu = c->b = c->mu = c->r = c->u = c->t = nullptr;
-  c->v[0] = c->v[1] = nullptr;
+  c->hval = c->mval = c->tval = c->q = c->mdiag = c->lu = c->b = c->mu = c->t = nullptr;
+  c->r[0] = c->r[1] = c->u[0] = c->u[1] = c->v[0] = c->v[1] = nullptr;
   c->ready = false;
   c->n = 0;
   c->nc = 0;
@@ -652,7 +681,6 @@ extern "C" gfc3dgpu_ctx* gfc3dgpu_ctx_create(int device) {
     gfc3dgpu_ctx_destroy(c);
     return nullptr;
   }
-  c->grid = std::min(GRID_MAX, c->sms * std::min(std::min(per_sm, per_sm_fast), 2));
   return c;
 }
 
@@ -878,10 +906,11 @@ extern "C" int gfc3dgpu_ctx_set_problem(gfc3dgpu_ctx* c, int64_t n, int nc, cons
   ok(put(&c->q, qv));
   ok(put(&c->b, bv));
   ok(put(&c->mu, muv));
-  ok(put(&c->r, zero_r));
-  ok(put(&c->u, std::vector<double>(std::max<long long>(m, 1), 0.0)));
-  ok(put(&c->v[0], zero_v));
-  ok(put(&c->v[1], zero_v));
+  for (int k = 0; k < 2; k++) {
+    ok(put(&c->r[k], zero_r));
+    ok(put(&c->u[k], std::vector<double>(std::max<long long>(m, 1), 0.0)));
+    ok(put(&c->v[k], zero_v));
+  }
   ok(put(&c->t, std::vector<double>(n, 0.0)));
   int singular = 0;
   if (diag) {
@@ -931,11 +960,16 @@ extern "C" int gfc3dgpu_ctx_set_problem(gfc3dgpu_ctx* c, int64_t n, int nc, cons
   c->maxcomp = maxcomp;
   c->nslab_d = (int)((n + 31) / 32);
   c->nslab_c = (int)nslab_c;
+  // a block a slab until every SM has one: fewer blocks make the barriers and
+  // the grid sums shorter
+  const long long work = std::max<long long>(std::max(c->nslab_d, c->nslab_c),
+                                             diag ? 0 : (maxcomp <= SMALL_COMPONENT ? (ncomp + 31) / 32 : ncomp));
+  c->grid = (int)std::max(1LL, std::min<long long>(std::min(c->sms, GRID_MAX), work));
   double s = 0.0;
   for (long long i = 0; i < n; i++) s += q[i] * q[i];
   c->norm_q = sqrt(s);
   c->bytes_iter = bytes;
-  c->vcur = 0;
+  c->cur = 0;
   c->trace_len = 0;
   c->ready = true;
   return 0;
@@ -950,11 +984,11 @@ extern "C" int gfc3dgpu_ctx_set_start(gfc3dgpu_ctx* c, const double* r, const do
   const long long m = 3LL * c->nc;
   if (m > 0) {
     if (r)
-      G2(cudaMemcpy(c->r, r, sizeof(double) * m, cudaMemcpyHostToDevice));
+      G2(cudaMemcpy(c->r[0], r, sizeof(double) * m, cudaMemcpyHostToDevice));
     else
-      G2(cudaMemset(c->r, 0, sizeof(double) * m));
+      G2(cudaMemset(c->r[0], 0, sizeof(double) * m));
   }
-  c->vcur = 0;
+  c->cur = 0;
   if (v)
     G2(cudaMemcpy(c->v[0], v, sizeof(double) * c->n, cudaMemcpyHostToDevice));
   else
@@ -993,11 +1027,12 @@ static Args args_of(gfc3dgpu_ctx* c) {
   a.tval = c->tval;
   a.b = c->b;
   a.mu = c->mu;
-  a.r = c->r;
-  a.u = c->u;
-  // the current velocity is v0 of the launch
-  a.v0 = c->v[c->vcur];
-  a.v1 = c->v[c->vcur ^ 1];
+  // the current iterate is buffer 0 of the launch
+  for (int k = 0; k < 2; k++) {
+    a.r[k] = c->r[c->cur ^ k];
+    a.u[k] = c->u[c->cur ^ k];
+    a.v[k] = c->v[c->cur ^ k];
+  }
   a.t = c->t;
   a.norm_q = c->norm_q;
   a.flags = c->flags;
@@ -1050,8 +1085,8 @@ extern "C" int gfc3dgpu_ctx_solve(gfc3dgpu_ctx* c, double tol, int max_iter, int
   float t = 0.f;
   const int rc = launch(c, a, out, &t);
   if (rc) return rc;
-  // v0 of the launch is buffer c->vcur; the result lies in v0 or v1
-  c->vcur ^= (int)out[3];
+  // buffer 0 of the launch is c->cur's; the result lies in buffer out[3]
+  c->cur ^= (int)out[3];
   if (iters) *iters = (int)out[0];
   if (error) *error = out[1];
   if (info) *info = (int)out[2];
@@ -1083,9 +1118,9 @@ extern "C" int gfc3dgpu_ctx_get(gfc3dgpu_ctx* c, double* r, double* u, double* v
   }
   G2(cudaSetDevice(c->device));
   const long long m = 3LL * c->nc;
-  if (r && m) G2(cudaMemcpy(r, c->r, sizeof(double) * m, cudaMemcpyDeviceToHost));
-  if (u && m) G2(cudaMemcpy(u, c->u, sizeof(double) * m, cudaMemcpyDeviceToHost));
-  if (v) G2(cudaMemcpy(v, c->v[c->vcur], sizeof(double) * c->n, cudaMemcpyDeviceToHost));
+  if (r && m) G2(cudaMemcpy(r, c->r[c->cur], sizeof(double) * m, cudaMemcpyDeviceToHost));
+  if (u && m) G2(cudaMemcpy(u, c->u[c->cur], sizeof(double) * m, cudaMemcpyDeviceToHost));
+  if (v) G2(cudaMemcpy(v, c->v[c->cur], sizeof(double) * c->n, cudaMemcpyDeviceToHost));
   return 0;
 }
 
