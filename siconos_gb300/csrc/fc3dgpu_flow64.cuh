@@ -22,24 +22,13 @@
 // error evaluation.
 #pragma once
 #include "fc3dgpu_coop64.cuh"
+#include "fc3dgpu_word128.cuh"
 
 namespace fc3dgpu {
 
 // Polls of a reaction before the back-off, and the back-off (ns).
 #define FC3D_FLOW64_SPIN 16
 #define FC3D_FLOW64_SLEEP_NS 100
-
-__device__ __forceinline__ void st_word128(double* p, unsigned long long lo, unsigned long long hi) {
-  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(lo),
-               "l"(hi)
-               : "memory");
-}
-__device__ __forceinline__ void ld_word128(const double* p, unsigned long long& lo, unsigned long long& hi) {
-  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
-               : "=l"(lo), "=l"(hi)
-               : "l"(p)
-               : "memory");
-}
 
 // A stamped reaction; false (x not set) before sweep `need` has written it.
 __device__ __forceinline__ bool ld_stamped64(const double* rs, int p, int need, double x[3]) {

@@ -4,9 +4,10 @@
 // row its blocks sorted by (original) column, the column stored permuted,
 // each a 5x5 column-major block; q, mu, mu_r, rho, r, u in permuted order.
 // One cooperative launch runs every sweep: a colour's contacts are spread
-// over the whole grid (five lanes a contact in FP64, one in FP32), a grid
-// barrier separates colours, and the
-// convergence logic runs on the device with the same bits in every block.
+// over the whole grid (five lanes a contact in FP64, one in FP32), a contact
+// waits for the reactions it reads (or, where the block pattern is not
+// symmetric, a grid barrier separates colours), and the convergence logic runs
+// on the device with the same bits in every block.
 // FP64 without FMA contraction, in the reference's operation order; in mixed
 // precision FP32 sweeps of the same loop run first and the FP64 loop starts
 // from their iterate.
@@ -23,6 +24,7 @@
 
 #include "rfc3dgpu.h"
 #include "rfc3dgpu_coop.cuh"
+#include "fc3dgpu_word128.cuh"
 
 extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 
@@ -34,6 +36,7 @@ constexpr int NT = 128;
 constexpr int MAXC = 128;
 constexpr int TRACE_CAP = 1 << 16;
 constexpr int MAX_BLOCKS = 1024;
+constexpr unsigned long long SPIN = 1ull << 22;  // polls of a dataflow wait
 
 // Kernel arguments; Real = double for the reference's loop, float for the
 // FP32 sweeps that precede it in mixed precision.
@@ -55,8 +58,13 @@ struct ArgsT {
   int local_max, max_iter;
   double* part;   // 2 slots x MAX_BLOCKS x 4 block partial sums
   double* trace;  // per-sweep light error, from trace[0]
-  double* out;    // [0] sweeps, [1] final error, [2] info, [3] last light error
+  double* out;    // [0] sweeps, [1] final error, [2] info (-1: a wait gave up), [3] last light error
   int trace_cap;  // entries of trace this launch may write
+  // dataflow sweeps: the reactions with the sweep that wrote them (null: by
+  // colours), contacts of a unit, polls of a wait
+  Real* rs;
+  int rows;
+  unsigned long long spin;
   // FP32 sweeps only: their stop rules on the light error
   double switch_tol;
   int stall_window;
@@ -415,7 +423,8 @@ struct Reduce {
 };
 
 // Sum of N values over the grid in a fixed order (warp tree, warps in
-// order, blocks in order): every block gets the same bits.  The partials go
+// order, blocks by lanes of one warp: one thread adding 152 blocks' values in
+// turn took 12 us): every block gets the same bits.  The partials go
 // through a two-slot ring in global memory: a block writes slot k & 1 only
 // after the barrier of call k - 1, which every block passes after reading
 // call k - 2's slot.  The barrier also orders all reaction updates before it.
@@ -430,21 +439,28 @@ __device__ void grid_sum(double v[N], const A& a, Reduce& R, cg::grid_group& g) 
   }
   __syncthreads();
   double* slot = a.part + (size_t)(R.calls & 1) * MAX_BLOCKS * 4;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < N; i++) {
-      double s = 0.0;
-      for (int k = 0; k < (int)(blockDim.x >> 5); k++) s += R.warp[k][i];
-      __stcg(&slot[4 * blockIdx.x + i], s);
-    }
+  if (threadIdx.x < N) {
+    double s = 0.0;
+    for (int k = 0; k < (int)(blockDim.x >> 5); k++) s += R.warp[k][threadIdx.x];
+    __stcg(&slot[4 * blockIdx.x + threadIdx.x], s);
   }
   grid_sync(g);
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < N; i++) {
-      double s = 0.0;
-      for (int b = 0; b < (int)gridDim.x; b++) s += __ldcg(&slot[4 * b + i]);
-      R.bcast[i] = s;
+  if (threadIdx.x < 32) {
+    double s[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) s[i] = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32)
+#pragma unroll
+      for (int i = 0; i < N; i++) s[i] += __ldcg(&slot[4 * b + i]);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < N; i++) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < N; i++) R.bcast[i] = s[i];
+      R.calls++;
     }
-    R.calls++;
   }
   __syncthreads();
 #pragma unroll
@@ -491,6 +507,35 @@ __device__ double full_error(const Args& a, Reduce& R, cg::grid_group& g) {
   return e;
 }
 
+// Contact p's new reaction rl (stored too) from its row sums s over the other
+// contacts, on one lane: the take-off shortcut or the one-contact Newton; v as
+// sweep_colours.
+template <typename Real>
+__device__ __forceinline__ void local_contact(const ArgsT<Real>& a, int p, const Real s[5], Real local_tol, double* v,
+                                              Real rl[5]) {
+  Real ql[5], old[5];
+  for (int i = 0; i < 5; i++) {
+    ql[i] = a.q[5 * (size_t)p + i] + s[i];
+    old[i] = __ldcg(&a.r[5 * (size_t)p + i]);
+    rl[i] = old[i];
+  }
+  if (ql[0] > -Eps<Real>::v()) {
+    for (int i = 0; i < 5; i++) rl[i] = Real(0.0);
+  } else {
+    Real M[25];
+    const Real* d = a.W + 25 * (size_t)(a.rp[p] + a.dpos[p]);
+    for (int i = 0; i < 25; i++) M[i] = __ldg(&d[i]);
+    local_nsn<Real>(M, ql, a.mu[p], a.mur[p], a.rho[p], rl, local_tol, a.local_max);
+  }
+  const Real d0 = old[0] - rl[0], d1 = old[1] - rl[1], d2 = old[2] - rl[2], d3 = old[3] - rl[3],
+             d4 = old[4] - rl[4];
+  v[0] += (double)(d0 * d0 + d1 * d1 + d2 * d2 + d3 * d3 + d4 * d4);
+  for (int i = 0; i < 5; i++) {
+    v[1] += (double)(rl[i] * rl[i]);
+    __stcg(&a.r[5 * (size_t)p + i], rl[i]);
+  }
+}
+
 // One sweep over the colours (rolling_friction_3d_nsgs.c:520-590 in colour
 // order): per contact q_loc = q_p + the row sums over the other contacts'
 // columns (in column order), the take-off shortcut or the one-contact
@@ -513,27 +558,8 @@ __device__ __forceinline__ void sweep_colours(const ArgsT<Real>& a, Real local_t
         for (int k = 0; k < 5; k++)
           for (int i = 0; i < 5; i++) s[i] += __ldg(&blk[i + 5 * k]) * x[k];
       }
-      Real ql[5], rl[5], old[5];
-      for (int i = 0; i < 5; i++) {
-        ql[i] = a.q[5 * (size_t)p + i] + s[i];
-        old[i] = __ldcg(&a.r[5 * (size_t)p + i]);
-        rl[i] = old[i];
-      }
-      if (ql[0] > -Eps<Real>::v()) {
-        for (int i = 0; i < 5; i++) rl[i] = Real(0.0);
-      } else {
-        Real M[25];
-        const Real* d = a.W + 25 * (size_t)(s0 + a.dpos[p]);
-        for (int i = 0; i < 25; i++) M[i] = __ldg(&d[i]);
-        local_nsn<Real>(M, ql, a.mu[p], a.mur[p], a.rho[p], rl, local_tol, a.local_max);
-      }
-      const Real d0 = old[0] - rl[0], d1 = old[1] - rl[1], d2 = old[2] - rl[2], d3 = old[3] - rl[3],
-                 d4 = old[4] - rl[4];
-      v[0] += (double)(d0 * d0 + d1 * d1 + d2 * d2 + d3 * d3 + d4 * d4);
-      for (int i = 0; i < 5; i++) {
-        v[1] += (double)(rl[i] * rl[i]);
-        __stcg(&a.r[5 * (size_t)p + i], rl[i]);
-      }
+      Real rl[5];
+      local_contact<Real>(a, p, s, local_tol, v, rl);
     }
     if (c + 1 < a.ncol) grid_sync(g);
   }
@@ -599,6 +625,210 @@ __device__ __forceinline__ void sweep_colours_coop(const Args& a, double local_t
   }
 }
 
+// ---- the sweeps as dataflow -------------------------------------------------
+// What bounds a sweep by colours: a colour takes as long as its slowest
+// contact (up to nine Newton iterations) however few need them, six contacts a
+// warp share the slowest one's control flow, and most SM quarters idle (1,000
+// contacts of a colour: 167 warps for 608 quarters).  Here a warp takes units
+// of one to six contacts and waits only for the reactions these read, each
+// stored with the number of the sweep that wrote it; no barrier inside a
+// sweep.  In a colour's order a contact reads the new reactions of lower
+// colours and the old ones of higher colours; the pattern is symmetric, so a
+// contact of a higher colour cannot write its new one before this contact has
+// written its own, and a stamp at least the one needed is the one needed.
+// us a sweep by colours and as dataflow, copies of the 21-contact rockfall
+// problem:
+//   FP64: 21 contacts 161, 130   2,100: 259, 216   21,000: 507, 401
+//   FP32: 21 contacts 82, 59     2,100: 130, 104   21,000: 147, 139
+
+// Polls of a reaction before the back-off, and the back-off (ns).
+#define RFC3D_FLOW_SPIN 16
+#define RFC3D_FLOW_SLEEP_NS 100
+
+// Component i of reaction p and its stamp: one 128-bit word in FP64.
+__device__ __forceinline__ void st_stamped(double* rs, int p, int i, double x, int stamp) {
+  fc3dgpu::st_word128(rs + 2 * (5 * (size_t)p + i), (unsigned long long)__double_as_longlong(x),
+                      (unsigned long long)(unsigned)stamp);
+}
+__device__ __forceinline__ bool ld_stamped(const double* rs, int p, int need, double x[5]) {
+  unsigned long long lo[5], hi[5];
+#pragma unroll
+  for (int i = 0; i < 5; i++) fc3dgpu::ld_word128(rs + 2 * (5 * (size_t)p + i), lo[i], hi[i]);
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < 5; i++) {
+    x[i] = __longlong_as_double((long long)lo[i]);
+    ok = ok && (int)hi[i] >= need;
+  }
+  return ok;
+}
+// In FP32 two words: components 0-2 and 3-4, each with the stamp.
+__device__ __forceinline__ void st_all_stamped(float* rs, int p, const float x[5], int stamp) {
+  auto pack = [](float lo, float hi) {
+    return (unsigned long long)__float_as_uint(lo) | (unsigned long long)__float_as_uint(hi) << 32;
+  };
+  const float s = __int_as_float(stamp);
+  fc3dgpu::st_word128(rs + 8 * (size_t)p, pack(x[0], x[1]), pack(x[2], s));
+  fc3dgpu::st_word128(rs + 8 * (size_t)p + 4, pack(x[3], x[4]), pack(0.f, s));
+}
+__device__ __forceinline__ bool ld_stamped(const float* rs, int p, int need, float x[5]) {
+  unsigned long long a, b, c, d;
+  fc3dgpu::ld_word128(rs + 8 * (size_t)p, a, b);
+  fc3dgpu::ld_word128(rs + 8 * (size_t)p + 4, c, d);
+  x[0] = __uint_as_float((unsigned)a);
+  x[1] = __uint_as_float((unsigned)(a >> 32));
+  x[2] = __uint_as_float((unsigned)b);
+  x[3] = __uint_as_float((unsigned)c);
+  x[4] = __uint_as_float((unsigned)(c >> 32));
+  return (int)(b >> 32) >= need && (int)(d >> 32) >= need;
+}
+__device__ __forceinline__ void st_all_stamped(double* rs, int p, const double x[5], int stamp) {
+#pragma unroll
+  for (int i = 0; i < 5; i++) st_stamped(rs, p, i, x[i], stamp);
+}
+
+// The reactions x[t] of the contacts j[t] as row p reads them in `sweep`
+// (j < 0: none); false when the wait gave up.
+template <typename Real, int CH>
+__device__ __forceinline__ bool wait_reactions(const ArgsT<Real>& a, const int (&j)[CH], int p, int sweep,
+                                               Real (&x)[CH][5]) {
+  unsigned late = 0;
+#pragma unroll
+  for (int t = 0; t < CH; t++)
+    if (j[t] >= 0) late |= (ld_stamped(a.rs, j[t], sweep - (j[t] > p ? 1 : 0), x[t]) ? 0u : 1u) << t;
+  for (unsigned long long n = 0; late; n++) {
+    if (n > a.spin) return false;
+    if (n > RFC3D_FLOW_SPIN) __nanosleep(RFC3D_FLOW_SLEEP_NS);
+#pragma unroll
+    for (int t = 0; t < CH; t++)
+      if ((late >> t & 1u) && ld_stamped(a.rs, j[t], sweep - (j[t] > p ? 1 : 0), x[t])) late &= ~(1u << t);
+  }
+  return true;
+}
+
+// Contacts [first, first + n) of a colour, five lanes each.  v[2] counts
+// waits that gave up (the sweep goes on, so that every block gets to the
+// barrier at its end).
+__device__ __forceinline__ void flow_unit(const Args& a, int first, int n, int sweep, double local_tol, double v[3]) {
+  const int lane = threadIdx.x & 31;
+  const bool spare = lane >= 5 * RFC3D_COOP_GROUPS;
+  RLane c;
+  const int grp = spare ? 0 : lane / 5;
+  c.base = 5 * grp;
+  c.i = lane - (spare ? 5 * RFC3D_COOP_GROUPS : c.base);
+  // groups without a contact repeat the first one without storing it
+  const bool have = !spare && grp < n;
+  const int p = have ? first + grp : first;
+  const int s0 = a.rp[p], len = a.rp[p + 1] - s0;
+  const int longest = __reduce_max_sync(0xffffffffu, len);
+  RProblem P;
+  const double* d = a.W + 25 * (size_t)(s0 + a.dpos[p]);
+#pragma unroll
+  for (int e = 0; e < 25; e++) P.M[e] = __ldg(&d[e]);
+  P.mu = a.mu[p];
+  P.mur = a.mur[p];
+  P.rho = a.rho[p];
+  const double q = a.q[5 * (size_t)p + c.i], old = __ldcg(&a.r[5 * (size_t)p + c.i]);
+  double s = 0.0;
+  bool ok = true;
+  constexpr int CH = 2;
+  for (int t0 = 0; t0 < longest; t0 += CH) {
+    int j[CH];
+    double w[CH][5], x[CH][5];
+#pragma unroll
+    for (int t = 0; t < CH; t++) {
+      const int sl = s0 + (t0 + t < len ? t0 + t : 0);
+      const int col = __ldg(&a.col[sl]);
+      j[t] = t0 + t < len && col != p ? col : -1;
+      const double* blk = a.W + 25 * (size_t)sl + c.i;
+#pragma unroll
+      for (int k = 0; k < 5; k++) w[t][k] = __ldg(&blk[5 * k]);
+    }
+    ok = wait_reactions<double, CH>(a, j, p, sweep, x) && ok;
+#pragma unroll
+    for (int t = 0; t < CH; t++)
+      if (j[t] >= 0)
+#pragma unroll
+        for (int k = 0; k < 5; k++) s += w[t][k] * x[t][k];
+  }
+  __syncwarp();
+  P.q = q + s;
+  const bool off = ie_lt(-DBL_EPSILON, rget(P.q, c.base));  // take-off
+  double rl = old;
+  if (rany(have && !off)) rlocal_solve(c, P, have && !off, DBL_EPSILON, local_tol, a.local_max, rl);
+  if (off) rl = 0.0;
+  if (have) {
+    st_stamped(a.rs, p, c.i, rl, sweep);
+    __stcg(&a.r[5 * (size_t)p + c.i], rl);
+  }
+  const double dr = old - rl;
+  const double d2 = rsum(c, dr * dr);
+  const double r2 = rsum(c, rl * rl);
+  if (have && c.i == 0) {
+    v[0] += d2;
+    v[1] += r2;
+  }
+  if (!ok) v[2] += 1.0;
+}
+
+// Contacts [first, first + n) of a colour, one lane each, in FP32
+__device__ __forceinline__ void flow_unit(const ArgsT<float>& a, int first, int n, int sweep, float local_tol,
+                                          double v[3]) {
+  const int lane = threadIdx.x & 31;
+  const bool have = lane < n;
+  const int p = first + (have ? lane : 0), s0 = a.rp[p], len = have ? a.rp[p + 1] - s0 : 0;
+  const int longest = __reduce_max_sync(0xffffffffu, len);
+  float s[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int t = 0; t < longest; t++) {
+    const int col = t < len ? a.col[s0 + t] : p;
+    const int j[1] = {col != p ? col : -1};
+    float x[1][5];
+    if (!wait_reactions<float, 1>(a, j, p, sweep, x)) v[2] += 1.0;
+    __syncwarp();  // the lanes left the wait one by one: together again
+    if (j[0] < 0) continue;
+    const float* blk = a.W + 25 * (size_t)(s0 + t);
+    for (int k = 0; k < 5; k++)
+      for (int i = 0; i < 5; i++) s[i] += __ldg(&blk[i + 5 * k]) * x[0][k];
+  }
+  __syncwarp();
+  if (have) {
+    float rl[5];
+    local_contact<float>(a, p, s, local_tol, v, rl);
+    st_all_stamped(a.rs, p, rl, sweep);
+  }
+  __syncwarp();
+}
+
+// One sweep: unit u of a colour goes to block u mod the grid, a block's units
+// in colour order to its warps in turn.
+template <typename Real, typename Unit>
+__device__ __forceinline__ void flow_sweep(const ArgsT<Real>& a, const Unit& unit) {
+  const int nw = blockDim.x >> 5, size = gridDim.x, rank = blockIdx.x;
+  int e = threadIdx.x >> 5;  // the warp's next unit among the block's
+  for (int c = 0; c < a.ncol; c++) {
+    const int p0 = a.cptr[c], n = a.cptr[c + 1] - p0, units = (n + a.rows - 1) / a.rows;
+    const int mine = rank < units ? (units - rank + size - 1) / size : 0;
+    for (; e < mine; e += nw) {
+      const int l = (rank + e * size) * a.rows;
+      unit(p0 + l, min(a.rows, n - l));
+    }
+    e -= mine;
+  }
+}
+
+// The start's reactions with sweep 0's stamp
+template <typename Real>
+__device__ __forceinline__ void flow_start(const ArgsT<Real>& a, cg::grid_group& g) {
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.nc; p += gridDim.x * blockDim.x) {
+    Real x[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) x[i] = __ldcg(&a.r[5 * (size_t)p + i]);
+    st_all_stamped(a.rs, p, x, 0);
+  }
+  grid_sync(g);
+}
+
+template <bool FLOW>
 __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
   __shared__ Reduce R;
   cg::grid_group g = cg::this_grid();
@@ -608,11 +838,21 @@ __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
   double tolerance = a.tol, err = 1., local_tol = a.local_tol;
   int iter = 0, not_conv = 1;
+  if (FLOW) flow_start(a, g);
   while (iter < a.max_iter && not_conv) {
     ++iter;
-    double v[2] = {0.0, 0.0};
-    sweep_colours_coop(a, local_tol, v, g);
-    grid_sum<2>(v, a, R, g);
+    double v[3] = {0.0, 0.0, 0.0};
+    if constexpr (FLOW) {
+      flow_sweep(a, [&](int first, int n) { flow_unit(a, first, n, iter, local_tol, v); });
+      grid_sum<3>(v, a, R, g);
+      if (v[2] != 0.0) {
+        if (lead) a.out[2] = -1.0;
+        return;
+      }
+    } else {
+      sweep_colours_coop(a, local_tol, v, g);
+      grid_sum<2>(v, a, R, g);
+    }
     err = sqrt(v[0]);
     const double nr = sqrt(v[1]);
     if (fabs(nr) > DBL_EPSILON) err /= nr;
@@ -647,6 +887,7 @@ __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
 // light error drops below switch_tol, makes no 1 % progress for
 // stall_window sweeps, turns non-finite (out[2] = 1) or the budget ends.
 // The FP64 loop then starts from their iterate.
+template <bool FLOW>
 __global__ void __launch_bounds__(NT) k_rfc3d_sweeps32(const ArgsT<float> a) {
   __shared__ Reduce R;
   cg::grid_group g = cg::this_grid();
@@ -656,11 +897,21 @@ __global__ void __launch_bounds__(NT) k_rfc3d_sweeps32(const ArgsT<float> a) {
   double err = INFINITY, best = INFINITY;
   int iter = 0, best_iter = 0;
   bool finite = true;
+  if (FLOW) flow_start(a, g);
   while (iter < a.max_iter) {
     ++iter;
-    double v[2] = {0.0, 0.0};
-    sweep_colours<float>(a, (float)a.local_tol, v, g);
-    grid_sum<2>(v, a, R, g);
+    double v[3] = {0.0, 0.0, 0.0};
+    if constexpr (FLOW) {
+      flow_sweep(a, [&](int first, int n) { flow_unit(a, first, n, iter, (float)a.local_tol, v); });
+      grid_sum<3>(v, a, R, g);
+      if (v[2] != 0.0) {
+        if (lead) a.out[2] = -1.0;
+        return;
+      }
+    } else {
+      sweep_colours<float>(a, (float)a.local_tol, v, g);
+      grid_sum<2>(v, a, R, g);
+    }
     err = sqrt(v[0]);
     const double nr = sqrt(v[1]);
     if (fabs(nr) > DBL_EPSILON) err /= nr;
@@ -756,14 +1007,17 @@ struct rfc3dgpu_ctx {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
   int nc = 0, ncol = 0, max_colour = 0, blocks = 1, threads = NT, blocks32 = 1, threads32 = NT;
+  int rows = 0, rows32 = 0;  // contacts of a unit of the dataflow sweeps (0: sweeps by colours)
   double norm_q = 0.0;
   std::vector<int> perm, iperm, colour;
   std::vector<double> rho_host;
   int *cptr = nullptr, *rp = nullptr, *col = nullptr, *dpos = nullptr;
-  double *W = nullptr, *q = nullptr, *mu = nullptr, *mur = nullptr, *rho = nullptr, *r = nullptr, *u = nullptr,
+  double *W = nullptr, *q = nullptr, *mu = nullptr, *mur = nullptr, *rho = nullptr, *r = nullptr, *rs = nullptr,
+         *u = nullptr,
          *part = nullptr, *trace = nullptr, *out = nullptr;
   // FP32 copies for the FP32 sweeps of mixed precision
-  float *W32 = nullptr, *q32 = nullptr, *mu32 = nullptr, *mur32 = nullptr, *rho32 = nullptr, *r32 = nullptr;
+  float *W32 = nullptr, *q32 = nullptr, *mu32 = nullptr, *mur32 = nullptr, *rho32 = nullptr, *r32 = nullptr,
+        *rs32 = nullptr;
   int trace_len = 0;
   // 1: FP64 sweeps only (default); 0: FP32 sweeps, then the FP64 loop
   int precision = 1;
@@ -787,12 +1041,12 @@ static const double LOCAL_TOL32 = 1e-6;
 
 static void free_problem(rfc3dgpu_ctx* c) {
   void* ptrs[] = {c->cptr, c->rp,  c->col, c->dpos, c->W,   c->q,    c->mu,    c->mur,   c->rho,
-                  c->r,    c->u,   c->W32, c->q32,  c->mu32, c->mur32, c->rho32, c->r32};
+                  c->r,    c->rs,  c->u,   c->W32, c->q32,  c->mu32, c->mur32, c->rho32, c->r32, c->rs32};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   c->cptr = c->rp = c->col = c->dpos = nullptr;
-  c->W = c->q = c->mu = c->mur = c->rho = c->r = c->u = nullptr;
-  c->W32 = c->q32 = c->mu32 = c->mur32 = c->rho32 = c->r32 = nullptr;
+  c->W = c->q = c->mu = c->mur = c->rho = c->r = c->rs = c->u = nullptr;
+  c->W32 = c->q32 = c->mu32 = c->mur32 = c->rho32 = c->r32 = c->rs32 = nullptr;
   c->nc = 0;
 }
 
@@ -907,6 +1161,7 @@ extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* 
   for (int i = 0; i < nc; i++) cptr[colour[i] + 1]++;
   for (int k = 0; k < ncol; k++) cptr[k + 1] += cptr[k];
   std::vector<int> rp(nc + 1, 0), col((size_t)nnzb), dpos(nc);
+  std::vector<int64_t> ocol((size_t)nnzb);  // the slots' original columns, ascending in a row
   std::vector<double> W((size_t)nnzb * 25), qp(5 * (size_t)nc), mup(nc), murp(nc), rhop(nc);
   c->rho_host.assign(nc, 0.0);
   std::vector<int64_t> order;
@@ -923,6 +1178,7 @@ extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* 
       const int64_t k = order[t];
       const int s = rp[p] + (int)t;
       col[s] = c->iperm[colidx[k]];
+      ocol[s] = colidx[k];
       memcpy(&W[25 * (size_t)s], &blocks[25 * k], 25 * sizeof(double));
       if (colidx[k] == i && dpos[p] < 0) dpos[p] = (int)t;
     }
@@ -932,6 +1188,10 @@ extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* 
     mup[p] = mu[i];
     murp[p] = mur[i];
   }
+  bool symmetric = true;
+  for (int p = 0; p < nc && symmetric; p++)
+    for (int s = rp[p]; s < rp[p + 1] && symmetric; s++)
+      symmetric = std::binary_search(ocol.begin() + rp[col[s]], ocol.begin() + rp[col[s] + 1], (int64_t)c->perm[p]);
   double s2 = 0.0;
   for (int64_t k = 0; k < 5LL * nc; k++) s2 += q[k] * q[k];
   c->norm_q = sqrt(s2);
@@ -947,6 +1207,7 @@ extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* 
   if (e == cudaSuccess) e = upload(&c->mur, murp);
   if (e == cudaSuccess) e = upload(&c->rho, rhop);
   if (e == cudaSuccess) e = upload(&c->r, zero);
+  if (e == cudaSuccess && symmetric) e = cudaMalloc((void**)&c->rs, sizeof(double) * 10 * (size_t)nc);
   if (e == cudaSuccess) e = upload(&c->u, zero);
   {
     auto f32 = [](const std::vector<double>& v) { return std::vector<float>(v.begin(), v.end()); };
@@ -956,6 +1217,7 @@ extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* 
     if (e == cudaSuccess) e = upload(&c->mur32, f32(murp));
     if (e == cudaSuccess) e = upload(&c->rho32, f32(rhop));
     if (e == cudaSuccess) e = upload(&c->r32, f32(zero));
+    if (e == cudaSuccess && symmetric) e = cudaMalloc((void**)&c->rs32, sizeof(float) * 8 * (size_t)nc);
   }
   if (e != cudaSuccess) {
     free_problem(c);
@@ -981,8 +1243,25 @@ extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* 
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
     blocks = std::max(1, std::min(blocks_of(threads), std::max(1, std::min(per_sm * sms, MAX_BLOCKS))));
   };
-  shape((const void*)k_rfc3d_nsgs, RFC3D_COOP_GROUPS, c->threads, c->blocks);
-  shape((const void*)k_rfc3d_sweeps32, 32, c->threads32, c->blocks32);
+  // dataflow: a unit of an average colour for every SM quarter, four warps a
+  // block, enough blocks for the largest colour's units
+  auto flow_shape = [&](const void* kernel, int most, int& rows, int& threads, int& blocks) {
+    const long long quarters = 4LL * ncol * sms;
+    rows = (int)std::min<long long>(most, std::max(1LL, (nc + quarters - 1) / quarters));
+    threads = NT;
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, NT, 0);
+    const int units = (c->max_colour + rows - 1) / rows;
+    blocks = std::max(1, std::min((units + 3) / 4, std::min(std::max(1, per_sm) * sms, MAX_BLOCKS)));
+  };
+  c->rows = c->rows32 = 0;
+  if (symmetric) {
+    flow_shape((const void*)k_rfc3d_nsgs<true>, RFC3D_COOP_GROUPS, c->rows, c->threads, c->blocks);
+    flow_shape((const void*)k_rfc3d_sweeps32<true>, 32, c->rows32, c->threads32, c->blocks32);
+  } else {
+    shape((const void*)k_rfc3d_nsgs<false>, RFC3D_COOP_GROUPS, c->threads, c->blocks);
+    shape((const void*)k_rfc3d_sweeps32<false>, 32, c->threads32, c->blocks32);
+  }
   return 0;
 }
 
@@ -1011,6 +1290,9 @@ static Args args_of(const rfc3dgpu_ctx* c) {
   a.mur = c->mur;
   a.rho = c->rho;
   a.r = c->r;
+  a.rs = c->rs;
+  a.rows = c->rows;
+  a.spin = SPIN;
   a.u = c->u;
   a.norm_q = c->norm_q;
   a.part = c->part;
@@ -1035,6 +1317,9 @@ static ArgsT<float> args32_of(const rfc3dgpu_ctx* c) {
   a.mur = c->mur32;
   a.rho = c->rho32;
   a.r = c->r32;
+  a.rs = c->rs32;
+  a.rows = c->rows32;
+  a.spin = SPIN;
   a.u = c->u;
   a.norm_q = c->norm_q;
   a.part = c->part;
@@ -1071,9 +1356,14 @@ extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, dou
     a.stall_window = c->stall;
     k_rfc3d_to_f32<<<(n5 + 255) / 256, 256, 0, c->stream>>>(n5, c->r, c->r32);
     KR(cudaGetLastError());
-    KR(launch(c, k_rfc3d_sweeps32, a, c->blocks32, c->threads32));
+    KR(c->rows32 ? launch(c, k_rfc3d_sweeps32<true>, a, c->blocks32, c->threads32)
+                 : launch(c, k_rfc3d_sweeps32<false>, a, c->blocks32, c->threads32));
     KR(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
     KR(cudaStreamSynchronize(c->stream));
+    if (out[2] < 0.0) {
+      fc3dgpu_set_error("rfc3dgpu_ctx_solve: a wait for a reaction reached its poll limit");
+      return NUMERICS_ERR_UNKNOWN;
+    }
     sweeps32 = (int)out[0];
     // a non-finite FP32 iterate is dropped: the FP64 loop starts where the
     // FP32 sweeps did
@@ -1089,10 +1379,15 @@ extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, dou
   a.local_max = local_max_iter;
   a.trace = c->trace + std::min(sweeps32, TRACE_CAP);
   a.trace_cap = TRACE_CAP - std::min(sweeps32, TRACE_CAP);
-  KR(launch(c, k_rfc3d_nsgs, a, c->blocks, c->threads));
+  KR(c->rows ? launch(c, k_rfc3d_nsgs<true>, a, c->blocks, c->threads)
+             : launch(c, k_rfc3d_nsgs<false>, a, c->blocks, c->threads));
   KR(cudaEventRecord(c->ev[1], c->stream));
   KR(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
   KR(cudaStreamSynchronize(c->stream));
+  if (out[2] < 0.0) {
+    fc3dgpu_set_error("rfc3dgpu_ctx_solve: a wait for a reaction reached its poll limit");
+    return NUMERICS_ERR_UNKNOWN;
+  }
   float t = 0.f;
   cudaEventElapsedTime(&t, c->ev[0], c->ev[1]);
   c->sweeps32 = sweeps32;

@@ -11,11 +11,11 @@
 // roots and comparisons run on the integer pipes, the point an iteration ends
 // at is the one the next starts from, and products with the structural zeros
 // of the velocity matrix (which can only change the sign of a zero) are left
-// out.  FP64 sweep, one lane -> five lanes a contact, copies of the rockfall
-// problem: 547 -> 161 us at 21 contacts, 892 -> 259 at 2,100, 1,015 -> 507 at
-// 21,000, 3,898 -> 3,009 at 210,000.  The FP32 sweeps stay on one lane: the
-// exchanges cost what they save there (83 and 86 us at 21 contacts, 147 and
-// 224 at 21,000).
+// out.  FP64 sweep by colours, one lane -> five lanes a contact, copies of
+// the rockfall problem: 547 -> 161 us at 21 contacts, 892 -> 259 at 2,100,
+// 1,015 -> 507 at 21,000, 3,898 -> 3,009 at 210,000.  The FP32 sweeps stay on
+// one lane: the exchanges cost what they save there (83 and 86 us at 21
+// contacts, 147 and 224 at 21,000).
 //
 // The control flow is the same for the whole warp: loops run until its last
 // contact is done, finished contacts keep their values, and the collectives
