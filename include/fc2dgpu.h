@@ -105,7 +105,8 @@ int fc2dgpu_ctx_colours(fc2dgpu_ctx *ctx, int32_t *colour);
  * cluster_blocks blocks (1..16; -1: a cooperative grid over every SM) of
  * `threads` threads (32..512, a multiple of 32), the reactions kept in HBM
  * (reactions = 1) or replicated in every cluster block's shared memory (2,
- * up to 13,312 contacts); 0 picks each from the problem (the default).
+ * up to 13,312 contacts); 0 picks each from the problem (the default; then
+ * larger problems on a symmetric pattern sweep as dataflow on a grid).
  * fc2dgpu_ctx_launch_shape reports a grid as minus its block count.  The
  * iterates do not depend on the shape; the reduction order of the errors
  * does. */

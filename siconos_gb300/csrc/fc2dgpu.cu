@@ -3,8 +3,9 @@
 // Layout: contacts permuted by colour (stable in contact order); per permuted
 // row its blocks in the caller's order (diagonal included, at dpos), each a
 // 2x2 column-major block, with the permuted column index; q, mu, r, u in
-// permuted order.  One thread-block cluster per problem, or a cooperative
-// grid over every SM when a colour is larger than a cluster (k_fc2d_nsgs).
+// permuted order.  One thread-block cluster per problem, or, for larger
+// colours, a cooperative grid over every SM, as dataflow where the block
+// pattern is symmetric (k_fc2d_nsgs).
 // FP64 without FMA contraction, in the reference's operation order.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -15,10 +16,12 @@
 
 #include <algorithm>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "fc2dgpu.h"
 #include "fc3dgpu_ieee64.cuh"
+#include "fc3dgpu_word128.cuh"
 
 extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 
@@ -32,6 +35,8 @@ constexpr int MAXC = 128;
 constexpr int TRACE_CAP = 1 << 16;
 constexpr size_t REP_MAX_BYTES = 208 * 1024;  // shared-memory copy of the reactions at most
 constexpr int GRID_MAX = 1024;                 // blocks of a cooperative grid at most
+constexpr int FLAG_STRIDE = 8;                 // words between the dataflow blocks' barrier flags
+constexpr unsigned long long SPIN = 1ull << 22;  // polls of a dataflow wait
 
 template <typename T>
 struct Vec2;
@@ -78,6 +83,12 @@ struct Args {
   int stall;              // FP32 phase: stop after this many sweeps without a new lowest error
   const double* before;   // out[] of the phase run before this one (or null)
   double* part;           // grid team: 2 x GRID_MAX x 4 block partial sums
+  // dataflow: the reactions with the sweep that wrote them, contacts of a
+  // unit, the blocks' barrier flags, where a wait that gave up is told
+  T* rs;
+  int rows;
+  unsigned* flags;
+  double* fail;
   double* trace;
   double* out;  // [0] sweeps, [1] final error, [2] info, [3] last light error
 };
@@ -87,9 +98,10 @@ struct Args {
 // shared memory.  A cooperative grid (every SM, for colours too large for a
 // cluster): grid barrier, partial sums through a ring in global memory.
 struct ClusterTeam {
-  static constexpr bool grid = false;
+  static constexpr bool grid = false, flow = false;
   cg::cluster_group cl;
-  __device__ ClusterTeam() : cl(cg::this_cluster()) {}
+  template <typename T>
+  __device__ explicit ClusterTeam(const Args<T>&) : cl(cg::this_cluster()) {}
   __device__ __forceinline__ int rank() const { return (int)cl.block_rank(); }
   __device__ __forceinline__ int size() const { return (int)cl.num_blocks(); }
   // barrier between colours: the hardware cluster barrier (about 670 cycles
@@ -114,9 +126,10 @@ struct ClusterTeam {
 };
 
 struct GridTeam {
-  static constexpr bool grid = true;
+  static constexpr bool grid = true, flow = false;
   cg::grid_group g;
-  __device__ GridTeam() : g(cg::this_grid()) {}
+  template <typename T>
+  __device__ explicit GridTeam(const Args<T>&) : g(cg::this_grid()) {}
   __device__ __forceinline__ int rank() const { return (int)blockIdx.x; }
   __device__ __forceinline__ int size() const { return (int)gridDim.x; }
   __device__ __forceinline__ void sync() {
@@ -128,6 +141,54 @@ struct GridTeam {
   __device__ __forceinline__ void sync_all() { sync(); }
   __device__ __forceinline__ void arrive() {}
   __device__ __forceinline__ void wait() { sync(); }
+};
+
+// A cooperative grid whose sweeps are dataflow: a barrier of flags (the sums
+// of a sweep pass one) whose waits, like those for reactions, end after SPIN
+// polls; `dead` (the same in the whole block) then ends the solve.
+struct FlowTeam {
+  static constexpr bool grid = true, flow = true;
+  unsigned* flags;
+  double* fail;
+  unsigned epoch = 0;
+  bool dead = false;
+  template <typename T>
+  __device__ explicit FlowTeam(const Args<T>& a) : flags(a.flags), fail(a.fail) {}
+  __device__ __forceinline__ int rank() const { return (int)blockIdx.x; }
+  __device__ __forceinline__ int size() const { return (int)gridDim.x; }
+  __device__ __forceinline__ void give_up() {
+    *(volatile double*)fail = 1.0;
+    dead = true;
+  }
+  __device__ __forceinline__ void sync() {
+    epoch++;
+    bool ok = true;
+    __syncthreads();
+    if (threadIdx.x < 32 && !dead && gridDim.x > 1) {
+      const int lane = threadIdx.x;
+      if (lane == 0)
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&flags[blockIdx.x * FLAG_STRIDE]), "r"(epoch)
+                     : "memory");
+      for (unsigned long long n = 0;; n++) {
+        bool all = true;
+#pragma unroll 8
+        for (int b = lane; b < (int)gridDim.x; b += 32) {
+          unsigned f;
+          asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(&flags[b * FLAG_STRIDE]) : "memory");
+          all &= f >= epoch;
+        }
+        if (__all_sync(0xffffffffu, all)) break;
+        if (n > SPIN) {
+          ok = false;
+          break;
+        }
+        if (n > 256) __nanosleep(32);
+      }
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    if (__syncthreads_or(!ok)) give_up();
+  }
+  __device__ __forceinline__ void sync_all() { sync(); }
 };
 
 // Where the sweep keeps the reactions.  HBM: read past L1 (ld.global.cg)
@@ -146,6 +207,14 @@ struct Reactions {
     if (REP) return rs[j];
     return __ldcg(reinterpret_cast<const V*>(rw) + j);
   }
+  // the reactions of a row's next slots (column -1: none)
+  template <int N>
+  __device__ __forceinline__ void gather(const int (&col)[N], int, V (&r)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      if (col[i] >= 0) r[i] = get(col[i]);
+  }
+  __device__ __forceinline__ bool any(bool more) const { return more; }
   template <typename Team>
   __device__ __forceinline__ void put(int j, T x0, T x1, Team& t) const {
     V v;
@@ -158,18 +227,17 @@ struct Reactions {
       __stcg(reinterpret_cast<V*>(rw) + j, v);
     }
   }
-};
-
-// Component `comp` alone of reaction j
-template <bool REP, typename Team>
-__device__ __forceinline__ void put_component(const Reactions<double, REP>& rx, int j, int comp, double x, Team& t) {
-  if constexpr (REP && !Team::grid) {
-    const int cs = t.size();
-    for (int k = 0; k < cs; k++) reinterpret_cast<double*>(t.cl.map_shared_rank(rx.rs, k))[2 * j + comp] = x;
-  } else {
-    __stcg(rx.rw + 2 * (size_t)j + comp, x);
+  // component `comp` alone
+  template <typename Team>
+  __device__ __forceinline__ void put_component(int j, int comp, T x, Team& t) const {
+    if constexpr (REP && !Team::grid) {
+      const int cs = t.size();
+      for (int k = 0; k < cs; k++) reinterpret_cast<T*>(t.cl.map_shared_rank(rs, k))[2 * j + comp] = x;
+    } else {
+      __stcg(rw + 2 * (size_t)j + comp, x);
+    }
   }
-}
+};
 
 // Team-wide sum of N values per thread, in a fixed order (xor-shuffle tree
 // in each warp, the warps in order, then the blocks in rank order), so every
@@ -229,6 +297,48 @@ __device__ __forceinline__ void team_sum2(double v[2], Reduce<double>& R, Team& 
   __syncthreads();
   v[0] = R.bcast[0];
   v[1] = R.bcast[1];
+  __syncthreads();
+}
+
+// The sum of N values over the dataflow grid, each step a tree.
+template <int N, typename T>
+__device__ __forceinline__ void flow_sum(T v[N], Reduce<T>& R, FlowTeam& team, double* gpart) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  auto tree = [&](T x) {
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    const T x = tree(v[i]);
+    if (lane == 0) R.warp[w][i] = x;
+  }
+  __syncthreads();
+  double* gslot = gpart + (size_t)(R.calls & 1) * GRID_MAX * 4;
+  if (threadIdx.x < N) {
+    T x = 0;
+    for (int k = 0; k < nw; k++) x += R.warp[k][threadIdx.x];
+    __stcg(&gslot[4 * blockIdx.x + threadIdx.x], (double)x);
+  }
+  team.sync();
+  if (w == 0) {
+    T x[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) x[i] = 0;
+    for (int b = lane; b < (int)gridDim.x; b += 32)
+#pragma unroll
+      for (int i = 0; i < N; i++) x[i] += (T)__ldcg(&gslot[4 * b + i]);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      x[i] = tree(x[i]);
+      if (lane == 0) R.bcast[i] = x[i];
+    }
+    if (lane == 0) R.calls++;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < N; i++) v[i] = R.bcast[i];
   __syncthreads();
 }
 
@@ -426,17 +536,15 @@ __device__ __forceinline__ void load_row(const Args<T>& a, int c, int k, int com
 // A contact of the FP32 sweep on one lane: its neighbours' reactions are
 // fetched together, then the products run in the row's order
 // (SBM_row_prod_no_diag_2x2: every block on the diagonal is left out).
-template <bool REP, typename Team>
-__device__ __forceinline__ void contact32(const Args<float>& a, const Reactions<float, REP>& rx, int k, Row<float>& x,
-                                          float& x0, float& x1, float P[2], Team& team) {
+template <typename RX, typename Team>
+__device__ __forceinline__ void contact32(const Args<float>& a, RX& rx, int k, bool act, Row<float>& x, float& x0,
+                                          float& x1, float P[2], Team& team) {
   const int p = x.p;
   const float2 old = rx.get(p);
   float ql[2] = {x.q.x, x.q.y};
   for (int t0 = 0;; t0 += FC2D_NB) {
     float2 r[FC2D_NB];
-#pragma unroll
-    for (int i = 0; i < FC2D_NB; i++)
-      if (x.col[i] >= 0) r[i] = rx.get(x.col[i]);
+    rx.gather(x.col, p, r);
 #pragma unroll
     for (int i = 0; i < FC2D_NB; i++)
       if (x.col[i] >= 0) {
@@ -445,7 +553,7 @@ __device__ __forceinline__ void contact32(const Args<float>& a, const Reactions<
         ql[0] += x.w[i].y * r[i].y;
         ql[1] += x.w[i].w * r[i].y;
       }
-    if (t0 + FC2D_NB >= x.slots) break;
+    if (!rx.any(t0 + FC2D_NB < x.slots)) break;
     load_slots(a, x, t0 + FC2D_NB, k & 31, 0);
   }
   const float W[4] = {x.d.x, x.d.y, x.d.z, x.d.w};
@@ -454,7 +562,7 @@ __device__ __forceinline__ void contact32(const Args<float>& a, const Reactions<
   local_solve<float>(W, x.det, ql, x.mu, P);
   x0 = old.x - P[0];
   x1 = old.y - P[1];
-  rx.put(p, P[0], P[1], team);
+  if (act) rx.put(p, P[0], P[1], team);
 }
 
 // A contact of the FP64 sweep on two lanes, one component each.  The sweep
@@ -463,33 +571,38 @@ __device__ __forceinline__ void contact32(const Args<float>& a, const Reactions<
 // the local solve run side by side; divisions and comparisons are the integer
 // forms of fc3dgpu_ieee64.cuh.  The bits are local_solve's.  Every lane of the
 // warp calls it; `act` false stores nothing.
-template <bool REP, typename Team>
-__device__ __forceinline__ void contact64(const Args<double>& a, const Reactions<double, REP>& rx, int k, int comp,
-                                          bool act, Row<double>& x, double& dx, double& pn, Team& team) {
+template <typename RX, typename Team>
+__device__ __forceinline__ void contact64(const Args<double>& a, RX& rx, int k, int comp, bool act,
+                                          Row<double>& x, double& dx, double& pn, Team& team) {
   using namespace fc3dgpu;
   const int p = x.p;
   const double2 o = rx.get(p);
   const double old = comp ? o.y : o.x;
+  double2 n, t;  // Wnn, Wtn; Wnt, Wtt
+  double mu, det;
+  auto block = [&]() {
+    n = __ldg(reinterpret_cast<const double2*>(a.D) + 2 * (size_t)p);
+    t = __ldg(reinterpret_cast<const double2*>(a.D) + 2 * (size_t)p + 1);
+    mu = __ldg(&a.mu[p]);
+    det = __ldg(&a.det[p]);
+  };
+  if (Team::flow) block();  // before the wait; the other teams' registers don't hold it
   double y = x.q;
   for (int t0 = 0;; t0 += FC2D_NB) {
     double2 r[FC2D_NB];
-#pragma unroll
-    for (int i = 0; i < FC2D_NB; i++)
-      if (x.col[i] >= 0) r[i] = rx.get(x.col[i]);
+    rx.gather(x.col, p, r);
 #pragma unroll
     for (int i = 0; i < FC2D_NB; i++)
       if (x.col[i] >= 0) {
         y += x.w[i].x * r[i].x;
         y += x.w[i].y * r[i].y;
       }
-    if (t0 + FC2D_NB >= x.slots) break;
+    if (!rx.any(t0 + FC2D_NB < x.slots)) break;
     load_slots(a, x, t0 + FC2D_NB, k & 31, comp);
   }
   const double z = __shfl_xor_sync(0xffffffffu, y, 1);
   const double q0 = comp ? z : y, q1 = comp ? y : z;
-  const double2 n = __ldg(reinterpret_cast<const double2*>(a.D) + 2 * (size_t)p);      // Wnn, Wtn
-  const double2 t = __ldg(reinterpret_cast<const double2*>(a.D) + 2 * (size_t)p + 1);  // Wnt, Wtt
-  const double mu = __ldg(&a.mu[p]), det = __ldg(&a.det[p]);
+  if (!Team::flow) block();
   double P = 0.0;
   const bool contact = !ie_positive(q0);
   // P = -(adjugate q) / D, component by component
@@ -510,14 +623,14 @@ __device__ __forceinline__ void contact64(const Args<double>& a, const Reactions
   }
   dx = old - P;
   pn = P;
-  if (act) put_component<REP, Team>(rx, p, comp, P, team);
+  if (act) rx.put_component(p, comp, P, team);
 }
 
 // All colours of one sweep; v gets this thread's sums |r_old - r_new|^2 and
 // |r_new|^2.  row: the static inputs of the thread's first contact of colour
 // 0, loaded; left loaded for the next sweep.
 template <bool REP, typename Team>
-__device__ __forceinline__ void sweep_colours(const Args<float>& a, const Reactions<float, REP>& rx, int g0, int G,
+__device__ __forceinline__ void sweep_colours(const Args<float>& a, Reactions<float, REP>& rx, int g0, int G,
                                               Row<float>& row, float v[2], Team& team) {
   auto size = [&](int c) { return __ldg(&a.cptr[c + 1]) - __ldg(&a.cptr[c]); };
   int n = size(0), next;
@@ -532,7 +645,7 @@ __device__ __forceinline__ void sweep_colours(const Args<float>& a, const Reacti
         v[1] += P[0] * P[0] + P[1] * P[1];
         load_row(a, c, k, 0, row);
       }
-      contact32(a, rx, k, row, x0, x1, P, team);
+      contact32(a, rx, k, true, row, x0, x1, P, team);
     }
     if (c + 1 < a.ncol) team.arrive();
     if (g0 < next) load_row(a, cn, g0, 0, row);
@@ -545,7 +658,7 @@ __device__ __forceinline__ void sweep_colours(const Args<float>& a, const Reacti
 }
 
 template <bool REP, typename Team>
-__device__ __forceinline__ void sweep_colours(const Args<double>& a, const Reactions<double, REP>& rx, int g0, int G,
+__device__ __forceinline__ void sweep_colours(const Args<double>& a, Reactions<double, REP>& rx, int g0, int G,
                                               Row<double>& row, double v[2], Team& team) {
   const int comp = g0 & 1, h0 = g0 >> 1, H = G >> 1;
   const int lead = (g0 & ~31) >> 1;  // the warp's first contact, present while any of the warp's is
@@ -572,6 +685,174 @@ __device__ __forceinline__ void sweep_colours(const Args<double>& a, const React
     v[1] += pn * pn;
     if (c + 1 < a.ncol) team.wait();
   }
+}
+
+// ---- the sweeps as dataflow -------------------------------------------------
+// What bounds a colour of a large problem is not its contacts but what stands
+// between two colours: a barrier over every SM and then the loads it releases.
+// Here a warp takes units of a few contacts and waits only for the reactions
+// these read, each stored with the number of the sweep that wrote it.  In a
+// colour's order a contact reads the new reactions of lower colours and the
+// old ones of higher colours; the pattern is symmetric, so a contact of a
+// higher colour cannot write its new one before this contact has written its
+// own, and a stamp at least the one needed is the one needed.  Granular
+// problems, us a sweep by colours and as dataflow: FP64 24.4 and 18.6 at 367
+// contacts, 34.7 and 26.2 at 7,002, 34.8 and 28.9 at 28,008, 63.2 and 35.1 at
+// 70,020; FP32 10.2 and 8.5, 14.1 and 11.9, 19.9 and 12.3, 22.3 and 13.0.
+// What is left is the chain of a colour's longest rows: with a warp a quarter
+// an instruction takes eight cycles and an FP64 one 64.
+
+// Polls of a reaction before the back-off, and the back-off (ns).
+#define FC2D_FLOW_SPIN 16
+#define FC2D_FLOW_SLEEP_NS 100
+
+// The stamped reactions beside the plain ones (which the error evaluation and
+// the end of the solve read): in FP32 one 128-bit word (x, y, stamp), in FP64
+// one for each component (value, stamp).
+template <typename T>
+struct FlowReactions {
+  using V = typename Vec2<T>::type;
+  static constexpr int L = sizeof(T) == sizeof(double) ? 2 : 1;  // words of a reaction
+  T* rw;
+  T* rs;
+  int sweep;
+  bool failed;
+  __device__ __forceinline__ V get(int j) const { return __ldcg(reinterpret_cast<const V*>(rw) + j); }
+  __device__ __forceinline__ bool any(bool more) const { return __any_sync(0xffffffffu, more); }
+  __device__ __forceinline__ void stamp(int j, V v, int at) const {
+    if constexpr (sizeof(T) == sizeof(float)) {
+      fc3dgpu::st_word128(rs + 4 * (size_t)j,
+                          (unsigned long long)__float_as_uint(v.x) | (unsigned long long)__float_as_uint(v.y) << 32,
+                          (unsigned long long)(unsigned)at);
+    } else {
+      fc3dgpu::st_word128(rs + 4 * (size_t)j, (unsigned long long)__double_as_longlong(v.x), (unsigned long long)at);
+      fc3dgpu::st_word128(rs + 4 * (size_t)j + 2, (unsigned long long)__double_as_longlong(v.y),
+                          (unsigned long long)at);
+    }
+  }
+  // Waits for the reactions of a row's next slots.  Every poll loads all of
+  // them without a branch between two loads (a slot without a column loads the
+  // contact's own word), so it costs one memory latency (with a branch a
+  // slot a sweep of 28,008 contacts took 15.1 us in FP32, 12.3 without).  A
+  // wait that gives up goes on with what is there: the block ends
+  // the solve after the sweep.
+  template <int N>
+  __device__ __forceinline__ void gather(const int (&col)[N], int p, V (&r)[N]) {
+    int from[N], need[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      from[i] = col[i] >= 0 ? col[i] : p;
+      need[i] = sweep - (col[i] >= 0 && col[i] < p ? 0 : 1);
+    }
+    for (unsigned long long n = 0;; n++) {
+      unsigned long long w[N][L][2];
+#pragma unroll
+      for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int k = 0; k < L; k++) fc3dgpu::ld_word128(rs + 4 * (size_t)from[i] + 2 * k, w[i][k][0], w[i][k][1]);
+      bool all = true;
+#pragma unroll
+      for (int i = 0; i < N; i++) {
+        bool there = true;
+#pragma unroll
+        for (int k = 0; k < L; k++) there = there && (int)(unsigned)w[i][k][1] >= need[i];
+        if constexpr (L == 1) {
+          r[i].x = __uint_as_float((unsigned)w[i][0][0]);
+          r[i].y = __uint_as_float((unsigned)(w[i][0][0] >> 32));
+        } else {
+          r[i].x = __longlong_as_double((long long)w[i][0][0]);
+          r[i].y = __longlong_as_double((long long)w[i][L - 1][0]);
+        }
+        all = all && there;
+      }
+      if (__all_sync(0xffffffffu, all || failed)) break;
+      if (n > SPIN) failed = true;
+      if (n > FC2D_FLOW_SPIN) __nanosleep(FC2D_FLOW_SLEEP_NS);
+    }
+  }
+  template <typename Team>
+  __device__ __forceinline__ void put(int j, T x0, T x1, Team&) const {
+    V v;
+    v.x = x0;
+    v.y = x1;
+    stamp(j, v, sweep);
+    __stcg(reinterpret_cast<V*>(rw) + j, v);
+  }
+  template <typename Team>
+  __device__ __forceinline__ void put_component(int j, int comp, T x, Team&) const {
+    fc3dgpu::st_word128(rs + 4 * (size_t)j + 2 * comp, (unsigned long long)__double_as_longlong(x),
+                        (unsigned long long)sweep);
+    __stcg(rw + 2 * (size_t)j + comp, x);
+  }
+};
+
+// The reactions of the solve's start (FP64) with sweep 0's stamps, and the
+// sweep's plain copy.
+template <typename T>
+__device__ __forceinline__ FlowReactions<T> open_flow(const Args<T>& a, FlowTeam& team) {
+  FlowReactions<T> fx{a.rw, a.rs, 0, false};
+  for (int j = team.rank() * blockDim.x + threadIdx.x; j < a.nc; j += team.size() * blockDim.x) {
+    const double2 x = __ldcg(reinterpret_cast<const double2*>(a.r) + j);
+    typename Vec2<T>::type v;
+    v.x = (T)x.x;
+    v.y = (T)x.y;
+    fx.stamp(j, v, 0);
+    if (sizeof(T) != sizeof(double)) __stcg(reinterpret_cast<typename Vec2<T>::type*>(a.rw) + j, v);
+  }
+  team.sync_all();
+  return fx;
+}
+
+// Contacts and this block's units of each colour: unit u of a colour goes to
+// block u mod the grid.
+struct FlowTable {
+  int n[MAXC], mine[MAXC];
+  template <typename T>
+  __device__ __forceinline__ void fill(const Args<T>& a, const FlowTeam& team) {
+    for (int c = threadIdx.x; c < a.ncol; c += blockDim.x) {
+      n[c] = a.cptr[c + 1] - a.cptr[c];
+      const int units = (n[c] + a.rows - 1) / a.rows, rank = team.rank(), size = team.size();
+      mine[c] = rank < units ? (units - rank + size - 1) / size : 0;
+    }
+    __syncthreads();
+  }
+};
+
+// One sweep, a block's units in colour order to its warps in turn.  Lane
+// groups without a contact repeat the unit's first one without storing it.
+template <typename T>
+__device__ __forceinline__ void flow_sweep(const Args<T>& a, FlowReactions<T>& fx, const FlowTable& tab, T v[2],
+                                           FlowTeam& team) {
+  constexpr int L = sizeof(T) == sizeof(double) ? 2 : 1;
+  const int lane = threadIdx.x & 31, comp = L == 2 ? lane & 1 : 0, i = lane / L, nw = blockDim.x >> 5;
+  int e = threadIdx.x >> 5;  // the warp's next unit among the block's
+  for (int c = 0; c < a.ncol; c++) {
+    const int n = tab.n[c], mine = tab.mine[c];
+    for (; e < mine; e += nw) {
+      const int k0 = (team.rank() + e * team.size()) * a.rows;
+      const bool act = i < a.rows && k0 + i < n;
+      const int k = act ? k0 + i : k0;
+      Row<T> row;
+      load_row(a, c, k, comp, row);
+      if constexpr (L == 2) {
+        double dx, pn;
+        contact64(a, fx, k, comp, act, row, dx, pn, team);
+        if (act) {
+          v[0] += dx * dx;
+          v[1] += pn * pn;
+        }
+      } else {
+        float x0, x1, P[2];
+        contact32(a, fx, k, act, row, x0, x1, P, team);
+        if (act) {
+          v[0] += x0 * x0 + x1 * x1;
+          v[1] += P[0] * P[0] + P[1] * P[1];
+        }
+      }
+    }
+    e -= mine;
+  }
+  if (__syncthreads_or(fx.failed)) team.give_up();
 }
 
 // Bring the FP64 reactions into the sweep's copy (replica or FP32 copy in
@@ -630,7 +911,8 @@ __device__ __forceinline__ void close_reactions(const Args<T>& a, const Reaction
 // (read by rows, each lane touched its own lines and a colour of 5,000
 // contacts queued on the L1's tags) and loaded before the barrier that
 // releases the colour; the light-error terms are summed behind the barrier's
-// arrival.  Granular problems, us a sweep before and after: FP64 37.4 and 24.6
+// arrival; above 64 contacts a colour the sweeps go as dataflow (above).  By
+// colours, granular problems, us a sweep before and after: FP64 37.4 and 24.6
 // at 367 contacts, 49.2 and 34.9 at 7,002, 75.3 and 34.4 at 28,008; FP32 12.5
 // and 10.1, 16.5 and 14.2, 26.7 and 20.3.  The hardware cluster barrier
 // (release / acquire) separates colours, the barrier of the error reduction
@@ -641,15 +923,23 @@ __device__ __forceinline__ void close_reactions(const Args<T>& a, const Reaction
 // A phase that follows another starts its sweep count, budget and trace
 // where the previous one stopped (read from the device, no host round trip).
 template <typename T, bool REP, typename Team>
-__global__ void __launch_bounds__(NT_MAX, 1) k_fc2d_nsgs(const Args<T> a) {
+__global__ void __launch_bounds__(Team::flow ? 256 : NT_MAX, 1) k_fc2d_nsgs(const Args<T> a) {
   using V = typename Vec2<T>::type;
   extern __shared__ __align__(16) unsigned char dsm[];
   V* rsm = reinterpret_cast<V*>(dsm);
   __shared__ Reduce<T> R;
-  Team team;
+  Team team(a);
   if (threadIdx.x == 0) R.calls = 0;
   __syncthreads();
-  const Reactions<T, REP> rx = open_reactions<T, REP>(a, rsm, team);
+  Reactions<T, REP> rx{nullptr, a.rw};
+  FlowReactions<T> fx{};
+  __shared__ typename std::conditional<Team::flow, FlowTable, char>::type tab;
+  if constexpr (Team::flow) {
+    tab.fill(a, team);
+    fx = open_flow(a, team);
+  } else {
+    rx = open_reactions<T, REP>(a, rsm, team);
+  }
   const int g0 = team.rank() * blockDim.x + threadIdx.x, G = team.size() * blockDim.x;
   const bool lead = team.rank() == 0 && threadIdx.x == 0;
   const int done = a.before ? (int)a.before[0] : 0;
@@ -657,18 +947,27 @@ __global__ void __launch_bounds__(NT_MAX, 1) k_fc2d_nsgs(const Args<T> a) {
   T tolerance = (T)a.tol, err = (T)INFINITY, best = (T)INFINITY;
   int iter = 0, not_conv = 1, since_best = 0;
   Row<T> row;
-  {
+  if constexpr (!Team::flow) {
     const int comp = sizeof(T) == sizeof(double) ? g0 & 1 : 0, k = sizeof(T) == sizeof(double) ? g0 >> 1 : g0;
     if (k < a.cptr[1] - a.cptr[0]) load_row(a, 0, k, comp, row);
   }
   while (iter < budget && not_conv) {
     ++iter;
     T v[2] = {0, 0};
-    sweep_colours(a, rx, g0, G, row, v, team);
+    if constexpr (Team::flow) {
+      fx.sweep = iter;
+      flow_sweep(a, fx, tab, v, team);
+    } else {
+      sweep_colours(a, rx, g0, G, row, v, team);
+    }
     if constexpr (sizeof(T) == sizeof(double))
       team_sum2(v, R, team, a.part);
+    else if constexpr (Team::flow)
+      flow_sum<2>(v, R, team, a.part);
     else
       team_sum<2>(v, R, team, a.part);
+    if constexpr (Team::flow)
+      if (team.dead) return;
     if constexpr (sizeof(T) == sizeof(double)) {
       const double nr = fc3dgpu::ie_sqrt(v[1]);
       err = fc3dgpu::ie_sqrt(v[0]);
@@ -694,6 +993,8 @@ __global__ void __launch_bounds__(NT_MAX, 1) k_fc2d_nsgs(const Args<T> a) {
       not_conv = 0;
       if constexpr (sizeof(T) == sizeof(double)) {
         const double full = full_error<REP>(a, rx, R, team);
+        if constexpr (Team::flow)
+          if (team.dead) return;
         if (full > a.tol) {
           tolerance = err / full * a.tol;
           not_conv = 1;
@@ -711,6 +1012,8 @@ __global__ void __launch_bounds__(NT_MAX, 1) k_fc2d_nsgs(const Args<T> a) {
       not_conv = 1;
     }
   }
+  if constexpr (Team::flow)
+    if (team.dead) return;
   if (lead) {
     a.out[0] = done + iter;
     a.out[1] = final_err;
@@ -724,7 +1027,7 @@ template <bool REP, typename Team>
 __global__ void __launch_bounds__(NT_MAX, 1) k_fc2d_error(const Args<double> a) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ Reduce<double> R;
-  Team team;
+  Team team(a);
   if (threadIdx.x == 0) R.calls = 0;
   __syncthreads();
   const Reactions<double, REP> rx = open_reactions<double, REP>(a, reinterpret_cast<double2*>(dsm), team);
@@ -743,8 +1046,8 @@ using namespace fc2dgpu;
 // A launch: a cluster of cs blocks, or a cooperative grid of `blocks`; the
 // reactions in HBM or replicated in shared memory.
 struct Shape {
-  bool grid = false, rep = false;
-  int cs = 1, nt = 128, blocks = 1;
+  bool grid = false, rep = false, flow = false;
+  int cs = 1, nt = 128, blocks = 1, rows = 1;
 };
 
 struct fc2dgpu_ctx {
@@ -765,7 +1068,9 @@ struct fc2dgpu_ctx {
   double *sW = nullptr, *D = nullptr;
   float *sW32 = nullptr, *D32 = nullptr;
   double *W = nullptr, *det = nullptr, *q = nullptr, *mu = nullptr, *r = nullptr, *u = nullptr, *trace = nullptr,
-         *out = nullptr, *part = nullptr;
+         *out = nullptr, *part = nullptr, *rs = nullptr;  // rs: stamped reactions of the dataflow, of either precision
+                                                                  // (a symmetric block pattern)
+  unsigned* flags = nullptr;
   // FP32 copies for the first phase of a mixed-precision solve
   float *W32 = nullptr, *det32 = nullptr, *q32 = nullptr, *mu32 = nullptr, *r32 = nullptr;
   int precision = 1;          // 0 FP32 sweeps + FP64 polish, 1 FP64 sweeps only
@@ -784,11 +1089,36 @@ struct fc2dgpu_ctx {
     }                                                                                     \
   } while (0)
 
+// Dataflow above this many contacts in the largest colour, where one block no
+// longer holds it at a contact a thread: with 41 contacts a sweep takes 8.3 us
+// in one block and 9.2 as dataflow in FP64 (6.3 and 7.5 mixed), with 131 on a
+// cluster 24.4 and 18.6 (FP32 10.2 and 8.5).
+constexpr int FLOW_FROM = 64;
+
 static void choose_shape(fc2dgpu_ctx* c);
+
+// Whether every block (i, j) has a block (j, i), as often: the rows' columns in
+// ascending order against the columns' rows, which two transpositions give.
+static bool symmetric_pattern(int nc, const std::vector<int>& rp, const std::vector<int>& col) {
+  auto transpose = [&](const std::vector<int>& p, const std::vector<int>& x, std::vector<int>& tp, std::vector<int>& t) {
+    tp.assign(nc + 1, 0);
+    for (int j : x) tp[j + 1]++;
+    for (int j = 0; j < nc; j++) tp[j + 1] += tp[j];
+    t.resize(x.size());
+    std::vector<int> at(tp.begin(), tp.end() - 1);
+    for (int i = 0; i < nc; i++)
+      for (int s = p[i]; s < p[i + 1]; s++) t[at[x[s]]++] = i;
+  };
+  std::vector<int> tp, t, sp, sorted;
+  transpose(rp, col, tp, t);
+  if (tp != rp) return false;
+  transpose(tp, t, sp, sorted);
+  return t == sorted;
+}
 
 static void free_problem(fc2dgpu_ctx* c) {
   void* ptrs[] = {c->cptr, c->rp, c->col, c->dpos, c->W, c->det, c->q, c->mu, c->r, c->u,
-                  c->sp, c->scol, c->slab, c->sW, c->D, c->sW32, c->D32, c->W32, c->det32, c->q32, c->mu32, c->r32};
+                  c->sp, c->scol, c->slab, c->sW, c->D, c->sW32, c->D32, c->W32, c->det32, c->q32, c->mu32, c->r32, c->rs};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   c->cptr = c->rp = c->col = c->dpos = nullptr;
@@ -798,6 +1128,7 @@ static void free_problem(fc2dgpu_ctx* c) {
   c->sW = c->D = nullptr;
   c->sW32 = c->D32 = nullptr;
   c->W32 = c->det32 = c->q32 = c->mu32 = c->r32 = nullptr;
+  c->rs = nullptr;
   c->nc = 0;
 }
 
@@ -808,6 +1139,7 @@ extern "C" void fc2dgpu_ctx_destroy(fc2dgpu_ctx* c) {
   if (c->trace) cudaFree(c->trace);
   if (c->out) cudaFree(c->out);
   if (c->part) cudaFree(c->part);
+  if (c->flags) cudaFree(c->flags);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -830,7 +1162,9 @@ extern "C" fc2dgpu_ctx* fc2dgpu_ctx_create(int device) {
   bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaEventCreate(&c->ev[0]) == cudaSuccess && cudaEventCreate(&c->ev[1]) == cudaSuccess &&
             cudaMalloc(&c->trace, sizeof(double) * TRACE_CAP) == cudaSuccess &&
-            cudaMalloc(&c->out, sizeof(double) * 8) == cudaSuccess &&
+            cudaMalloc(&c->out, sizeof(double) * 9) == cudaSuccess &&
+            cudaMemset(c->out, 0, sizeof(double) * 9) == cudaSuccess &&
+            cudaMalloc(&c->flags, sizeof(unsigned) * GRID_MAX * FLAG_STRIDE) == cudaSuccess &&
             cudaMalloc(&c->part, sizeof(double) * 2 * GRID_MAX * 4) == cudaSuccess;
   if (!ok) {
     fc3dgpu_set_error("fc2dgpu_ctx_create: set-up failed (%s)", cudaGetErrorString(cudaGetLastError()));
@@ -1009,6 +1343,13 @@ extern "C" int fc2dgpu_ctx_set_problem(fc2dgpu_ctx* c, int nc, const int64_t* ro
   c->singular = singular;
   c->max_colour = 0;
   for (int k = 0; k < ncol; k++) c->max_colour = std::max(c->max_colour, cptr[k + 1] - cptr[k]);
+  if (c->max_colour > FLOW_FROM && symmetric_pattern(nc, rp, col) &&
+      cudaMalloc(&c->rs, sizeof(double) * 4 * (size_t)nc) != cudaSuccess) {
+    cudaGetLastError();
+    free_problem(c);
+    fc3dgpu_set_error("fc2dgpu_ctx_set_problem: out of device memory");
+    return NUMERICS_ERR_UNKNOWN;
+  }
   choose_shape(c);
   return 0;
 }
@@ -1133,7 +1474,35 @@ static Shape grid_shape(fc2dgpu_ctx* c, int nt, int lanes) {
   return s;
 }
 
+// Units of as few contacts as give every SM quarter one of an average colour;
+// a block an SM, of eight warps where the largest colour has more units than
+// quarters, else of four.
+static Shape flow_shape(fc2dgpu_ctx* c, int most) {
+  Shape s;
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+  const long long quarters = 4LL * c->ncol * sms;
+  s.grid = s.flow = true;
+  s.rows = (int)std::min<long long>(most, std::max(1LL, (c->nc + quarters - 1) / quarters));
+  const int units = (c->max_colour + s.rows - 1) / s.rows;
+  s.nt = units > 4 * sms ? 256 : 128;
+  s.blocks = std::max(1, std::min((units + s.nt / 32 - 1) / (s.nt / 32), std::min(sms, GRID_MAX)));
+  return s;
+}
+
+static void choose_flow(fc2dgpu_ctx* c) {
+  if (!c->rs || c->cs_req != 0 || c->nt_req != 0 || c->rep_req != 0) return;
+  c->s32 = flow_shape(c, 32);
+  c->s64 = flow_shape(c, 16);
+}
+
+static void choose_blocks(fc2dgpu_ctx* c);
 static void choose_shape(fc2dgpu_ctx* c) {
+  choose_blocks(c);
+  choose_flow(c);
+}
+
+static void choose_blocks(fc2dgpu_ctx* c) {
   if (c->cs_req < 0 || (c->cs_req == 0 && c->rep_req != 2 && c->max_colour > GRID_FROM)) {
     c->s32 = grid_shape(c, c->nt_req, 1);
     c->s64 = c->cs_req < 0 ? c->s32 : grid_shape(c, c->nt_req, 2);
@@ -1241,6 +1610,9 @@ static Args<double> args64(const fc2dgpu_ctx* c) {
   a.trace = c->trace;
   a.out = c->out;
   a.part = c->part;
+  a.rs = c->rs;
+  a.flags = c->flags;
+  a.fail = c->out + 8;
   return a;
 }
 
@@ -1269,6 +1641,9 @@ static Args<float> args32(const fc2dgpu_ctx* c) {
   a.trace = c->trace;
   a.out = c->out + 4;
   a.part = c->part;
+  a.rs = reinterpret_cast<float*>(c->rs);
+  a.flags = c->flags;
+  a.fail = c->out + 8;
   return a;
 }
 
@@ -1347,19 +1722,30 @@ extern "C" int fc2dgpu_ctx_solve(fc2dgpu_ctx* c, double tol, int max_iter, int e
     b.switch_tol = c->switch_tol > 0.0 ? c->switch_tol : std::max(tol, 1e-6);
     b.stall = c->stall;
     const Shape& s = c->s32;
-    K2(s.grid  ? launch_grid(c, s, k_fc2d_nsgs<float, false, GridTeam>, b)
+    b.rows = s.rows;
+    if (s.flow) K2(cudaMemsetAsync(c->flags, 0, sizeof(unsigned) * GRID_MAX * FLAG_STRIDE, c->stream));
+    K2(s.flow  ? launch_grid(c, s, k_fc2d_nsgs<float, false, FlowTeam>, b)
+       : s.grid ? launch_grid(c, s, k_fc2d_nsgs<float, false, GridTeam>, b)
        : s.rep ? launch(c, s, k_fc2d_nsgs<float, true, ClusterTeam>, b, sizeof(float2) * (size_t)c->nc)
                : launch(c, s, k_fc2d_nsgs<float, false, ClusterTeam>, b, 0));
     a.before = c->out + 4;
   }
   const Shape& s = c->s64;
-  K2(s.grid  ? launch_grid(c, s, k_fc2d_nsgs<double, false, GridTeam>, a)
+  a.rows = s.rows;
+  if (s.flow) K2(cudaMemsetAsync(c->flags, 0, sizeof(unsigned) * GRID_MAX * FLAG_STRIDE, c->stream));
+  K2(s.flow  ? launch_grid(c, s, k_fc2d_nsgs<double, false, FlowTeam>, a)
+     : s.grid ? launch_grid(c, s, k_fc2d_nsgs<double, false, GridTeam>, a)
      : s.rep ? launch(c, s, k_fc2d_nsgs<double, true, ClusterTeam>, a, rep_bytes(c))
              : launch(c, s, k_fc2d_nsgs<double, false, ClusterTeam>, a, 0));
   K2(cudaEventRecord(c->ev[1], c->stream));
-  double out[8];
+  double out[9];
   K2(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
   K2(cudaStreamSynchronize(c->stream));
+  if (out[8] != 0.0) {
+    K2(cudaMemset(c->out, 0, sizeof(double) * 9));
+    fc3dgpu_set_error("fc2dgpu_ctx_solve: a wait reached its poll limit");
+    return NUMERICS_ERR_UNKNOWN;
+  }
   float t = 0.f;
   cudaEventElapsedTime(&t, c->ev[0], c->ev[1]);
   if (iters) *iters = (int)out[0];

@@ -1,7 +1,8 @@
 """The 2D sweeps' automatic launches over their range: FP64 on two threads a
 contact in one block, in clusters and on the grid, rows longer than the eight
 slots fetched together, and colours that end inside a warp; the FP64 sweeps
-and the FP32 ones bit for bit the oracle's in colour order."""
+and the FP32 ones bit for bit the oracle's in colour order.  As dataflow (a
+symmetric pattern): units from one contact to as many as a warp takes."""
 import numpy as np
 import pytest
 
@@ -9,6 +10,17 @@ from test_fc2d_oracle import load_fc2d, tiled2d
 from test_gpu_fc2d import _ctx, _order, sn  # noqa: F401
 
 pytestmark = pytest.mark.gpu
+
+
+def _one_sided(P, drop):
+    """P without its `drop`-th block off the diagonal (the transpose stays): the
+    sweeps go by colours."""
+    from dataclasses import replace
+    row = np.repeat(np.arange(P.nc), np.diff(P.rowptr))
+    keep = np.ones(len(row), bool)
+    keep[np.flatnonzero(row != P.colidx)[drop]] = False
+    return replace(P, rowptr=np.concatenate([[0], np.cumsum(np.bincount(row[keep], minlength=P.nc))]),
+                   colidx=P.colidx[keep], blocks=P.blocks[keep])
 
 
 def _dense_rows(O, nc, seed):
@@ -30,10 +42,15 @@ def _dense_rows(O, nc, seed):
 
 @pytest.mark.parametrize("problem,copies", [("FrictionContactProblem00031", 1), ("FrictionContactProblem00727", 1),
                                             ("FrictionContactProblem00727", 9),
-                                            ("fc2d_granularflowonwall_07002_00801", 1), ("dense", 90)])
-def test_sweeps_bit_exact(sn, problem, copies):  # noqa: F811
+                                            ("fc2d_granularflowonwall_07002_00801", 1),
+                                            ("fc2d_granularflowonwall_07002_00801", 10), ("dense", 90),
+                                            ("dense", 700)])
+@pytest.mark.parametrize("one_sided", [False, True])
+def test_sweeps_bit_exact(sn, problem, copies, one_sided):  # noqa: F811
     import oracle as O
     P = _dense_rows(O, copies, 3) if problem == "dense" else tiled2d(load_fc2d("fc2d_" + problem)[0], copies, 4)
+    if one_sided:
+        P = _one_sided(P, 0)
     ctx = _ctx(sn, P)
     _, colour = ctx.colours()
     res = ctx.solve(0.0, 8)
