@@ -270,7 +270,7 @@ int fc3dgpu_ctx_sync(fc3dgpu_ctx *ctx, int neighbourhood);
  * colours); 0 the coloured kernel above.  The same sweep either way.  Applies
  * with one lane per contact, in FP32 when no slab has more than 16
  * off-diagonal slots, in FP64 (bit-exact arithmetic, no timeline) on a
- * symmetric pattern with at most 110 contacts a colour and SM.  Returns the
+ * symmetric pattern with at most 150 contacts a colour and SM.  Returns the
  * previous setting. */
 int fc3dgpu_ctx_flow(fc3dgpu_ctx *ctx, int on);
 /* Warps per block of the dataflow sweep: 8, 10 or 12 (0: the default, 10,

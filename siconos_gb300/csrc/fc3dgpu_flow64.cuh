@@ -10,8 +10,8 @@
 // the block pattern is symmetric here too).  Each colour's units are dealt
 // over all blocks, so every SM quarter has work of each colour.  us a sweep by colours and as
 // dataflow (lattices of n contacts, 6 colours):
-//   42: 130, 88    2,800: 244, 140    11,600: 263, 200    40,935: 296, 257
-//   68,688: 408, 325    96,780: 453, 410    125,840: 483, 488    163,584: 541, 594
+//   42: 130, 85    2,800: 244, 138    11,600: 263, 190    40,935: 296, 236
+//   68,688: 408, 305    96,780: 453, 392    125,840: 483, 475    163,584: 541, 594
 // Beyond FC3D_FLOW64_MAX contacts a colour and block the sweeps go by colours:
 // the FP64 pipe is then full either way and one lane a contact needs it less.
 //
@@ -30,15 +30,18 @@ namespace fc3dgpu {
 #define FC3D_FLOW64_SPIN 16
 #define FC3D_FLOW64_SLEEP_NS 100
 
-// A stamped reaction; false (x not set) before sweep `need` has written it.
+// The reaction in the two words w; false before sweep `need` has written it.
+__device__ __forceinline__ bool take_stamped64(const unsigned long long w[4], int need, double x[3]) {
+  x[0] = __longlong_as_double((long long)w[0]);
+  x[1] = __longlong_as_double((long long)((w[1] & 0xffffffffull) | (w[3] << 32)));
+  x[2] = __longlong_as_double((long long)w[2]);
+  return (int)(w[1] >> 32) >= need && (int)(w[3] >> 32) >= need;
+}
 __device__ __forceinline__ bool ld_stamped64(const double* rs, int p, int need, double x[3]) {
-  unsigned long long a0, a1, b0, b1;
-  ld_word128(rs + 4 * (size_t)p, a0, a1);
-  ld_word128(rs + 4 * (size_t)p + 2, b0, b1);
-  x[0] = __longlong_as_double((long long)a0);
-  x[1] = __longlong_as_double((long long)((a1 & 0xffffffffull) | (b1 << 32)));
-  x[2] = __longlong_as_double((long long)b0);
-  return (int)(a1 >> 32) >= need && (int)(b1 >> 32) >= need;
+  unsigned long long w[4];
+  ld_word128(rs + 4 * (size_t)p, w[0], w[1]);
+  ld_word128(rs + 4 * (size_t)p + 2, w[2], w[3]);
+  return take_stamped64(w, need, x);
 }
 // Word `w` (0 or 1) of the stamped reaction p
 __device__ __forceinline__ void st_stamped64(double* rs, int p, int w, const double x[3], int stamp) {
@@ -82,7 +85,7 @@ __device__ __forceinline__ bool flow64_unit(const SweepArgs<double>& a, int p0, 
   const double o = __ldcg(&a.r[(size_t)p * FC3D_RSTRIDE + c.i]);
   double acc = a.q[((size_t)sl * 3 + c.i) * FC3D_SLAB + k];
   bool ok = true;
-  constexpr int CH = 6;
+  constexpr int CH = 5;
   for (int t0 = 0; t0 < nsmax && ok; t0 += CH) {
     int pj[CH];
     double wv[CH][3], rv[CH][3];
@@ -106,10 +109,20 @@ __device__ __forceinline__ bool flow64_unit(const SweepArgs<double>& a, int p0, 
         break;
       }
       if (polls > FC3D_FLOW64_SPIN) __nanosleep(FC3D_FLOW64_SLEEP_NS);
+      // a poll's loads are predicated, without a branch between them, so it
+      // costs one memory latency (40,935 contacts: 257 us a sweep with
+      // branches, 242 without, 236 with five slots at once in place of six)
+      unsigned long long w[CH][4];
+#pragma unroll
+      for (int t = 0; t < CH; t++) {
+        ld_word128_if(late >> t & 1u, a.rs + 4 * (size_t)pj[t], w[t][0], w[t][1]);
+        ld_word128_if(late >> t & 1u, a.rs + 4 * (size_t)pj[t] + 2, w[t][2], w[t][3]);
+      }
 #pragma unroll
       for (int t = 0; t < CH; t++)
-        if ((late >> t & 1u) && ld_stamped64(a.rs, pj[t], sweep - (pj[t] > p ? 1 : 0), rv[t])) late &= ~(1u << t);
+        if ((late >> t & 1u) && take_stamped64(w[t], sweep - (pj[t] > p ? 1 : 0), rv[t])) late &= ~(1u << t);
     }
+    __syncwarp();  // the lanes left the wait one by one: together again
 #pragma unroll
     for (int t = 0; t < CH; t++)
       if (t0 + t < ns) {

@@ -24,7 +24,7 @@
 #define FC3D_MAX_COLOURS 128
 // Contacts a colour and block up to which the FP64 sweeps go as dataflow
 // (measured in fc3dgpu_flow64.cuh)
-#define FC3D_FLOW64_MAX 110
+#define FC3D_FLOW64_MAX 150
 
 namespace fc3dgpu {
 

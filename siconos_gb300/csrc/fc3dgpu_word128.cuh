@@ -18,4 +18,15 @@ __device__ __forceinline__ void ld_word128(const void* p, unsigned long long& lo
                : "memory");
 }
 
+// The same where `yes`, else lo and hi as they are: a predicated load, so that
+// several of them are in flight together.
+__device__ __forceinline__ void ld_word128_if(bool yes, const void* p, unsigned long long& lo, unsigned long long& hi) {
+  asm volatile(
+      "{\n .reg .pred q;\n .reg .b128 t;\n setp.ne.u32 q, %3, 0;\n mov.b128 t, {%0, %1};\n"
+      " @q ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+      : "+l"(lo), "+l"(hi)
+      : "l"(p), "r"((unsigned)yes)
+      : "memory");
+}
+
 }  // namespace fc3dgpu

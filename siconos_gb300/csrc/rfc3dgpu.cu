@@ -688,22 +688,26 @@ __device__ __forceinline__ void st_all_stamped(double* rs, int p, const double x
 }
 
 // The reactions x[t] of the contacts j[t] as row p reads them in `sweep`
-// (j < 0: none); false when the wait gave up.
+// (j < 0: none); false when the wait gave up.  Called by the whole warp.  A
+// poll loads all of them without a branch between two loads (none: the row's
+// own), so it costs one memory latency.
 template <typename Real, int CH>
 __device__ __forceinline__ bool wait_reactions(const ArgsT<Real>& a, const int (&j)[CH], int p, int sweep,
                                                Real (&x)[CH][5]) {
-  unsigned late = 0;
+  int from[CH], need[CH];
 #pragma unroll
-  for (int t = 0; t < CH; t++)
-    if (j[t] >= 0) late |= (ld_stamped(a.rs, j[t], sweep - (j[t] > p ? 1 : 0), x[t]) ? 0u : 1u) << t;
-  for (unsigned long long n = 0; late; n++) {
+  for (int t = 0; t < CH; t++) {
+    from[t] = j[t] >= 0 ? j[t] : p;
+    need[t] = sweep - (j[t] >= 0 && j[t] < p ? 0 : 1);
+  }
+  for (unsigned long long n = 0;; n++) {
+    bool ok = true;
+#pragma unroll
+    for (int t = 0; t < CH; t++) ok = ld_stamped(a.rs, from[t], need[t], x[t]) && ok;
+    if (__all_sync(0xffffffffu, ok)) return true;
     if (n > a.spin) return false;
     if (n > RFC3D_FLOW_SPIN) __nanosleep(RFC3D_FLOW_SLEEP_NS);
-#pragma unroll
-    for (int t = 0; t < CH; t++)
-      if ((late >> t & 1u) && ld_stamped(a.rs, j[t], sweep - (j[t] > p ? 1 : 0), x[t])) late &= ~(1u << t);
   }
-  return true;
 }
 
 // Contacts [first, first + n) of a colour, five lanes each.  v[2] counts
@@ -784,7 +788,6 @@ __device__ __forceinline__ void flow_unit(const ArgsT<float>& a, int first, int 
     const int j[1] = {col != p ? col : -1};
     float x[1][5];
     if (!wait_reactions<float, 1>(a, j, p, sweep, x)) v[2] += 1.0;
-    __syncwarp();  // the lanes left the wait one by one: together again
     if (j[0] < 0) continue;
     const float* blk = a.W + 25 * (size_t)(s0 + t);
     for (int k = 0; k < 5; k++)
