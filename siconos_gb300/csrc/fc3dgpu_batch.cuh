@@ -2,7 +2,6 @@
 //
 // The problems are one block-diagonal union layout (rows permuted by
 // problem, then colour, each (problem, colour) group padded to 32-row slabs).
-// problem, then colour, each (problem, colour) group padded to 32-row slabs).
 // A problem is solved by one block, or by a team of blocks that splits every
 // colour's slabs evenly and meets at a bounded barrier of its own between
 // colours; blocks without a team, and teams that are done, pull problems one
@@ -16,8 +15,13 @@
 // latency chain, so a batch with few problems is as slow as its largest
 // problem on one SM; the teams (batch_plan in fc3dgpu_ctx.cu) give the large
 // problems the idle SMs.  48 lattices of 130 to 8,901 contacts, 100 FP32
-// sweeps: 28.3 ms one block each, 7.6 ms in teams; 200 lattices, 30 sweeps:
-// 11.1 and 7.2 ms; in FP64, 48 lattices and 100 sweeps, 50 ms in teams.
+// sweeps: 28.3 ms one block each, 7.6 ms in teams by colours, 4.3 as dataflow
+// (fc3dgpu_batch_flow.cuh); 200 lattices, 30 sweeps: 11.1, 7.2 and 3.3 ms.
+// In FP64, us a sweep in teams by colours and as dataflow: 2 lattices 279 and
+// 214, 10: 294 and 240, 24: 385 and 326; with more than 110 contacts a colour
+// and block the FP64 pipes are full either way (40 lattices 463 and 489), and
+// so they are with one block a problem (100 small lattices 443 and 455 with
+// the same line there): those of up to 40 contacts a colour are dataflow.
 #pragma once
 #include "fc3dgpu_batch_args.cuh"
 #include "fc3dgpu_sweep.cuh"
@@ -120,14 +124,29 @@ __device__ __forceinline__ bool scene_full_error(const BatchArgs<Real>& b, int p
 }
 
 // How a block sweeps a problem's colours.  ColourSweep: colour by colour, the
-// team's barrier between them (the sums' barrier closes the last one).
+// team's barrier between them (the sums' barrier closes the last one); in FP64
+// as dataflow (fc3dgpu_flow64.cuh) where stamped reactions are given and the
+// team's blocks have few contacts of a colour.
 template <typename Real>
 struct ColourSweep {
   typename RangeList<Real>::type& wk;
-  __device__ __forceinline__ void open(const BatchArgs<Real>&, const int*, int, const BatchTeam&) {}
-  __device__ __forceinline__ bool sweep(const BatchArgs<Real>& b, const int* sptr, int ncol, int, Real local_tol,
+  int rows;  // of a dataflow unit, 0: by colours
+  __device__ __forceinline__ void open(const BatchArgs<Real>& b, const int* sptr, int ncol, const BatchTeam& t) {
+    rows = 0;
+#ifndef FC3D_FAST_F64
+    if constexpr (sizeof(Real) == sizeof(double))
+      if (b.base.rs && (sptr[ncol] - sptr[0]) * FC3D_SLAB <=
+                           ncol * (t.size > 1 ? FC3D_BATCH_FLOW64_MAX * t.size : FC3D_BATCH_FLOW64_ALONE))
+        rows = flow64_rows(sptr, ncol, t.size);
+#endif
+  }
+  __device__ __forceinline__ bool sweep(const BatchArgs<Real>& b, const int* sptr, int ncol, int sweep, Real local_tol,
                                         double acc[3], BatchTeam& t) {
     const SweepArgs<Real>& a = b.base;
+#ifndef FC3D_FAST_F64
+    if constexpr (sizeof(Real) == sizeof(double))
+      if (rows > 0) return flow64_sweep(a, sptr, ncol, rows, t.rank, t.size, sweep, local_tol, acc[0], acc[1]);
+#endif
     for (int c = 0; c < ncol; c++) {
       const int s0 = sptr[c], n = sptr[c + 1] - s0;
       process_range<Real>(a, s0 + n * t.rank / t.size, s0 + n * (t.rank + 1) / t.size, local_tol, acc[0], acc[1], wk,
@@ -286,7 +305,7 @@ __device__ __forceinline__ void batch_problems(const BatchArgs<Real>& b, Sweep& 
 template <typename Real>
 __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_batch_kernel(const BatchArgs<Real> b) {
   __shared__ typename RangeList<Real>::type wk;
-  ColourSweep<Real> sw = {wk};
+  ColourSweep<Real> sw = {wk, 0};
   batch_problems<Real>(b, sw);
 }
 

@@ -6,6 +6,10 @@
 #define FC3D_BATCH_BLOCKS 1024
 // Warps of a block of the FP32 batched kernel
 #define FC3D_BATCH_WARPS32 10
+// Contacts a colour and block up to which a problem's FP64 sweeps go as
+// dataflow: of a team's blocks, of a block alone (measured in fc3dgpu_batch.cuh)
+#define FC3D_BATCH_FLOW64_MAX 110
+#define FC3D_BATCH_FLOW64_ALONE 40
 
 namespace fc3dgpu {
 

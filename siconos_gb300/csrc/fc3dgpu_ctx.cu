@@ -2506,6 +2506,11 @@ static int record_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
     b.scene_out_prev = mixed ? c->sout32 : nullptr;
     const int which = p->precision >= 2 ? 2 : 1;
     if (int rc = attach_teams(c, b, which)) return rc;
+    if (which == 1 && c->flow_on && c->symmetric == 1) {
+      k_stamp64<<<grid1d(c->npad + 1), 256, 0, s>>>(c->npad, c->r64, c->rs64);
+      CK(cudaGetLastError());
+      b.base.rs = c->rs64;
+    }
     if (which == 2)
       CK(fc3dgpu_launch_batch_f64_fast(&b, c->batch_plans[2].grid, s));
     else
@@ -2539,6 +2544,10 @@ extern "C" int fc3dgpu_ctx_solve_batch(fc3dgpu_ctx* c, const fc3dgpu_params* p, 
     }
     int resident[3];
     if (int rc = prepare_batch_flow(c, &resident[0])) return rc;
+    if (c->flow_on) {
+      if (int rc = look_symmetric(c)) return rc;
+      if (c->symmetric == 1) CK(ensure(&c->rs64, &c->rs64_cap, ((size_t)c->npad + 1) * 4));
+    }
     CK(batch_grid_f64(&resident[1]));
     CK(fc3dgpu_batch_grid_f64_fast(&resident[2]));
     CK(ensure(&c->steams, &c->steams_cap, (size_t)3 * FC3D_BATCH_BLOCKS));

@@ -9,13 +9,14 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dims", [[(20, 19, 9), (3, 3, 2), (12, 11, 6)], [(2, 2, 1), (25, 24, 12)]],
                          ids=["three", "tiny-and-large"])
-@pytest.mark.parametrize("precision,flow", [(0, True), (0, False), (1, True)], ids=["fp32", "fp32-colours", "fp64"])
+@pytest.mark.parametrize("precision,flow", [(0, True), (0, False), (1, True), (1, False)],
+                         ids=["fp32", "fp32-colours", "fp64", "fp64-colours"])
 def test_team_equals_solo_bitwise(gpu, dims, precision, flow):
     from siconos_gb300 import scene
     from siconos_gb300.device import DeviceSolver
     scs = [scene.lattice(*d, seed=50 + k, mu=0.3 + 0.2 * k) for k, d in enumerate(dims)]
     kw = dict(tol=1e-300, max_iter=12, precision=precision, fp32_only=1 - precision)
-    gpu.flow(flow)  # the FP32 sweeps as dataflow, or colour by colour
+    gpu.flow(flow)  # the sweeps as dataflow, or colour by colour
     try:
         gpu.load_batch(scs)
         st = gpu.solve_batch(**kw)
@@ -23,7 +24,7 @@ def test_team_equals_solo_bitwise(gpu, dims, precision, flow):
         gpu.flow(True)
     rb, ub = gpu.get_batch()
     solo = DeviceSolver(0)
-    solo.flow(False)  # the coloured FP32 kernel, whose stop rules the batch has (the dataflow stops a sweep later)
+    solo.flow(False)  # the coloured kernels, whose stop rules the batch has (the dataflow stops a sweep later)
     for k, s in enumerate(scs):
         solo.load(s)
         one = solo.solve(lanes=1, **kw)
