@@ -32,7 +32,9 @@ struct FlowSweep {
     slab0 = sptr[0];
     const int n = sptr[ncol] - slab0;
     tw = t.size * FC3D_BATCH_WARPS32;
-    gw = t.rank * FC3D_BATCH_WARPS32 + (threadIdx.x >> 5);
+    // a colour's units over the team's blocks first (warps first: 2 lattices 1.48
+    // ms for 30 sweeps, 1.38 so; 48 lattices, 100 sweeps 4.33 and 4.13)
+    gw = (threadIdx.x >> 5) * t.size + t.rank;
     for (sh = 0; sh < 5 && (n << (sh + 1)) <= tw;) sh++;
     units = n << sh;
     if (gw < units) {
