@@ -15,8 +15,8 @@
 // latency chain, so a batch with few problems is as slow as its largest
 // problem on one SM; the teams (batch_plan in fc3dgpu_ctx.cu) give the large
 // problems the idle SMs.  48 lattices of 130 to 8,901 contacts, 100 FP32
-// sweeps: 28.3 ms one block each, 7.6 ms in teams by colours, 4.3 as dataflow
-// (fc3dgpu_batch_flow.cuh); 200 lattices, 30 sweeps: 11.1, 7.2 and 3.3 ms.
+// sweeps: 28.3 ms one block each, 7.6 ms in teams by colours, 3.6 as dataflow
+// (fc3dgpu_batch_flow.cuh); 200 lattices, 30 sweeps: 11.1, 7.2 and 3.0 ms.
 // In FP64, us a sweep in teams by colours and as dataflow: 2 lattices 279 and
 // 214, 10: 294 and 240, 24: 385 and 326; with more than 110 contacts a colour
 // and block the FP64 pipes are full either way (40 lattices 463 and 489), and
@@ -66,47 +66,63 @@ __device__ __forceinline__ bool team_sync(BatchTeam& t, unsigned* flags, unsigne
   return s_ok != 0;
 }
 
-// Sums of three values per thread over the team in a fixed order (warp tree,
-// warps in order, blocks in order), the same bits in every thread.  The block
-// sums of a team go through a ring of two slots in global memory: a block
-// writes slot k & 1 only after the barrier of call k - 1, which every block
-// passes after reading call k - 2's slot.
+// Sums of three values per thread over the team in a fixed order (warps, then
+// the block's warps, then the team's blocks, each a butterfly that carries the
+// three values; all but the first by one warp), the same bits in every thread;
+// LIGHT: out[0] alone, the light error of the sums 0 and 1.  The block sums of
+// a team go through a ring of two slots in global memory: a block writes slot
+// k & 1 only after the barrier of call k - 1, which every block passes after
+// reading call k - 2's slot.
 struct TeamSum {
   double warp[FC3D_BLOCK_MAX / 32][3];
+  double out[3];
 };
-template <typename Real>
+template <bool LIGHT, typename Real>
 __device__ __forceinline__ bool team_reduce3(const BatchArgs<Real>& b, BatchTeam& t, TeamSum& S, double v[3],
                                              double out[3]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = lane >> 3, k = lane & 7;
+  {
+    // value 0 in lane 0, 1 in lane 8, 2 in lane 16
+    const bool b16 = lane & 16, b8 = lane & 8;
+    const double x = (b16 ? v[2] : v[0]) + __shfl_xor_sync(full, b16 ? v[0] : v[2], 16);
+    const double y = v[1] + __shfl_xor_sync(full, v[1], 16);
+    double z = (b8 ? y : x) + __shfl_xor_sync(full, b8 ? x : y, 8);
 #pragma unroll
-  for (int i = 0; i < 3; i++) {
-    double x = v[i];
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) S.warp[w][i] = x;
+    for (int o = 4; o >= 1; o >>= 1) z += __shfl_xor_sync(full, z, o);
+    if (k == 0 && i < 3) S.warp[w][i] = z;
   }
   __syncthreads();
-  double s[3] = {0.0, 0.0, 0.0};
-  for (int k = 0; k < (int)(blockDim.x >> 5); k++)
-#pragma unroll
-    for (int i = 0; i < 3; i++) s[i] += S.warp[k][i];
-  if (t.size == 1) {
-#pragma unroll
-    for (int i = 0; i < 3; i++) out[i] = s[i];
-    __syncthreads();
-    return true;
-  }
   double* ring = b.team_part + (size_t)(t.epoch & 1) * FC3D_BATCH_BLOCKS * 4;
-  if (threadIdx.x == 0)
+  double y = 0.0;
+  if (w == 0) {
+    if (i < 3)
+      for (int q = k; q < (int)(blockDim.x >> 5); q += 8) y += S.warp[q][i];
 #pragma unroll
-    for (int i = 0; i < 3; i++) __stcg(&ring[4 * blockIdx.x + i], s[i]);
-  if (!team_sync(t, b.base.barrier, b.base.spin_limit, b.base.status)) return false;
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    double x = 0.0;
-    for (int k = 0; k < t.size; k++) x += __ldcg(&ring[4 * (t.first + k) + i]);
-    out[i] = x;
+    for (int o = 4; o >= 1; o >>= 1) y += __shfl_xor_sync(full, y, o);
+    if (t.size > 1 && k == 0 && i < 3) __stcg(&ring[4 * blockIdx.x + i], y);
   }
+  if (t.size > 1 && !team_sync(t, b.base.barrier, b.base.spin_limit, b.base.status)) return false;
+  if (w == 0) {
+    if (t.size > 1) {
+      y = 0.0;
+      if (i < 3)
+        for (int q = k; q < t.size; q += 8) y += __ldcg(&ring[4 * (t.first + q) + i]);
+#pragma unroll
+      for (int o = 4; o >= 1; o >>= 1) y += __shfl_xor_sync(full, y, o);
+    }
+    if (LIGHT) {
+      // the second sum to lane 16, where warp_light_error takes it
+      const double second = __shfl_sync(full, y, 8);
+      y = warp_light_error(lane == 16 ? second : y);
+      if (lane == 0) S.out[0] = y;
+    } else if (k == 0 && i < 3) {
+      S.out[i] = y;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < (LIGHT ? 1 : 3); q++) out[q] = S.out[q];
   return true;
 }
 
@@ -115,10 +131,10 @@ __device__ __forceinline__ bool scene_full_error(const BatchArgs<Real>& b, int p
                                                  BatchTeam& t, TeamSum& S, double& full) {
   double v[3], s[3];
   full_error_rows(b.base, v, p0, p1, t.rank * blockDim.x + threadIdx.x, t.size * blockDim.x);
-  if (!team_reduce3(b, t, S, v, s)) return false;
-  double e = sqrt(s[0]);
-  const double scal = fmax(norm_q, fmax(sqrt(s[2]), sqrt(s[1])));
-  if (fabs(scal) > DBL_EPSILON) e /= scal;
+  if (!team_reduce3<false>(b, t, S, v, s)) return false;
+  double e = ie_sqrt(s[0]);
+  const double scal = fmax(norm_q, fmax(ie_sqrt(s[2]), ie_sqrt(s[1])));
+  if (fabs(scal) > DBL_EPSILON) e = ie_div(e, scal);
   full = e;
   return true;
 }
@@ -193,10 +209,8 @@ __device__ __forceinline__ bool solve_scene(const BatchArgs<Real>& b, int scene,
     double acc[3] = {0.0, 0.0, 0.0};
     if (!sw.sweep(b, sptr, ncol, sweep, (Real)local_tol, acc, t)) return false;
     double s[3];
-    if (!team_reduce3(b, t, S, acc, s)) return false;
-    incr = sqrt(s[0]);
-    const double nr = sqrt(s[1]);
-    if (fabs(nr) > DBL_EPSILON) incr /= nr;
+    if (!team_reduce3<true>(b, t, S, acc, s)) return false;
+    incr = s[0];
     bool stop = false;
     if (a.mode == 1) {
       if (incr < working) {

@@ -2,8 +2,8 @@
 // the single-problem dataflow kernel does (fc3dgpu_flow.cuh), with no barrier
 // between colours.  What bounds a sweep of the colour-by-colour form is its
 // six barriers with a load, product, list and solve phase each (76 us a sweep
-// for the largest of 48 lattices in teams, 42 us as dataflow; 512 lattices, 30
-// sweeps: 13.4 and 7.1 ms).  Needs a symmetric block
+// for the largest of 48 lattices in teams, 36 us as dataflow; 512 lattices, 30
+// sweeps: 13.4 and 6.8 ms).  Needs a symmetric block
 // pattern (stamped reactions) and slabs that fit the warps' buffers; the
 // colour-by-colour form stays for the others.
 #pragma once

@@ -144,30 +144,36 @@ __device__ __forceinline__ bool flow_full_error(const SweepArgs<float>& a, unsig
   return true;
 }
 
-// Wait until every block's flag shows epoch e (bounded; warp 0 polls, then
-// an acquire fence and a block barrier).  False when the wait gave up or a
-// timeout anywhere is on record: one value for the whole block (read once,
-// shared), so every warp leaves the sweep loop at the same barrier.
+// One warp waits until every block's flag shows epoch e (bounded), then an
+// acquire fence.  False when the wait gave up or a timeout anywhere is on
+// record (the same in all its lanes).
+__device__ __forceinline__ bool grid_poll(const unsigned* flags, unsigned e, unsigned long long limit, int* status) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long n = 0;
+  int ok = 1;
+  for (;;) {
+    bool mine = true;
+    for (int b = lane; b < (int)gridDim.x; b += 32)
+      mine &= (ld_relaxed_u32(&flags[b * FC3D_FLAG_STRIDE]) >= e);
+    if (__all_sync(0xffffffffu, mine)) break;
+    if (++n > limit) {
+      ok = 0;
+      if (lane == 0) atomicOr(status, 1);
+      break;
+    }
+    if (n > 256) __nanosleep(32);
+  }
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  ok = ok && !(*(volatile int*)status & 1);
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+// ... for the whole block (warp 0 polls): one value, read once and shared, so
+// every warp leaves the sweep loop at the same barrier.
 __device__ __forceinline__ bool grid_wait(const unsigned* flags, unsigned e, unsigned long long limit, int* status) {
   __shared__ int s_ok;
   if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    unsigned long long n = 0;
-    int ok = 1;
-    for (;;) {
-      bool mine = true;
-      for (int b = lane; b < (int)gridDim.x; b += 32)
-        mine &= (ld_relaxed_u32(&flags[b * FC3D_FLAG_STRIDE]) >= e);
-      if (__all_sync(0xffffffffu, mine)) break;
-      if (++n > limit) {
-        ok = 0;
-        if (lane == 0) atomicOr(status, 1);
-        break;
-      }
-      if (n > 256) __nanosleep(32);
-    }
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    if (lane == 0) s_ok = ok && !(*(volatile int*)status & 1);
+    const bool ok = grid_poll(flags, e, limit, status);
+    if (threadIdx.x == 0) s_ok = ok;
   }
   __syncthreads();
   return s_ok != 0;
@@ -468,16 +474,15 @@ __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<f
   int sweep = 0, best_sweep = 0;
   bool converged = false, aborted = false, stopped = false;
   const double target = fmax(a.user_tol, a.switch_tol);
+  // by one warp, after every block's end of sweep j
   auto light_error = [&](int j) {
-    double sm[2];
-    grid_sum<2>(f.part, (j & 3) * 2, sm);
-    double e = sqrt(sm[0]);
-    const double nr = sqrt(sm[1]);
-    if (fabs(nr) > DBL_EPSILON) e /= nr;
-    if (a.trace && blockIdx.x == 0 && threadIdx.x == 0 && a.trace_base + j - 1 < a.trace_cap)
-      a.trace[a.trace_base + j - 1] = e;
+    const double e = grid_light_error(f.part, (j & 3) * 2);
+    if (a.trace && blockIdx.x == 0 && lane == 0 && a.trace_base + j - 1 < a.trace_cap) a.trace[a.trace_base + j - 1] = e;
     return e;
   };
+  enum Act { GO_ON, STOP, CHECK, GIVE_UP };
+  __shared__ int s_act;
+  __shared__ double s_e;
   // the full error of the current iterate once every block ended sweep j
   // (epoch e_end); adapts the working tolerance as the coloured kernel does
   auto full_check = [&](double incr_j, unsigned e_end) {
@@ -543,32 +548,54 @@ __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<f
       if (tl) tl[4] = globaltimer_ns();
       if (!STAMP) flow_signal(f, x.d0, x.d1, x.dep0, x.dep1, lane);
     }
-    flow_block_sum<2, NW>(acc, f.part + blockIdx.x * 8 + (sweep & 3) * 2);
+    block_sum2(acc, f.part + blockIdx.x * 8 + (sweep & 3) * 2);
     e_prev = e_last;
     e_last = ++epoch;
-    if (threadIdx.x == 0) st_release_u32(&a.barrier[blockIdx.x * FC3D_FLAG_STRIDE], e_last);
-    if (sweep < 2) continue;
-    if (!grid_wait(a.barrier, e_prev, a.spin_limit, a.status)) {
+    if (w == 0) {
+      __syncwarp();
+      if (lane == 0) st_release_u32(&a.barrier[blockIdx.x * FC3D_FLAG_STRIDE], e_last);
+    }
+    if (sweep < 2) {
+      __syncthreads();
+      continue;
+    }
+    // warp 0 decides for the block
+    if (w == 0) {
+      int act = GO_ON;
+      double e1 = 0.0;
+      if (!grid_poll(a.barrier, e_prev, a.spin_limit, a.status)) {
+        act = GIVE_UP;
+      } else {
+        // the FP32 accelerator's stop rules on sweep - 1, as the coloured
+        // kernel applies them to each sweep
+        e1 = light_error(sweep - 1);
+        if (!(e1 == e1)) {
+          if (lane == 0) atomicOr(a.status, 2);
+          act = STOP;
+        }
+        if (e1 < a.switch_tol) act = STOP;
+        if (e1 < 0.99 * best) {
+          best = e1;
+          best_sweep = sweep - 1;
+        } else if (a.stall_window > 0 && sweep - 1 - best_sweep >= a.stall_window) {
+          act = STOP;
+        }
+        if (act == GO_ON && e1 < working) act = CHECK;
+      }
+      if (lane == 0) {
+        s_act = act;
+        s_e = e1;
+      }
+    }
+    __syncthreads();
+    const int act = s_act;
+    if (act == GIVE_UP) {
       aborted = true;
       break;
     }
-    // the FP32 accelerator's stop rules on sweep - 1, as the coloured
-    // kernel applies them to each sweep
-    const double e1 = light_error(sweep - 1);
-    bool stop = false;
-    if (!(e1 == e1)) {
-      if (threadIdx.x == 0) atomicOr(a.status, 2);
-      stop = true;
-    }
-    if (e1 < a.switch_tol) stop = true;
-    if (e1 < 0.99 * best) {
-      best = e1;
-      best_sweep = sweep - 1;
-    } else if (a.stall_window > 0 && sweep - 1 - best_sweep >= a.stall_window) {
-      stop = true;
-    }
-    if (!stop && e1 < working) {
-      if (!full_check(e1, e_last)) {
+    bool stop = act == STOP;
+    if (act == CHECK) {
+      if (!full_check(s_e, e_last)) {
         aborted = true;
         break;
       }
@@ -585,7 +612,13 @@ __global__ void __launch_bounds__(NW * 32, 1) nsgs_flow_kernel(const SweepArgs<f
     if (!grid_wait(a.barrier, e_last, a.spin_limit, a.status)) {
       aborted = true;
     } else {
-      incr = light_error(sweep);
+      if (w == 0) {
+        const double e = light_error(sweep);
+        if (lane == 0) s_e = e;
+      }
+      __syncthreads();
+      incr = s_e;
+      __syncthreads();
       if (!stopped) {
         bool stop = false;
         if (!(incr == incr)) {

@@ -17,6 +17,7 @@
 #include <cfloat>
 #include <cuda_runtime.h>
 
+#include "fc3dgpu_ieee64.cuh"
 #include "fc3dgpu_layout.cuh"
 #include "fc3dgpu_coop64.cuh"
 
@@ -143,6 +144,57 @@ __device__ __forceinline__ void block_sum(double v[N], double* out_partials) {
     out_partials[threadIdx.x] = s;
   }
   __syncthreads();
+}
+
+// The light error's sums.  An FP64 addition holds an SM quarter's pipe for 64
+// cycles, so what all warps of a block compute alike (sums over warps and
+// blocks, roots, the quotient) is dear at the end of every sweep.  Here each
+// butterfly carries both values (half the lanes each) and one warp does the
+// rest.  us a sweep before and after: 42 contacts FP32 23.8 and 21.3, FP64 85
+// and 83; 2 batched lattices FP32 46 and 36; the large FP32 dataflow, whose
+// blocks end a sweep at different times, the same.
+//
+// Both values of every lane summed over the warp: value 0 in lane 0, value 1
+// in lane 16.
+__device__ __forceinline__ double warp_sum2(double v0, double v1) {
+  const bool hi = threadIdx.x & 16;
+  double x = (hi ? v1 : v0) + __shfl_xor_sync(0xffffffffu, hi ? v0 : v1, 16);
+#pragma unroll
+  for (int o = 8; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+// ... over the block (at most 16 warps), written by warp 0 to out[0], out[1].
+// `sh` is free again after the block's next barrier.
+__device__ __forceinline__ void block_sum2(const double v[2], double* out) {
+  __shared__ double sh[16][2];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = lane & 15;
+  const double x = warp_sum2(v[0], v[1]);
+  if (k == 0) sh[w][lane >> 4] = x;
+  __syncthreads();
+  if (w == 0) {
+    double y = k < (int)(blockDim.x >> 5) ? sh[k][lane >> 4] : 0.0;
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    if (k == 0) out[lane >> 4] = y;
+  }
+}
+// sqrt(s0 / s1) as the reference forms it, by one warp from lane 0's and lane
+// 16's sums; the same in all its lanes.
+__device__ __forceinline__ double warp_light_error(double sum) {
+  const double root = ie_sqrt(sum);
+  const double e = __shfl_sync(0xffffffffu, root, 0), nr = __shfl_sync(0xffffffffu, root, 16);
+  return fabs(nr) > DBL_EPSILON ? ie_div(e, nr) : e;
+}
+// The light error from every block's partials in slots slot0 and slot0 + 1, by
+// one warp
+__device__ __forceinline__ double grid_light_error(const double* partials, int slot0) {
+  const int lane = threadIdx.x & 31;
+  double y = 0.0;
+#pragma unroll 5
+  for (int b = lane & 15; b < (int)gridDim.x; b += 16) y += __ldcg(&partials[b * 8 + slot0 + (lane >> 4)]);
+#pragma unroll
+  for (int o = 8; o >= 1; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+  return warp_light_error(y);
 }
 
 // Sum slot k of every block's partials in a fixed order; every block gets
@@ -1228,7 +1280,7 @@ __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_kernel(const Sw
     if constexpr (FLOW) {
       if (!flow64_sweep(a, a.sptr, a.ncol, rows64, blockIdx.x, gridDim.x, sweep, local_tol, acc[0],
                         acc[1])) return;
-      block_sum<2>(acc, a.partials + blockIdx.x * 8);
+      block_sum2(acc, a.partials + blockIdx.x * 8);
       if (!grid_barrier(a.barrier, epoch, a.spin_limit, a.status)) return;
     }
     for (int c = 0; c < (FLOW ? 0 : a.ncol); c++) {
@@ -1271,7 +1323,7 @@ __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_kernel(const Sw
           }
         }
       }
-      if (c == a.ncol - 1) block_sum<2>(acc, a.partials + blockIdx.x * 8);
+      if (c == a.ncol - 1) block_sum2(acc, a.partials + blockIdx.x * 8);
       if (tl) a.timeline[((size_t)c * gridDim.x + blockIdx.x) * FC3D_TL_STRIDE + 1] = globaltimer_ns();
       const bool ok = (local_sync && c < a.ncol - 1)
                           ? nbr_barrier(a.barrier, epoch, a.nbr + a.nbr_ptr[blockIdx.x],
@@ -1282,11 +1334,14 @@ __global__ void __launch_bounds__(BlockDim<Real>::value, 1) nsgs_kernel(const Sw
         return;
       }
     }
-    double s[2];
-    grid_sum<2>(a.partials, 0, s);
-    incr = sqrt(s[0]);
-    const double nr = sqrt(s[1]);
-    if (fabs(nr) > DBL_EPSILON) incr /= nr;
+    __shared__ double s_incr;
+    if (threadIdx.x < 32) {
+      const double e = grid_light_error(a.partials, 0);
+      if (lane == 0) s_incr = e;
+    }
+    __syncthreads();
+    incr = s_incr;
+    __syncthreads();
     if (a.trace && blockIdx.x == 0 && threadIdx.x == 0 && a.trace_base + sweep - 1 < a.trace_cap)
       a.trace[a.trace_base + sweep - 1] = incr;
     bool stop = false;
