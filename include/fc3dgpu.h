@@ -273,8 +273,8 @@ int fc3dgpu_ctx_sync(fc3dgpu_ctx *ctx, int neighbourhood);
  * symmetric pattern with at most 150 contacts a colour and SM.  Returns the
  * previous setting. */
 int fc3dgpu_ctx_flow(fc3dgpu_ctx *ctx, int on);
-/* Warps per block of the dataflow sweep: 8, 10 or 12 (0: the default, 10,
- * or the autotuner's choice); fewer when the per-warp buffers of the current
+/* Warps per block of the dataflow sweep: 8, 10 or 12 (0: the default, by the
+ * number of slabs, or the autotuner's choice); fewer when the per-warp buffers of the current
  * layout do not fit.  Returns the previous request. */
 int fc3dgpu_ctx_flow_warps(fc3dgpu_ctx *ctx, int nw);
 /* Measuring autotuner of the sweep variant, run at the first solve of a new

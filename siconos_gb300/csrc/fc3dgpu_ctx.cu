@@ -1570,6 +1570,8 @@ extern "C" int fc3dgpu_ctx_flow(fc3dgpu_ctx* c, int on) {
   return old;
 }
 
+static int default_flow_warps(const fc3dgpu_ctx* c);
+
 extern "C" int fc3dgpu_ctx_flow_warps(fc3dgpu_ctx* c, int nw) {
   if (!c) return -1;
   if (nw != 0 && nw != 8 && nw != 10 && nw != 12) {
@@ -1580,7 +1582,7 @@ extern "C" int fc3dgpu_ctx_flow_warps(fc3dgpu_ctx* c, int nw) {
   c->flow_want = nw;
   if (c->flow_state == 1) {
     if (cudaSetDevice(c->device) != cudaSuccess) return NUMERICS_ERR_UNKNOWN;
-    const int got = fc3dgpu::flow_warps(c->flow_maxslot, nw);
+    const int got = fc3dgpu::flow_warps(c->flow_maxslot, default_flow_warps(c));
     if (got > 0) c->flow_nw = got;
   }
   return old;
@@ -1839,25 +1841,32 @@ static int prepare_batch_flow(fc3dgpu_ctx* c, int* resident) {
   return 0;
 }
 
-// Column-slab lists of the dataflow sweep for the current layout; leaves
-// c->flow_state 1 when the sweep applies, -1 when not (slabs longer than
-// FC3D_FLOW_MAXSLOT or than the per-warp buffers allow).
-static int prepare_flow(fc3dgpu_ctx* c) {
+// Warps a block of the FP32 dataflow where none are asked for: 10, or on
+// stamped reactions 8 or 12 where that takes a tenth less by rounds of slabs
+// times a round's time, which grows about as the warps plus two.  us a sweep
+// with 8, 10 and 12 warps, the choice last: 57,800 contacts 30.5, 36.6, 31.4
+// (12); 68,688 30.3, 33.1, 37.8 (8); 96,780 35.2, 31.2, 32.2 (10); 109,368 32.9,
+// 35.4, 32.1 (12); 164,400 36.0, 38.0, 36.0 (12); 216,346 36.4, 38.9, 39.7 (10);
+// 260,288 42.5, 41.3, 42.6 (10).  Up to a slab a warp, 10.
+static int default_flow_warps(const fc3dgpu_ctx* c) {
+  if (c->flow_want > 0 || c->symmetric != 1 || c->nslab <= 10LL * c->nsm) return c->flow_want;
+  auto cost = [&](int nw) {
+    const long long warps = (long long)nw * c->nsm;
+    return (c->nslab + warps - 1) / warps * (nw + 2);
+  };
+  const int other = cost(8) < cost(12) ? 8 : 12;
+  return 10 * cost(other) <= 9 * cost(10) ? other : 10;
+}
+
+// The neighbour-slab lists and arrival counters of the dataflow sweep for a
+// pattern that is not symmetric.
+static int build_flow_lists(fc3dgpu_ctx* c) {
   using namespace fc3dgpu;
-  if (c->flow_state != 0) return 0;
-  c->flow_state = -1;
-  if (c->nscenes > 0 || c->ncol < 2 || c->nslab <= 0) return 0;
-  int maxslot = 0;
-  for (int s = 0; s < c->nslab; s++) maxslot = std::max(maxslot, c->slab_nslot_h[s]);
-  if (maxslot > FC3D_FLOW_MAXSLOT) return 0;
-  const int nw = flow_warps(maxslot, c->flow_want);
-  if (nw == 0) return 0;
   cudaStream_t s = c->stream;
   const int nslab = c->nslab;
   CK(ensure(&c->flow_dptr, &c->flow_dptr_cap, (size_t)nslab + 1));
   CK(ensure(&c->flow_done, &c->flow_done_cap, (size_t)nslab));
   CK(ensure(&c->flow_sptr, &c->flow_sptr_cap, FC3D_MAX_COLOURS + 1));
-  CK(ensure(&c->flow_part, &c->flow_part_cap, 1024 * 8));
   CK(cudaMemcpyAsync(c->flow_sptr, c->sptr, sizeof(int) * (FC3D_MAX_COLOURS + 1), cudaMemcpyHostToDevice, s));
   // column-slab counts, their prefix sum on the host, then the lists
   CK(build_flow_deps(nslab, c->npad, c->ncol, c->flow_sptr, c->perm, c->slab_nslot, c->slab_off, c->col, nullptr,
@@ -1910,8 +1919,30 @@ static int prepare_flow(fc3dgpu_ctx* c) {
   CK(cudaMemcpyAsync(c->flow_dptr, sptr_sym.data(), sizeof(int) * (nslab + 1), cudaMemcpyHostToDevice, s));
   if (!sym.empty()) CK(cudaMemcpyAsync(c->flow_dep, sym.data(), sizeof(int) * sym.size(), cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(c->flow_need, need.data(), sizeof(int2) * nslab, cudaMemcpyHostToDevice, s));
-  if (int rc = prepare_records(c)) return rc;
+  CK(cudaStreamSynchronize(s));
   c->launches += 2;
+  return 0;
+}
+
+// What the dataflow sweep needs of the current layout; leaves
+// c->flow_state 1 when the sweep applies, -1 when not (slabs longer than
+// FC3D_FLOW_MAXSLOT or than the per-warp buffers allow).
+static int prepare_flow(fc3dgpu_ctx* c) {
+  using namespace fc3dgpu;
+  if (c->flow_state != 0) return 0;
+  c->flow_state = -1;
+  if (c->nscenes > 0 || c->ncol < 2 || c->nslab <= 0) return 0;
+  int maxslot = 0;
+  for (int s = 0; s < c->nslab; s++) maxslot = std::max(maxslot, c->slab_nslot_h[s]);
+  if (maxslot > FC3D_FLOW_MAXSLOT) return 0;
+  if (flow_warps(maxslot, 8) == 0) return 0;
+  CK(ensure(&c->flow_part, &c->flow_part_cap, 1024 * 8));
+  if (int rc = prepare_records(c)) return rc;
+  // stamped reactions (a symmetric pattern) need no lists of neighbour slabs
+  if (c->symmetric != 1)
+    if (int rc = build_flow_lists(c)) return rc;
+  const int nw = flow_warps(maxslot, default_flow_warps(c));
+  if (nw == 0) return 0;
   c->flow_nw = nw;
   c->flow_maxslot = maxslot;
   c->flow_state = 1;
@@ -2022,7 +2053,7 @@ static int autotune(fc3dgpu_ctx* c, const fc3dgpu_params* p) {
   }
   if (!all) best64 = 0.f;  // one lane per contact, unmeasured
   c->flow_want = want;
-  if (c->flow_state == 1) c->flow_nw = c->tune_flow ? c->tune_nw : flow_warps(c->flow_maxslot, want);
+  if (c->flow_state == 1) c->flow_nw = c->tune_flow ? c->tune_nw : flow_warps(c->flow_maxslot, default_flow_warps(c));
   c->timeline = tl;
   c->timeline_sweep = tls;
   c->counters_on = cnt;
@@ -2190,7 +2221,7 @@ static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
         while (f.split < 5 && ((long long)c->nslab << (f.split + 1)) <= (long long)sms * c->flow_nw) f.split++;
       }
-      CK(cudaMemsetAsync(c->flow_done, 0, sizeof(unsigned) * c->nslab, s));
+      if (!f.stamped) CK(cudaMemsetAsync(c->flow_done, 0, sizeof(unsigned) * c->nslab, s));
       CK(pack_flow_records(c->nslab, c->slab_off, c->slab_nslot, c->W32, c->col, c->q32, c->D32, c->mu32, c->rho32,
                            c->flow_rec_off, c->flow_rec, s));
       c->launches++;
