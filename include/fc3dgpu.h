@@ -270,12 +270,12 @@ int fc3dgpu_ctx_sync(fc3dgpu_ctx *ctx, int neighbourhood);
  * colours); 0 the coloured kernel above.  The same sweep either way.  Applies
  * with one lane per contact, in FP32 when no slab has more than 16
  * off-diagonal slots, in FP64 (bit-exact arithmetic, no timeline) on a
- * symmetric pattern with at most 150 contacts a colour and SM.  Returns the
- * previous setting. */
+ * symmetric pattern (rows of at most 64 blocks off the diagonal) with at most
+ * 150 contacts a colour and SM.  Returns the previous setting. */
 int fc3dgpu_ctx_flow(fc3dgpu_ctx *ctx, int on);
 /* Warps per block of the dataflow sweep: 8, 10 or 12 (0: the default, by the
- * number of slabs, or the autotuner's choice); fewer when the per-warp buffers of the current
- * layout do not fit.  Returns the previous request. */
+ * number of slabs, or the autotuner's choice); fewer when the per-warp
+ * buffers of the current layout do not fit.  Returns the previous request. */
 int fc3dgpu_ctx_flow_warps(fc3dgpu_ctx *ctx, int nw);
 /* Measuring autotuner of the sweep variant, run at the first solve of a new
  * structure with automatic lanes (fc3dgpu_params.lanes = 0): it times a few

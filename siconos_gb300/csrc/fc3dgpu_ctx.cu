@@ -1791,9 +1791,17 @@ static size_t staging_sizes(fc3dgpu_ctx* c, int grid, unsigned* wb, unsigned* cb
 }
 
 // c->symmetric of the current layout: every block has its transpose's place
-// in W (the stamped dataflow sweeps need it).
+// in W (the stamped dataflow sweeps need it).  A row's search goes through its
+// neighbours' slabs, so its time goes with the square of the longest row: from
+// 64 blocks on (rows of a few hundred took milliseconds) the pattern counts as
+// not symmetric and the sweeps go by colours.
 static int look_symmetric(fc3dgpu_ctx* c) {
   if (c->symmetric >= 0) return 0;
+  for (int t = 0; t < c->nslab; t++)
+    if (c->slab_nslot_h[t] > 64) {
+      c->symmetric = 0;
+      return 0;
+    }
   cudaStream_t s = c->stream;
   int missing = 0;
   CK(fc3dgpu::check_flow_symmetric(c->npad, c->perm, c->slab_nslot, c->slab_off, c->col, c->scratch, s));

@@ -36,8 +36,8 @@ def test_lattices(gpu, dims, warps):
 
 @pytest.mark.parametrize("nc,degree", [(40, 11), (700, 12), (700, 13)])
 def test_long_rows(gpu, nc, degree):
-    """A ring where every contact is tied to its `degree` nearest (11 to 13
-    blocks off the diagonal, more colours than a lattice)."""
+    """A ring where every contact is tied to its `degree` nearest (more colours
+    than a lattice; from 65 blocks on the pattern is not looked at)."""
     g = np.random.default_rng(nc + degree)
     near = [d for k in range(1, degree // 2 + 1) for d in (k, -k)] + ([nc // 2] if degree % 2 else [])
     blocks, cols, rowptr = {}, [], [0]
