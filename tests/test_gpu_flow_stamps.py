@@ -1,22 +1,24 @@
 """The dataflow sweep on stamped reactions at the edges of its splits of a
 slab (from one row a warp to several slabs a warp) and with rows longer than
-the slots gathered together: the coloured kernel's iterates bit for bit."""
+the slots gathered together, in FP32 and in FP64 (from one contact a unit to
+ten): the coloured kernel's iterates bit for bit."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-def _both(gpu, load, sweeps):
+def _both(gpu, load, sweeps, precision=0):
+    how = dict(precision=1) if precision else dict(fp32_only=1, switch_tol=0.0)
     out = []
     for on in (True, False):
         gpu.flow(on)
         try:
             load()
-            st = gpu.solve(tol=1e-300, max_iter=sweeps, fp32_only=1, lanes=1, switch_tol=0.0, stall_window=0)
+            st = gpu.solve(tol=1e-300, max_iter=sweeps, lanes=1, stall_window=0, **how)
         finally:
             gpu.flow(True)
-        out.append((st["sweeps32"], gpu.get()[0]))
+        out.append((st["sweeps32"], st["sweeps64"], gpu.get()[0]))
     return out
 
 
@@ -27,15 +29,27 @@ def test_lattices(gpu, dims, warps):
     sc = lattice(*dims, seed=9)
     gpu.flow_warps(warps)
     try:
-        (n, r), (m, want) = _both(gpu, lambda: gpu.load(sc), 15)
+        (n, k, r), (m, j, want) = _both(gpu, lambda: gpu.load(sc), 15)
     finally:
         gpu.flow_warps(0)
+    assert (n, k) == (m, j)
+    np.testing.assert_array_equal(r, want)
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 1), (3, 3, 2), (12, 11, 9), (19, 18, 11), (30, 31, 15), (44, 44, 22),
+                                  (46, 46, 23)])
+def test_lattices_fp64(gpu, dims):
+    """On both sides of the line beyond which the sweeps go by colours too."""
+    from siconos_gb300.scene import lattice
+    sc = lattice(*dims, seed=9)
+    (_, n, r), (_, m, want) = _both(gpu, lambda: gpu.load(sc), 10, precision=1)
     assert n == m
     np.testing.assert_array_equal(r, want)
 
 
-@pytest.mark.parametrize("nc,degree", [(40, 11), (700, 12), (700, 13)])
-def test_long_rows(gpu, nc, degree):
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("nc,degree", [(40, 4), (40, 5), (40, 11), (700, 12), (700, 13), (150, 64), (150, 66)])
+def test_long_rows(gpu, nc, degree, precision):
     """A ring where every contact is tied to its `degree` nearest (more colours
     than a lattice; from 65 blocks on the pattern is not looked at)."""
     g = np.random.default_rng(nc + degree)
@@ -63,6 +77,6 @@ def test_long_rows(gpu, nc, degree):
         gpu.set_q_mu(q, mu)
         gpu.set_r(np.zeros(3 * nc))
 
-    (n, r), (m, want) = _both(gpu, load, 15)
-    assert n == m
+    (n, k, r), (m, j, want) = _both(gpu, load, 15, precision)
+    assert (n, k) == (m, j)
     np.testing.assert_array_equal(r, want)
