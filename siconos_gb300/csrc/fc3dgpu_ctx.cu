@@ -1555,17 +1555,20 @@ extern "C" int fc3dgpu_ctx_staging(fc3dgpu_ctx* c, int on) {
   return old;
 }
 
+// The batch's launches are recorded with their arguments: a setting that goes
+// into these has them recorded anew.
+static void drop_batch_graph(fc3dgpu_ctx* c) {
+  if (c->batch_graph) cudaGraphExecDestroy(c->batch_graph);
+  c->batch_graph = nullptr;
+}
+
 // Slab-dataflow FP32 sweep (no barriers between colours): on (1, default)
 // or off (0, the coloured persistent kernel).  Returns the previous setting.
 extern "C" int fc3dgpu_ctx_flow(fc3dgpu_ctx* c, int on) {
   if (!c) return -1;
   const int old = c->flow_on;
   c->flow_on = on ? 1 : 0;
-  if (old != c->flow_on && c->batch_graph) {
-    // recorded for the other form
-    cudaGraphExecDestroy(c->batch_graph);
-    c->batch_graph = nullptr;
-  }
+  if (old != c->flow_on) drop_batch_graph(c);
   c->batch_flow = 0;
   return old;
 }
@@ -1596,6 +1599,7 @@ extern "C" unsigned long long fc3dgpu_ctx_spin_limit(fc3dgpu_ctx* c, unsigned lo
   if (!c) return 0;
   const unsigned long long old = c->spin_limit;
   c->spin_limit = polls;
+  if (old != polls) drop_batch_graph(c);
   return old;
 }
 

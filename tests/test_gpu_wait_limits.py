@@ -1,0 +1,39 @@
+"""Device waits with a limit of one poll: every form of the sweeps gives up with
+an error, and with the default limit the context solves as before."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _gives_up_and_recovers(gpu, solve):
+    want = solve()
+    old = gpu.spin_limit(1)
+    try:
+        with pytest.raises(RuntimeError):
+            solve()
+    finally:
+        gpu.spin_limit(old)
+    np.testing.assert_array_equal(solve(), want)
+
+
+def _batch(gpu, precision):
+    from siconos_gb300.scene import lattice
+    gpu.load_batch([lattice(*d, seed=40 + k) for k, d in enumerate([(20, 19, 9), (3, 3, 2), (12, 11, 6)])])
+
+    def solve():
+        gpu.zero_r()
+        gpu.solve_batch(tol=1e-300, max_iter=12, precision=precision, fp32_only=1 - precision)
+        return gpu.get()[0]
+
+    return solve
+
+
+@pytest.mark.parametrize("flow", [True, False], ids=["dataflow", "colours"])
+def test_batch_fp32(gpu, flow):
+    """The limit set after the batch's launches were recorded counts too."""
+    gpu.flow(flow)
+    try:
+        _gives_up_and_recovers(gpu, _batch(gpu, 0))
+    finally:
+        gpu.flow(True)
