@@ -122,7 +122,9 @@ __device__ __forceinline__ bool flow64_unit(const SweepArgs<double>& a, int p0, 
       for (int t = 0; t < CH; t++)
         if ((late >> t & 1u) && take_stamped64(w[t], sweep - (pj[t] > p ? 1 : 0), rv[t])) late &= ~(1u << t);
     }
-    __syncwarp();  // the lanes left the wait one by one: together again
+    // the lanes left the wait one by one: together again, and all of them leave
+    // the loop when one gave up
+    ok = __all_sync(0xffffffffu, ok);
 #pragma unroll
     for (int t = 0; t < CH; t++)
       if (t0 + t < ns) {
@@ -131,7 +133,7 @@ __device__ __forceinline__ bool flow64_unit(const SweepArgs<double>& a, int p0, 
         acc += wv[t][2] * rv[t][2];
       }
   }
-  if (!__all_sync(0xffffffffu, ok)) return false;
+  if (!ok) return false;
   P.q = acc;
   const bool off = ie_lt(-DBL_EPSILON, coop_get(acc, c.base));  // take-off
   const bool act = have && !off;

@@ -37,3 +37,21 @@ def test_batch_fp32(gpu, flow):
         _gives_up_and_recovers(gpu, _batch(gpu, 0))
     finally:
         gpu.flow(True)
+
+
+@pytest.mark.parametrize("dims", [(3, 3, 2), (19, 18, 11)])
+def test_fp64(gpu, dims):
+    """From one contact a unit to several; rows of more than one round of slots."""
+    from siconos_gb300.scene import lattice
+    gpu.load(lattice(*dims, seed=2))
+
+    def solve():
+        gpu.zero_r()
+        gpu.solve(tol=1e-300, max_iter=12, precision=1, lanes=1)
+        return gpu.get()[0]
+
+    _gives_up_and_recovers(gpu, solve)
+
+
+def test_batch_fp64(gpu):
+    _gives_up_and_recovers(gpu, _batch(gpu, 1))
