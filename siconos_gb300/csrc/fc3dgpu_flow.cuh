@@ -284,7 +284,8 @@ __device__ __forceinline__ void flow_own_r(const SweepArgs<float>& a, int s, int
 // light-error sums are left to the caller, after the slab's release.
 // STAMP: the columns' reactions are loaded until their stamps are those
 // sweep `sweep` needs (this sweep's of an earlier colour, a smaller row; the
-// last one's of a later colour); false when the poll limit ran out.  refill
+// last one's of a later colour, and of the row itself, which a second block on
+// its diagonal reads); false when the poll limit ran out.  refill
 // is false when the buffer already holds the next slab (the same one).
 template <bool STAMP>
 __device__ __forceinline__ bool flow_slab(const SweepArgs<float>& a, const FlowArgs& f, int s, const FlowNext& next,
@@ -319,7 +320,7 @@ __device__ __forceinline__ bool flow_slab(const SweepArgs<float>& a, const FlowA
 #pragma unroll
         for (int k = 0; k < CH; k++) {
           pj[k] = t0 + k < ns ? Cs[(t0 + k) * FC3D_SLAB + rl] : a.npad;
-          need[k] = sweep - (pj[k] > p ? 1 : 0);
+          need[k] = sweep - (pj[k] >= p ? 1 : 0);
           const Stamped v = ld_stamped(a.r, pj[k]);
           rv[k][0] = v.x[0];
           rv[k][1] = v.x[1];

@@ -97,10 +97,11 @@ __device__ __forceinline__ bool flow64_unit(const SweepArgs<double>& a, int p0, 
 #pragma unroll
       for (int e = 0; e < 3; e++) wv[t][e] = t0 + t < ns ? __ldg(&wp[3 * e * FC3D_SLAB]) : 0.0;
     }
+    // (a second block on the diagonal reads the row's own last reaction)
     unsigned late = 0;
 #pragma unroll
     for (int t = 0; t < CH; t++)
-      late |= (ld_stamped64(a.rs, pj[t], sweep - (pj[t] > p ? 1 : 0), rv[t]) ? 0u : 1u) << t;
+      late |= (ld_stamped64(a.rs, pj[t], sweep - (pj[t] >= p ? 1 : 0), rv[t]) ? 0u : 1u) << t;
     unsigned long long polls = 0;
     while (late) {
       if (++polls > a.spin_limit) {
@@ -120,7 +121,7 @@ __device__ __forceinline__ bool flow64_unit(const SweepArgs<double>& a, int p0, 
       }
 #pragma unroll
       for (int t = 0; t < CH; t++)
-        if ((late >> t & 1u) && take_stamped64(w[t], sweep - (pj[t] > p ? 1 : 0), rv[t])) late &= ~(1u << t);
+        if ((late >> t & 1u) && take_stamped64(w[t], sweep - (pj[t] >= p ? 1 : 0), rv[t])) late &= ~(1u << t);
     }
     // the lanes left the wait one by one: together again, and all of them leave
     // the loop when one gave up
