@@ -2295,7 +2295,7 @@ static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st
     if (!(converged32 && a.max_sweeps == 0)) {
       if (a.max_sweeps > 0) {
         CK(cudaMemsetAsync(c->cost, 0, (size_t)c->npad, s));
-        if (lanes64 == 1 && !fast64 && c->flow_on && !c->timeline)
+        if (lanes64 == 1 && !fast64 && c->flow_on && !a.timeline)
           if (int rc = attach_flow64(c, a)) return rc;
       }
       CK(cudaMemsetAsync(c->barrier, 0, FC3D_BARRIER_WORDS * sizeof(unsigned), s));

@@ -1,0 +1,30 @@
+"""Timeline records and work counters: what they record, and the sweeps of a
+context on which they were switched on and off again."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def own(built_lib):
+    from siconos_gb300.device import DeviceSolver
+    d = DeviceSolver(0)
+    yield d
+    d.close()
+
+
+def test_fp64_sweeps_after_a_timeline(own):
+    """The dataflow's sweeps start with one launch more (the stamps): before a
+    timeline was armed, not while it is, and again after it was switched off."""
+    from siconos_gb300.scene import lattice
+    own.load(lattice(6, 6, 4, seed=1))
+    n = []
+    for arm in (None, 2, 0):
+        if arm is not None:
+            own.timeline(arm)
+        own.zero_r()
+        before = own.launches()
+        own.solve(tol=1e-300, max_iter=4, precision=1, lanes=1)
+        n.append(own.launches() - before)
+    assert n[1] == n[0] - 1 and n[2] == n[0]
