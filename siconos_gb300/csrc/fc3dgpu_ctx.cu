@@ -2376,6 +2376,11 @@ extern "C" int fc3dgpu_ctx_counters(fc3dgpu_ctx* c, int enable, unsigned long lo
     CK(cudaStreamSynchronize(c->stream));
   }
   CK(cudaMemsetAsync(c->counters, 0, 8 * sizeof(unsigned long long), c->stream));
+  if (!c->counters_on != !enable) {
+    // the batch's FP32 dataflow does not count
+    drop_batch_graph(c);
+    c->batch_flow = 0;
+  }
   c->counters_on = enable;
   return 0;
 }

@@ -28,3 +28,25 @@ def test_fp64_sweeps_after_a_timeline(own):
         own.solve(tol=1e-300, max_iter=4, precision=1, lanes=1)
         n.append(own.launches() - before)
     assert n[1] == n[0] - 1 and n[2] == n[0]
+
+
+def test_counters_of_a_batch_between_solves(own):
+    """Switched on after a first batch solve they count its FP32 sweeps (one
+    local solve or take-off a contact and sweep), switched off nothing; the
+    reactions are the same throughout."""
+    from siconos_gb300.scene import lattice
+    own.load_batch([lattice(8, 7, 5, seed=1), lattice(3, 3, 2, seed=2)])
+    kw = dict(tol=1e-300, max_iter=10, fp32_only=1, switch_tol=0.0, stall_window=0)
+
+    def solve():
+        own.zero_r()
+        own.solve_batch(**kw)
+        return own.get()[0]
+
+    want = solve()
+    own.counters(True)
+    np.testing.assert_array_equal(solve(), want)
+    on = own.counters(False)
+    np.testing.assert_array_equal(solve(), want)
+    assert 0 < on["solves"] <= 10 * own.nc and on["newton"] > 0
+    assert own.counters(False)["solves"] == 0
