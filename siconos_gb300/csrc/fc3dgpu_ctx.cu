@@ -2227,8 +2227,8 @@ static int solve_impl(fc3dgpu_ctx* c, const fc3dgpu_params* p, fc3dgpu_stats* st
       f.rec = c->flow_rec;
       f.rec_off = c->flow_rec_off;
       f.stamped = c->symmetric == 1 ? 1 : 0;
-      f.split = 0;
-      if (f.stamped) {
+      f.split = 0;  // (a timeline is recorded by whole slabs)
+      if (f.stamped && !a.timeline) {
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
         while (f.split < 5 && ((long long)c->nslab << (f.split + 1)) <= (long long)sms * c->flow_nw) f.split++;

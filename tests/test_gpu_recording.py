@@ -50,3 +50,26 @@ def test_counters_of_a_batch_between_solves(own):
     np.testing.assert_array_equal(solve(), want)
     assert 0 < on["solves"] <= 10 * own.nc and on["newton"] > 0
     assert own.counters(False)["solves"] == 0
+
+
+@pytest.mark.parametrize("dims", [(3, 3, 2), (12, 11, 9)])
+def test_timeline_of_a_slab(own, dims):
+    """Scenes small enough for a slab's rows to be spread over several warps: one
+    record a slab all the same, its stamps in order, and the local solves of all
+    slabs those that the sweep by colours counts."""
+    from siconos_gb300.scene import lattice
+    own.load(lattice(*dims, seed=6))
+    kw = dict(tol=1e-300, max_iter=8, fp32_only=1, lanes=1, switch_tol=0.0, stall_window=0)
+    records = {}
+    for on in (True, False):
+        own.flow(on)
+        own.timeline(5)
+        own.zero_r()
+        own.solve(**kw)
+        records[on] = own.timeline(0).reshape(-1, 8)
+    slabs = records[True][records[True][:, 0] > 0]
+    n = own.nc
+    assert (n + 31) // 32 <= len(slabs) <= n
+    for a, b in ((0, 1), (1, 2), (2, 3), (3, 6), (6, 7), (7, 4)):
+        assert (slabs[:, a] <= slabs[:, b]).all(), (a, b)
+    assert slabs[:, 5].sum() == records[False][:, 3].sum() > 0
