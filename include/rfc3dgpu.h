@@ -94,6 +94,9 @@ int rfc3dgpu_ctx_rho(rfc3dgpu_ctx *ctx, double *rho);
 int rfc3dgpu_ctx_set_precision(rfc3dgpu_ctx *ctx, int precision, double switch_tol, int stall_window);
 /* FP32 and FP64 sweeps of the last solve. */
 int rfc3dgpu_ctx_last_sweeps(rfc3dgpu_ctx *ctx, int *sweeps32, int *sweeps64);
+/* Poll limit of a wait for a reaction in the dataflow sweeps (0: the default of
+ * 2^22 polls); a wait that reaches it ends the solve with an error. */
+int rfc3dgpu_ctx_spin_limit(rfc3dgpu_ctx *ctx, unsigned long long polls);
 
 #ifdef __cplusplus
 }

@@ -36,7 +36,7 @@ constexpr int NT = 128;
 constexpr int MAXC = 128;
 constexpr int TRACE_CAP = 1 << 16;
 constexpr int MAX_BLOCKS = 1024;
-constexpr unsigned long long SPIN = 1ull << 22;  // polls of a dataflow wait
+constexpr unsigned long long SPIN = 1ull << 22;  // polls of a dataflow wait where no limit is set
 
 // Kernel arguments; Real = double for the reference's loop, float for the
 // FP32 sweeps that precede it in mixed precision.
@@ -688,12 +688,14 @@ __device__ __forceinline__ void st_all_stamped(double* rs, int p, const double x
 }
 
 // The reactions x[t] of the contacts j[t] as row p reads them in `sweep`
-// (j < 0: none); false when the wait gave up.  Called by the whole warp.  A
-// poll loads all of them without a branch between two loads (none: the row's
-// own), so it costs one memory latency.
+// (j < 0: none).  Called by the whole warp.  A poll loads all of them without a
+// branch between two loads (none: the row's own), so it costs one memory
+// latency.  A wait that gives up sets `failed` (in the whole warp) and goes on
+// with what is there, as every later one of the warp then does at once: the
+// sweep goes on, so that every block gets to the barrier at its end.
 template <typename Real, int CH>
-__device__ __forceinline__ bool wait_reactions(const ArgsT<Real>& a, const int (&j)[CH], int p, int sweep,
-                                               Real (&x)[CH][5]) {
+__device__ __forceinline__ void wait_reactions(const ArgsT<Real>& a, const int (&j)[CH], int p, int sweep,
+                                               Real (&x)[CH][5], bool& failed) {
   int from[CH], need[CH];
 #pragma unroll
   for (int t = 0; t < CH; t++) {
@@ -704,16 +706,15 @@ __device__ __forceinline__ bool wait_reactions(const ArgsT<Real>& a, const int (
     bool ok = true;
 #pragma unroll
     for (int t = 0; t < CH; t++) ok = ld_stamped(a.rs, from[t], need[t], x[t]) && ok;
-    if (__all_sync(0xffffffffu, ok)) return true;
-    if (n > a.spin) return false;
+    if (__all_sync(0xffffffffu, ok || failed)) return;
+    if (n > a.spin) failed = true;
     if (n > RFC3D_FLOW_SPIN) __nanosleep(RFC3D_FLOW_SLEEP_NS);
   }
 }
 
-// Contacts [first, first + n) of a colour, five lanes each.  v[2] counts
-// waits that gave up (the sweep goes on, so that every block gets to the
-// barrier at its end).
-__device__ __forceinline__ void flow_unit(const Args& a, int first, int n, int sweep, double local_tol, double v[3]) {
+// Contacts [first, first + n) of a colour, five lanes each
+__device__ __forceinline__ void flow_unit(const Args& a, int first, int n, int sweep, double local_tol, double v[3],
+                                          bool& failed) {
   const int lane = threadIdx.x & 31;
   const bool spare = lane >= 5 * RFC3D_COOP_GROUPS;
   RLane c;
@@ -734,7 +735,6 @@ __device__ __forceinline__ void flow_unit(const Args& a, int first, int n, int s
   P.rho = a.rho[p];
   const double q = a.q[5 * (size_t)p + c.i], old = __ldcg(&a.r[5 * (size_t)p + c.i]);
   double s = 0.0;
-  bool ok = true;
   constexpr int CH = 2;
   for (int t0 = 0; t0 < longest; t0 += CH) {
     int j[CH];
@@ -748,7 +748,7 @@ __device__ __forceinline__ void flow_unit(const Args& a, int first, int n, int s
 #pragma unroll
       for (int k = 0; k < 5; k++) w[t][k] = __ldg(&blk[5 * k]);
     }
-    ok = wait_reactions<double, CH>(a, j, p, sweep, x) && ok;
+    wait_reactions<double, CH>(a, j, p, sweep, x, failed);
 #pragma unroll
     for (int t = 0; t < CH; t++)
       if (j[t] >= 0)
@@ -772,12 +772,11 @@ __device__ __forceinline__ void flow_unit(const Args& a, int first, int n, int s
     v[0] += d2;
     v[1] += r2;
   }
-  if (!ok) v[2] += 1.0;
 }
 
 // Contacts [first, first + n) of a colour, one lane each, in FP32
 __device__ __forceinline__ void flow_unit(const ArgsT<float>& a, int first, int n, int sweep, float local_tol,
-                                          double v[3]) {
+                                          double v[3], bool& failed) {
   const int lane = threadIdx.x & 31;
   const bool have = lane < n;
   const int p = first + (have ? lane : 0), s0 = a.rp[p], len = have ? a.rp[p + 1] - s0 : 0;
@@ -787,7 +786,7 @@ __device__ __forceinline__ void flow_unit(const ArgsT<float>& a, int first, int 
     const int col = t < len ? a.col[s0 + t] : p;
     const int j[1] = {col != p ? col : -1};
     float x[1][5];
-    if (!wait_reactions<float, 1>(a, j, p, sweep, x)) v[2] += 1.0;
+    wait_reactions<float, 1>(a, j, p, sweep, x, failed);
     if (j[0] < 0) continue;
     const float* blk = a.W + 25 * (size_t)(s0 + t);
     for (int k = 0; k < 5; k++)
@@ -846,7 +845,9 @@ __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
     ++iter;
     double v[3] = {0.0, 0.0, 0.0};
     if constexpr (FLOW) {
-      flow_sweep(a, [&](int first, int n) { flow_unit(a, first, n, iter, local_tol, v); });
+      bool failed = false;
+      flow_sweep(a, [&](int first, int n) { flow_unit(a, first, n, iter, local_tol, v, failed); });
+      v[2] = failed ? 1.0 : 0.0;
       grid_sum<3>(v, a, R, g);
       if (v[2] != 0.0) {
         if (lead) a.out[2] = -1.0;
@@ -905,7 +906,9 @@ __global__ void __launch_bounds__(NT) k_rfc3d_sweeps32(const ArgsT<float> a) {
     ++iter;
     double v[3] = {0.0, 0.0, 0.0};
     if constexpr (FLOW) {
-      flow_sweep(a, [&](int first, int n) { flow_unit(a, first, n, iter, (float)a.local_tol, v); });
+      bool failed = false;
+      flow_sweep(a, [&](int first, int n) { flow_unit(a, first, n, iter, (float)a.local_tol, v, failed); });
+      v[2] = failed ? 1.0 : 0.0;
       grid_sum<3>(v, a, R, g);
       if (v[2] != 0.0) {
         if (lead) a.out[2] = -1.0;
@@ -1024,6 +1027,7 @@ struct rfc3dgpu_ctx {
   int trace_len = 0;
   // 1: FP64 sweeps only (default); 0: FP32 sweeps, then the FP64 loop
   int precision = 1;
+  unsigned long long spin = SPIN;
   double switch_tol = 0.0;  // FP32 sweeps end below this light error (0: max(tol, 1e-6))
   int stall = 64;
   int sweeps32 = 0, sweeps64 = 0;
@@ -1295,7 +1299,7 @@ static Args args_of(const rfc3dgpu_ctx* c) {
   a.r = c->r;
   a.rs = c->rs;
   a.rows = c->rows;
-  a.spin = SPIN;
+  a.spin = c->spin;
   a.u = c->u;
   a.norm_q = c->norm_q;
   a.part = c->part;
@@ -1322,7 +1326,7 @@ static ArgsT<float> args32_of(const rfc3dgpu_ctx* c) {
   a.r = c->r32;
   a.rs = c->rs32;
   a.rows = c->rows32;
-  a.spin = SPIN;
+  a.spin = c->spin;
   a.u = c->u;
   a.norm_q = c->norm_q;
   a.part = c->part;
@@ -1418,6 +1422,12 @@ extern "C" int rfc3dgpu_ctx_last_sweeps(rfc3dgpu_ctx* c, int* sweeps32, int* swe
   if (!c) return NUMERICS_ERR_INVALID_ARGUMENT;
   if (sweeps32) *sweeps32 = c->sweeps32;
   if (sweeps64) *sweeps64 = c->sweeps64;
+  return 0;
+}
+
+extern "C" int rfc3dgpu_ctx_spin_limit(rfc3dgpu_ctx* c, unsigned long long polls) {
+  if (!c) return NUMERICS_ERR_INVALID_ARGUMENT;
+  c->spin = polls ? polls : SPIN;
   return 0;
 }
 

@@ -326,6 +326,7 @@ ABI = {
     "gfc3dgpu_ctx_info": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), _DP,
                                     C.POINTER(C.c_int)]),
     "gfc3dgpu_ctx_spin_limit": (C.c_int, [C.c_void_p, C.c_ulonglong]),
+    "rfc3dgpu_ctx_spin_limit": (C.c_int, [C.c_void_p, C.c_ulonglong]),
     "gfc3dgpu_ctx_set_arithmetic": (C.c_int, [C.c_void_p, C.c_int]),
     "fc3dgpu_lattice_global_sizes": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
     "fc3dgpu_lattice_fill_global": (C.c_int, [C.c_void_p, C.c_double, C.c_double, _I64, _I64, _F64, _I64, _I64, _F64, _F64,
@@ -877,6 +878,10 @@ class RollingContext:
         """0: FP32 sweeps, then the reference's FP64 loop from their iterate;
         1: FP64 sweeps only (the default of a context)."""
         _check(lib().rfc3dgpu_ctx_set_precision(self.ctx, precision, switch_tol, stall_window))
+
+    def spin_limit(self, polls: int):
+        """Polls before a wait of the dataflow sweeps gives up (0: default)."""
+        _check(lib().rfc3dgpu_ctx_spin_limit(self.ctx, polls))
 
     def last_sweeps(self):
         """(FP32 sweeps, FP64 sweeps) of the last solve."""

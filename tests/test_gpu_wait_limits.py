@@ -55,3 +55,30 @@ def test_fp64(gpu, dims):
 
 def test_batch_fp64(gpu):
     _gives_up_and_recovers(gpu, _batch(gpu, 1))
+
+
+def _context_recovers(ctx, n, solve):
+    def run():
+        ctx.set_r(np.zeros(n))
+        solve()
+        return ctx.get_r_u()[0]
+
+    want = run()
+    ctx.spin_limit(1)
+    with pytest.raises(RuntimeError, match="poll limit"):
+        run()
+    ctx.spin_limit(0)
+    np.testing.assert_array_equal(run(), want)
+    ctx.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("copies", [1, 100])
+def test_rolling(built_lib, copies, precision):
+    import siconos_gb300.numerics as sn
+    from test_gpu_rfc3d import _ctx
+    from test_rfc3d_oracle import load_rfc3d, tiled
+    T = tiled(load_rfc3d("rfc3d_rockfall_21_54029")[0], copies, 7)
+    ctx = _ctx(sn, T)
+    ctx.set_precision(precision)
+    _context_recovers(ctx, 5 * T.nc, lambda: ctx.solve(0.0, 6))
