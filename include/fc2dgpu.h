@@ -112,6 +112,9 @@ int fc2dgpu_ctx_colours(fc2dgpu_ctx *ctx, int32_t *colour);
  * does. */
 int fc2dgpu_ctx_set_launch(fc2dgpu_ctx *ctx, int cluster_blocks, int threads, int reactions);
 int fc2dgpu_ctx_launch_shape(fc2dgpu_ctx *ctx, int *cluster_blocks, int *threads, int *reactions);
+/* Poll limit of a wait in the dataflow sweeps (0: the default of 2^22 polls); a
+ * wait that reaches it ends the solve with an error. */
+int fc2dgpu_ctx_spin_limit(fc2dgpu_ctx *ctx, unsigned long long polls);
 /* Per-sweep light error of the last solve (cap entries); returns how many. */
 int fc2dgpu_ctx_trace(fc2dgpu_ctx *ctx, double *out, int cap);
 

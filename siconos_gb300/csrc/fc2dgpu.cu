@@ -36,7 +36,7 @@ constexpr int TRACE_CAP = 1 << 16;
 constexpr size_t REP_MAX_BYTES = 208 * 1024;  // shared-memory copy of the reactions at most
 constexpr int GRID_MAX = 1024;                 // blocks of a cooperative grid at most
 constexpr int FLAG_STRIDE = 8;                 // words between the dataflow blocks' barrier flags
-constexpr unsigned long long SPIN = 1ull << 22;  // polls of a dataflow wait
+constexpr unsigned long long SPIN = 1ull << 22;  // polls of a dataflow wait where no limit is set
 
 template <typename T>
 struct Vec2;
@@ -89,6 +89,7 @@ struct Args {
   int rows;
   unsigned* flags;
   double* fail;
+  unsigned long long spin;  // polls of a wait
   double* trace;
   double* out;  // [0] sweeps, [1] final error, [2] info, [3] last light error
 };
@@ -144,16 +145,17 @@ struct GridTeam {
 };
 
 // A cooperative grid whose sweeps are dataflow: a barrier of flags (the sums
-// of a sweep pass one) whose waits, like those for reactions, end after SPIN
+// of a sweep pass one) whose waits, like those for reactions, end after `spin`
 // polls; `dead` (the same in the whole block) then ends the solve.
 struct FlowTeam {
   static constexpr bool grid = true, flow = true;
   unsigned* flags;
   double* fail;
+  unsigned long long spin;
   unsigned epoch = 0;
   bool dead = false;
   template <typename T>
-  __device__ explicit FlowTeam(const Args<T>& a) : flags(a.flags), fail(a.fail) {}
+  __device__ explicit FlowTeam(const Args<T>& a) : flags(a.flags), fail(a.fail), spin(a.spin) {}
   __device__ __forceinline__ int rank() const { return (int)blockIdx.x; }
   __device__ __forceinline__ int size() const { return (int)gridDim.x; }
   __device__ __forceinline__ void give_up() {
@@ -178,7 +180,7 @@ struct FlowTeam {
           all &= f >= epoch;
         }
         if (__all_sync(0xffffffffu, all)) break;
-        if (n > SPIN) {
+        if (n > spin) {
           ok = false;
           break;
         }
@@ -717,6 +719,7 @@ struct FlowReactions {
   T* rs;
   int sweep;
   bool failed;
+  unsigned long long spin;
   __device__ __forceinline__ V get(int j) const { return __ldcg(reinterpret_cast<const V*>(rw) + j); }
   __device__ __forceinline__ bool any(bool more) const { return __any_sync(0xffffffffu, more); }
   __device__ __forceinline__ void stamp(int j, V v, int at) const {
@@ -766,7 +769,7 @@ struct FlowReactions {
         all = all && there;
       }
       if (__all_sync(0xffffffffu, all || failed)) break;
-      if (n > SPIN) failed = true;
+      if (n > spin) failed = true;
       if (n > FC2D_FLOW_SPIN) __nanosleep(FC2D_FLOW_SLEEP_NS);
     }
   }
@@ -790,7 +793,7 @@ struct FlowReactions {
 // sweep's plain copy.
 template <typename T>
 __device__ __forceinline__ FlowReactions<T> open_flow(const Args<T>& a, FlowTeam& team) {
-  FlowReactions<T> fx{a.rw, a.rs, 0, false};
+  FlowReactions<T> fx{a.rw, a.rs, 0, false, a.spin};
   for (int j = team.rank() * blockDim.x + threadIdx.x; j < a.nc; j += team.size() * blockDim.x) {
     const double2 x = __ldcg(reinterpret_cast<const double2*>(a.r) + j);
     typename Vec2<T>::type v;
@@ -1073,6 +1076,7 @@ struct fc2dgpu_ctx {
   unsigned* flags = nullptr;
   // FP32 copies for the first phase of a mixed-precision solve
   float *W32 = nullptr, *det32 = nullptr, *q32 = nullptr, *mu32 = nullptr, *r32 = nullptr;
+  unsigned long long spin = SPIN;
   int precision = 1;          // 0 FP32 sweeps + FP64 polish, 1 FP64 sweeps only
   double switch_tol = 0.0;    // FP32 phase stops below this light error (0: max(tol, 1e-6))
   int stall = 64;             // ... or after this many sweeps without a new lowest error
@@ -1613,6 +1617,7 @@ static Args<double> args64(const fc2dgpu_ctx* c) {
   a.rs = c->rs;
   a.flags = c->flags;
   a.fail = c->out + 8;
+  a.spin = c->spin;
   return a;
 }
 
@@ -1644,6 +1649,7 @@ static Args<float> args32(const fc2dgpu_ctx* c) {
   a.rs = reinterpret_cast<float*>(c->rs);
   a.flags = c->flags;
   a.fail = c->out + 8;
+  a.spin = c->spin;
   return a;
 }
 
@@ -1662,6 +1668,12 @@ extern "C" int fc2dgpu_ctx_last_sweeps(fc2dgpu_ctx* c, int* sweeps32, int* sweep
   if (!c) return NUMERICS_ERR_INVALID_ARGUMENT;
   if (sweeps32) *sweeps32 = c->sweeps32;
   if (sweeps64) *sweeps64 = c->sweeps64;
+  return 0;
+}
+
+extern "C" int fc2dgpu_ctx_spin_limit(fc2dgpu_ctx* c, unsigned long long polls) {
+  if (!c) return NUMERICS_ERR_INVALID_ARGUMENT;
+  c->spin = polls ? polls : SPIN;
   return 0;
 }
 

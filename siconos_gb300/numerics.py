@@ -327,6 +327,7 @@ ABI = {
                                     C.POINTER(C.c_int)]),
     "gfc3dgpu_ctx_spin_limit": (C.c_int, [C.c_void_p, C.c_ulonglong]),
     "rfc3dgpu_ctx_spin_limit": (C.c_int, [C.c_void_p, C.c_ulonglong]),
+    "fc2dgpu_ctx_spin_limit": (C.c_int, [C.c_void_p, C.c_ulonglong]),
     "gfc3dgpu_ctx_set_arithmetic": (C.c_int, [C.c_void_p, C.c_int]),
     "fc3dgpu_lattice_global_sizes": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
     "fc3dgpu_lattice_fill_global": (C.c_int, [C.c_void_p, C.c_double, C.c_double, _I64, _I64, _F64, _I64, _I64, _F64, _F64,
@@ -747,6 +748,10 @@ class Fc2dContext:
         cs, nt, rx = C.c_int(), C.c_int(), C.c_int()
         _check(lib().fc2dgpu_ctx_launch_shape(self.ctx, C.byref(cs), C.byref(nt), C.byref(rx)))
         return cs.value, nt.value, rx.value
+
+    def spin_limit(self, polls: int):
+        """Polls before a wait of the dataflow sweeps gives up (0: default)."""
+        _check(lib().fc2dgpu_ctx_spin_limit(self.ctx, polls))
 
     def trace(self, cap: int) -> np.ndarray:
         out = np.zeros(max(cap, 1))

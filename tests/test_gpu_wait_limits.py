@@ -82,3 +82,16 @@ def test_rolling(built_lib, copies, precision):
     ctx = _ctx(sn, T)
     ctx.set_precision(precision)
     _context_recovers(ctx, 5 * T.nc, lambda: ctx.solve(0.0, 6))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("problem,copies", [("FrictionContactProblem00727", 1),
+                                            ("fc2d_granularflowonwall_07002_00801", 4)])
+def test_2d(built_lib, problem, copies, precision):
+    import siconos_gb300.numerics as sn
+    from test_fc2d_oracle import load_fc2d, tiled2d
+    from test_gpu_fc2d import _ctx
+    P = tiled2d(load_fc2d("fc2d_" + problem)[0], copies, 4)
+    ctx = _ctx(sn, P)
+    ctx.set_precision(precision, 1e-30, 1 << 20)
+    _context_recovers(ctx, 2 * P.nc, lambda: ctx.solve(1e-300, 8))
