@@ -111,30 +111,30 @@ __global__ void __launch_bounds__(3 * CH) k_error_noalloc(int nc, long long nnz,
         badl = 1;
       } else {
         // blocks four at a time: their columns, then their values and
-        // reactions, are requested together; a column out of range reads
-        // contact 0 and flags the input
+        // reactions, are requested together; a column out of range (-1, as
+        // behind the row's end) is left out and flags the input
         constexpr int U = 4;
         for (long long b = b0; b < b1; b += U) {
           long long j[U];
           double wv[U][3], rv[U][3];
 #pragma unroll
           for (int k = 0; k < U; k++) {
-            j[k] = b + k < b1 ? __ldg(&colidx[b + k]) : 0;
+            j[k] = b + k < b1 ? __ldg(&colidx[b + k]) : -1;
             if (j[k] < 0 || j[k] >= nc) {
-              badl = 1;
-              j[k] = 0;
+              if (b + k < b1) badl = 1;
+              j[k] = -1;
             }
           }
 #pragma unroll
           for (int k = 0; k < U; k++)
 #pragma unroll
             for (int e = 0; e < 3; e++) {
-              wv[k][e] = b + k < b1 ? __ldg(&blocks[9 * (b + k) + 3 * e + comp]) : 0.0;
-              rv[k][e] = b + k < b1 ? __ldg(&r[3 * j[k] + e]) : 0.0;
+              wv[k][e] = j[k] >= 0 ? __ldg(&blocks[9 * (b + k) + 3 * e + comp]) : 0.0;
+              rv[k][e] = j[k] >= 0 ? __ldg(&r[3 * j[k] + e]) : 0.0;
             }
 #pragma unroll
           for (int k = 0; k < U; k++)
-            if (b + k < b1)
+            if (j[k] >= 0)
 #pragma unroll
               for (int e = 0; e < 3; e++) u = fma(wv[k][e], rv[k][e], u);
         }
