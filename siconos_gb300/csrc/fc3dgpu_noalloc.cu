@@ -48,8 +48,10 @@ static_assert(MAX_CHUNKS * LARGE_CHUNK == FC3DGPU_NOALLOC_MAX_CONTACTS, "limit m
 static_assert(SMALL_MAX / SMALL_CHUNK <= MAX_CHUNKS, "the scratch holds the small chunks");
 // 3 partial sums per chunk, then one 256-byte line of SLOTS completion slots
 // (ticket, bad-input flag).  A call takes the next slot; a launch that
-// completes leaves its slot at zero and clears the one half a turn ahead,
-// which makes an interrupted launch harmless.
+// completes leaves its slot at zero and clears the one half a turn ahead, so
+// what an interrupted launch leaves is gone before its slot's turn comes again.
+// A call that is captured keeps its slot in every replay: there a copy
+// operation clears the slot before each launch.
 constexpr int SLOTS = 16;
 constexpr int SCRATCH_DOUBLES = 3 * MAX_CHUNKS + 32;
 static_assert(SCRATCH_DOUBLES * 8 == FC3DGPU_NOALLOC_SCRATCH_BYTES, "header states the scratch size");
@@ -319,6 +321,15 @@ extern "C" int fc3dgpu_compute_error_device(int nc, int64_t nnz, const int64_t* 
   int rc = setup(dev, &scratch, &sms, &slot);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();  // the launch reports it
+  if (capture == cudaStreamCaptureStatusActive) {
+    e = cudaMemsetAsync(scratch + 3 * MAX_CHUNKS + slot, 0, 2 * sizeof(unsigned), s);
+    if (e != cudaSuccess) {
+      fc3dgpu_set_error("fc3dgpu_compute_error_device: %s", cudaGetErrorString(e));
+      return NUMERICS_ERR_UNKNOWN;
+    }
+  }
   auto launch = [&](auto kernel, int chunk, int per_sm) {
     const int nchunks = (nc + chunk - 1) / chunk;
     int grid = per_sm * sms;
