@@ -16,18 +16,19 @@ def own(built_lib):
 
 def test_fp64_sweeps_after_a_timeline(own):
     """The dataflow's sweeps start with one launch more (the stamps): before a
-    timeline was armed, not while it is, and again after it was switched off."""
+    timeline was armed, not while it is, and again after it was switched off.
+    The first solve, which also looks at the pattern, is not counted."""
     from siconos_gb300.scene import lattice
     own.load(lattice(6, 6, 4, seed=1))
     n = []
-    for arm in (None, 2, 0):
+    for arm in (None, None, 2, 0):
         if arm is not None:
             own.timeline(arm)
         own.zero_r()
         before = own.launches()
         own.solve(tol=1e-300, max_iter=4, precision=1, lanes=1)
         n.append(own.launches() - before)
-    assert n[1] == n[0] - 1 and n[2] == n[0]
+    assert n[2] == n[1] - 1 and n[3] == n[1]
 
 
 def test_counters_of_a_batch_between_solves(own):
