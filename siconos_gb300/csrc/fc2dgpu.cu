@@ -15,6 +15,8 @@
 #include <string.h>
 
 #include <algorithm>
+#include <memory>
+#include <new>
 #include <numeric>
 #include <type_traits>
 #include <vector>
@@ -1053,7 +1055,43 @@ struct Shape {
   int cs = 1, nt = 128, blocks = 1, rows = 1;
 };
 
-struct fc2dgpu_ctx {
+// Arrays side by side in one allocation; from base nullptr only their length.
+struct Pool {
+  char* base;
+  size_t at;
+  template <typename T>
+  void take(T*& p, size_t n) {
+    p = base ? reinterpret_cast<T*>(base + at) : nullptr;
+    at += (sizeof(T) * n + 255) / 256 * 256;
+  }
+};
+
+// What a problem sends to the device (Args), with FP32 copies for the first
+// phase of a mixed-precision solve.  Filled on the host in one buffer of the
+// device's layout, so that it takes one copy.
+struct Uploaded {
+  int *cptr = nullptr, *rp = nullptr, *col = nullptr, *dpos = nullptr, *sp = nullptr;
+  int2* slab = nullptr;
+  double *W = nullptr, *det = nullptr, *q = nullptr, *mu = nullptr;
+  float *det32 = nullptr, *q32 = nullptr, *mu32 = nullptr;
+  void carve(Pool& pool, int nc, size_t nnzb, int ncol, int nslab) {
+    pool.take(cptr, ncol + 1);
+    pool.take(rp, (size_t)nc + 1);
+    pool.take(col, nnzb);
+    pool.take(dpos, nc);
+    pool.take(sp, ncol + 1);
+    pool.take(slab, nslab);
+    pool.take(W, 4 * nnzb);
+    pool.take(det, nc);
+    pool.take(q, 2 * (size_t)nc);
+    pool.take(mu, nc);
+    pool.take(det32, nc);
+    pool.take(q32, 2 * (size_t)nc);
+    pool.take(mu32, nc);
+  }
+};
+
+struct fc2dgpu_ctx : Uploaded {
   int device = 0;
   int cs_req = 0, nt_req = 0;  // launch shape asked for (0 = automatic)
   int rep_req = 0;             // reactions: 0 automatic, 1 in HBM, 2 replicated in shared memory
@@ -1065,17 +1103,15 @@ struct fc2dgpu_ctx {
   bool singular = false;
   double norm_q = 0.0;
   std::vector<int> perm, iperm, colour;
-  int *cptr = nullptr, *rp = nullptr, *col = nullptr, *dpos = nullptr;
-  int *sp = nullptr, *scol = nullptr;
-  int2* slab = nullptr;
-  double *sW = nullptr, *D = nullptr;
-  float *sW32 = nullptr, *D32 = nullptr;
-  double *W = nullptr, *det = nullptr, *q = nullptr, *mu = nullptr, *r = nullptr, *u = nullptr, *trace = nullptr,
-         *out = nullptr, *part = nullptr, *rs = nullptr;  // rs: stamped reactions of the dataflow, of either precision
-                                                                  // (a symmetric block pattern)
+  void* pool = nullptr;  // holds the arrays of Uploaded and the next seven
+  size_t pool_bytes = 0;
+  int* scol = nullptr;
+  double *sW = nullptr, *D = nullptr, *r = nullptr, *u = nullptr;
+  float *sW32 = nullptr, *D32 = nullptr, *r32 = nullptr;
+  double* rs = nullptr;  // stamped reactions of the dataflow, of either precision (a symmetric block pattern)
+  void* work = nullptr;  // holds the next four
+  double *trace = nullptr, *out = nullptr, *part = nullptr;
   unsigned* flags = nullptr;
-  // FP32 copies for the first phase of a mixed-precision solve
-  float *W32 = nullptr, *det32 = nullptr, *q32 = nullptr, *mu32 = nullptr, *r32 = nullptr;
   unsigned long long spin = SPIN;
   int precision = 1;          // 0 FP32 sweeps + FP64 polish, 1 FP64 sweeps only
   double switch_tol = 0.0;    // FP32 phase stops below this light error (0: max(tol, 1e-6))
@@ -1101,38 +1137,47 @@ constexpr int FLOW_FROM = 64;
 
 static void choose_shape(fc2dgpu_ctx* c);
 
-// Whether every block (i, j) has a block (j, i), as often: the rows' columns in
-// ascending order against the columns' rows, which two transpositions give.
-static bool symmetric_pattern(int nc, const std::vector<int>& rp, const std::vector<int>& col) {
-  auto transpose = [&](const std::vector<int>& p, const std::vector<int>& x, std::vector<int>& tp, std::vector<int>& t) {
+// Whether every block (i, j) has a block (j, i), as often (the dataflow needs
+// it).  On the device a row looks itself up in its neighbours' rows, so the work
+// goes with the square of a row's length: for rows of up to this many blocks.
+constexpr int SYMMETRIC_ROWS = 64;
+
+__global__ void k_one_sided(int nc, const int* __restrict__ rp, const int* __restrict__ col, int* __restrict__ one_sided) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= nc) return;
+  auto count = [&](int row, int of) {
+    int n = 0;
+    for (int k = rp[row]; k < rp[row + 1]; k++) n += col[k] == of;
+    return n;
+  };
+  for (int k = rp[p]; k < rp[p + 1]; k++)
+    if (count(col[k], p) != count(p, col[k])) *one_sided = 1;
+}
+
+// On the host for longer rows: the columns' rows in ascending order, which a
+// transposition gives, against the rows' sorted columns, which a second one
+// gives.
+static bool symmetric_pattern(int nc, const int* rp, const int* col) {
+  auto transpose = [&](const int* p, const int* x, std::vector<int>& tp, std::vector<int>& t) {
     tp.assign(nc + 1, 0);
-    for (int j : x) tp[j + 1]++;
+    for (int k = 0; k < p[nc]; k++) tp[x[k] + 1]++;
     for (int j = 0; j < nc; j++) tp[j + 1] += tp[j];
-    t.resize(x.size());
+    t.resize(p[nc]);
     std::vector<int> at(tp.begin(), tp.end() - 1);
     for (int i = 0; i < nc; i++)
-      for (int s = p[i]; s < p[i + 1]; s++) t[at[x[s]]++] = i;
+      for (int k = p[i]; k < p[i + 1]; k++) t[at[x[k]]++] = i;
   };
   std::vector<int> tp, t, sp, sorted;
   transpose(rp, col, tp, t);
-  if (tp != rp) return false;
-  transpose(tp, t, sp, sorted);
+  if (!std::equal(tp.begin(), tp.end(), rp)) return false;
+  transpose(tp.data(), t.data(), sp, sorted);
   return t == sorted;
 }
 
 static void free_problem(fc2dgpu_ctx* c) {
-  void* ptrs[] = {c->cptr, c->rp, c->col, c->dpos, c->W, c->det, c->q, c->mu, c->r, c->u,
-                  c->sp, c->scol, c->slab, c->sW, c->D, c->sW32, c->D32, c->W32, c->det32, c->q32, c->mu32, c->r32, c->rs};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
-  c->cptr = c->rp = c->col = c->dpos = nullptr;
-  c->W = c->det = c->q = c->mu = c->r = c->u = nullptr;
-  c->sp = c->scol = nullptr;
-  c->slab = nullptr;
-  c->sW = c->D = nullptr;
-  c->sW32 = c->D32 = nullptr;
-  c->W32 = c->det32 = c->q32 = c->mu32 = c->r32 = nullptr;
-  c->rs = nullptr;
+  if (c->pool) cudaFree(c->pool);
+  c->pool = nullptr;
+  c->pool_bytes = 0;
   c->nc = 0;
 }
 
@@ -1140,10 +1185,7 @@ extern "C" void fc2dgpu_ctx_destroy(fc2dgpu_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   free_problem(c);
-  if (c->trace) cudaFree(c->trace);
-  if (c->out) cudaFree(c->out);
-  if (c->part) cudaFree(c->part);
-  if (c->flags) cudaFree(c->flags);
+  if (c->work) cudaFree(c->work);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -1163,13 +1205,20 @@ extern "C" fc2dgpu_ctx* fc2dgpu_ctx_create(int device) {
   }
   fc2dgpu_ctx* c = new fc2dgpu_ctx();
   c->device = device;
+  auto carve = [&](Pool p) {
+    p.take(c->trace, TRACE_CAP);
+    p.take(c->out, 9);
+    p.take(c->part, 2 * GRID_MAX * 4);
+    p.take(c->flags, GRID_MAX * FLAG_STRIDE);
+    return p.at;
+  };
   bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaEventCreate(&c->ev[0]) == cudaSuccess && cudaEventCreate(&c->ev[1]) == cudaSuccess &&
-            cudaMalloc(&c->trace, sizeof(double) * TRACE_CAP) == cudaSuccess &&
-            cudaMalloc(&c->out, sizeof(double) * 9) == cudaSuccess &&
-            cudaMemset(c->out, 0, sizeof(double) * 9) == cudaSuccess &&
-            cudaMalloc(&c->flags, sizeof(unsigned) * GRID_MAX * FLAG_STRIDE) == cudaSuccess &&
-            cudaMalloc(&c->part, sizeof(double) * 2 * GRID_MAX * 4) == cudaSuccess;
+            cudaMalloc(&c->work, carve(Pool{nullptr, 0})) == cudaSuccess;
+  if (ok) {
+    carve(Pool{static_cast<char*>(c->work), 0});
+    ok = cudaMemsetAsync(c->out, 0, sizeof(double) * 9, c->stream) == cudaSuccess;
+  }
   if (!ok) {
     fc3dgpu_set_error("fc2dgpu_ctx_create: set-up failed (%s)", cudaGetErrorString(cudaGetLastError()));
     fc2dgpu_ctx_destroy(c);
@@ -1178,12 +1227,40 @@ extern "C" fc2dgpu_ctx* fc2dgpu_ctx_create(int device) {
   return c;
 }
 
-template <typename T>
-static cudaError_t upload(T** d, const std::vector<T>& h) {
-  cudaError_t e = cudaMalloc((void**)d, sizeof(T) * (h.empty() ? 1 : h.size()));
-  if (e != cudaSuccess) return e;
-  if (!h.empty()) e = cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice);
-  return e;
+// The sweeps' coalesced copy of the rows (Args::slab), one thread a row.  Built
+// here from the uploaded rows: on the host, with an upload each in both
+// precisions, it took longer than the rest of the layout (70,020 contacts:
+// T2D ms, T2D now).
+__global__ void k_slab_rows(int ncol, const int* __restrict__ cptr, const int* __restrict__ sp,
+                            const int2* __restrict__ slab, const int* __restrict__ rp, const int* __restrict__ col,
+                            const int* __restrict__ dpos, const double* __restrict__ W, int* __restrict__ scol,
+                            double* __restrict__ sW, float* __restrict__ sW32, double* __restrict__ D,
+                            float* __restrict__ D32) {
+  const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (b >= sp[ncol]) return;
+  int c = 0;
+  while (sp[c + 1] <= b) c++;
+  const int p = cptr[c] + (b - sp[c]) * 32 + lane;
+  const int2 s = slab[b];
+  auto put = [&](size_t e, int j, double a00, double a01, double a10, double a11) {
+    scol[e] = j;
+    reinterpret_cast<double2*>(sW)[2 * e] = make_double2(a00, a01);
+    reinterpret_cast<double2*>(sW)[2 * e + 1] = make_double2(a10, a11);
+    reinterpret_cast<float4*>(sW32)[e] = make_float4((float)a00, (float)a01, (float)a10, (float)a11);
+  };
+  int t = 0;
+  if (p < cptr[c + 1]) {
+    for (int k = rp[p]; k < rp[p + 1]; k++) {
+      const double* w = W + 4 * (size_t)k;
+      if (col[k] != p) put((size_t)(s.x + t++) * 32 + lane, col[k], w[0], w[2], w[1], w[3]);
+    }
+    const double* d = W + 4 * (size_t)(rp[p] + dpos[p]);
+    for (int i = 0; i < 4; i++) {
+      D[4 * (size_t)p + i] = d[i];
+      D32[4 * (size_t)p + i] = (float)d[i];
+    }
+  }
+  for (; t < s.y; t++) put((size_t)(s.x + t) * 32 + lane, -1, 0.0, 0.0, 0.0, 0.0);
 }
 
 extern "C" int fc2dgpu_ctx_set_problem(fc2dgpu_ctx* c, int nc, const int64_t* rowptr, const int64_t* colidx,
@@ -1232,128 +1309,127 @@ extern "C" int fc2dgpu_ctx_set_problem(fc2dgpu_ctx* c, int nc, const int64_t* ro
     fc3dgpu_set_error("fc2dgpu_ctx_set_problem: cudaSetDevice failed");
     return NUMERICS_ERR_UNKNOWN;
   }
-  free_problem(c);
+  c->nc = 0;
   c->colour.assign(colour.begin(), colour.end());
   c->perm.resize(nc);
   std::iota(c->perm.begin(), c->perm.end(), 0);
   std::stable_sort(c->perm.begin(), c->perm.end(), [&](int x, int y) { return colour[x] < colour[y]; });
   c->iperm.resize(nc);
   for (int p = 0; p < nc; p++) c->iperm[c->perm[p]] = p;
-  std::vector<int> cptr(ncol + 1, 0);
-  for (int i = 0; i < nc; i++) cptr[colour[i] + 1]++;
-  for (int k = 0; k < ncol; k++) cptr[k + 1] += cptr[k];
-  std::vector<int> rp(nc + 1, 0), col((size_t)nnzb), dpos(nc);
-  std::vector<double> W((size_t)nnzb * 4), det(nc), qp(2 * (size_t)nc), mup(nc);
-  bool singular = false;
-  for (int p = 0; p < nc; p++) {
-    const int i = c->perm[p];
-    const int64_t k0 = rowptr[i], k1 = rowptr[i + 1];
-    rp[p + 1] = rp[p] + (int)(k1 - k0);
-    for (int64_t k = k0; k < k1; k++) {
-      const int s = rp[p] + (int)(k - k0);
-      col[s] = c->iperm[colidx[k]];
-      for (int e = 0; e < 4; e++) W[4 * (size_t)s + e] = blocks[4 * k + e];
-    }
-    dpos[p] = dposo[i];
-    const double* b = &blocks[4 * (rowptr[i] + dposo[i])];
-    det[p] = b[0] * b[3] - b[1] * b[2];
-    if (det[p] < DBL_EPSILON) singular = true;
-    qp[2 * p] = q[2 * i];
-    qp[2 * p + 1] = q[2 * i + 1];
-    mup[p] = mu[i];
+  // the rows' slabs by colour (Args::slab)
+  std::vector<int> size(ncol, 0);
+  for (int i = 0; i < nc; i++) size[colour[i]]++;
+  c->max_colour = *std::max_element(size.begin(), size.end());
+  int nslab = 0;
+  for (int n : size) nslab += (n + 31) / 32;
+  Uploaded h;
+  Pool measure = {nullptr, 0};
+  h.carve(measure, nc, nnzb, ncol, nslab);
+  const size_t sent = measure.at;
+  const std::unique_ptr<char[]> host(new (std::nothrow) char[sent]);
+  if (!host) {
+    fc3dgpu_set_error("fc2dgpu_ctx_set_problem: out of host memory");
+    return NUMERICS_ERR_MEMORY;
   }
+  Pool pool = {host.get(), 0};
+  h.carve(pool, nc, nnzb, ncol, nslab);
+  h.cptr[0] = h.sp[0] = 0;
+  for (int k = 0; k < ncol; k++) {
+    h.cptr[k + 1] = h.cptr[k] + size[k];
+    h.sp[k + 1] = h.sp[k] + (size[k] + 31) / 32;
+  }
+  bool singular = false;
+  size_t slots = 0;
+  int longest = 0;
+  h.rp[0] = 0;
+  for (int k = 0; k < ncol; k++)
+    for (int b = h.sp[k]; b < h.sp[k + 1]; b++) {
+      int most = 0;  // blocks off the diagonal of the slab's longest row
+      for (int p = h.cptr[k] + 32 * (b - h.sp[k]); p < std::min(h.cptr[k] + 32 * (b + 1 - h.sp[k]), h.cptr[k + 1]); p++) {
+        const int i = c->perm[p];
+        const int64_t k0 = rowptr[i], k1 = rowptr[i + 1];
+        int off = 0;
+        for (int64_t s = k0; s < k1; s++) {
+          const size_t at = (size_t)h.rp[p] + (size_t)(s - k0);
+          h.col[at] = c->iperm[colidx[s]];
+          off += colidx[s] != i;
+          for (int e = 0; e < 4; e++) h.W[4 * at + e] = blocks[4 * s + e];
+        }
+        h.rp[p + 1] = h.rp[p] + (int)(k1 - k0);
+        longest = std::max(longest, (int)(k1 - k0));
+        most = std::max(most, off);
+        h.dpos[p] = dposo[i];
+        const double* d = &blocks[4 * (k0 + dposo[i])];
+        h.det[p] = d[0] * d[3] - d[1] * d[2];
+        // of the rounded block, in FP32
+        h.det32[p] = (float)d[0] * (float)d[3] - (float)d[1] * (float)d[2];
+        if (h.det[p] < DBL_EPSILON) singular = true;
+        for (int e = 0; e < 2; e++) {
+          h.q[2 * (size_t)p + e] = q[2 * (size_t)i + e];
+          h.q32[2 * (size_t)p + e] = (float)q[2 * (size_t)i + e];
+        }
+        h.mu[p] = mu[i];
+        h.mu32[p] = (float)mu[i];
+      }
+      h.slab[b] = make_int2((int)slots, most);
+      slots += most;
+    }
   double s2 = 0.0;
   for (int64_t k = 0; k < 2LL * nc; k++) s2 += q[k] * q[k];
   c->norm_q = sqrt(s2);
-  std::vector<double> zero(2 * (size_t)nc, 0.0);
+  // the device's arrays, in the allocation of the problem before where that is
+  // of about the size
+  int* one_sided = nullptr;
+  auto carve = [&](Pool p) {
+    c->carve(p, nc, nnzb, ncol, nslab);
+    p.take(c->scol, slots * 32);
+    p.take(c->sW, slots * 128);
+    p.take(c->sW32, slots * 128);
+    p.take(c->D, 4 * (size_t)nc);
+    p.take(c->D32, 4 * (size_t)nc);
+    p.take(c->rs, c->max_colour > FLOW_FROM ? 4 * (size_t)nc : 0);
+    // zero from here on
+    p.take(c->r, 2 * (size_t)nc);
+    p.take(c->u, 2 * (size_t)nc);
+    p.take(c->r32, 2 * (size_t)nc);
+    p.take(one_sided, 1);
+    return p.at;
+  };
+  const size_t bytes = carve(Pool{nullptr, 0});
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = upload(&c->cptr, cptr);
-  if (e == cudaSuccess) e = upload(&c->rp, rp);
-  if (e == cudaSuccess) e = upload(&c->col, col);
-  if (e == cudaSuccess) e = upload(&c->dpos, dpos);
-  if (e == cudaSuccess) e = upload(&c->W, W);
-  if (e == cudaSuccess) e = upload(&c->det, det);
-  if (e == cudaSuccess) e = upload(&c->q, qp);
-  if (e == cudaSuccess) e = upload(&c->mu, mup);
-  if (e == cudaSuccess) e = upload(&c->r, zero);
-  if (e == cudaSuccess) e = upload(&c->u, zero);
-  // FP32 copies; the determinants of the rounded blocks, in FP32
-  {
-    std::vector<float> W32(W.begin(), W.end()), det32(nc), q32(qp.begin(), qp.end()), mu32(mup.begin(), mup.end());
-    for (int p = 0; p < nc; p++) {
-      const float* b = &W32[4 * ((size_t)rp[p] + dpos[p])];
-      det32[p] = b[0] * b[3] - b[1] * b[2];
-    }
-    std::vector<float> zero32(2 * (size_t)nc, 0.0f);
-    if (e == cudaSuccess) e = upload(&c->W32, W32);
-    if (e == cudaSuccess) e = upload(&c->det32, det32);
-    if (e == cudaSuccess) e = upload(&c->q32, q32);
-    if (e == cudaSuccess) e = upload(&c->mu32, mu32);
-    if (e == cudaSuccess) e = upload(&c->r32, zero32);
+  if (bytes > c->pool_bytes || bytes < c->pool_bytes / 2) {
+    free_problem(c);
+    e = cudaMalloc(&c->pool, bytes);
+    c->pool_bytes = e == cudaSuccess ? bytes : 0;
+    if (e != cudaSuccess) c->pool = nullptr;
   }
-  // the sweeps' coalesced copy of the rows (Args::slab)
-  {
-    std::vector<int> sp(ncol + 1, 0);
-    for (int k = 0; k < ncol; k++) sp[k + 1] = sp[k] + (cptr[k + 1] - cptr[k] + 31) / 32;
-    std::vector<int2> slab(sp[ncol]);
-    int slots = 0;
-    auto off_diagonal = [&](int p) {
-      int n = 0;
-      for (int s = rp[p]; s < rp[p + 1]; s++) n += col[s] != p;
-      return n;
-    };
-    for (int k = 0; k < ncol; k++)
-      for (int b = sp[k]; b < sp[k + 1]; b++) {
-        const int p0 = cptr[k] + 32 * (b - sp[k]), p1 = std::min(p0 + 32, cptr[k + 1]);
-        int m = 0;
-        for (int p = p0; p < p1; p++) m = std::max(m, off_diagonal(p));
-        slab[b] = make_int2(slots, m);
-        slots += m;
-      }
-    std::vector<int> scol((size_t)slots * 32, -1);
-    std::vector<double> sW((size_t)slots * 128, 0.0), D(4 * (size_t)nc);
-    for (int k = 0; k < ncol; k++)
-      for (int p = cptr[k]; p < cptr[k + 1]; p++) {
-        const int b = sp[k] + (p - cptr[k]) / 32, lane = (p - cptr[k]) % 32;
-        size_t slot = (size_t)slab[b].x;
-        for (int s = rp[p]; s < rp[p + 1]; s++) {
-          if (col[s] == p) continue;
-          const size_t x = slot++ * 32 + lane;
-          scol[x] = col[s];
-          const double* w = &W[4 * (size_t)s];
-          sW[4 * x] = w[0];
-          sW[4 * x + 1] = w[2];
-          sW[4 * x + 2] = w[1];
-          sW[4 * x + 3] = w[3];
-        }
-        for (int i = 0; i < 4; i++) D[4 * (size_t)p + i] = W[4 * ((size_t)rp[p] + dpos[p]) + i];
-      }
-    const std::vector<float> sW32(sW.begin(), sW.end()), D32(D.begin(), D.end());
-    if (e == cudaSuccess) e = upload(&c->sp, sp);
-    if (e == cudaSuccess) e = upload(&c->slab, slab);
-    if (e == cudaSuccess) e = upload(&c->scol, scol);
-    if (e == cudaSuccess) e = upload(&c->sW, sW);
-    if (e == cudaSuccess) e = upload(&c->D, D);
-    if (e == cudaSuccess) e = upload(&c->sW32, sW32);
-    if (e == cudaSuccess) e = upload(&c->D32, D32);
+  int mismatch = 0;
+  if (e == cudaSuccess) {
+    cudaStream_t st = c->stream;
+    carve(Pool{static_cast<char*>(c->pool), 0});
+    e = cudaMemcpyAsync(c->pool, host.get(), sent, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->r, 0, (size_t)((char*)(one_sided + 1) - (char*)c->r), st);
+    k_slab_rows<<<(nslab * 32 + 255) / 256, 256, 0, st>>>(ncol, c->cptr, c->sp, c->slab, c->rp, c->col, c->dpos, c->W,
+                                                          c->scol, c->sW, c->sW32, c->D, c->D32);
+    if (c->max_colour > FLOW_FROM && longest <= SYMMETRIC_ROWS) {
+      k_one_sided<<<(nc + 255) / 256, 256, 0, st>>>(nc, c->rp, c->col, one_sided);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(&mismatch, one_sided, sizeof(int), cudaMemcpyDeviceToHost, st);
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    const cudaError_t done = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = done;
   }
   if (e != cudaSuccess) {
+    cudaGetLastError();
     free_problem(c);
     fc3dgpu_set_error("fc2dgpu_ctx_set_problem: %s", cudaGetErrorString(e));
     return NUMERICS_ERR_UNKNOWN;
   }
+  if (c->max_colour <= FLOW_FROM || mismatch || (longest > SYMMETRIC_ROWS && !symmetric_pattern(nc, h.rp, h.col)))
+    c->rs = nullptr;
   c->nc = nc;
   c->ncol = ncol;
   c->singular = singular;
-  c->max_colour = 0;
-  for (int k = 0; k < ncol; k++) c->max_colour = std::max(c->max_colour, cptr[k + 1] - cptr[k]);
-  if (c->max_colour > FLOW_FROM && symmetric_pattern(nc, rp, col) &&
-      cudaMalloc(&c->rs, sizeof(double) * 4 * (size_t)nc) != cudaSuccess) {
-    cudaGetLastError();
-    free_problem(c);
-    fc3dgpu_set_error("fc2dgpu_ctx_set_problem: out of device memory");
-    return NUMERICS_ERR_UNKNOWN;
-  }
   choose_shape(c);
   return 0;
 }
@@ -1494,19 +1570,12 @@ static Shape flow_shape(fc2dgpu_ctx* c, int most) {
   return s;
 }
 
-static void choose_flow(fc2dgpu_ctx* c) {
-  if (!c->rs || c->cs_req != 0 || c->nt_req != 0 || c->rep_req != 0) return;
-  c->s32 = flow_shape(c, 32);
-  c->s64 = flow_shape(c, 16);
-}
-
-static void choose_blocks(fc2dgpu_ctx* c);
 static void choose_shape(fc2dgpu_ctx* c) {
-  choose_blocks(c);
-  choose_flow(c);
-}
-
-static void choose_blocks(fc2dgpu_ctx* c) {
+  if (c->rs && c->cs_req == 0 && c->nt_req == 0 && c->rep_req == 0) {
+    c->s32 = flow_shape(c, 32);
+    c->s64 = flow_shape(c, 16);
+    return;
+  }
   if (c->cs_req < 0 || (c->cs_req == 0 && c->rep_req != 2 && c->max_colour > GRID_FROM)) {
     c->s32 = grid_shape(c, c->nt_req, 1);
     c->s64 = c->cs_req < 0 ? c->s32 : grid_shape(c, c->nt_req, 2);
@@ -1630,7 +1699,6 @@ static Args<float> args32(const fc2dgpu_ctx* c) {
   a.rp = c->rp;
   a.col = c->col;
   a.dpos = c->dpos;
-  a.W = c->W32;
   a.sp = c->sp;
   a.slab = c->slab;
   a.scol = c->scol;
