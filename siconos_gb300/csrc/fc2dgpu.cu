@@ -101,7 +101,7 @@ struct Args {
 // shared memory.  A cooperative grid (every SM, for colours too large for a
 // cluster): grid barrier, partial sums through a ring in global memory.
 struct ClusterTeam {
-  static constexpr bool grid = false, flow = false;
+  static constexpr bool grid = false, flow = false, alone = false;
   cg::cluster_group cl;
   template <typename T>
   __device__ explicit ClusterTeam(const Args<T>&) : cl(cg::this_cluster()) {}
@@ -129,7 +129,7 @@ struct ClusterTeam {
 };
 
 struct GridTeam {
-  static constexpr bool grid = true, flow = false;
+  static constexpr bool grid = true, flow = false, alone = false;
   cg::grid_group g;
   template <typename T>
   __device__ explicit GridTeam(const Args<T>&) : g(cg::this_grid()) {}
@@ -146,11 +146,21 @@ struct GridTeam {
   __device__ __forceinline__ void wait() { sync(); }
 };
 
+// The same with FP64 contacts on one lane each (sweep_alone).
+struct ClusterAlone : ClusterTeam {
+  static constexpr bool alone = true;
+  using ClusterTeam::ClusterTeam;
+};
+struct GridAlone : GridTeam {
+  static constexpr bool alone = true;
+  using GridTeam::GridTeam;
+};
+
 // A cooperative grid whose sweeps are dataflow: a barrier of flags (the sums
 // of a sweep pass one) whose waits, like those for reactions, end after `spin`
 // polls; `dead` (the same in the whole block) then ends the solve.
 struct FlowTeam {
-  static constexpr bool grid = true, flow = true;
+  static constexpr bool grid = true, flow = true, alone = false;
   unsigned* flags;
   double* fail;
   unsigned long long spin;
@@ -691,6 +701,70 @@ __device__ __forceinline__ void sweep_colours(const Args<double>& a, Reactions<d
   }
 }
 
+// local_solve with the integer forms of its divisions and comparisons
+__device__ __forceinline__ void local_solve64(const double2 n, const double2 t, double det, const double q[2],
+                                              double mu, double P[2]) {
+  using namespace fc3dgpu;
+  if (ie_positive(q[0])) {
+    P[0] = P[1] = 0.0;
+    return;
+  }
+  ie_div2(-(t.y * q[0] - t.x * q[1]), -(-n.y * q[0] + n.x * q[1]), ie_den(det), P[0], P[1]);
+  const double muPn = mu * P[0];
+  if (ie_lt(muPn, ie_abs(P[1]))) {
+    const bool back = ie_lt(P[1], -muPn);
+    P[0] = ie_div(-q[0], back ? n.x - mu * t.x : n.x + mu * t.x);
+    P[1] = (back ? -mu : mu) * P[0];
+  }
+}
+
+// The FP64 sweep with a contact a lane, where a requested launch leaves a thread
+// more than ALONE_FROM contacts of a colour: two lanes a contact then take twice
+// the rounds, each with the whole chain of a contact.
+template <bool REP, typename Team>
+__device__ __forceinline__ void sweep_alone(const Args<double>& a, Reactions<double, REP>& rx, int g0, int G,
+                                            double v[2], Team& team) {
+  constexpr int NB = 4;  // slots loaded together
+  for (int c = 0; c < a.ncol; c++) {
+    const int p0 = __ldg(&a.cptr[c]), n = __ldg(&a.cptr[c + 1]) - p0;
+    for (int k = g0; k < n; k += G) {
+      const int p = p0 + k;
+      const int2 s = __ldg(&a.slab[__ldg(&a.sp[c]) + (k >> 5)]);
+      const double2 old = rx.get(p), q = __ldg(reinterpret_cast<const double2*>(a.q) + p);
+      double y[2] = {q.x, q.y};
+      for (int t0 = 0; t0 < s.y; t0 += NB) {
+        int col[NB];
+        double2 w[NB][2], r[NB];
+#pragma unroll
+        for (int i = 0; i < NB; i++) {
+          const size_t e = (size_t)(s.x + (t0 + i < s.y ? t0 + i : t0)) * 32 + (k & 31);
+          col[i] = t0 + i < s.y ? __ldg(&a.scol[e]) : -1;
+          w[i][0] = __ldg(reinterpret_cast<const double2*>(a.sW) + 2 * e);
+          w[i][1] = __ldg(reinterpret_cast<const double2*>(a.sW) + 2 * e + 1);
+        }
+        rx.gather(col, p, r);
+#pragma unroll
+        for (int i = 0; i < NB; i++)
+          if (col[i] >= 0) {
+            y[0] += w[i][0].x * r[i].x;
+            y[1] += w[i][1].x * r[i].x;
+            y[0] += w[i][0].y * r[i].y;
+            y[1] += w[i][1].y * r[i].y;
+          }
+      }
+      const double2 wn = __ldg(reinterpret_cast<const double2*>(a.D) + 2 * (size_t)p);
+      const double2 wt = __ldg(reinterpret_cast<const double2*>(a.D) + 2 * (size_t)p + 1);
+      double P[2];
+      local_solve64(wn, wt, __ldg(&a.det[p]), y, __ldg(&a.mu[p]), P);
+      const double x0 = old.x - P[0], x1 = old.y - P[1];
+      v[0] += x0 * x0 + x1 * x1;
+      v[1] += P[0] * P[0] + P[1] * P[1];
+      rx.put(p, P[0], P[1], team);
+    }
+    if (c + 1 < a.ncol) team.sync();
+  }
+}
+
 // ---- the sweeps as dataflow -------------------------------------------------
 // What bounds a colour of a large problem is not its contacts but what stands
 // between two colours: a barrier over every SM and then the loads it releases.
@@ -952,7 +1026,7 @@ __global__ void __launch_bounds__(Team::flow ? 256 : NT_MAX, 1) k_fc2d_nsgs(cons
   T tolerance = (T)a.tol, err = (T)INFINITY, best = (T)INFINITY;
   int iter = 0, not_conv = 1, since_best = 0;
   Row<T> row;
-  if constexpr (!Team::flow) {
+  if constexpr (!Team::flow && !Team::alone) {
     const int comp = sizeof(T) == sizeof(double) ? g0 & 1 : 0, k = sizeof(T) == sizeof(double) ? g0 >> 1 : g0;
     if (k < a.cptr[1] - a.cptr[0]) load_row(a, 0, k, comp, row);
   }
@@ -962,6 +1036,8 @@ __global__ void __launch_bounds__(Team::flow ? 256 : NT_MAX, 1) k_fc2d_nsgs(cons
     if constexpr (Team::flow) {
       fx.sweep = iter;
       flow_sweep(a, fx, tab, v, team);
+    } else if constexpr (Team::alone) {
+      sweep_alone(a, rx, g0, G, v, team);
     } else {
       sweep_colours(a, rx, g0, G, row, v, team);
     }
@@ -1052,6 +1128,7 @@ using namespace fc2dgpu;
 // reactions in HBM or replicated in shared memory.
 struct Shape {
   bool grid = false, rep = false, flow = false;
+  bool alone = false;  // FP64: a contact a lane
   int cs = 1, nt = 128, blocks = 1, rows = 1;
 };
 
@@ -1539,6 +1616,13 @@ constexpr int GRID_FROM = CS_MAX * NT_MAX;
 // where the grid's barriers alone take 8 more than the cluster's).
 constexpr int GRID64_FROM = 1000;
 
+// Contacts of the largest colour a thread from which FP64 contacts are one
+// lane's.  ms for 40 sweeps on two lanes and on one, by contacts a thread: 1.2
+// (2,048 threads) 2.25 and 2.47, 1.2 (77,824) 4.39 and 5.13, 3.1 (77,824) 8.39 and
+// 8.85; 4.7 (512) 4.48 and 3.78, 4.7 (2,048) 6.17 and 5.63, 12 (8,192) 24.7 and 22.2,
+// 19 (128) 14.7 and 11.4, 76 (128) 60.1 and 45.3.
+constexpr int ALONE_FROM = 4;
+
 static Shape grid_shape(fc2dgpu_ctx* c, int nt, int lanes) {
   Shape s;
   int sms = 0, per_sm = 0;
@@ -1570,12 +1654,18 @@ static Shape flow_shape(fc2dgpu_ctx* c, int most) {
   return s;
 }
 
+static void choose_blocks(fc2dgpu_ctx* c);
 static void choose_shape(fc2dgpu_ctx* c) {
   if (c->rs && c->cs_req == 0 && c->nt_req == 0 && c->rep_req == 0) {
     c->s32 = flow_shape(c, 32);
     c->s64 = flow_shape(c, 16);
     return;
   }
+  choose_blocks(c);
+  c->s64.alone = c->max_colour > (long long)ALONE_FROM * (c->s64.grid ? c->s64.blocks : c->s64.cs) * c->s64.nt;
+}
+
+static void choose_blocks(fc2dgpu_ctx* c) {
   if (c->cs_req < 0 || (c->cs_req == 0 && c->rep_req != 2 && c->max_colour > GRID_FROM)) {
     c->s32 = grid_shape(c, c->nt_req, 1);
     c->s64 = c->cs_req < 0 ? c->s32 : grid_shape(c, c->nt_req, 2);
@@ -1813,10 +1903,15 @@ extern "C" int fc2dgpu_ctx_solve(fc2dgpu_ctx* c, double tol, int max_iter, int e
   const Shape& s = c->s64;
   a.rows = s.rows;
   if (s.flow) K2(cudaMemsetAsync(c->flags, 0, sizeof(unsigned) * GRID_MAX * FLAG_STRIDE, c->stream));
-  K2(s.flow  ? launch_grid(c, s, k_fc2d_nsgs<double, false, FlowTeam>, a)
-     : s.grid ? launch_grid(c, s, k_fc2d_nsgs<double, false, GridTeam>, a)
-     : s.rep ? launch(c, s, k_fc2d_nsgs<double, true, ClusterTeam>, a, rep_bytes(c))
-             : launch(c, s, k_fc2d_nsgs<double, false, ClusterTeam>, a, 0));
+  if (s.alone)
+    K2(s.grid  ? launch_grid(c, s, k_fc2d_nsgs<double, false, GridAlone>, a)
+       : s.rep ? launch(c, s, k_fc2d_nsgs<double, true, ClusterAlone>, a, rep_bytes(c))
+               : launch(c, s, k_fc2d_nsgs<double, false, ClusterAlone>, a, 0));
+  else
+    K2(s.flow  ? launch_grid(c, s, k_fc2d_nsgs<double, false, FlowTeam>, a)
+       : s.grid ? launch_grid(c, s, k_fc2d_nsgs<double, false, GridTeam>, a)
+       : s.rep ? launch(c, s, k_fc2d_nsgs<double, true, ClusterTeam>, a, rep_bytes(c))
+               : launch(c, s, k_fc2d_nsgs<double, false, ClusterTeam>, a, 0));
   K2(cudaEventRecord(c->ev[1], c->stream));
   double out[9];
   K2(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));

@@ -75,3 +75,24 @@ def test_problems_in_turn(sn):  # noqa: F811
             ctx.nc = nc
         _check(sn, ctx, P)
     ctx.close()
+
+
+@pytest.mark.parametrize("copies,shape", [(9, (1, 32, 1)), (9, (1, 64, 2)), (9, (2, 32, 2)), (9, (16, 32, 1)),
+                                          (1, (1, 32, 0)), (1, (1, 64, 0)), (4, (1, 128, 2)), (4, (1, 160, 1)),
+                                          (1100, (-1, 32, 0))])
+def test_more_contacts_than_threads(sn, copies, shape):  # noqa: F811
+    """Requested launches on both sides of the line from which FP64 contacts are
+    one lane's (four a thread; 131 contacts in the largest colour of a copy)."""
+    import oracle as O
+    from test_fc2d_oracle import load_fc2d, tiled2d
+    P = tiled2d(load_fc2d("fc2d_FrictionContactProblem00727")[0], copies, 4)
+    ctx = _ctx(sn, P)
+    _, colour = ctx.colours()
+    ctx.set_launch(*shape)
+    res = ctx.solve(0.0, 6)
+    r, u = ctx.get_r_u()
+    ctx.close()
+    ref = O.fc2d_nsgs_port(P, tol=0.0, maxiter=6, order=_order(colour))
+    np.testing.assert_array_equal(r, ref.r)
+    np.testing.assert_array_equal(u, ref.u)
+    assert res["error"] == pytest.approx(ref.error, rel=1e-12, abs=0)
