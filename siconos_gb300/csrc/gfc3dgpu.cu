@@ -619,7 +619,7 @@ struct gfc3dgpu_ctx {
 static void free_problem(gfc3dgpu_ctx* c) {
   void* ptrs[] = {c->hoff, c->moff, c->toff, c->luoff, c->hns, c->hcol, c->mns, c->mcol, c->tns, c->tcol,
                   c->cptr, c->cdof, c->piv, c->hval, c->mval, c->tval, c->q, c->mdiag, c->lu, c->b,
-                  c->mu, c->r[0], c->r[1], c->u[0], c->u[1], c->v[0], c->v[1], c->t};
+                  c->mu, c->r[0], c->u[0], c->v[0], c->v[1], c->t};  // r[1] and u[1] lie behind r[0] and u[0]
   for (void* p : ptrs)
     if (p) cudaFree(p);
   c->hoff = c->moff = c->toff = c->luoff = nullptr;
@@ -880,7 +880,7 @@ extern "C" int gfc3dgpu_ctx_set_problem(gfc3dgpu_ctx* c, int64_t n, int nc, cons
   }
   free_problem(c);
   std::vector<double> qv(q, q + n), bv(b ? b : q, b ? b + m : q), muv(mu ? mu : q, mu ? mu + nc : q);
-  std::vector<double> zero_r(m + 1, 0.0), zero_v(n + 1, 0.0);
+  const std::vector<double> zero_v(n + 1, 0.0);
   std::vector<long long> mp64(Mp, Mp + n + 1);
   std::vector<int> mi32(Mi, Mi + Mp[n]);
   std::vector<double> mx64(Mx, Mx + Mp[n]);
@@ -906,11 +906,15 @@ extern "C" int gfc3dgpu_ctx_set_problem(gfc3dgpu_ctx* c, int64_t n, int nc, cons
   ok(put(&c->q, qv));
   ok(put(&c->b, bv));
   ok(put(&c->mu, muv));
-  for (int k = 0; k < 2; k++) {
-    ok(put(&c->r[k], zero_r));
-    ok(put(&c->u[k], std::vector<double>(std::max<long long>(m, 1), 0.0)));
-    ok(put(&c->v[k], zero_v));
-  }
+  // both buffers of r and of u in one allocation each (an allocation and copy
+  // takes 10 us)
+  const long long pitch = (m + 1 + 31) / 32 * 32;
+  const std::vector<double> zero_pair(2 * pitch, 0.0);
+  ok(put(&c->r[0], zero_pair));
+  ok(put(&c->u[0], zero_pair));
+  c->r[1] = c->r[0] + pitch;
+  c->u[1] = c->u[0] + pitch;
+  for (int k = 0; k < 2; k++) ok(put(&c->v[k], zero_v));
   ok(put(&c->t, std::vector<double>(n, 0.0)));
   int singular = 0;
   if (diag) {
