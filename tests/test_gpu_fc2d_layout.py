@@ -49,11 +49,13 @@ def _check(sn, ctx, P):  # noqa: F811
     np.testing.assert_array_equal(ctx.get_r_u()[0], want)
 
 
-@pytest.mark.parametrize("rows", [20, 64, 65, 100])
+@pytest.mark.parametrize("nc,rows", [(300, 20), (300, 64), (300, 100), (2698, 52), (2698, 53), (3000, 64), (3000, 65),
+                                     (3000, 100)])
 @pytest.mark.parametrize("change", ["none", "drop", "double"])
-def test_pattern(sn, rows, change):  # noqa: F811
+def test_pattern(sn, nc, rows, change):  # noqa: F811
+    """Looked at by the device from 8,192 blocks on, with rows of up to 64."""
     import oracle as O
-    P = _hub(O, 300, rows, change)
+    P = _hub(O, nc, rows, change)
     ctx = _ctx(sn, P)
     assert (ctx.launch_shape()[0] < 0) == (change == "none")  # a grid: dataflow
     _check(sn, ctx, P)
