@@ -107,8 +107,10 @@ int fc2dgpu_ctx_colours(fc2dgpu_ctx *ctx, int32_t *colour);
  * (reactions = 1) or replicated in every cluster block's shared memory (2,
  * up to 13,312 contacts); 0 picks each from the problem (the default; then
  * larger problems on a symmetric pattern sweep as dataflow on a grid).
- * fc2dgpu_ctx_launch_shape reports a grid as minus its block count.  The
- * iterates do not depend on the shape; the reduction order of the errors
+ * fc2dgpu_ctx_launch_shape reports the launch that a solve of the context's
+ * precision starts with (FP64 sweeps, or in mixed precision the FP32 ones,
+ * whose automatic launch may be another), a grid as minus its block count.
+ * The iterates do not depend on the shape; the reduction order of the errors
  * does. */
 int fc2dgpu_ctx_set_launch(fc2dgpu_ctx *ctx, int cluster_blocks, int threads, int reactions);
 int fc2dgpu_ctx_launch_shape(fc2dgpu_ctx *ctx, int *cluster_blocks, int *threads, int *reactions);

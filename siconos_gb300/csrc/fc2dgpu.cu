@@ -1747,9 +1747,10 @@ extern "C" int fc2dgpu_ctx_set_launch(fc2dgpu_ctx* c, int cluster_blocks, int th
 
 extern "C" int fc2dgpu_ctx_launch_shape(fc2dgpu_ctx* c, int* cluster_blocks, int* threads, int* reactions) {
   if (!c) return NUMERICS_ERR_INVALID_ARGUMENT;
-  if (cluster_blocks) *cluster_blocks = c->s32.grid ? -c->s32.blocks : c->s32.cs;
-  if (threads) *threads = c->s32.nt;
-  if (reactions) *reactions = c->s32.rep ? 2 : 1;
+  const Shape& s = c->precision == 0 ? c->s32 : c->s64;
+  if (cluster_blocks) *cluster_blocks = s.grid ? -s.blocks : s.cs;
+  if (threads) *threads = s.nt;
+  if (reactions) *reactions = s.rep ? 2 : 1;
   return 0;
 }
 

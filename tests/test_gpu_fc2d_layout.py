@@ -98,3 +98,21 @@ def test_more_contacts_than_threads(sn, copies, shape):  # noqa: F811
     np.testing.assert_array_equal(r, ref.r)
     np.testing.assert_array_equal(u, ref.u)
     assert res["error"] == pytest.approx(ref.error, rel=1e-12, abs=0)
+
+
+@pytest.mark.parametrize("problem,copies", [("FrictionContactProblem00727", 9), ("FrictionContactProblem00071", 1)])
+def test_launch_shape_is_that_of_the_precision(sn, problem, copies):  # noqa: F811
+    """By colours: FP64 goes to a grid above 1,000 contacts a colour and takes two
+    threads a contact, FP32 has a cluster and one."""
+    from test_fc2d_oracle import load_fc2d, tiled2d
+    from test_gpu_fc2d_shapes import _one_sided
+    P = _one_sided(tiled2d(load_fc2d("fc2d_" + problem)[0], copies, 4), 0)
+    ctx = _ctx(sn, P)
+    fp64 = ctx.launch_shape()
+    ctx.set_precision(0)
+    fp32 = ctx.launch_shape()
+    ctx.close()
+    if copies > 1:
+        assert fp64[0] < 0 < fp32[0]
+    else:
+        assert fp64 == (1, 2 * fp32[1], 2) and fp32[0] == 1
