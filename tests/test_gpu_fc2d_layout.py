@@ -57,6 +57,7 @@ def test_pattern(sn, nc, rows, change):  # noqa: F811
     import oracle as O
     P = _hub(O, nc, rows, change)
     ctx = _ctx(sn, P)
+    ctx.set_precision(0)  # by colours FP32 sweeps of so few contacts have a cluster
     assert (ctx.launch_shape()[0] < 0) == (change == "none")  # a grid: dataflow
     _check(sn, ctx, P)
     ctx.close()
