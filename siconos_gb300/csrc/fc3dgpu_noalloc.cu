@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(3 * CH) k_error_noalloc(int nc, long long nnz,
           for (int k = 0; k < U; k++)
 #pragma unroll
             for (int e = 0; e < 3; e++) {
-              wv[k][e] = j[k] >= 0 ? __ldg(&blocks[9 * (b + k) + 3 * e + comp]) : 0.0;
-              rv[k][e] = j[k] >= 0 ? __ldg(&r[3 * j[k] + e]) : 0.0;
+              wv[k][e] = b + k < b1 ? __ldg(&blocks[9 * (b + k) + 3 * e + comp]) : 0.0;
+              rv[k][e] = b + k < b1 ? __ldg(&r[3 * (j[k] < 0 ? 0 : j[k]) + e]) : 0.0;
             }
 #pragma unroll
           for (int k = 0; k < U; k++)
