@@ -675,7 +675,9 @@ static cudaError_t ensure(T** p, size_t* cap, size_t n) {
 // down to m rounds, with the smallest m for which the blocks suffice.  With
 // more problems than blocks no m does; then the problems above 1.25 times the
 // mean load of a block are split down to that and the others stay one block
-// each in the queue.  slabs: slabs of a colour per problem, decreasing.
+// each in the queue.  slabs: slabs of a colour per problem, decreasing (from
+// the contacts, as if every problem had six colours, the sphere lattices' number:
+// only the problems' proportions and the rounding to rounds depend on it).
 struct BatchPlan {
   int grid = 0, team_scenes = 0;
   std::vector<int4> teams;  // one entry per block, empty without teams
@@ -1796,9 +1798,9 @@ static size_t staging_sizes(fc3dgpu_ctx* c, int grid, unsigned* wb, unsigned* cb
 
 // c->symmetric of the current layout: every block has its transpose's place
 // in W (the stamped dataflow sweeps need it).  A row's search goes through its
-// neighbours' slabs, so its time goes with the square of the longest row: from
-// 64 blocks on (rows of a few hundred took milliseconds) the pattern counts as
-// not symmetric and the sweeps go by colours.
+// neighbours' slabs, so its time goes with the square of the longest row: with
+// more than 64 blocks in one (rows of a few hundred took milliseconds) the
+// pattern counts as not symmetric and the sweeps go by colours.
 static int look_symmetric(fc3dgpu_ctx* c) {
   if (c->symmetric >= 0) return 0;
   for (int t = 0; t < c->nslab; t++)
@@ -1859,7 +1861,8 @@ static int prepare_batch_flow(fc3dgpu_ctx* c, int* resident) {
 // with 8, 10 and 12 warps, the choice last: 57,800 contacts 30.5, 36.6, 31.4
 // (12); 68,688 30.3, 33.1, 37.8 (8); 96,780 35.2, 31.2, 32.2 (10); 109,368 32.9,
 // 35.4, 32.1 (12); 164,400 36.0, 38.0, 36.0 (12); 216,346 36.4, 38.9, 39.7 (10);
-// 260,288 42.5, 41.3, 42.6 (10).  Up to a slab a warp, 10.
+// 260,288 42.5, 41.3, 42.6 (10).  Of these the model misses the best by 7 % at
+// 216,346 contacts and by 3 % at 57,800.  Up to a slab a warp, 10.
 static int default_flow_warps(const fc3dgpu_ctx* c) {
   if (c->flow_want > 0 || c->symmetric != 1 || c->nslab <= 10LL * c->nsm) return c->flow_want;
   auto cost = [&](int nw) {

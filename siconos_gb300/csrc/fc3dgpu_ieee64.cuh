@@ -45,7 +45,9 @@ __device__ __forceinline__ double ie_double(uint64_t x) { return __longlong_as_d
 #define IE_SLOW static __device__ __noinline__
 #else
 // host versions, for the tests: the seeds with a settable error in units of
-// the last place, since the device's approximations are not exact
+// the last place, since the device's approximations are not exact (at most 1
+// unit for the reciprocal, 2^-22.9 or 2.1 units for the reciprocal root; the
+// results are right up to 3)
 #include <math.h>
 #include <string.h>
 static int ie_host_seed_ulps = 0;
