@@ -38,10 +38,13 @@ extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 namespace fc3dgpu {
 namespace noalloc {
 
-// Contacts per chunk: 64, or 256 where 64 would make more chunks than the
-// last block sums quickly (and than the scratch holds).
+// Contacts per chunk: 64, which spreads few contacts over the SMs, or 256 where 64
+// would make more chunks than the last block sums quickly (and, beyond 2^20
+// contacts, than the scratch holds).  us a call with 64 and 256: 480 contacts 12.4
+// and 24.6, 40,935 24.6 and 39.0, 94,400 43.1 and 53.3, 320,400 151.6 and 149.6,
+// 509,600 238 and 222, 968,352 444 and 390.
 constexpr int SMALL_CHUNK = 64, LARGE_CHUNK = 256;
-constexpr int SMALL_MAX = 1 << 19;  // contacts
+constexpr int SMALL_MAX = 1 << 18;  // contacts
 static int chunk_of(int nc) { return nc <= SMALL_MAX ? SMALL_CHUNK : LARGE_CHUNK; }
 constexpr int MAX_CHUNKS = FC3DGPU_NOALLOC_MAX_CONTACTS / LARGE_CHUNK;
 static_assert(MAX_CHUNKS * LARGE_CHUNK == FC3DGPU_NOALLOC_MAX_CONTACTS, "limit must be a multiple of the chunk");
