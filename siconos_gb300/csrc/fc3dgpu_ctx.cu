@@ -16,6 +16,7 @@
 
 #include "fc3dgpu_batch_args.cuh"
 #include "fc3dgpu_sweep_launch.h"
+#include "fc3dgpu_copy.h"
 #include "fc3dgpu_fast64.h"
 #include "fc3dgpu_layout.cuh"
 #include "fc3dgpu_local64.cuh"
@@ -2455,9 +2456,14 @@ extern "C" int fc3dgpu_colour(int nc, const int64_t* rowptr, const int64_t* coli
     rc = NUMERICS_ERR_MEMORY;
   }
   if (!rc) {
-    cudaMemcpy(c->rowptr, rowptr, sizeof(long long) * (nc + 1), cudaMemcpyHostToDevice);
-    cudaMemcpy(c->colidx, colidx, sizeof(long long) * nnzb, cudaMemcpyHostToDevice);
-    rc = colour_device(c, nc, nnzb, kind);
+    cudaError_t e = copy_to_device(c->rowptr, rowptr, sizeof(long long) * (nc + 1), c->stream);
+    if (e == cudaSuccess) e = copy_to_device(c->colidx, colidx, sizeof(long long) * nnzb, c->stream);
+    if (e == cudaSuccess) {
+      rc = colour_device(c, nc, nnzb, kind);
+    } else {
+      fc3dgpu_set_error("fc3dgpu_colour: %s", cudaGetErrorString(e));
+      rc = NUMERICS_ERR_UNKNOWN;
+    }
     if (rc >= 0 && cudaMemcpy(colour, c->colour, sizeof(int) * nc, cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = NUMERICS_ERR_UNKNOWN;
   }
