@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "fc2dgpu.h"
+#include "fc3dgpu_copy.h"
 #include "fc3dgpu_ieee64.cuh"
 #include "fc3dgpu_word128.cuh"
 
@@ -1537,11 +1538,11 @@ extern "C" int fc2dgpu_ctx_set_q_mu(fc2dgpu_ctx* c, const double* q, const doubl
     mup[p] = mu[i];
   }
   K2(cudaSetDevice(c->device));
-  K2(cudaMemcpy(c->q, qp.data(), sizeof(double) * qp.size(), cudaMemcpyHostToDevice));
-  K2(cudaMemcpy(c->mu, mup.data(), sizeof(double) * mup.size(), cudaMemcpyHostToDevice));
+  K2(copy_to_device(c->q, qp.data(), sizeof(double) * qp.size(), c->stream));
+  K2(copy_to_device(c->mu, mup.data(), sizeof(double) * mup.size(), c->stream));
   const std::vector<float> q32(qp.begin(), qp.end()), mu32(mup.begin(), mup.end());
-  K2(cudaMemcpy(c->q32, q32.data(), sizeof(float) * q32.size(), cudaMemcpyHostToDevice));
-  K2(cudaMemcpy(c->mu32, mu32.data(), sizeof(float) * mu32.size(), cudaMemcpyHostToDevice));
+  K2(copy_to_device(c->q32, q32.data(), sizeof(float) * q32.size(), c->stream));
+  K2(copy_to_device(c->mu32, mu32.data(), sizeof(float) * mu32.size(), c->stream));
   c->norm_q = sqrt(s2);
   return 0;
 }
@@ -1554,7 +1555,7 @@ extern "C" int fc2dgpu_ctx_set_r(fc2dgpu_ctx* c, const double* r) {
     rp[2 * (size_t)c->iperm[i] + 1] = r[2 * i + 1];
   }
   K2(cudaSetDevice(c->device));
-  K2(cudaMemcpy(c->r, rp.data(), sizeof(double) * rp.size(), cudaMemcpyHostToDevice));
+  K2(copy_to_device(c->r, rp.data(), sizeof(double) * rp.size(), c->stream));
   return 0;
 }
 
@@ -1923,7 +1924,7 @@ extern "C" int fc2dgpu_ctx_solve(fc2dgpu_ctx* c, double tol, int max_iter, int e
   K2(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
   K2(cudaStreamSynchronize(c->stream));
   if (out[8] != 0.0) {
-    K2(cudaMemset(c->out, 0, sizeof(double) * 9));
+    K2(cudaMemsetAsync(c->out, 0, sizeof(double) * 9, c->stream));
     fc3dgpu_set_error("fc2dgpu_ctx_solve: a wait reached its poll limit");
     return NUMERICS_ERR_UNKNOWN;
   }
