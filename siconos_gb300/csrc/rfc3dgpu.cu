@@ -24,6 +24,7 @@
 
 #include "rfc3dgpu.h"
 #include "rfc3dgpu_coop.cuh"
+#include "fc3dgpu_copy.h"
 #include "fc3dgpu_word128.cuh"
 
 extern "C" void fc3dgpu_set_error(const char* fmt, ...);
@@ -1103,11 +1104,9 @@ extern "C" rfc3dgpu_ctx* rfc3dgpu_ctx_create(int device) {
 }
 
 template <typename T>
-static cudaError_t upload(T** d, const std::vector<T>& h) {
-  cudaError_t e = cudaMalloc((void**)d, sizeof(T) * (h.empty() ? 1 : h.size()));
-  if (e != cudaSuccess) return e;
-  if (!h.empty()) e = cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice);
-  return e;
+static cudaError_t upload(const rfc3dgpu_ctx* c, T** d, const std::vector<T>& h) {
+  const cudaError_t e = cudaMalloc((void**)d, sizeof(T) * (h.empty() ? 1 : h.size()));
+  return e == cudaSuccess ? copy_to_device(*d, h.data(), sizeof(T) * h.size(), c->stream) : e;
 }
 
 extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* rowptr, const int64_t* colidx,
@@ -1204,26 +1203,26 @@ extern "C" int rfc3dgpu_ctx_set_problem(rfc3dgpu_ctx* c, int nc, const int64_t* 
   c->norm_q = sqrt(s2);
   std::vector<double> zero(5 * (size_t)nc, 0.0);
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = upload(&c->cptr, cptr);
-  if (e == cudaSuccess) e = upload(&c->rp, rp);
-  if (e == cudaSuccess) e = upload(&c->col, col);
-  if (e == cudaSuccess) e = upload(&c->dpos, dpos);
-  if (e == cudaSuccess) e = upload(&c->W, W);
-  if (e == cudaSuccess) e = upload(&c->q, qp);
-  if (e == cudaSuccess) e = upload(&c->mu, mup);
-  if (e == cudaSuccess) e = upload(&c->mur, murp);
-  if (e == cudaSuccess) e = upload(&c->rho, rhop);
-  if (e == cudaSuccess) e = upload(&c->r, zero);
+  if (e == cudaSuccess) e = upload(c, &c->cptr, cptr);
+  if (e == cudaSuccess) e = upload(c, &c->rp, rp);
+  if (e == cudaSuccess) e = upload(c, &c->col, col);
+  if (e == cudaSuccess) e = upload(c, &c->dpos, dpos);
+  if (e == cudaSuccess) e = upload(c, &c->W, W);
+  if (e == cudaSuccess) e = upload(c, &c->q, qp);
+  if (e == cudaSuccess) e = upload(c, &c->mu, mup);
+  if (e == cudaSuccess) e = upload(c, &c->mur, murp);
+  if (e == cudaSuccess) e = upload(c, &c->rho, rhop);
+  if (e == cudaSuccess) e = upload(c, &c->r, zero);
   if (e == cudaSuccess && symmetric) e = cudaMalloc((void**)&c->rs, sizeof(double) * 10 * (size_t)nc);
-  if (e == cudaSuccess) e = upload(&c->u, zero);
+  if (e == cudaSuccess) e = upload(c, &c->u, zero);
   {
     auto f32 = [](const std::vector<double>& v) { return std::vector<float>(v.begin(), v.end()); };
-    if (e == cudaSuccess) e = upload(&c->W32, f32(W));
-    if (e == cudaSuccess) e = upload(&c->q32, f32(qp));
-    if (e == cudaSuccess) e = upload(&c->mu32, f32(mup));
-    if (e == cudaSuccess) e = upload(&c->mur32, f32(murp));
-    if (e == cudaSuccess) e = upload(&c->rho32, f32(rhop));
-    if (e == cudaSuccess) e = upload(&c->r32, f32(zero));
+    if (e == cudaSuccess) e = upload(c, &c->W32, f32(W));
+    if (e == cudaSuccess) e = upload(c, &c->q32, f32(qp));
+    if (e == cudaSuccess) e = upload(c, &c->mu32, f32(mup));
+    if (e == cudaSuccess) e = upload(c, &c->mur32, f32(murp));
+    if (e == cudaSuccess) e = upload(c, &c->rho32, f32(rhop));
+    if (e == cudaSuccess) e = upload(c, &c->r32, f32(zero));
     if (e == cudaSuccess && symmetric) e = cudaMalloc((void**)&c->rs32, sizeof(float) * 8 * (size_t)nc);
   }
   if (e != cudaSuccess) {
@@ -1278,7 +1277,7 @@ extern "C" int rfc3dgpu_ctx_set_r(rfc3dgpu_ctx* c, const double* r) {
   for (int i = 0; i < c->nc; i++)
     for (int a = 0; a < 5; a++) rp[5 * (size_t)c->iperm[i] + a] = r[5 * (size_t)i + a];
   KR(cudaSetDevice(c->device));
-  KR(cudaMemcpy(c->r, rp.data(), sizeof(double) * rp.size(), cudaMemcpyHostToDevice));
+  KR(copy_to_device(c->r, rp.data(), sizeof(double) * rp.size(), c->stream));
   return 0;
 }
 
