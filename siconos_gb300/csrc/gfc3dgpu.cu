@@ -51,6 +51,7 @@
 #include <numeric>
 #include <vector>
 
+#include "fc3dgpu_copy.h"
 #include "fc3dgpu_local64.cuh"
 #include "fc3dgpu_sweep.cuh"
 #include "gfc3dgpu.h"
@@ -685,11 +686,9 @@ extern "C" gfc3dgpu_ctx* gfc3dgpu_ctx_create(int device) {
 }
 
 template <typename T>
-static cudaError_t put(T** d, const std::vector<T>& h) {
-  cudaError_t e = cudaMalloc((void**)d, sizeof(T) * std::max<size_t>(h.size(), 1));
-  if (e != cudaSuccess) return e;
-  if (h.empty()) return cudaSuccess;
-  return cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice);
+static cudaError_t put(const gfc3dgpu_ctx* c, T** d, const std::vector<T>& h) {
+  const cudaError_t e = cudaMalloc((void**)d, sizeof(T) * std::max<size_t>(h.size(), 1));
+  return e == cudaSuccess ? copy_to_device(*d, h.data(), sizeof(T) * h.size(), c->stream) : e;
 }
 
 // Rows of a CSR matrix as 32-row slot-major slabs; padding gets value 0 and
@@ -891,49 +890,49 @@ extern "C" int gfc3dgpu_ctx_set_problem(gfc3dgpu_ctx* c, int64_t n, int nc, cons
   auto ok = [&](cudaError_t x) {
     if (e == cudaSuccess) e = x;
   };
-  ok(put(&c->hoff, hoff));
-  ok(put(&c->hns, hns));
-  ok(put(&c->hcol, hcol));
-  ok(put(&c->hval, hval));
-  ok(put(&c->moff, moff));
-  ok(put(&c->mns, mns));
-  ok(put(&c->mcol, mcol));
-  ok(put(&c->mval, mval));
-  ok(put(&c->toff, toff));
-  ok(put(&c->tns, tns));
-  ok(put(&c->tcol, tcol));
-  ok(put(&c->tval, tval));
-  ok(put(&c->q, qv));
-  ok(put(&c->b, bv));
-  ok(put(&c->mu, muv));
+  ok(put(c, &c->hoff, hoff));
+  ok(put(c, &c->hns, hns));
+  ok(put(c, &c->hcol, hcol));
+  ok(put(c, &c->hval, hval));
+  ok(put(c, &c->moff, moff));
+  ok(put(c, &c->mns, mns));
+  ok(put(c, &c->mcol, mcol));
+  ok(put(c, &c->mval, mval));
+  ok(put(c, &c->toff, toff));
+  ok(put(c, &c->tns, tns));
+  ok(put(c, &c->tcol, tcol));
+  ok(put(c, &c->tval, tval));
+  ok(put(c, &c->q, qv));
+  ok(put(c, &c->b, bv));
+  ok(put(c, &c->mu, muv));
   // both buffers of r and of u in one allocation each (an allocation and copy
   // takes 10 us)
   const long long pitch = (m + 1 + 31) / 32 * 32;
   const std::vector<double> zero_pair(2 * pitch, 0.0);
-  ok(put(&c->r[0], zero_pair));
-  ok(put(&c->u[0], zero_pair));
+  ok(put(c, &c->r[0], zero_pair));
+  ok(put(c, &c->u[0], zero_pair));
   c->r[1] = c->r[0] + pitch;
   c->u[1] = c->u[0] + pitch;
-  for (int k = 0; k < 2; k++) ok(put(&c->v[k], zero_v));
-  ok(put(&c->t, std::vector<double>(n, 0.0)));
+  for (int k = 0; k < 2; k++) ok(put(c, &c->v[k], zero_v));
+  ok(put(c, &c->t, std::vector<double>(n, 0.0)));
   int singular = 0;
   if (diag) {
-    ok(put(&c->mdiag, mdiag));
+    ok(put(c, &c->mdiag, mdiag));
     for (long long i = 0; i < n; i++)
       if (mdiag[i] == 0.0) singular = 1;
   } else {
-    ok(put(&c->cptr, cptr));
-    ok(put(&c->cdof, cdof));
-    ok(put(&c->luoff, luoff));
-    ok(put(&c->piv, std::vector<int>(n, 0)));
-    ok(put(&c->lu, std::vector<double>(luoff[ncomp], 0.0)));
-    ok(put(&d_mp, mp64));
-    ok(put(&d_mi, mi32));
-    ok(put(&d_mx, mx64));
-    ok(put(&d_comp, comp_of));
-    ok(put(&d_local, local));
+    ok(put(c, &c->cptr, cptr));
+    ok(put(c, &c->cdof, cdof));
+    ok(put(c, &c->luoff, luoff));
+    ok(put(c, &c->piv, std::vector<int>(n, 0)));
+    ok(put(c, &c->lu, std::vector<double>(luoff[ncomp], 0.0)));
+    ok(put(c, &d_mp, mp64));
+    ok(put(c, &d_mi, mi32));
+    ok(put(c, &d_mx, mx64));
+    ok(put(c, &d_comp, comp_of));
+    ok(put(c, &d_local, local));
     if (e == cudaSuccess) {
-      ok(cudaMemset(c->status, 0, sizeof(int)));
+      ok(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
       k_scatter_m<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, d_mp, d_mi, d_mx, d_comp, d_local,
                                                                        c->cptr, c->luoff, c->lu);
       ok(cudaGetLastError());
@@ -988,15 +987,16 @@ extern "C" int gfc3dgpu_ctx_set_start(gfc3dgpu_ctx* c, const double* r, const do
   const long long m = 3LL * c->nc;
   if (m > 0) {
     if (r)
-      G2(cudaMemcpy(c->r[0], r, sizeof(double) * m, cudaMemcpyHostToDevice));
+      G2(copy_to_device(c->r[0], r, sizeof(double) * m, c->stream));
     else
-      G2(cudaMemset(c->r[0], 0, sizeof(double) * m));
+      G2(cudaMemsetAsync(c->r[0], 0, sizeof(double) * m, c->stream));
   }
   c->cur = 0;
   if (v)
-    G2(cudaMemcpy(c->v[0], v, sizeof(double) * c->n, cudaMemcpyHostToDevice));
+    G2(copy_to_device(c->v[0], v, sizeof(double) * c->n, c->stream));
   else
-    G2(cudaMemset(c->v[0], 0, sizeof(double) * c->n));
+    G2(cudaMemsetAsync(c->v[0], 0, sizeof(double) * c->n, c->stream));
+  G2(cudaStreamSynchronize(c->stream));
   return 0;
 }
 
