@@ -14,6 +14,7 @@
 
 #include "fc2dgpu_percolour.h"
 #include "fc3dgpu.h"
+#include "fc3dgpu_copy.h"
 
 extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 
@@ -149,10 +150,9 @@ extern "C" void fc2dgpu_percolour_destroy(fc2dgpu_percolour* h) {
 }
 
 template <typename T>
-static cudaError_t put(T** d, const std::vector<T>& v) {
-  cudaError_t e = cudaMalloc((void**)d, sizeof(T) * std::max<size_t>(v.size(), 1));
-  if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
-  return e;
+static cudaError_t put(const fc2dgpu_percolour* h, T** d, const std::vector<T>& v) {
+  const cudaError_t e = cudaMalloc((void**)d, sizeof(T) * std::max<size_t>(v.size(), 1));
+  return e == cudaSuccess ? copy_to_device(*d, v.data(), sizeof(T) * v.size(), h->stream) : e;
 }
 
 // The local-solve kernel of colour range [lo, hi): this file's, or the loaded
@@ -257,16 +257,16 @@ static int setup(fc2dgpu_percolour* h, int colour_kind) {
     mup[p] = h->mu[i];
   }
   KP(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-  KP(put(&h->d_ci, ci));
-  KP(put(&h->d_val, val));
-  KP(put(&h->d_Wd, Wd));
-  KP(put(&h->d_det, det));
-  KP(put(&h->d_q, qp));
-  KP(put(&h->d_mu, mup));
+  KP(put(h, &h->d_ci, ci));
+  KP(put(h, &h->d_val, val));
+  KP(put(h, &h->d_Wd, Wd));
+  KP(put(h, &h->d_det, det));
+  KP(put(h, &h->d_q, qp));
+  KP(put(h, &h->d_mu, mup));
   KP(cudaMalloc(&h->d_z, sizeof(double) * 2 * nc));
   KP(cudaMalloc(&h->d_y, sizeof(double) * 2 * nc));
   KP(cudaMalloc(&h->d_sum, sizeof(double) * 2));
-  KP(cudaMemset(h->d_z, 0, sizeof(double) * 2 * nc));
+  KP(cudaMemsetAsync(h->d_z, 0, sizeof(double) * 2 * nc, h->stream));
   SP(cusparseCreate(&h->sp));
   SP(cusparseSetStream(h->sp, h->stream));
   SP(cusparseCreateDnVec(&h->zvec, 2 * (int64_t)nc, h->d_z, CUDA_R_64F));
@@ -283,7 +283,7 @@ static int setup(fc2dgpu_percolour* h, int colour_kind) {
     std::vector<int64_t> rpc(2 * (size_t)n + 1);
     for (size_t k = 0; k <= 2 * (size_t)n; k++) rpc[k] = rp[2 * (size_t)lo + k] - first;
     int64_t* d_rpc = nullptr;
-    KP(put(&d_rpc, rpc));
+    KP(put(h, &d_rpc, rpc));
     h->bufs.push_back(d_rpc);
     SP(cusparseCreateCsr(&h->mats[c], 2 * (int64_t)n, 2 * (int64_t)nc, last - first, d_rpc, h->d_ci + first,
                          h->d_val + first, CUSPARSE_INDEX_64I, CUSPARSE_INDEX_64I, CUSPARSE_INDEX_BASE_ZERO,
@@ -441,9 +441,9 @@ extern "C" int fc2dgpu_percolour_use_bsr(fc2dgpu_percolour* h, int on) {
       rp.push_back((int)ci.size() - base);
     }
     h->bsr_cnnz[h->ncol] = (int)ci.size();
-    KP(put(&h->d_brp, rp));
-    KP(put(&h->d_bci, ci));
-    KP(put(&h->d_bval, val));
+    KP(put(h, &h->d_brp, rp));
+    KP(put(h, &h->d_bci, ci));
+    KP(put(h, &h->d_bval, val));
     SP(cusparseCreateMatDescr(&h->descr));
     SP(cusparseSetMatIndexBase(h->descr, CUSPARSE_INDEX_BASE_ZERO));
     SP(cusparseSetMatType(h->descr, CUSPARSE_MATRIX_TYPE_GENERAL));
@@ -462,7 +462,7 @@ extern "C" int fc2dgpu_percolour_solve(fc2dgpu_percolour* h, const double* r0, d
       zp[2 * (size_t)h->iperm[i]] = r0[2 * i];
       zp[2 * (size_t)h->iperm[i] + 1] = r0[2 * i + 1];
     }
-  KP(cudaMemcpy(h->d_z, zp.data(), sizeof(double) * zp.size(), cudaMemcpyHostToDevice));
+  KP(copy_to_device(h->d_z, zp.data(), sizeof(double) * zp.size(), h->stream));
   const auto t0 = std::chrono::steady_clock::now();
   double tolerance = tol, err = INFINITY;
   int iter = 0, not_conv = 1;
