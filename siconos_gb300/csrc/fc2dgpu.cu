@@ -23,6 +23,7 @@
 
 #include "fc2dgpu.h"
 #include "fc3dgpu_copy.h"
+#include "fc3dgpu_grid_count.cuh"
 #include "fc3dgpu_ieee64.cuh"
 #include "fc3dgpu_word128.cuh"
 
@@ -38,7 +39,6 @@ constexpr int MAXC = 128;
 constexpr int TRACE_CAP = 1 << 16;
 constexpr size_t REP_MAX_BYTES = 208 * 1024;  // shared-memory copy of the reactions at most
 constexpr int GRID_MAX = 1024;                 // blocks of a cooperative grid at most
-constexpr int FLAG_STRIDE = 8;                 // words between the dataflow blocks' barrier flags
 constexpr unsigned long long SPIN = 1ull << 22;  // polls of a dataflow wait where no limit is set
 
 template <typename T>
@@ -87,10 +87,10 @@ struct Args {
   const double* before;   // out[] of the phase run before this one (or null)
   double* part;           // grid team: 2 x GRID_MAX x 4 block partial sums
   // dataflow: the reactions with the sweep that wrote them, contacts of a
-  // unit, the blocks' barrier flags, where a wait that gave up is told
+  // unit, the grid barrier's count, where a wait that gave up is told
   T* rs;
   int rows;
-  unsigned* flags;
+  unsigned* arrived;
   double* fail;
   unsigned long long spin;  // polls of a wait
   double* trace;
@@ -131,17 +131,17 @@ struct ClusterTeam {
 
 struct GridTeam {
   static constexpr bool grid = true, flow = false, alone = false;
-  cg::grid_group g;
+  unsigned* arrived;
+  double* fail;
+  unsigned long long spin;
+  fc3dgpu::GridCount g;
   template <typename T>
-  __device__ explicit GridTeam(const Args<T>&) : g(cg::this_grid()) {}
+  __device__ explicit GridTeam(const Args<T>& a) : arrived(a.arrived), fail(a.fail), spin(a.spin) {}
+  __device__ __forceinline__ bool dead() const { return g.dead; }
+  __device__ __forceinline__ void give_up() { g.give_up(*this); }
+  __device__ __forceinline__ void sync() { g.sync(*this); }
   __device__ __forceinline__ int rank() const { return (int)blockIdx.x; }
   __device__ __forceinline__ int size() const { return (int)gridDim.x; }
-  __device__ __forceinline__ void sync() {
-    if (gridDim.x == 1)
-      __syncthreads();
-    else
-      g.sync();
-  }
   __device__ __forceinline__ void sync_all() { sync(); }
   __device__ __forceinline__ void arrive() {}
   __device__ __forceinline__ void wait() { sync(); }
@@ -157,53 +157,11 @@ struct GridAlone : GridTeam {
   using GridTeam::GridTeam;
 };
 
-// A cooperative grid whose sweeps are dataflow: a barrier of flags (the sums
-// of a sweep pass one) whose waits, like those for reactions, end after `spin`
-// polls; `dead` (the same in the whole block) then ends the solve.
-struct FlowTeam {
-  static constexpr bool grid = true, flow = true, alone = false;
-  unsigned* flags;
-  double* fail;
-  unsigned long long spin;
-  unsigned epoch = 0;
-  bool dead = false;
-  template <typename T>
-  __device__ explicit FlowTeam(const Args<T>& a) : flags(a.flags), fail(a.fail), spin(a.spin) {}
-  __device__ __forceinline__ int rank() const { return (int)blockIdx.x; }
-  __device__ __forceinline__ int size() const { return (int)gridDim.x; }
-  __device__ __forceinline__ void give_up() {
-    *(volatile double*)fail = 1.0;
-    dead = true;
-  }
-  __device__ __forceinline__ void sync() {
-    epoch++;
-    bool ok = true;
-    __syncthreads();
-    if (threadIdx.x < 32 && !dead && gridDim.x > 1) {
-      const int lane = threadIdx.x;
-      if (lane == 0)
-        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&flags[blockIdx.x * FLAG_STRIDE]), "r"(epoch)
-                     : "memory");
-      for (unsigned long long n = 0;; n++) {
-        bool all = true;
-#pragma unroll 8
-        for (int b = lane; b < (int)gridDim.x; b += 32) {
-          unsigned f;
-          asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(f) : "l"(&flags[b * FLAG_STRIDE]) : "memory");
-          all &= f >= epoch;
-        }
-        if (__all_sync(0xffffffffu, all)) break;
-        if (n > spin) {
-          ok = false;
-          break;
-        }
-        if (n > 256) __nanosleep(32);
-      }
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    }
-    if (__syncthreads_or(!ok)) give_up();
-  }
-  __device__ __forceinline__ void sync_all() { sync(); }
+// A cooperative grid whose sweeps are dataflow: the sums of a sweep pass its one
+// barrier; the waits for reactions give up as the barrier's do.
+struct FlowTeam : GridTeam {
+  static constexpr bool flow = true;
+  using GridTeam::GridTeam;
 };
 
 // Where the sweep keeps the reactions.  HBM: read past L1 (ld.global.cg)
@@ -1048,8 +1006,8 @@ __global__ void __launch_bounds__(Team::flow ? 256 : NT_MAX, 1) k_fc2d_nsgs(cons
       flow_sum<2>(v, R, team, a.part);
     else
       team_sum<2>(v, R, team, a.part);
-    if constexpr (Team::flow)
-      if (team.dead) return;
+    if constexpr (Team::grid)
+      if (team.dead()) return;
     if constexpr (sizeof(T) == sizeof(double)) {
       const double nr = fc3dgpu::ie_sqrt(v[1]);
       err = fc3dgpu::ie_sqrt(v[0]);
@@ -1075,8 +1033,8 @@ __global__ void __launch_bounds__(Team::flow ? 256 : NT_MAX, 1) k_fc2d_nsgs(cons
       not_conv = 0;
       if constexpr (sizeof(T) == sizeof(double)) {
         const double full = full_error<REP>(a, rx, R, team);
-        if constexpr (Team::flow)
-          if (team.dead) return;
+        if constexpr (Team::grid)
+          if (team.dead()) return;
         if (full > a.tol) {
           tolerance = err / full * a.tol;
           not_conv = 1;
@@ -1094,8 +1052,8 @@ __global__ void __launch_bounds__(Team::flow ? 256 : NT_MAX, 1) k_fc2d_nsgs(cons
       not_conv = 1;
     }
   }
-  if constexpr (Team::flow)
-    if (team.dead) return;
+  if constexpr (Team::grid)
+    if (team.dead()) return;
   if (lead) {
     a.out[0] = done + iter;
     a.out[1] = final_err;
@@ -1189,7 +1147,7 @@ struct fc2dgpu_ctx : Uploaded {
   double* rs = nullptr;  // stamped reactions of the dataflow, of either precision (a symmetric block pattern)
   void* work = nullptr;  // holds the next four
   double *trace = nullptr, *out = nullptr, *part = nullptr;
-  unsigned* flags = nullptr;
+  unsigned* arrived = nullptr;
   unsigned long long spin = SPIN;
   int precision = 1;          // 0 FP32 sweeps + FP64 polish, 1 FP64 sweeps only
   double switch_tol = 0.0;    // FP32 phase stops below this light error (0: max(tol, 1e-6))
@@ -1291,7 +1249,7 @@ extern "C" fc2dgpu_ctx* fc2dgpu_ctx_create(int device) {
     p.take(c->trace, TRACE_CAP);
     p.take(c->out, 9);
     p.take(c->part, 2 * GRID_MAX * 4);
-    p.take(c->flags, GRID_MAX * FLAG_STRIDE);
+    p.take(c->arrived, 1);
     return p.at;
   };
   bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
@@ -1781,7 +1739,7 @@ static Args<double> args64(const fc2dgpu_ctx* c) {
   a.out = c->out;
   a.part = c->part;
   a.rs = c->rs;
-  a.flags = c->flags;
+  a.arrived = c->arrived;
   a.fail = c->out + 8;
   a.spin = c->spin;
   return a;
@@ -1812,7 +1770,7 @@ static Args<float> args32(const fc2dgpu_ctx* c) {
   a.out = c->out + 4;
   a.part = c->part;
   a.rs = reinterpret_cast<float*>(c->rs);
-  a.flags = c->flags;
+  a.arrived = c->arrived;
   a.fail = c->out + 8;
   a.spin = c->spin;
   return a;
@@ -1836,6 +1794,13 @@ extern "C" int fc2dgpu_ctx_last_sweeps(fc2dgpu_ctx* c, int* sweeps32, int* sweep
   return 0;
 }
 
+// The error of a launch whose waits gave up.
+static int gave_up(fc2dgpu_ctx* c, const char* who) {
+  K2(cudaMemsetAsync(c->out, 0, sizeof(double) * 9, c->stream));
+  fc3dgpu_set_error("%s: a wait reached its poll limit", who);
+  return NUMERICS_ERR_UNKNOWN;
+}
+
 extern "C" int fc2dgpu_ctx_spin_limit(fc2dgpu_ctx* c, unsigned long long polls) {
   if (!c) return NUMERICS_ERR_INVALID_ARGUMENT;
   c->spin = polls ? polls : SPIN;
@@ -1851,11 +1816,15 @@ extern "C" int fc2dgpu_ctx_compute_error(fc2dgpu_ctx* c, double norm_q, double* 
   Args<double> a = args64(c);
   a.norm_q = norm_q;
   const Shape& s = c->s64;
+  if (s.grid) K2(cudaMemsetAsync(c->arrived, 0, sizeof(unsigned), c->stream));
   K2(s.grid  ? launch_grid(c, s, k_fc2d_error<false, GridTeam>, a)
      : s.rep ? launch(c, s, k_fc2d_error<true, ClusterTeam>, a, rep_bytes(c))
              : launch(c, s, k_fc2d_error<false, ClusterTeam>, a, 0));
-  K2(cudaMemcpyAsync(error, c->out + 1, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  double out[9];
+  K2(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
   K2(cudaStreamSynchronize(c->stream));
+  if (out[8] != 0.0) return gave_up(c, "fc2dgpu_ctx_compute_error");
+  *error = out[1];
   return 0;
 }
 
@@ -1900,7 +1869,7 @@ extern "C" int fc2dgpu_ctx_solve(fc2dgpu_ctx* c, double tol, int max_iter, int e
     b.stall = c->stall;
     const Shape& s = c->s32;
     b.rows = s.rows;
-    if (s.flow) K2(cudaMemsetAsync(c->flags, 0, sizeof(unsigned) * GRID_MAX * FLAG_STRIDE, c->stream));
+    if (s.grid) K2(cudaMemsetAsync(c->arrived, 0, sizeof(unsigned), c->stream));
     K2(s.flow  ? launch_grid(c, s, k_fc2d_nsgs<float, false, FlowTeam>, b)
        : s.grid ? launch_grid(c, s, k_fc2d_nsgs<float, false, GridTeam>, b)
        : s.rep ? launch(c, s, k_fc2d_nsgs<float, true, ClusterTeam>, b, sizeof(float2) * (size_t)c->nc)
@@ -1909,7 +1878,7 @@ extern "C" int fc2dgpu_ctx_solve(fc2dgpu_ctx* c, double tol, int max_iter, int e
   }
   const Shape& s = c->s64;
   a.rows = s.rows;
-  if (s.flow) K2(cudaMemsetAsync(c->flags, 0, sizeof(unsigned) * GRID_MAX * FLAG_STRIDE, c->stream));
+  if (s.grid) K2(cudaMemsetAsync(c->arrived, 0, sizeof(unsigned), c->stream));
   if (s.alone)
     K2(s.grid  ? launch_grid(c, s, k_fc2d_nsgs<double, false, GridAlone>, a)
        : s.rep ? launch(c, s, k_fc2d_nsgs<double, true, ClusterAlone>, a, rep_bytes(c))
@@ -1923,11 +1892,7 @@ extern "C" int fc2dgpu_ctx_solve(fc2dgpu_ctx* c, double tol, int max_iter, int e
   double out[9];
   K2(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
   K2(cudaStreamSynchronize(c->stream));
-  if (out[8] != 0.0) {
-    K2(cudaMemsetAsync(c->out, 0, sizeof(double) * 9, c->stream));
-    fc3dgpu_set_error("fc2dgpu_ctx_solve: a wait reached its poll limit");
-    return NUMERICS_ERR_UNKNOWN;
-  }
+  if (out[8] != 0.0) return gave_up(c, "fc2dgpu_ctx_solve");
   float t = 0.f;
   cudaEventElapsedTime(&t, c->ev[0], c->ev[1]);
   if (iters) *iters = (int)out[0];

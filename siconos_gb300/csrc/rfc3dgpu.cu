@@ -11,7 +11,6 @@
 // FP64 without FMA contraction, in the reference's operation order; in mixed
 // precision FP32 sweeps of the same loop run first and the FP64 loop starts
 // from their iterate.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
@@ -25,13 +24,13 @@
 #include "rfc3dgpu.h"
 #include "rfc3dgpu_coop.cuh"
 #include "fc3dgpu_copy.h"
+#include "fc3dgpu_grid_count.cuh"
 #include "fc3dgpu_word128.cuh"
 
 extern "C" void fc3dgpu_set_error(const char* fmt, ...);
 
 namespace rfc3dgpu {
 
-namespace cg = cooperative_groups;
 
 constexpr int NT = 128;
 constexpr int MAXC = 128;
@@ -59,7 +58,9 @@ struct ArgsT {
   int local_max, max_iter;
   double* part;   // 2 slots x MAX_BLOCKS x 4 block partial sums
   double* trace;  // per-sweep light error, from trace[0]
-  double* out;    // [0] sweeps, [1] final error, [2] info (-1: a wait gave up), [3] last light error
+  double* out;    // [0] sweeps, [1] final error, [2] info, [3] last light error
+  unsigned* arrived;  // the grid barrier's count, zero at the launch
+  double* fail;     // where a wait that gave up is told
   int trace_cap;  // entries of trace this launch may write
   // dataflow sweeps: the reactions with the sweep that wrote them (null: by
   // colours), contacts of a unit, polls of a wait
@@ -410,13 +411,6 @@ __device__ __forceinline__ void local_nsn(const Real* M, const Real* q, Real mu,
 
 // ---- grid-wide pieces ------------------------------------------------------
 
-__device__ __forceinline__ void grid_sync(cg::grid_group& g) {
-  if (gridDim.x == 1)
-    __syncthreads();
-  else
-    g.sync();
-}
-
 struct Reduce {
   double warp[NT / 32][4];
   double bcast[4];
@@ -430,7 +424,7 @@ struct Reduce {
 // after the barrier of call k - 1, which every block passes after reading
 // call k - 2's slot.  The barrier also orders all reaction updates before it.
 template <int N, typename A>
-__device__ void grid_sum(double v[N], const A& a, Reduce& R, cg::grid_group& g) {
+__device__ void grid_sum(double v[N], const A& a, Reduce& R, fc3dgpu::GridCount& g) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < N; i++) {
@@ -445,7 +439,7 @@ __device__ void grid_sum(double v[N], const A& a, Reduce& R, cg::grid_group& g) 
     for (int k = 0; k < (int)(blockDim.x >> 5); k++) s += R.warp[k][threadIdx.x];
     __stcg(&slot[4 * blockIdx.x + threadIdx.x], s);
   }
-  grid_sync(g);
+  g.sync(a);
   if (threadIdx.x < 32) {
     double s[N];
 #pragma unroll
@@ -471,7 +465,7 @@ __device__ void grid_sum(double v[N], const A& a, Reduce& R, cg::grid_group& g) 
 
 // rolling_friction_3d_compute_error (rolling_friction_3d_compute_error.c:
 // 58-110): u = 1.0 q + 1.0 (row sums of W r in column order)
-__device__ double full_error(const Args& a, Reduce& R, cg::grid_group& g) {
+__device__ double full_error(const Args& a, Reduce& R, fc3dgpu::GridCount& g) {
   double v[3] = {0.0, 0.0, 0.0};
   const int g0 = blockIdx.x * blockDim.x + threadIdx.x, G = gridDim.x * blockDim.x;
   for (int p = g0; p < a.nc; p += G) {
@@ -544,7 +538,7 @@ __device__ __forceinline__ void local_contact(const ArgsT<Real>& a, int p, const
 // sum |r_new|^2 (in the precision of the sweep, summed in FP64).
 template <typename Real>
 __device__ __forceinline__ void sweep_colours(const ArgsT<Real>& a, Real local_tol, double v[2],
-                                              cg::grid_group& g) {
+                                              fc3dgpu::GridCount& g) {
   const int g0 = blockIdx.x * blockDim.x + threadIdx.x, G = gridDim.x * blockDim.x;
   for (int c = 0; c < a.ncol; c++) {
     for (int p = a.cptr[c] + g0; p < a.cptr[c + 1]; p += G) {
@@ -562,14 +556,14 @@ __device__ __forceinline__ void sweep_colours(const ArgsT<Real>& a, Real local_t
       Real rl[5];
       local_contact<Real>(a, p, s, local_tol, v, rl);
     }
-    if (c + 1 < a.ncol) grid_sync(g);
+    if (c + 1 < a.ncol) g.sync(a);
   }
 }
 
 // sweep_colours in FP64, five lanes a contact and six contacts a warp
 // (rfc3dgpu_coop.cuh).
 __device__ __forceinline__ void sweep_colours_coop(const Args& a, double local_tol, double v[2],
-                                                   cg::grid_group& g) {
+                                                   fc3dgpu::GridCount& g) {
   const int lane = threadIdx.x & 31;
   const bool spare = lane >= 5 * RFC3D_COOP_GROUPS;
   RLane c;
@@ -622,7 +616,7 @@ __device__ __forceinline__ void sweep_colours_coop(const Args& a, double local_t
         }
       }
     }
-    if (col + 1 < a.ncol) grid_sync(g);
+    if (col + 1 < a.ncol) g.sync(a);
   }
 }
 
@@ -821,20 +815,20 @@ __device__ __forceinline__ void flow_sweep(const ArgsT<Real>& a, const Unit& uni
 
 // The start's reactions with sweep 0's stamp
 template <typename Real>
-__device__ __forceinline__ void flow_start(const ArgsT<Real>& a, cg::grid_group& g) {
+__device__ __forceinline__ void flow_start(const ArgsT<Real>& a, fc3dgpu::GridCount& g) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < a.nc; p += gridDim.x * blockDim.x) {
     Real x[5];
 #pragma unroll
     for (int i = 0; i < 5; i++) x[i] = __ldcg(&a.r[5 * (size_t)p + i]);
     st_all_stamped(a.rs, p, x, 0);
   }
-  grid_sync(g);
+  g.sync(a);
 }
 
 template <bool FLOW>
 __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
   __shared__ Reduce R;
-  cg::grid_group g = cg::this_grid();
+  fc3dgpu::GridCount g;
   if (threadIdx.x == 0) R.calls = 0;
   __syncthreads();
   const int g0 = blockIdx.x * blockDim.x + threadIdx.x, G = gridDim.x * blockDim.x;
@@ -850,14 +844,12 @@ __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
       flow_sweep(a, [&](int first, int n) { flow_unit(a, first, n, iter, local_tol, v, failed); });
       v[2] = failed ? 1.0 : 0.0;
       grid_sum<3>(v, a, R, g);
-      if (v[2] != 0.0) {
-        if (lead) a.out[2] = -1.0;
-        return;
-      }
+      if (v[2] != 0.0) g.give_up(a);
     } else {
       sweep_colours_coop(a, local_tol, v, g);
       grid_sum<2>(v, a, R, g);
     }
+    if (g.dead) return;
     err = sqrt(v[0]);
     const double nr = sqrt(v[1]);
     if (fabs(nr) > DBL_EPSILON) err /= nr;
@@ -867,6 +859,7 @@ __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
     if (err < tolerance) {
       not_conv = 0;
       const double full = full_error(a, R, g);
+      if (g.dead) return;
       if (full > a.tol) {
         if (err < DBL_EPSILON)
           local_tol = fmax(local_tol / 100., DBL_EPSILON * 1e-6);
@@ -878,6 +871,7 @@ __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
   }
   const double light = err;
   err = full_error(a, R, g);
+  if (g.dead) return;
   not_conv = !(err < a.tol);
   if (lead) {
     a.out[0] = iter;
@@ -895,7 +889,7 @@ __global__ void __launch_bounds__(NT) k_rfc3d_nsgs(const Args a) {
 template <bool FLOW>
 __global__ void __launch_bounds__(NT) k_rfc3d_sweeps32(const ArgsT<float> a) {
   __shared__ Reduce R;
-  cg::grid_group g = cg::this_grid();
+  fc3dgpu::GridCount g;
   if (threadIdx.x == 0) R.calls = 0;
   __syncthreads();
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
@@ -911,14 +905,12 @@ __global__ void __launch_bounds__(NT) k_rfc3d_sweeps32(const ArgsT<float> a) {
       flow_sweep(a, [&](int first, int n) { flow_unit(a, first, n, iter, (float)a.local_tol, v, failed); });
       v[2] = failed ? 1.0 : 0.0;
       grid_sum<3>(v, a, R, g);
-      if (v[2] != 0.0) {
-        if (lead) a.out[2] = -1.0;
-        return;
-      }
+      if (v[2] != 0.0) g.give_up(a);
     } else {
       sweep_colours<float>(a, (float)a.local_tol, v, g);
       grid_sum<2>(v, a, R, g);
     }
+    if (g.dead) return;
     err = sqrt(v[0]);
     const double nr = sqrt(v[1]);
     if (fabs(nr) > DBL_EPSILON) err /= nr;
@@ -952,11 +944,11 @@ __global__ void k_rfc3d_to_f64(int n, const float* __restrict__ x, double* __res
 
 __global__ void __launch_bounds__(NT) k_rfc3d_error(const Args a) {
   __shared__ Reduce R;
-  cg::grid_group g = cg::this_grid();
+  fc3dgpu::GridCount g;
   if (threadIdx.x == 0) R.calls = 0;
   __syncthreads();
   const double e = full_error(a, R, g);
-  if (blockIdx.x == 0 && threadIdx.x == 0) a.out[1] = e;
+  if (!g.dead && blockIdx.x == 0 && threadIdx.x == 0) a.out[1] = e;
 }
 
 }  // namespace rfc3dgpu
@@ -1029,6 +1021,7 @@ struct rfc3dgpu_ctx {
   // 1: FP64 sweeps only (default); 0: FP32 sweeps, then the FP64 loop
   int precision = 1;
   unsigned long long spin = SPIN;
+  unsigned* arrived = nullptr;
   double switch_tol = 0.0;  // FP32 sweeps end below this light error (0: max(tol, 1e-6))
   int stall = 64;
   int sweeps32 = 0, sweeps64 = 0;
@@ -1062,7 +1055,7 @@ extern "C" void rfc3dgpu_ctx_destroy(rfc3dgpu_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   free_problem(c);
-  void* ptrs[] = {c->part, c->trace, c->out};
+  void* ptrs[] = {c->part, c->trace, c->out, c->arrived};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto& e : c->ev)
@@ -1094,7 +1087,9 @@ extern "C" rfc3dgpu_ctx* rfc3dgpu_ctx_create(int device) {
             cudaEventCreate(&c->ev[0]) == cudaSuccess && cudaEventCreate(&c->ev[1]) == cudaSuccess &&
             cudaMalloc(&c->part, sizeof(double) * 2 * MAX_BLOCKS * 4) == cudaSuccess &&
             cudaMalloc(&c->trace, sizeof(double) * TRACE_CAP) == cudaSuccess &&
-            cudaMalloc(&c->out, sizeof(double) * 8) == cudaSuccess;
+            cudaMalloc(&c->arrived, sizeof(unsigned)) == cudaSuccess &&
+            cudaMalloc(&c->out, sizeof(double) * 8) == cudaSuccess &&
+            cudaMemsetAsync(c->out, 0, sizeof(double) * 8, c->stream) == cudaSuccess;
   if (!ok) {
     fc3dgpu_set_error("rfc3dgpu_ctx_create: set-up failed (%s)", cudaGetErrorString(cudaGetLastError()));
     rfc3dgpu_ctx_destroy(c);
@@ -1299,6 +1294,8 @@ static Args args_of(const rfc3dgpu_ctx* c) {
   a.rs = c->rs;
   a.rows = c->rows;
   a.spin = c->spin;
+  a.arrived = c->arrived;
+  a.fail = c->out + 4;
   a.u = c->u;
   a.norm_q = c->norm_q;
   a.part = c->part;
@@ -1326,6 +1323,8 @@ static ArgsT<float> args32_of(const rfc3dgpu_ctx* c) {
   a.rs = c->rs32;
   a.rows = c->rows32;
   a.spin = c->spin;
+  a.arrived = c->arrived;
+  a.fail = c->out + 4;
   a.u = c->u;
   a.norm_q = c->norm_q;
   a.part = c->part;
@@ -1338,7 +1337,18 @@ static ArgsT<float> args32_of(const rfc3dgpu_ctx* c) {
 template <typename K, typename A>
 static cudaError_t launch(rfc3dgpu_ctx* c, K kernel, A& a, int blocks, int threads) {
   void* params[] = {&a};
+  if (blocks > 1) {
+    const cudaError_t e = cudaMemsetAsync(c->arrived, 0, sizeof(unsigned), c->stream);
+    if (e != cudaSuccess) return e;
+  }
   return cudaLaunchCooperativeKernel((const void*)kernel, dim3(blocks), dim3(threads), params, 0, c->stream);
+}
+
+// The error of a launch whose waits gave up.
+static int gave_up(rfc3dgpu_ctx* c, const char* who) {
+  KR(cudaMemsetAsync(c->out, 0, sizeof(double) * 8, c->stream));
+  fc3dgpu_set_error("%s: a wait reached its poll limit", who);
+  return NUMERICS_ERR_UNKNOWN;
 }
 
 extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, double local_tol, int local_max_iter,
@@ -1350,7 +1360,7 @@ extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, dou
   KR(cudaSetDevice(c->device));
   const int n5 = 5 * c->nc;
   KR(cudaEventRecord(c->ev[0], c->stream));
-  double out[4];
+  double out[5];
   int sweeps32 = 0;
   if (c->precision == 0 && max_iter > 0) {
     // FP32 sweeps from the current reaction, then the FP64 loop from theirs
@@ -1366,10 +1376,7 @@ extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, dou
                  : launch(c, k_rfc3d_sweeps32<false>, a, c->blocks32, c->threads32));
     KR(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
     KR(cudaStreamSynchronize(c->stream));
-    if (out[2] < 0.0) {
-      fc3dgpu_set_error("rfc3dgpu_ctx_solve: a wait for a reaction reached its poll limit");
-      return NUMERICS_ERR_UNKNOWN;
-    }
+    if (out[4] != 0.0) return gave_up(c, "rfc3dgpu_ctx_solve");
     sweeps32 = (int)out[0];
     // a non-finite FP32 iterate is dropped: the FP64 loop starts where the
     // FP32 sweeps did
@@ -1390,10 +1397,7 @@ extern "C" int rfc3dgpu_ctx_solve(rfc3dgpu_ctx* c, double tol, int max_iter, dou
   KR(cudaEventRecord(c->ev[1], c->stream));
   KR(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
   KR(cudaStreamSynchronize(c->stream));
-  if (out[2] < 0.0) {
-    fc3dgpu_set_error("rfc3dgpu_ctx_solve: a wait for a reaction reached its poll limit");
-    return NUMERICS_ERR_UNKNOWN;
-  }
+  if (out[4] != 0.0) return gave_up(c, "rfc3dgpu_ctx_solve");
   float t = 0.f;
   cudaEventElapsedTime(&t, c->ev[0], c->ev[1]);
   c->sweeps32 = sweeps32;
@@ -1436,8 +1440,11 @@ extern "C" int rfc3dgpu_ctx_compute_error(rfc3dgpu_ctx* c, double norm_q, double
   Args a = args_of(c);
   a.norm_q = norm_q;
   KR(launch(c, k_rfc3d_error, a, c->blocks, c->threads));
-  KR(cudaMemcpyAsync(error, c->out + 1, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  double out[5];
+  KR(cudaMemcpyAsync(out, c->out, sizeof(out), cudaMemcpyDeviceToHost, c->stream));
   KR(cudaStreamSynchronize(c->stream));
+  if (out[4] != 0.0) return gave_up(c, "rfc3dgpu_ctx_compute_error");
+  *error = out[1];
   return 0;
 }
 

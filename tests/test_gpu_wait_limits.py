@@ -95,3 +95,30 @@ def test_2d(built_lib, problem, copies, precision):
     ctx = _ctx(sn, P)
     ctx.set_precision(precision, 1e-30, 1 << 20)
     _context_recovers(ctx, 2 * P.nc, lambda: ctx.solve(1e-300, 8))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("dim", [2, 5])
+def test_grid_barriers(built_lib, dim, precision):
+    """By colours (a pattern that is not symmetric) on a grid: the barriers
+    between colours, and that of an error evaluation."""
+    import siconos_gb300.numerics as sn
+    if dim == 2:
+        from test_fc2d_oracle import load_fc2d, tiled2d
+        from test_gpu_fc2d import _ctx
+        from test_gpu_fc2d_shapes import _one_sided
+        T = _one_sided(tiled2d(load_fc2d("fc2d_fc2d_granularflowonwall_07002_00801")[0], 4, 4), 0)
+    else:
+        from test_gpu_rfc3d import _ctx
+        from test_gpu_rolling_lanes import _one_sided
+        from test_rfc3d_oracle import load_rfc3d, tiled
+        T = _one_sided(tiled(load_rfc3d("rfc3d_rockfall_21_54029")[0], 100, 7), 0)
+    ctx = _ctx(sn, T)
+    ctx.set_precision(precision, 1e-30, 1 << 20)
+    error = ctx.compute_error(1.0)
+    ctx.spin_limit(1)
+    with pytest.raises(RuntimeError, match="poll limit"):
+        ctx.compute_error(1.0)
+    ctx.spin_limit(0)
+    assert ctx.compute_error(1.0) == error
+    _context_recovers(ctx, dim * T.nc, lambda: ctx.solve(1e-300, 6))
