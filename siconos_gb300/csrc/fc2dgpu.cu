@@ -1909,8 +1909,8 @@ extern "C" int fc2dgpu_ctx_get_r_u(fc2dgpu_ctx* c, double* r, double* u) {
   if (!c || c->nc == 0) return NUMERICS_ERR_INVALID_ARGUMENT;
   K2(cudaSetDevice(c->device));
   std::vector<double> rp(2 * (size_t)c->nc), up(2 * (size_t)c->nc);
-  K2(cudaMemcpy(rp.data(), c->r, sizeof(double) * rp.size(), cudaMemcpyDeviceToHost));
-  K2(cudaMemcpy(up.data(), c->u, sizeof(double) * up.size(), cudaMemcpyDeviceToHost));
+  K2(copy_to_host(rp.data(), c->r, sizeof(double) * rp.size(), c->stream));
+  K2(copy_to_host(up.data(), c->u, sizeof(double) * up.size(), c->stream));
   for (int i = 0; i < c->nc; i++) {
     const size_t p = (size_t)c->iperm[i];
     if (r) {
@@ -1936,6 +1936,6 @@ extern "C" int fc2dgpu_ctx_trace(fc2dgpu_ctx* c, double* out, int cap) {
   const int n = std::min(cap, c->trace_len);
   if (n <= 0 || !out) return 0;
   K2(cudaSetDevice(c->device));
-  K2(cudaMemcpy(out, c->trace, sizeof(double) * n, cudaMemcpyDeviceToHost));
+  K2(copy_to_host(out, c->trace, sizeof(double) * n, c->stream));
   return n;
 }

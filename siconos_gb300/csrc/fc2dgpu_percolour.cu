@@ -386,7 +386,7 @@ static double host_full_error(fc2dgpu_percolour* h) {
 
 static int pull_z(fc2dgpu_percolour* h) {
   std::vector<double> zp(2 * (size_t)h->nc);
-  KP(cudaMemcpy(zp.data(), h->d_z, sizeof(double) * zp.size(), cudaMemcpyDeviceToHost));
+  KP(copy_to_host(zp.data(), h->d_z, sizeof(double) * zp.size(), h->stream));
   for (int i = 0; i < h->nc; i++) {
     h->z[2 * (size_t)i] = zp[2 * (size_t)h->iperm[i]];
     h->z[2 * (size_t)i + 1] = zp[2 * (size_t)h->iperm[i] + 1];

@@ -2464,7 +2464,7 @@ extern "C" int fc3dgpu_colour(int nc, const int64_t* rowptr, const int64_t* coli
       fc3dgpu_set_error("fc3dgpu_colour: %s", cudaGetErrorString(e));
       rc = NUMERICS_ERR_UNKNOWN;
     }
-    if (rc >= 0 && cudaMemcpy(colour, c->colour, sizeof(int) * nc, cudaMemcpyDeviceToHost) != cudaSuccess)
+    if (rc >= 0 && copy_to_host(colour, c->colour, sizeof(int) * nc, c->stream) != cudaSuccess)
       rc = NUMERICS_ERR_UNKNOWN;
   }
   fc3dgpu_ctx_destroy(c);

@@ -1122,9 +1122,9 @@ extern "C" int gfc3dgpu_ctx_get(gfc3dgpu_ctx* c, double* r, double* u, double* v
   }
   G2(cudaSetDevice(c->device));
   const long long m = 3LL * c->nc;
-  if (r && m) G2(cudaMemcpy(r, c->r[c->cur], sizeof(double) * m, cudaMemcpyDeviceToHost));
-  if (u && m) G2(cudaMemcpy(u, c->u[c->cur], sizeof(double) * m, cudaMemcpyDeviceToHost));
-  if (v) G2(cudaMemcpy(v, c->v[c->cur], sizeof(double) * c->n, cudaMemcpyDeviceToHost));
+  if (r && m) G2(copy_to_host(r, c->r[c->cur], sizeof(double) * m, c->stream));
+  if (u && m) G2(copy_to_host(u, c->u[c->cur], sizeof(double) * m, c->stream));
+  if (v) G2(copy_to_host(v, c->v[c->cur], sizeof(double) * c->n, c->stream));
   return 0;
 }
 
@@ -1133,7 +1133,7 @@ extern "C" int gfc3dgpu_ctx_trace(gfc3dgpu_ctx* c, double* out, int cap) {
   const int n = std::min(cap, c->trace_len);
   if (n <= 0 || !out) return 0;
   G2(cudaSetDevice(c->device));
-  G2(cudaMemcpy(out, c->trace, sizeof(double) * n, cudaMemcpyDeviceToHost));
+  G2(copy_to_host(out, c->trace, sizeof(double) * n, c->stream));
   return n;
 }
 

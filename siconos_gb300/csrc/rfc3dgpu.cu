@@ -1452,8 +1452,8 @@ extern "C" int rfc3dgpu_ctx_get_r_u(rfc3dgpu_ctx* c, double* r, double* u) {
   if (!c || c->nc == 0) return NUMERICS_ERR_INVALID_ARGUMENT;
   KR(cudaSetDevice(c->device));
   std::vector<double> rp(5 * (size_t)c->nc), up(5 * (size_t)c->nc);
-  KR(cudaMemcpy(rp.data(), c->r, sizeof(double) * rp.size(), cudaMemcpyDeviceToHost));
-  KR(cudaMemcpy(up.data(), c->u, sizeof(double) * up.size(), cudaMemcpyDeviceToHost));
+  KR(copy_to_host(rp.data(), c->r, sizeof(double) * rp.size(), c->stream));
+  KR(copy_to_host(up.data(), c->u, sizeof(double) * up.size(), c->stream));
   for (int i = 0; i < c->nc; i++)
     for (int a = 0; a < 5; a++) {
       const size_t p = 5 * (size_t)c->iperm[i] + a;
@@ -1480,6 +1480,6 @@ extern "C" int rfc3dgpu_ctx_trace(rfc3dgpu_ctx* c, double* out, int cap) {
   const int n = std::min(cap, c->trace_len);
   if (n <= 0 || !out) return 0;
   KR(cudaSetDevice(c->device));
-  KR(cudaMemcpy(out, c->trace, sizeof(double) * n, cudaMemcpyDeviceToHost));
+  KR(copy_to_host(out, c->trace, sizeof(double) * n, c->stream));
   return n;
 }
