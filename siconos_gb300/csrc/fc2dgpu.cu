@@ -733,9 +733,9 @@ __device__ __forceinline__ void sweep_alone(const Args<double>& a, Reactions<dou
 // old ones of higher colours; the pattern is symmetric, so a contact of a
 // higher colour cannot write its new one before this contact has written its
 // own, and a stamp at least the one needed is the one needed.  Granular
-// problems, us a sweep by colours and as dataflow: FP64 24.4 and 18.6 at 367
-// contacts, 34.7 and 26.2 at 7,002, 34.8 and 28.9 at 28,008, 63.2 and 35.1 at
-// 70,020; FP32 10.2 and 8.5, 14.1 and 11.9, 19.9 and 12.3, 22.3 and 13.0.
+// problems, us a sweep by colours and as dataflow: FP64 24.4 and 18.0 at 367
+// contacts, 32.0 and 24.7 at 7,002, 32.1 and 27.3 at 28,008, 60.7 and 33.6 at
+// 70,020; FP32 10.2 and 7.7, 14.4 and 9.9, 19.8 and 10.4, 21.5 and 11.2.
 // What is left is the chain of a colour's longest rows: with a warp a quarter
 // an instruction takes eight cycles and an FP64 one 64.
 
@@ -950,9 +950,9 @@ __device__ __forceinline__ void close_reactions(const Args<T>& a, const Reaction
 // contacts queued on the L1's tags) and loaded before the barrier that
 // releases the colour; the light-error terms are summed behind the barrier's
 // arrival; above 64 contacts a colour the sweeps go as dataflow (above).  By
-// colours, granular problems, us a sweep before and after: FP64 37.4 and 24.6
-// at 367 contacts, 49.2 and 34.9 at 7,002, 75.3 and 34.4 at 28,008; FP32 12.5
-// and 10.1, 16.5 and 14.2, 26.7 and 20.3.  The hardware cluster barrier
+// colours, granular problems, us a sweep before and after: FP64 37.0 and 24.4
+// at 367 contacts, 48.9 and 32.0 at 7,002, 74.7 and 32.1 at 28,008; FP32 12.0
+// and 10.2, 16.2 and 14.4, 25.8 and 19.8.  The hardware cluster barrier
 // (release / acquire) separates colours, the barrier of the error reduction
 // closing the last one, and the convergence logic runs on the device with the
 // same bits in every block.
@@ -1166,9 +1166,9 @@ struct fc2dgpu_ctx : Uploaded {
   } while (0)
 
 // Dataflow above this many contacts in the largest colour, where one block no
-// longer holds it at a contact a thread: with 41 contacts a sweep takes 8.3 us
-// in one block and 9.2 as dataflow in FP64 (6.3 and 7.5 mixed), with 131 on a
-// cluster 24.4 and 18.6 (FP32 10.2 and 8.5).
+// longer holds it at a contact a thread: with 41 contacts a sweep takes 12.6 us
+// in one block and 13.5 as dataflow in FP64 (11.5 and 12.5 mixed), with 131 on a
+// cluster 24.4 and 18.0 (FP32 10.2 and 7.7).
 constexpr int FLOW_FROM = 64;
 
 static void choose_shape(fc2dgpu_ctx* c);
@@ -1571,19 +1571,19 @@ static bool cluster_fits(fc2dgpu_ctx* c, int cs, int nt, bool rep) {
 }
 
 // A colour with more contacts than a full cluster has threads (16 x 512)
-// goes to a cooperative grid over every SM instead (grid barrier, about
-// 1-2 us, instead of the cluster's 0.3 us; the FP64 pipes of all SMs).
+// goes to a cooperative grid over every SM instead (a barrier over all of them
+// instead of the cluster's 0.3 us; the FP64 pipes of all SMs).
 constexpr int GRID_FROM = CS_MAX * NT_MAX;
 // In FP64 the FP64 units of a cluster's SMs bound a colour from far fewer
-// contacts (cluster and grid, us a sweep: 40.7 and 35.2 with 2,401 contacts in
-// the largest colour, 67.5 and 34.6 with 4,828; 26 on a cluster with 514,
-// where the grid's barriers alone take 8 more than the cluster's).
+// contacts (cluster and grid, us a sweep: 41.3 and 32.0 with 2,401 contacts in
+// the largest colour, 54.1 and 32.1 with 4,828; with 514 the cluster's 25.6
+// against 37.8 on the grid).
 constexpr int GRID64_FROM = 1000;
 
 // Contacts of the largest colour a thread from which FP64 contacts are one
 // lane's.  ms for 40 sweeps on two lanes and on one, by contacts a thread: 1.2
-// (2,048 threads) 2.25 and 2.47, 1.2 (77,824) 4.39 and 5.13, 3.1 (77,824) 8.39 and
-// 8.85; 4.7 (512) 4.48 and 3.78, 4.7 (2,048) 6.17 and 5.63, 12 (8,192) 24.7 and 22.2,
+// (2,048 threads) 2.25 and 2.47, 2.5 (77,824) 7.21 and 7.45; 6.2 (77,824) 15.0 and
+// 14.7, 4.7 (512) 4.48 and 3.78, 4.7 (2,048) 6.17 and 5.63, 12 (8,192) 24.7 and 22.2,
 // 19 (128) 14.7 and 11.4, 76 (128) 60.1 and 45.3.
 constexpr int ALONE_FROM = 4;
 

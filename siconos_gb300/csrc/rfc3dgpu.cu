@@ -632,9 +632,10 @@ __device__ __forceinline__ void sweep_colours_coop(const Args& a, double local_t
 // contact of a higher colour cannot write its new one before this contact has
 // written its own, and a stamp at least the one needed is the one needed.
 // us a sweep by colours and as dataflow, copies of the 21-contact rockfall
-// problem:
-//   FP64: 21 contacts 161, 130   2,100: 259, 216   21,000: 507, 401
-//   FP32: 21 contacts 82, 59     2,100: 130, 104   21,000: 147, 139
+// problem, sweeps 10 to 60 from zero:
+//   FP64: 21 contacts 136, 93    2,100: 228, 186   21,000: 430, 351
+//   FP32: 21 contacts 71, 47     2,100: 125, 100   21,000: 127, 134
+//   210,000: FP64 2,598, 2,480   FP32 285, 269
 
 // Polls of a reaction before the back-off, and the back-off (ns).
 #define RFC3D_FLOW_SPIN 16
